@@ -6,10 +6,13 @@ point raises, and every compute call needs a CUDA device.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libquantforge_rt.so")
+HOST_PATH = os.path.join(HERE, "lib", "_qf_host.so")  # native host path of the operators (csrc/qf_host.cpp)
 
 QF_OK = 0
 QF_F16, QF_BF16, QF_F32 = 0, 1, 2
@@ -101,6 +104,23 @@ def load() -> ctypes.CDLL:
     lib.qf_w4a16_linear_allgather.argtypes = [vp, vp, dp, vp, vp, vp, vp, vp, vp, sz, vp]
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def load_host():
+    """Load the native host path of the operators, or raise."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise ImportError(f"{HOST_PATH} is missing: build it with `python -m quantforge_b200.build`.")
+        loader = importlib.machinery.ExtensionFileLoader("_qf_host", HOST_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_qf_host", loader))
+        loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def status_name(status: int) -> str:

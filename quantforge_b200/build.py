@@ -1,14 +1,16 @@
-"""Builds libquantforge_rt.so (CUDA kernels + C ABI) for sm_100a with nvcc, in-tree.
+"""Builds libquantforge_rt.so (CUDA kernels + C ABI) for sm_100a with nvcc, and _qf_host.so (the native host path of
+the Python operators, a CPython extension over torch's C++ API) with g++, in-tree.
 
     python -m quantforge_b200.build [--force] [--verbose]
 
-nvcc cross-compiles without a GPU.  The shared library lands in quantforge_b200/lib/.
+nvcc cross-compiles without a GPU.  The shared libraries land in quantforge_b200/lib/.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -30,23 +32,31 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found")
 
 
+def _older(path: str, deps) -> bool:
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
+
+
+def _headers() -> list:
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + \
+        [os.path.join(ROOT, "include", "quantforge_rt.h"), os.path.abspath(__file__)]
+
+
 def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", "quantforge_rt.h"),
-                                                                os.path.abspath(__file__)]
-    return any(os.path.getmtime(d) > t for d in deps)
+    return _older(LIB_PATH, _headers() + [os.path.join(CSRC, f) for f in SOURCES])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
+        build_host()
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)
     objs = []
     procs = []
     for src in SOURCES:
         obj = os.path.join(LIB_DIR, src.replace(".cu", ".o"))
+        objs.append(obj)
+        if not force and not verbose and not _older(obj, _headers() + [os.path.join(CSRC, src)]):
+            continue
         cmd = [_nvcc(), *NVCC_FLAGS, "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-c",
                os.path.join(CSRC, src), "-o", obj]
         if verbose:
@@ -54,7 +64,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd.insert(2, "-v")
             print(" ".join(cmd), flush=True)
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-        objs.append(obj)
     failed = False
     for src, pr in procs:
         out, _ = pr.communicate()
@@ -66,7 +75,30 @@ def build(force: bool = False, verbose: bool = False) -> str:
     link = [_nvcc(), "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a",
             "-Xcompiler", "-fPIC", "-lcudart_static", "-ldl", "-lpthread", "-lrt"]
     subprocess.run(link, check=True)
+    build_host(force)
     return LIB_PATH
+
+
+HOST_SRC = os.path.join(CSRC, "qf_host.cpp")
+HOST_PATH = os.path.join(LIB_DIR, "_qf_host.so")
+
+
+def build_host(force: bool = False) -> str:
+    """Builds the native host path (part of build(): it links against libquantforge_rt.so)."""
+    if not force and not _older(HOST_PATH, [HOST_SRC, os.path.join(ROOT, "include", "quantforge_rt.h")]):
+        return HOST_PATH
+    import torch
+    from torch.utils import cpp_extension
+    includes = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(ROOT, "include"),
+                                                os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+                    f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                    *[f for i in includes for f in ("-isystem", i)], HOST_SRC, "-o", HOST_PATH,
+                    "-L", LIB_DIR, "-lquantforge_rt", "-Wl,-rpath,$ORIGIN",
+                    "-L", torch_lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"],
+                   check=True)
+    return HOST_PATH
 
 
 OPT_SRC = os.path.join(HERE, "opt", "quantforge_opt.cpp")

@@ -1,0 +1,347 @@
+// Native host path of the Python operators: what quantforge_b200/ops.py does around one C-ABI call (reading the
+// tensors, checking them, allocating the result, finding stream and workspace, filling the descriptor), without the
+// interpreter. Only the ordinary case is handled here: CUDA tensors of one device, contiguous, right shapes and types,
+// a workspace that this stream already has. Whatever differs - an argument in error included - returns None, and
+// ops.py takes the call from the start: it makes the copies and allocations that are needed, and raises what it has to.
+//
+// Why: the interpreter needed 15 to 17 us per linear (attribute reads, two foreign calls, a device context manager,
+// ctypes conversions), more than the kernels of small layers take on the GPU.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <unordered_map>
+#include <vector>
+
+#include "quantforge_rt.h"
+
+namespace {
+
+using at::ScalarType;
+using at::Tensor;
+
+constexpr int kMaxDevices = 64;
+qf_ctx *g_ctx[kMaxDevices] = {nullptr};  // ops.py registers a device's context when it creates it
+
+// The workspaces that ops.py has made, by device and stream, ascending in size. The tensors live in ops.py.
+struct Buffer {
+    size_t bytes;
+    void *ptr;
+};
+struct StreamKey {
+    int device;
+    cudaStream_t stream;
+    bool operator==(const StreamKey &o) const { return device == o.device && stream == o.stream; }
+};
+struct StreamKeyHash {
+    size_t operator()(const StreamKey &k) const { return std::hash<void *>()((void *)k.stream) * 31u + (size_t)k.device; }
+};
+std::unordered_map<StreamKey, std::vector<Buffer>, StreamKeyHash> g_workspaces;
+
+bool find_workspace(int device, cudaStream_t stream, size_t need, void **ptr, size_t *bytes) {
+    *ptr = nullptr;
+    *bytes = 0;
+    if (need == 0) return true;
+    const auto it = g_workspaces.find(StreamKey{device, stream});
+    if (it == g_workspaces.end()) return false;
+    for (const Buffer &b : it->second)
+        if (b.bytes >= need) {
+            *ptr = b.ptr;
+            *bytes = b.bytes;
+            return true;
+        }
+    return false;
+}
+
+int type_code(ScalarType t) {
+    return t == at::kHalf ? QF_F16 : t == at::kBFloat16 ? QF_BF16 : t == at::kFloat ? QF_F32 : -1;
+}
+bool is_byte(ScalarType t) { return t == at::kChar || t == at::kByte; }
+
+// A plain contiguous CUDA tensor on `device` (-1: any; then `device` becomes its device).
+const Tensor *cuda_tensor(PyObject *o, int *device) {
+    if (!THPVariable_Check(o)) return nullptr;
+    const Tensor &t = THPVariable_Unpack(o);
+    if (!t.is_cuda() || t.layout() != at::kStrided || !t.is_contiguous() || !t.has_storage() ||
+        t.key_set().has(c10::DispatchKey::Python) || t.is_conj() || t.is_neg())
+        return nullptr;
+    const int d = t.get_device();
+    if (*device >= 0 && d != *device) return nullptr;
+    *device = d;
+    return &t;
+}
+
+bool shape_is(const Tensor &t, int64_t a, int64_t b) { return t.dim() == 2 && t.size(0) == a && t.size(1) == b; }
+
+// The device must be the current one and must have a context.
+bool ready(int device) {
+    return device >= 0 && device < kMaxDevices && g_ctx[device] != nullptr && c10::cuda::current_device() == device;
+}
+
+cudaStream_t stream_of(int device) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
+
+Tensor empty(at::IntArrayRef size, ScalarType type, int device) {
+    return at::detail::empty_cuda(size, type, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), std::nullopt);
+}
+
+// A small integer argument; false leaves no error set.
+bool as_int(PyObject *o, long long *v) {
+    if (!PyLong_Check(o)) return false;
+    *v = PyLong_AsLongLong(o);
+    if (*v == -1 && PyErr_Occurred()) {
+        PyErr_Clear();
+        return false;
+    }
+    return true;
+}
+bool attr_int(PyObject *o, PyObject *name, long long *v) {
+    PyObject *a = PyObject_GetAttr(o, name);
+    if (!a) {
+        PyErr_Clear();
+        return false;
+    }
+    const bool ok = as_int(a, v);
+    Py_DECREF(a);
+    return ok;
+}
+
+// Zero points [G, N]: none (constant), int8, or packed four-bit codes.
+bool read_zeros(PyObject *o, int64_t G, int64_t N, int *device, qf_linear_desc *d, const void **ptr) {
+    *ptr = nullptr;
+    if (o == Py_None) {
+        d->zero_mode = QF_ZERO_CONST;
+        return true;
+    }
+    const Tensor *z = cuda_tensor(o, device);
+    if (!z) return false;
+    if (z->scalar_type() == at::kChar && shape_is(*z, G, N)) d->zero_mode = QF_ZERO_I8;
+    else if (z->scalar_type() == at::kInt && N % 8 == 0 && shape_is(*z, G, N / 8)) d->zero_mode = QF_ZERO_U4;
+    else return false;
+    *ptr = z->const_data_ptr();
+    return true;
+}
+
+// Packed weights [N, K/2] bytes or [N, K/8] words, scales [K/group, N], zeros. `K` < 0: taken from the weights.
+bool read_weights(PyObject *qw_o, PyObject *sc_o, PyObject *z_o, int *device, qf_linear_desc *d, int64_t K,
+                  const void **qw_ptr, const void **sc_ptr, const void **z_ptr, ScalarType *act) {
+    const Tensor *qw = cuda_tensor(qw_o, device), *sc = cuda_tensor(sc_o, device);
+    if (!qw || !sc || qw->dim() != 2) return false;
+    const int64_t per = is_byte(qw->scalar_type()) ? 2 : qw->scalar_type() == at::kInt ? 8 : 0;
+    if (per == 0) return false;
+    d->N = qw->size(0);
+    d->K = qw->size(1) * per;
+    if (K >= 0 && d->K != K) return false;
+    if (d->group_size <= 0 || d->K % d->group_size != 0) return false;
+    *act = sc->scalar_type();
+    if (*act != at::kHalf && *act != at::kBFloat16) return false;
+    const int64_t G = d->K / d->group_size;
+    if (!shape_is(*sc, G, d->N)) return false;
+    d->act_dtype = type_code(*act);
+    *qw_ptr = qw->const_data_ptr();
+    *sc_ptr = sc->const_data_ptr();
+    return read_zeros(z_o, G, d->N, device, d, z_ptr);
+}
+
+// Allocates or checks the result, finds the workspace and makes the call. None where any of it does not apply.
+PyObject *finish(qf_linear_desc *d, int device, const Tensor &x, const void *qw, const void *sc, const void *z,
+                 PyObject *out_dtype_o, PyObject *out_o, PyObject *residual_o) {
+    ScalarType out_type = x.scalar_type();
+    if (out_dtype_o != Py_None) {
+        if (!THPDtype_Check(out_dtype_o)) Py_RETURN_NONE;
+        out_type = ((THPDtype *)out_dtype_o)->scalar_type;
+    }
+    d->out_dtype = type_code(out_type);
+    if (d->out_dtype < 0 || d->M <= 0) Py_RETURN_NONE;
+    const int64_t cols = d->epilogue == QF_EPI_SILU_MUL ? d->N / 2 : d->N;
+    const void *res = nullptr;
+    if (residual_o != Py_None) {
+        const Tensor *r = cuda_tensor(residual_o, &device);
+        if (!r) Py_RETURN_NONE;
+        if (d->epilogue == QF_EPI_RESIDUAL_ADD && (!shape_is(*r, d->M, cols) || r->scalar_type() != out_type)) Py_RETURN_NONE;
+        res = r->const_data_ptr();
+    } else if (d->epilogue == QF_EPI_RESIDUAL_ADD) {
+        Py_RETURN_NONE;
+    }
+    if (!ready(device)) Py_RETURN_NONE;
+    const cudaStream_t stream = stream_of(device);
+    void *ws;
+    size_t ws_bytes;
+    if (!find_workspace(device, stream, qf_w4a16_workspace_bytes(d), &ws, &ws_bytes)) Py_RETURN_NONE;
+    if (out_o != Py_None) {
+        const Tensor *y = cuda_tensor(out_o, &device);
+        if (!y || !shape_is(*y, d->M, cols) || y->scalar_type() != out_type) Py_RETURN_NONE;
+        if (qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y->data_ptr(), res, ws, ws_bytes, stream) != QF_OK)
+            Py_RETURN_NONE;
+        Py_INCREF(out_o);
+        return out_o;
+    }
+    Tensor y = empty({d->M, cols}, out_type, device);
+    if (qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y.data_ptr(), res, ws, ws_bytes, stream) != QF_OK)
+        Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(y));
+}
+
+// ------------------------------------------------------------------------------------------------
+// entry points (positional arguments only; None = not handled here)
+// ------------------------------------------------------------------------------------------------
+PyObject *s_blob, *s_N, *s_K, *s_group, *s_act, *s_zmode, *s_zconst;  // interned attribute names of SlabWeight
+
+// linear(x, qweight, scales, zeros, group_size, zero_const, out_dtype, path, split_k, out, weight_layout, epilogue, residual)
+PyObject *linear_impl(PyObject *const *a) {
+    int device = -1;
+    const Tensor *x = cuda_tensor(a[0], &device);
+    if (!x || x->dim() != 2) Py_RETURN_NONE;
+    qf_linear_desc d = {};
+    long long group, zero_const, path, split_k, layout, epilogue;
+    if (!as_int(a[8], &split_k) || !as_int(a[11], &epilogue)) Py_RETURN_NONE;
+    d.M = x->size(0);
+    d.split_k = (int32_t)split_k;
+    d.epilogue = (int32_t)epilogue;
+    const void *qw, *sc = nullptr, *z = nullptr;
+    if (THPVariable_Check(a[1])) {
+        ScalarType act;
+        if (!as_int(a[4], &group) || !as_int(a[5], &zero_const) || !as_int(a[7], &path) || !as_int(a[10], &layout)) Py_RETURN_NONE;
+        if (group > INT32_MAX || zero_const < -128 || zero_const > 127) Py_RETURN_NONE;
+        d.group_size = (int32_t)group;
+        d.path = (int32_t)path;
+        d.weight_layout = (int32_t)layout;
+        if (!read_weights(a[1], a[2], a[3], &device, &d, x->size(1), &qw, &sc, &z, &act) || act != x->scalar_type()) Py_RETURN_NONE;
+        if (d.zero_mode == QF_ZERO_CONST) d.zero_const = (int32_t)zero_const;
+    } else {
+        // a SlabWeight: blob, shape and converter facts come from the object
+        PyObject *blob_o = PyObject_GetAttr(a[1], s_blob);
+        if (!blob_o) {
+            PyErr_Clear();
+            Py_RETURN_NONE;
+        }
+        const Tensor *blob = cuda_tensor(blob_o, &device);
+        qw = blob ? blob->const_data_ptr() : nullptr;  // the object keeps the tensor alive for the call
+        const size_t have = blob ? (size_t)blob->nbytes() : 0;
+        Py_DECREF(blob_o);
+        PyObject *act_o = PyObject_GetAttr(a[1], s_act);
+        if (!act_o) PyErr_Clear();
+        const bool act_ok = act_o && THPDtype_Check(act_o) && ((THPDtype *)act_o)->scalar_type == x->scalar_type();
+        Py_XDECREF(act_o);
+        long long N, K, zmode;
+        if (!qw || !act_ok || !attr_int(a[1], s_N, &N) || !attr_int(a[1], s_K, &K) || !attr_int(a[1], s_group, &group) ||
+            !attr_int(a[1], s_zmode, &zmode) || !attr_int(a[1], s_zconst, &zero_const))
+            Py_RETURN_NONE;
+        if (x->size(1) != K || have < qf_prepack_bytes(QF_LAYOUT_GEMV_SLAB, N, K)) Py_RETURN_NONE;
+        d.N = N;
+        d.K = K;
+        d.group_size = (int32_t)group;
+        d.act_dtype = type_code(x->scalar_type());
+        d.zero_mode = (int32_t)zmode;
+        d.zero_const = (int32_t)zero_const;
+        d.path = QF_PATH_AUTO;
+        d.weight_layout = QF_LAYOUT_GEMV_SLAB;
+    }
+    return finish(&d, device, *x, qw, sc, z, a[6], a[9], a[12]);
+}
+
+// gemv(x, w_packed, scale, zero_point): per-channel quantisation
+PyObject *gemv_impl(PyObject *const *a) {
+    int device = -1;
+    const Tensor *x = cuda_tensor(a[0], &device), *w = cuda_tensor(a[1], &device), *sc = cuda_tensor(a[2], &device),
+                 *z = cuda_tensor(a[3], &device);
+    if (!x || !w || !sc || !z || x->dim() != 2 || w->dim() != 2 || !is_byte(w->scalar_type())) Py_RETURN_NONE;
+    qf_linear_desc d = {};
+    d.M = x->size(0);
+    d.K = x->size(1);
+    d.N = w->size(0);
+    const ScalarType act = x->scalar_type();
+    if ((act != at::kHalf && act != at::kBFloat16) || sc->scalar_type() != act || z->scalar_type() != at::kChar) Py_RETURN_NONE;
+    if (w->size(1) * 2 != d.K || sc->numel() != d.N || z->numel() != d.N || d.K > INT32_MAX) Py_RETURN_NONE;
+    d.group_size = (int32_t)d.K;
+    d.act_dtype = type_code(act);
+    d.zero_mode = QF_ZERO_I8;
+    return finish(&d, device, *x, w->const_data_ptr(), sc->const_data_ptr(), z->const_data_ptr(), Py_None, Py_None, Py_None);
+}
+
+// unpack(packed)
+PyObject *unpack_impl(PyObject *const *a) {
+    int device = -1;
+    const Tensor *p = cuda_tensor(a[0], &device);
+    if (!p || p->dim() < 1 || !is_byte(p->scalar_type()) || p->numel() == 0 || !ready(device)) Py_RETURN_NONE;
+    c10::SmallVector<int64_t, 5> shape(p->sizes().begin(), p->sizes().end());
+    const int64_t cols = shape.back();
+    shape.back() = cols * 2;
+    Tensor out = empty(shape, at::kChar, device);
+    if (qf_unpack_int4(g_ctx[device], p->const_data_ptr(), out.data_ptr(), p->numel() / cols, cols, stream_of(device)) != QF_OK)
+        Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(out));
+}
+
+// dequant(qweight, scales, zeros, group_size, zero_const)
+PyObject *dequant_impl(PyObject *const *a) {
+    int device = -1;
+    qf_linear_desc d = {};
+    long long group, zero_const;
+    if (!as_int(a[3], &group) || !as_int(a[4], &zero_const) || group > INT32_MAX || zero_const < -128 || zero_const > 127)
+        Py_RETURN_NONE;
+    d.M = 1;
+    d.group_size = (int32_t)group;
+    const void *qw, *sc, *z;
+    ScalarType act;
+    if (!read_weights(a[0], a[1], a[2], &device, &d, -1, &qw, &sc, &z, &act) || !ready(device)) Py_RETURN_NONE;
+    if (d.zero_mode == QF_ZERO_CONST) d.zero_const = (int32_t)zero_const;
+    d.out_dtype = d.act_dtype;
+    Tensor out = empty({d.N, d.K}, act, device);
+    if (qf_dequant_w4(g_ctx[device], &d, qw, sc, z, out.data_ptr(), stream_of(device)) != QF_OK) Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(out));
+}
+
+template <PyObject *(*F)(PyObject *const *), Py_ssize_t N>
+PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
+    if (n != N) {
+        PyErr_SetString(PyExc_TypeError, "wrong number of arguments");
+        return nullptr;
+    }
+    try {
+        return F(args);
+    } catch (const std::exception &) {  // no memory, for one: ops.py meets the same and says so
+        Py_RETURN_NONE;
+    }
+}
+
+// set_ctx(device, handle)
+PyObject *set_ctx_impl(PyObject *const *a) {
+    long long device, handle;
+    if (!as_int(a[0], &device) || !as_int(a[1], &handle)) Py_RETURN_NONE;
+    if (device >= 0 && device < kMaxDevices) g_ctx[device] = (qf_ctx *)(intptr_t)handle;
+    Py_RETURN_NONE;
+}
+
+// add_workspace(device, stream, pointer, bytes)
+PyObject *add_workspace_impl(PyObject *const *a) {
+    long long device, stream, ptr, bytes;
+    if (!as_int(a[0], &device) || !as_int(a[1], &stream) || !as_int(a[2], &ptr) || !as_int(a[3], &bytes)) Py_RETURN_NONE;
+    g_workspaces[StreamKey{(int)device, (cudaStream_t)(intptr_t)stream}].push_back(Buffer{(size_t)bytes, (void *)(intptr_t)ptr});
+    Py_RETURN_NONE;
+}
+
+#define QF_FAST(name, fn, n) {name, (PyCFunction)(void (*)(void))(entry<fn, n>), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    QF_FAST("linear", linear_impl, 13), QF_FAST("gemv", gemv_impl, 4),       QF_FAST("unpack", unpack_impl, 1),
+    QF_FAST("dequant", dequant_impl, 5), QF_FAST("set_ctx", set_ctx_impl, 2), QF_FAST("add_workspace", add_workspace_impl, 4),
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_qf_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__qf_host(void) {
+    s_blob = PyUnicode_InternFromString("blob");
+    s_N = PyUnicode_InternFromString("N");
+    s_K = PyUnicode_InternFromString("K");
+    s_group = PyUnicode_InternFromString("group_size");
+    s_act = PyUnicode_InternFromString("act_dtype");
+    s_zmode = PyUnicode_InternFromString("zero_mode");
+    s_zconst = PyUnicode_InternFromString("zero_const");
+    return PyModule_Create(&module);
+}

@@ -4,6 +4,10 @@ The names and argument meaning of `pack_int4`, `unpack_int4` and `gemv_int4` fol
 reference's python/quantforge/baseline.py (:17-31, :34-49, :52-72).  Every compute call goes
 through the C ABI into hand-written sm_100a kernels; tensors on the CPU are rejected (there is
 no CPU implementation in this package).
+
+The hot operators first offer the call to the native host path (csrc/qf_host.cpp), which serves the ordinary case in
+2 to 4 us instead of the 15 to 20 us the statements below take; it answers None where anything is out of the ordinary
+(first call on a stream, copies to make, an argument in error), and the Python code then takes the call from the start.
 """
 from __future__ import annotations
 
@@ -20,6 +24,14 @@ from ._lib import (QF_BF16, QF_EPI_NONE, QF_EPI_RESIDUAL_ADD, QF_EPI_SILU_MUL, Q
 _DT = {torch.float16: QF_F16, torch.bfloat16: QF_BF16, torch.float32: QF_F32}
 _ctxs: dict[int, ctypes.c_void_p] = {}
 _workspaces: dict[tuple[int, int], list] = {}
+_fast = None  # the native host path, loaded on first use
+
+
+def _native():
+    global _fast
+    if _fast is None:
+        _fast = _lib.load_host()
+    return _fast
 
 
 def _ctx(device: torch.device) -> ctypes.c_void_p:
@@ -33,6 +45,7 @@ def _ctx(device: torch.device) -> ctypes.c_void_p:
         if st != 0:
             raise QuantForgeError(st, _lib.status_name(st), f"qf_ctx_create(device={idx}) failed")
         _ctxs[idx] = h
+        _native().set_ctx(idx, h.value)
     return _ctxs[idx]
 
 
@@ -98,6 +111,9 @@ def pack_zeros_u4(zeros: torch.Tensor) -> torch.Tensor:
 # --------------------------------------------------------------------------------------------
 def unpack_int4(packed: torch.Tensor) -> torch.Tensor:
     """int8[..., n] -> int8[..., 2n]: out[2i] = b & 0xF, out[2i+1] = (b >> 4) & 0xF (logical shift)."""
+    out = (_fast or _native()).unpack(packed)
+    if out is not None:
+        return out
     dev = _need_cuda(packed)
     if packed.dtype not in (torch.int8, torch.uint8):
         raise TypeError("unpack_int4 expects int8 (or uint8) packed bytes")
@@ -154,6 +170,7 @@ def _workspace(dev: torch.device, nbytes: int) -> Optional[torch.Tensor]:
             return ws
     ws = torch.zeros(max(nbytes, 4 << 20), dtype=torch.uint8, device=dev)
     bufs.append(ws)
+    _native().add_workspace(key[0], key[1], ws.data_ptr(), ws.numel())
     return ws
 
 
@@ -280,6 +297,10 @@ def w4a16_linear(x: torch.Tensor, qweight, scales: Optional[torch.Tensor] = None
     scales   same dtype as x, [K/group_size, N]
     zeros    None (constant `zero_const`), int8 [G, N] or packed int32 [G, N/8] (pack_zeros_u4)
     """
+    y = (_fast or _native()).linear(x, qweight, scales, zeros, group_size, zero_const, out_dtype, path, split_k, out,
+                                    weight_layout, epilogue, residual)
+    if y is not None:
+        return y
     if isinstance(qweight, SlabWeight):
         w = qweight
         dev = _need_cuda(x, w.blob, residual)
@@ -467,6 +488,9 @@ def w4a16_linear_host(x_host: torch.Tensor, qweight: torch.Tensor, scales: torch
 def dequant_w4(qweight: torch.Tensor, scales: torch.Tensor, zeros: Optional[torch.Tensor] = None,
                group_size: int = 128, zero_const: int = 8) -> torch.Tensor:
     """qf.dequant(qf.unpack(qweight)) materialised: W[N, K] in the dtype of `scales`."""
+    out = (_fast or _native()).dequant(qweight, scales, zeros, group_size, zero_const)
+    if out is not None:
+        return out
     dev = _need_cuda(qweight, scales, zeros)
     N = qweight.shape[0]
     K = qweight.shape[1] * (8 if qweight.dtype == torch.int32 else 2)
@@ -529,6 +553,9 @@ def gemv_int4(x: torch.Tensor, w_packed: torch.Tensor, scale: torch.Tensor, zero
     x (M, K) f16, w_packed (N, K/2) int8, per-output-channel scale (N,) f16 and zero_point (N,) int8.
     Per-channel quantisation is the group_size == K case of the group-wise kernel.
     """
+    y = (_fast or _native()).gemv(x, w_packed, scale, zero_point)
+    if y is not None:
+        return y
     K = x.shape[1]
     return w4a16_linear(x, w_packed, scale.reshape(1, -1).to(x.dtype), zero_point.reshape(1, -1).to(torch.int8),
                         group_size=K, out_dtype=x.dtype)
@@ -555,6 +582,10 @@ class W4A16Linear:
 
     def __call__(self, x: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                  out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        y = (_fast or _native()).linear(x, self.qweight, self.scales, self.zeros, self.group_size, self.zero_const,
+                                        out_dtype, QF_PATH_AUTO, 0, out, self.weight_layout, QF_EPI_NONE, None)
+        if y is not None:
+            return y
         return w4a16_linear(x, self.qweight, self.scales, self.zeros, self.group_size, self.zero_const, out_dtype,
                             out=out, weight_layout=self.weight_layout)
 
