@@ -136,6 +136,22 @@ const char *qf_last_error(const qf_ctx *ctx);
 int qf_unpack_int4(qf_ctx *ctx, const void *packed_i8, void *out_i8, int64_t rows, int64_t packed_cols, void *stream);
 
 /*
+ * The inverse, python/quantforge/baseline.py:17-31 `pack_int4`: codes int8[2 * n_bytes] -> out int8[n_bytes],
+ * out[i] = (codes[2i] & 0xF) | (codes[2i+1] & 0xF) << 4. `codes` 16-byte, `out` 8-byte aligned. Zero points of one byte each
+ * [G, N] become the QF_ZERO_U4 words [G, N/8] by the same call.
+ */
+int qf_pack_int4(qf_ctx *ctx, const void *codes_i8, void *out_i8, int64_t n_bytes, void *stream);
+
+/*
+ * Group-wise quantisation of weight[N, K] (qf_dtype `dtype`, 16-byte aligned): codes int8[N, K] in 0..15, scales [G, N] in
+ * `scale_dtype` (QF_F16 or QF_BF16), zeros int8[G, N] in 0..15 (not written when `symmetric`: the zero is the constant 8).
+ * group_size: a multiple of 4 that divides K. The arithmetic is fp32: scale = (max - min) / 15 or max|w| / 7, at least
+ * 2^-14, rounded to scale_dtype before the codes are chosen. No reference counterpart (it starts from codes).
+ */
+int qf_quantize_w4(qf_ctx *ctx, const void *weight, int dtype, int64_t N, int64_t K, int group_size, int symmetric,
+                   void *codes_i8, void *scales, int scale_dtype, void *zeros_i8_or_null, void *stream);
+
+/*
  * qf.dequant(qf.unpack(w))  materialised (the fused elementwise op of
  * lib/Transforms/FuseUnpackDequant.cpp:209-304; dequant arithmetic
  * lib/Transforms/LowerDequantToArith.cpp:141-159; zp==0 path

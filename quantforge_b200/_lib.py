@@ -31,6 +31,7 @@ EXPORTS = [
     "qf_comm_create", "qf_comm_export", "qf_comm_connect", "qf_comm_destroy", "qf_w4a16_linear_allreduce",
     "qf_w4a16_linear_allgather", "qf_w4a16_linear_host_async", "qf_w4a16_linear_fused", "qf_w4a16_linear_batched",
     "qf_prepack_bytes", "qf_prepack_gemv_slab", "qf_unpack_gemv_slab", "qf_repack_kn_to_canonical",
+    "qf_pack_int4", "qf_quantize_w4",
 ]
 QF_COMM_HANDLE_BYTES = 64
 
@@ -75,6 +76,8 @@ def load() -> ctypes.CDLL:
     lib.qf_last_error.restype = ctypes.c_char_p
     lib.qf_last_error.argtypes = [vp]
     lib.qf_unpack_int4.argtypes = [vp, vp, vp, i64, i64, vp]
+    lib.qf_pack_int4.argtypes = [vp, vp, vp, i64, vp]
+    lib.qf_quantize_w4.argtypes = [vp, vp, ctypes.c_int, i64, i64, ctypes.c_int, ctypes.c_int, vp, vp, ctypes.c_int, vp, vp]
     lib.qf_dequant_w4.argtypes = [vp, dp, vp, vp, vp, vp, vp]
     lib.qf_w4a16_workspace_bytes.restype = sz
     lib.qf_w4a16_workspace_bytes.argtypes = [dp]

@@ -302,6 +302,36 @@ int qf_unpack_int4(qf_ctx *ctx, const void *packed_i8, void *out_i8, int64_t row
     return launch_unpack(ctx, packed_i8, out_i8, rows, packed_cols, (cudaStream_t)stream);
 }
 
+int qf_pack_int4(qf_ctx *ctx, const void *codes_i8, void *out_i8, int64_t n_bytes, void *stream) {
+    if (!ctx) return QF_ERR_BAD_ARG;
+    if (n_bytes < 0) return fail(ctx, QF_ERR_BAD_ARG, "negative extent");
+    if (n_bytes == 0) return QF_OK;
+    if (!codes_i8 || !out_i8) return fail(ctx, QF_ERR_BAD_ARG, "null tensor pointer");
+    if (!aligned16(codes_i8) || ((uintptr_t)out_i8 & 7u))
+        return fail(ctx, QF_ERR_BAD_ARG, "codes must be 16-byte and the output 8-byte aligned");
+    int st = check_current_device(ctx);
+    if (st != QF_OK) return st;
+    return launch_pack(ctx, codes_i8, out_i8, n_bytes, (cudaStream_t)stream);
+}
+
+int qf_quantize_w4(qf_ctx *ctx, const void *weight, int dtype, int64_t N, int64_t K, int group_size, int symmetric,
+                   void *codes_i8, void *scales, int scale_dtype, void *zeros_i8_or_null, void *stream) {
+    if (!ctx) return QF_ERR_BAD_ARG;
+    if (N <= 0 || K <= 0 || group_size <= 0 || group_size % 4 != 0 || K % group_size != 0 || K > INT32_MAX)
+        return fail(ctx, QF_ERR_BAD_ARG, "group_size must be a multiple of 4 that divides K");
+    if (N * (K / group_size) > INT32_MAX) return fail(ctx, QF_ERR_BAD_ARG, "too many groups");
+    if (dtype != QF_F16 && dtype != QF_BF16 && dtype != QF_F32) return fail(ctx, QF_ERR_UNSUPPORTED, "unknown weight type");
+    if (scale_dtype != QF_F16 && scale_dtype != QF_BF16)
+        return fail(ctx, QF_ERR_UNSUPPORTED, "scales are QF_F16 or QF_BF16");
+    if (!weight || !codes_i8 || !scales || (!symmetric && !zeros_i8_or_null))
+        return fail(ctx, QF_ERR_BAD_ARG, "null tensor pointer");
+    if (!aligned16(weight) || !aligned16(codes_i8)) return fail(ctx, QF_ERR_BAD_ARG, "device pointers must be 16-byte aligned");
+    int st = check_current_device(ctx);
+    if (st != QF_OK) return st;
+    return launch_quantize(ctx, weight, dtype, N, K, group_size, symmetric != 0, codes_i8, scales, scale_dtype,
+                           zeros_i8_or_null, (cudaStream_t)stream);
+}
+
 int qf_dequant_w4(qf_ctx *ctx, const qf_linear_desc *desc, const void *qweight, const void *scales,
                   const void *qzeros_or_null, void *w_out, void *stream) {
     if (!ctx) return QF_ERR_BAD_ARG;

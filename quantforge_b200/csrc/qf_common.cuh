@@ -201,6 +201,9 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why);
 
 // kernels (defined in their own translation units)
 int launch_unpack(qf_ctx *ctx, const void *packed, void *out, int64_t rows, int64_t packed_cols, cudaStream_t s);
+int launch_pack(qf_ctx *ctx, const void *codes, void *out, int64_t n_bytes, cudaStream_t s);
+int launch_quantize(qf_ctx *ctx, const void *w, int dtype, int64_t N, int64_t K, int group, bool symmetric, void *codes,
+                    void *scales, int scale_dtype, void *zeros, cudaStream_t s);
 int launch_dequant(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const void *scales, const void *zeros,
                    void *w_out, cudaStream_t s);
 int launch_gemv(qf_ctx *ctx, const qf_linear_desc *d, const Plan &p, const void *X, const void *qw,

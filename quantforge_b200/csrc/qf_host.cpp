@@ -296,6 +296,94 @@ PyObject *dequant_impl(PyObject *const *a) {
     return THPVariable_Wrap(std::move(out));
 }
 
+// pack(codes): int8 [..., 2n] -> int8 [..., n]
+PyObject *pack_impl(PyObject *const *a) {
+    int device = -1;
+    const Tensor *c = cuda_tensor(a[0], &device);
+    if (!c || c->dim() < 1 || c->scalar_type() != at::kChar || c->numel() == 0 || c->sizes().back() % 2 != 0 || !ready(device))
+        Py_RETURN_NONE;
+    c10::SmallVector<int64_t, 5> shape(c->sizes().begin(), c->sizes().end());
+    shape.back() /= 2;
+    Tensor out = empty(shape, at::kChar, device);
+    if (qf_pack_int4(g_ctx[device], c->const_data_ptr(), out.data_ptr(), out.numel(), stream_of(device)) != QF_OK) Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(out));
+}
+
+// pack_zeros(zeros): int8 [G, N] -> int32 [G, N/8]
+PyObject *pack_zeros_impl(PyObject *const *a) {
+    int device = -1;
+    const Tensor *z = cuda_tensor(a[0], &device);
+    if (!z || z->dim() != 2 || z->scalar_type() != at::kChar || z->numel() == 0 || z->size(1) % 8 != 0 || !ready(device))
+        Py_RETURN_NONE;
+    Tensor out = empty({z->size(0), z->size(1) / 8}, at::kInt, device);
+    if (qf_pack_int4(g_ctx[device], z->const_data_ptr(), out.data_ptr(), z->numel() / 2, stream_of(device)) != QF_OK)
+        Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(out));
+}
+
+// quantize(weight, group_size, symmetric, scale_dtype) -> (codes, scales, zeros or None)
+PyObject *quantize_impl(PyObject *const *a) {
+    int device = -1;
+    const Tensor *w = cuda_tensor(a[0], &device);
+    long long group;
+    if (!w || w->dim() != 2 || w->numel() == 0 || type_code(w->scalar_type()) < 0 || !as_int(a[1], &group) || !PyBool_Check(a[2]) ||
+        !THPDtype_Check(a[3]) || !ready(device))
+        Py_RETURN_NONE;
+    const ScalarType st = ((THPDtype *)a[3])->scalar_type;
+    const int64_t N = w->size(0), K = w->size(1);
+    if ((st != at::kHalf && st != at::kBFloat16) || group <= 0 || group > INT32_MAX || K % group != 0) Py_RETURN_NONE;
+    const bool sym = a[2] == Py_True;
+    Tensor codes = empty({N, K}, at::kChar, device), scales = empty({K / group, N}, st, device), zeros;
+    if (!sym) zeros = empty({K / group, N}, at::kChar, device);
+    if (qf_quantize_w4(g_ctx[device], w->const_data_ptr(), type_code(w->scalar_type()), N, K, (int)group, sym, codes.data_ptr(),
+                       scales.data_ptr(), type_code(st), sym ? nullptr : zeros.data_ptr(), stream_of(device)) != QF_OK)
+        Py_RETURN_NONE;
+    PyObject *c = THPVariable_Wrap(std::move(codes)), *s = THPVariable_Wrap(std::move(scales));
+    PyObject *z = sym ? Py_NewRef(Py_None) : THPVariable_Wrap(std::move(zeros));
+    return Py_BuildValue("(NNN)", c, s, z);
+}
+
+// prepack_slab(qweight, scales, zeros, group_size, zero_const) -> (blob, N, K, zero_mode)
+PyObject *prepack_slab_impl(PyObject *const *a) {
+    int device = -1;
+    qf_linear_desc d = {};
+    long long group, zero_const;
+    if (!as_int(a[3], &group) || !as_int(a[4], &zero_const) || group > INT32_MAX || zero_const < -128 || zero_const > 127)
+        Py_RETURN_NONE;
+    d.M = 1;
+    d.group_size = (int32_t)group;
+    const void *qw, *sc, *z;
+    ScalarType act;
+    if (!read_weights(a[0], a[1], a[2], &device, &d, -1, &qw, &sc, &z, &act) || !ready(device)) Py_RETURN_NONE;
+    d.zero_const = (int32_t)zero_const;
+    d.out_dtype = d.act_dtype;
+    d.weight_layout = QF_LAYOUT_GEMV_SLAB;
+    const size_t bytes = qf_prepack_bytes(QF_LAYOUT_GEMV_SLAB, d.N, d.K);
+    if (bytes == 0) Py_RETURN_NONE;
+    Tensor blob = empty({(int64_t)bytes}, at::kByte, device);
+    if (qf_prepack_gemv_slab(g_ctx[device], &d, qw, sc, z, blob.data_ptr(), stream_of(device)) != QF_OK) Py_RETURN_NONE;
+    return Py_BuildValue("(NLLi)", THPVariable_Wrap(std::move(blob)), (long long)d.N, (long long)d.K, (int)d.zero_mode);
+}
+
+// prepack(qweight, to_canonical, layout)
+PyObject *prepack_impl(PyObject *const *a) {
+    int device = -1;
+    const Tensor *q = cuda_tensor(a[0], &device);
+    long long layout;
+    if (!q || q->dim() != 2 || q->numel() == 0 || !PyBool_Check(a[1]) || !as_int(a[2], &layout) || !ready(device)) Py_RETURN_NONE;
+    const int64_t per = is_byte(q->scalar_type()) ? 2 : q->scalar_type() == at::kInt ? 8 : 0;
+    if (per == 0 || (int64_t)q->nbytes() % 4 != 0) Py_RETURN_NONE;
+    Tensor out = empty(q->sizes(), q->scalar_type(), device);
+    const int back = a[1] == Py_True ? 1 : 0;
+    const int st = layout == QF_LAYOUT_TILED
+                       ? qf_prepack_w4_tiled(g_ctx[device], q->const_data_ptr(), out.data_ptr(), q->size(0), q->size(1) * per, back,
+                                             stream_of(device))
+                       : qf_prepack_w4(g_ctx[device], q->const_data_ptr(), out.data_ptr(), (int64_t)q->nbytes() / 4, back,
+                                       stream_of(device));
+    if (st != QF_OK) Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(out));
+}
+
 template <PyObject *(*F)(PyObject *const *), Py_ssize_t N>
 PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (n != N) {
@@ -328,6 +416,8 @@ PyObject *add_workspace_impl(PyObject *const *a) {
 #define QF_FAST(name, fn, n) {name, (PyCFunction)(void (*)(void))(entry<fn, n>), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     QF_FAST("linear", linear_impl, 13), QF_FAST("gemv", gemv_impl, 4),       QF_FAST("unpack", unpack_impl, 1),
+    QF_FAST("pack", pack_impl, 1),       QF_FAST("pack_zeros", pack_zeros_impl, 1), QF_FAST("quantize", quantize_impl, 4),
+    QF_FAST("prepack_slab", prepack_slab_impl, 5), QF_FAST("prepack", prepack_impl, 3),
     QF_FAST("dequant", dequant_impl, 5), QF_FAST("set_ctx", set_ctx_impl, 2), QF_FAST("add_workspace", add_workspace_impl, 4),
     {nullptr, nullptr, 0, nullptr}};
 

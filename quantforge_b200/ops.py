@@ -75,6 +75,19 @@ def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
 
 
+def _offer(fn, t: torch.Tensor, *args):
+    """fn(t, *args) of the native host path for a layout helper that also works without it: None where it does not
+    apply. A device's first such call creates its context."""
+    out = fn(t, *args)
+    if out is None and (t.device.index if t.device.index is not None else torch.cuda.current_device()) not in _ctxs:
+        try:
+            _ctx(t.device)
+        except QuantForgeError:  # not a device this library runs on
+            return None
+        out = fn(t, *args)
+    return out
+
+
 def launch_count() -> int:
     """Kernel launches enqueued by the runtime library since it was loaded."""
     return int(_lib.load().qf_launch_count())
@@ -89,6 +102,10 @@ def pack_int4(weights: torch.Tensor) -> torch.Tensor:
         raise TypeError("pack_int4 expects an int8 tensor of codes")
     if weights.shape[-1] % 2 != 0:
         raise ValueError("last dim must be even")
+    if weights.is_cuda:
+        packed = _offer((_fast or _native()).pack, weights)
+        if packed is not None:
+            return packed
     low = weights[..., 0::2] & 0x0F
     high = weights[..., 1::2] & 0x0F
     return (low | (high << 4)).to(torch.int8)
@@ -99,6 +116,10 @@ def pack_zeros_u4(zeros: torch.Tensor) -> torch.Tensor:
     G, N = zeros.shape
     if N % 8 != 0:
         raise ValueError("N must be a multiple of 8")
+    if zeros.is_cuda:
+        packed = _offer((_fast or _native()).pack_zeros, zeros)
+        if packed is not None:
+            return packed
     z = zeros.to(torch.int64).reshape(G, N // 8, 8) & 0xF
     shifts = torch.arange(8, device=zeros.device, dtype=torch.int64) * 4
     words = (z << shifts).sum(dim=-1)
@@ -217,6 +238,10 @@ class SlabWeight:
 def prepack_gemv_slab(qweight: torch.Tensor, scales: torch.Tensor, zeros: Optional[torch.Tensor] = None,
                       group_size: int = 128, zero_const: int = 8) -> SlabWeight:
     """One-time prepack of canonical weights (+ scales, zeros) for the streaming GEMV kernel (M <= 32)."""
+    made = (_fast or _native()).prepack_slab(qweight, scales, zeros, group_size, zero_const)
+    if made is not None:
+        blob, N, K, zero_mode = made
+        return SlabWeight(blob, N, K, group_size, scales.dtype, zero_mode, int(zero_const))
     dev = _need_cuda(qweight, scales, zeros)
     N = qweight.shape[0]
     K = qweight.shape[1] * (8 if qweight.dtype == torch.int32 else 2)
@@ -511,6 +536,9 @@ def prepack_w4(qweight: torch.Tensor, to_canonical: bool = False, layout: int = 
 
     The result has the shape and dtype of the input; only the order of the 4-bit codes changes.
     """
+    out = (_fast or _native()).prepack(qweight, to_canonical, layout)
+    if out is not None:
+        return out
     dev = _need_cuda(qweight)
     qweight = qweight.contiguous()
     if layout == QF_LAYOUT_TILED:

@@ -4,7 +4,8 @@
     qweight = pack_int4(codes)                      # int8 [N, K/2], the canonical layout of the runtime
     qzeros  = pack_zeros_u4(zeros)                  # int32 [G, N/8]   (asymmetric only)
 
-Layout helpers only (plain torch ops, any device); nothing here is on the inference hot path. The packing rule is the
+Layout helpers (any device); nothing here is on the inference hot path. Plain torch ops on the CPU, one kernel per call on
+CUDA tensors (csrc/qf_quantize.cu, the same fp32 arithmetic step for step). The packing rule is the
 reference's `pack_int4` (python/quantforge/baseline.py:17-31); quantisation itself has no counterpart in the reference,
 which starts from already-quantised codes.
 """
@@ -14,6 +15,7 @@ from typing import Optional, Tuple
 
 import torch
 
+from . import ops
 from .ops import pack_int4, pack_zeros_u4  # noqa: F401  (re-exported for convenience)
 
 
@@ -33,6 +35,10 @@ def quantize_w4(weight: torch.Tensor, group_size: int = 128, symmetric: bool = F
         raise ValueError("K must be a multiple of group_size")
     if scale_dtype is None:
         scale_dtype = weight.dtype if weight.dtype in (torch.float16, torch.bfloat16) else torch.float16
+    if weight.is_cuda:
+        made = ops._offer(ops._native().quantize, weight, group_size, bool(symmetric), scale_dtype)
+        if made is not None:
+            return made
     G = K // group_size
     w = weight.float().reshape(N, G, group_size)
     if symmetric:
