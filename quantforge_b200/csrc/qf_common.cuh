@@ -288,6 +288,21 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     return r;
 }
 
+// Nibble order inside a word: canonical c0 c1 .. c7 <-> pair-interleaved c0 c2 c4 c6 c1 c3 c5 c7 (lowest nibble first).
+__device__ __forceinline__ uint32_t even_nibbles(uint32_t w) {  // nibbles 0, 2, 4, 6 -> the low half
+    w &= 0x0f0f0f0fu;
+    w = (w | (w >> 4)) & 0x00ff00ffu;
+    return (w | (w >> 8)) & 0xffffu;
+}
+__device__ __forceinline__ uint32_t spread_nibbles(uint32_t h) {  // the inverse
+    h = (h | (h << 8)) & 0x00ff00ffu;
+    return (h | (h << 4)) & 0x0f0f0f0fu;
+}
+__device__ __forceinline__ uint32_t interleave_word(uint32_t w) { return even_nibbles(w) | (even_nibbles(w >> 4) << 16); }
+__device__ __forceinline__ uint32_t deinterleave_word(uint32_t w) {
+    return spread_nibbles(w & 0xffffu) | (spread_nibbles(w >> 16) << 4);
+}
+
 // 16-bit float bit patterns of small integers (exact in both formats for |v| <= 256).
 __device__ __forceinline__ uint32_t int_to_f16_bits(int v) {
     return (uint32_t)__half_as_ushort(__int2half_rn(v));

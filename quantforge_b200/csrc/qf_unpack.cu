@@ -131,26 +131,7 @@ int launch_pack(qf_ctx *ctx, const void *codes, void *out, int64_t n_bytes, cuda
     return QF_OK;
 }
 
-// Nibble permutation inside each word. canonical nibbles c0..c7 -> interleaved c0 c2 c4 c6 c1 c3 c5 c7.
-__device__ __forceinline__ uint32_t interleave_word(uint32_t w) {
-    uint32_t r = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        r |= ((w >> (8 * i)) & 0xFu) << (4 * i);            // even codes -> nibbles 0..3
-        r |= ((w >> (8 * i + 4)) & 0xFu) << (4 * (i + 4));  // odd codes  -> nibbles 4..7
-    }
-    return r;
-}
-__device__ __forceinline__ uint32_t deinterleave_word(uint32_t w) {
-    uint32_t r = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        r |= ((w >> (4 * i)) & 0xFu) << (8 * i);
-        r |= ((w >> (4 * (i + 4))) & 0xFu) << (8 * i + 4);
-    }
-    return r;
-}
-
+// Nibble permutation inside each word: qf_prepack_w4.
 __global__ void __launch_bounds__(256) prepack_kernel(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
                                                       int64_t n_words, int to_canonical) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -170,34 +151,31 @@ int launch_prepack(qf_ctx *ctx, const void *in, void *out, int64_t n_words, int 
 }
 
 // canonical word (n, j) <-> tiled word ((nt * KB + kb) * 128 + r) * 16 + w, n = nt*128 + r, j = kb*16 + w.
-__global__ void __launch_bounds__(256) prepack_tiled_kernel(const uint32_t *__restrict__ in,
-                                                            uint32_t *__restrict__ out, int64_t N, int64_t K,
-                                                            int to_canonical) {
-    const int64_t words_per_row = K >> 3;
-    const int64_t KB = K >> 7;
-    const int64_t total = N * words_per_row;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        // i enumerates the TILED order so that the side written (or read) in bulk is contiguous
-        const int64_t w = i & 15;
-        const int64_t r = (i >> 4) & 127;
-        const int64_t blk = i >> 11;
-        const int64_t kb = blk % KB;
-        const int64_t nt = blk / KB;
-        const int64_t canon = (nt * 128 + r) * words_per_row + kb * 16 + w;
+// A block moves one tile (8 KB, contiguous on the tiled side): two 16-byte pieces per thread, four threads to the 64
+// bytes of a row.
+__global__ void __launch_bounds__(256) prepack_tiled_kernel(const uint4 *__restrict__ in, uint4 *__restrict__ out,
+                                                            int KB, int to_canonical) {
+    const int nt = (int)(blockIdx.x / (unsigned)KB), kb = (int)(blockIdx.x % (unsigned)KB);
+    const int64_t tile = (int64_t)blockIdx.x * 512;
+    const int64_t canon0 = ((int64_t)nt * 128 * KB + kb) * 4;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = h * 256 + (int)threadIdx.x;
+        const int64_t canon = canon0 + (int64_t)(i >> 2) * KB * 4 + (i & 3);
+        uint4 v = in[to_canonical ? tile + i : canon];
         if (to_canonical)
-            out[canon] = deinterleave_word(in[i]);
+            v = make_uint4(deinterleave_word(v.x), deinterleave_word(v.y), deinterleave_word(v.z), deinterleave_word(v.w));
         else
-            out[i] = interleave_word(in[canon]);
+            v = make_uint4(interleave_word(v.x), interleave_word(v.y), interleave_word(v.z), interleave_word(v.w));
+        out[to_canonical ? canon : tile + i] = v;
     }
 }
 
 int launch_prepack_tiled(qf_ctx *ctx, const void *in, void *out, int64_t N, int64_t K, int to_canonical,
                          cudaStream_t s) {
-    const int64_t total = N * (K / 8);
-    int64_t blocks = (total + 255) / 256;
-    if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-    prepack_tiled_kernel<<<(unsigned)blocks, 256, 0, s>>>((const uint32_t *)in, (uint32_t *)out, N, K, to_canonical);
+    const int64_t tiles = (N / 128) * (K / 128);
+    if (tiles > INT32_MAX) return fail(ctx, QF_ERR_UNSUPPORTED, "matrix too large");
+    prepack_tiled_kernel<<<(unsigned)tiles, 256, 0, s>>>((const uint4 *)in, (uint4 *)out, (int)(K / 128), to_canonical);
     g_launch_count.fetch_add(1);
     QF_CUDA_TRY(ctx, cudaGetLastError());
     return QF_OK;
