@@ -144,12 +144,14 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
             p->ws_counter_bytes = 0;
         }
     } else {
-        const int bn = d->M <= 16 ? 16 : d->M <= 32 ? 32 : d->M <= 64 ? 64 : d->M <= 128 ? 128 : 256;
+        // As few batch tiles as a width of 256 allows, all of one width: the smallest multiple of 16 that covers M. (Tiles
+        // of 16, 32, 64, 128 or 256 rows ran M = 777 as 1024 rows; 777 x 4096 x 4096 f16, canonical: 38.5 -> 35.1 us.)
+        p->m_tiles = d->M > 256 ? (int)((d->M + 255) / 256) : 1;
+        const int64_t rows = d->M > p->m_tiles ? (d->M + p->m_tiles - 1) / p->m_tiles : 1;
+        const int bn = (int)((rows + 15) / 16 * 16);
         const int bk = gemm_block_k(bn);
         const int kblocks = (int)(d->K / bk);
         p->bn = bn;
-        p->m_tiles = (int)((d->M + bn - 1) / bn);
-        if (p->m_tiles < 1) p->m_tiles = 1;
         const int64_t tiles = (int64_t)p->m_tiles * (d->N / 128);
         int split;
         if (d->split_k > 0) {

@@ -3,7 +3,7 @@
 // Computes Y^T = W . X^T tile by tile so that the DEQUANTISED WEIGHTS are the MMA's A operand and
 // live only in tensor memory (TMEM):
 //   MMA M = 128 output features (weight rows, one per TMEM lane)
-//   MMA N = BN  rows of X (the batch), 16..256
+//   MMA N = the batch tile's rows of X, a multiple of 16 up to the instantiation's BN (16..256)
 //   MMA K = 16  per instruction, BK codes per pipeline stage
 //
 // Roles inside a CTA (320 threads):
@@ -66,6 +66,7 @@ struct GemmParams {
     int group_size;
     int zero_mode, zero_const;
     int out_dtype;
+    int bn;                // batch rows of a tile: a multiple of 16, at most the instantiation's BN (the MMA's N)
     int kblocks;           // K / BK
     int kblocks_per_split;
     int split_k;
@@ -261,7 +262,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     const int kb1 = min(kb0 + p.kblocks_per_split, p.kblocks);
     const int nkb = kb1 - kb0;
     const int64_t n0 = (int64_t)n_tile * 128;
-    const int64_t m0 = (int64_t)m_tile * BN;
+    const int64_t m0 = (int64_t)m_tile * p.bn;
 
     if (tid == 0) {
         s_abort = 0;
@@ -297,7 +298,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         // The whole warp runs the loop (uniform control flow); one elected lane issues the copies.
         const bool leader = elect_one();
         const uint32_t zbytes = p.zero_mode == QF_ZERO_U4 ? 64u : p.zero_mode == QF_ZERO_I8 ? 128u : 0u;
-        const uint32_t tx_bytes = C::STAGE_BYTES + 256u + zbytes;
+        const uint32_t tx_bytes = C::W_STAGE_BYTES + (uint32_t)(BK / 64) * (uint32_t)p.bn * 128u + 256u + zbytes;
         const int group_kb = p.group_size / BK;  // k-blocks per quantisation group (>= 1)
         const int gi = kb0 / group_kb;
         const uint8_t *sc_ptr = (const uint8_t *)(p.scales + n0) + (size_t)gi * p.N * 2;
@@ -359,7 +360,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         // ------------------------------ MMA issuer ------------------------------
         const bool leader = elect_one();
         const uint32_t idesc = (1u << 4) | ((BF16 ? 1u : 0u) << 7) | ((BF16 ? 1u : 0u) << 10) |
-                               ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+                               ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         const uint64_t desc_hi = make_b_desc(0) & 0xFFFFFFFF00000000ull;
         const uint32_t desc_lo_const = (uint32_t)(make_b_desc(0) & 0xFFFFFFFFull);
         int s = 0, a = 0;
@@ -450,11 +451,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             // this rank has finished and advanced the epoch
             unsigned ar_epoch = 0u;
             if constexpr (EXCH) ar_epoch = exch_read_epoch(ar);
-            constexpr int COLS_PER_WG = BN / 2;
-            const int64_t Mp = (int64_t)gridDim.x * BN;
+            const int cols_per_wg = p.bn >> 1;
+            const int64_t Mp = (int64_t)gridDim.x * p.bn;
 #pragma unroll 1
-            for (int c8 = 0; c8 < COLS_PER_WG / 8; ++c8) {
-                const int col = wg * COLS_PER_WG + c8 * 8;
+            for (int c8 = 0; c8 < cols_per_wg >> 3; ++c8) {
+                const int col = wg * cols_per_wg + c8 * 8;
                 uint32_t r[8];
                 tmem_ld8(lane_taddr + col, r);
                 tmem_wait_ld();
@@ -504,7 +505,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         cluster_sync_all();  // all partial tiles are in shared memory
         if (!s_abort) {
             // each block sums its share of the tile from all blocks in split order and writes the output
-            const int units = 32 * BN;  // float4 units of the tile
+            const int units = 32 * p.bn;  // float4 units of the tile
             const int per = (units + p.split_k - 1) / p.split_k;
             const int u_end = min(units, (split + 1) * per);
             for (int u = split * per + tid; u < u_end; u += GEMM_THREADS) {
@@ -577,9 +578,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 __threadfence();
                 // Each thread owns 4 consecutive output columns (one 16-byte load per split) and keeps 4 splits in
                 // flight, so the reduction is not a chain of dependent L2 round trips.
-                const int64_t Mp = (int64_t)gridDim.x * BN;
+                const int64_t Mp = (int64_t)gridDim.x * p.bn;
                 const size_t split_stride = (size_t)Mp * p.N;
-                for (int u = tid; u < 32 * BN; u += GEMM_THREADS) {
+                for (int u = tid; u < 32 * p.bn; u += GEMM_THREADS) {
                     const int nl = (u & 31) * 4;
                     const int64_t m = m0 + (u >> 5);
                     const bool silu = !EXCH && p.epilogue == QF_EPI_SILU_MUL;
@@ -623,7 +624,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             // Cross-GPU step: every element of the tile has been pushed to all ranks (above, or in the epilogue);
             // collect the other ranks' values for the same elements and write the output. The pairs carry their
             // own arrival token, so no block-level synchronisation separates the pushes from the collects.
-            if (!exch_collect_tile(ar, ar_epoch, m0, BN, n0, 128, p.M, p.N, p.Y, p.out_dtype, tid, GEMM_THREADS,
+            if (!exch_collect_tile(ar, ar_epoch, m0, p.bn, n0, 128, p.M, p.N, p.Y, p.out_dtype, tid, GEMM_THREADS,
                                    abort_flag))
                 s_abort = 1;
             __syncthreads();
@@ -706,6 +707,9 @@ static int get_tensor_map(qf_ctx *ctx, CUtensorMap *out, const void *ptr, int ki
     return QF_OK;
 }
 
+// Instantiation (widest batch tile) that serves a batch tile of bn rows.
+static int gemm_tile_of(int bn) { return bn <= 16 ? 16 : bn <= 32 ? 32 : bn <= 64 ? 64 : bn <= 128 ? 128 : 256; }
+
 constexpr bool gemm_has_exchange(int bn) { return bn <= 64; }  // the cross-GPU exchange serves decode batches only
 
 template <bool BF16, int BN>
@@ -750,8 +754,10 @@ static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan
                             tiled ? (uint64_t)d->N * (uint64_t)(d->K / 128) : (uint64_t)d->N, C::W_ROW_BYTES, 128,
                             C::BK == 128 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     if (st != QF_OK) return st;
-    st = get_tensor_map(ctx, &tx, X, 1, (uint64_t)d->K, (uint64_t)d->M, 64, BN, CU_TENSOR_MAP_SWIZZLE_128B);
+    st = get_tensor_map(ctx, &tx, X, 1, (uint64_t)d->K, (uint64_t)d->M, 64, (uint32_t)plan.bn,
+                        CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != QF_OK) return st;
+    p.bn = plan.bn;
     p.kblocks = (int)(d->K / C::BK);
     p.kblocks_per_split = plan.chunks_per_split;
     dim3 grid((unsigned)plan.m_tiles, (unsigned)(d->N / 128), (unsigned)plan.split_k);
@@ -792,7 +798,7 @@ static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan
 template <bool BF16>
 static int gemm_launch_dt(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan, const void *X, const void *qw,
                           GemmParams &p, cudaStream_t s, const ArParams *ar) {
-    switch (plan.bn) {
+    switch (gemm_tile_of(plan.bn)) {
         case 16: return gemm_launch_bn<BF16, 16>(ctx, d, plan, X, qw, p, s, ar);
         case 32: return gemm_launch_bn<BF16, 32>(ctx, d, plan, X, qw, p, s, ar);
         case 64: return gemm_launch_bn<BF16, 64>(ctx, d, plan, X, qw, p, s, ar);
