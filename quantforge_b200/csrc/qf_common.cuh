@@ -288,6 +288,12 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     return r;
 }
 
+__device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+
 // Nibble order inside a word: canonical c0 c1 .. c7 <-> pair-interleaved c0 c2 c4 c6 c1 c3 c5 c7 (lowest nibble first).
 __device__ __forceinline__ uint32_t even_nibbles(uint32_t w) {  // nibbles 0, 2, 4, 6 -> the low half
     w &= 0x0f0f0f0fu;
@@ -356,6 +362,40 @@ __device__ __forceinline__ void dequant8(uint32_t w, const ZeroScale<BF16> &zs, 
         p[3] = mul_f16x2(fma_f16x2(v3, 0x2c002c00u, zs.zfma), zs.s2);
     }
 }
+
+// The same weights, bit for bit, with one shift instead of three in bf16 (13 instructions as in f16): the odd nibbles are used
+// where they stand. w & 0x00f000f0 read as bf16 is c * 2^-129 (three mantissa bits and the lowest exponent bit: the spacing
+// of the numbers is the same on both sides of the smallest normal one), so fma(v, 2^127, -z/4) = (c - z) / 4 exactly, and the
+// multiply by 4s rounds the same product as one by s. A scale whose fourfold is not a finite bf16 (2^126 and more) would lose
+// the weights it can still hold, so such a scale takes the other form: `wide`, uniform over the warp that asks.
+// Used where the ALU pipe and the issue slots bound the conversion (tcgen05 kernel: 32 bf16 layers at 16 rows 1715 -> 1637 us,
+// 64 x 14336 x 4096 17.3 -> 16.9 us); the streaming GEMV kernel, bound by the packed-half pipe, measured 1 to 2 % slower with
+// it (8192 x 57344 at M = 1: 57.5 -> 58.9 us) and keeps the form above.
+template <bool BF16>
+struct ShortConvert {
+    ZeroScale<BF16> zs;
+    uint32_t zq, s4;
+    bool wide;
+    __device__ __forceinline__ void set(int z, uint32_t scale_bits) {  // all 32 lanes
+        zs.set(z, scale_bits);
+        if (BF16) {
+            zq = fma_bf16x2(zs.zsub, 0xbe80be80u, 0x42004200u);  // -(128 + z) / 4 + 32, exact
+            s4 = mul_bf16x2(zs.s2, 0x40804080u);
+            wide = __any_sync(0xffffffffu, (scale_bits & 0x7fffu) >= 0x7e80u);  // |s| >= 2^126
+        }
+    }
+    __device__ __forceinline__ void operator()(uint32_t w, uint32_t (&p)[4]) const {
+        if (BF16) {
+            const uint32_t w8 = w >> 8;
+            p[0] = mul_bf16x2(sub_bf16x2(lop3_and_or(w, 0x000f000fu, 0x43004300u), zs.zsub), zs.s2);
+            p[1] = mul_bf16x2(fma_bf16x2(w & 0x00f000f0u, 0x7f007f00u, zq), s4);
+            p[2] = mul_bf16x2(sub_bf16x2(lop3_and_or(w8, 0x000f000fu, 0x43004300u), zs.zsub), zs.s2);
+            p[3] = mul_bf16x2(fma_bf16x2(w8 & 0x00f000f0u, 0x7f007f00u, zq), s4);
+        } else {
+            dequant8<BF16>(w, zs, p);
+        }
+    }
+};
 
 // Zero point of (group gi, column n) for the three storage modes.
 template <int ZMODE>

@@ -143,6 +143,11 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3])
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -186,6 +191,11 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t smem_addr) {
     return d;
 }
 
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -199,25 +209,26 @@ __device__ __forceinline__ int load_zero_rt(const void *zeros, int zmode, int zc
     return load_zero<QF_ZERO_I8>(zeros, zconst, gi, n, N);
 }
 
+// (c0,c4)(c1,c5)(c2,c6)(c3,c7) -> (c0,c1)(c2,c3)(c4,c5)(c6,c7)
+__device__ __forceinline__ void reorder8(uint32_t (&p)[4]) {
+    const uint32_t lo0 = prmt(p[0], p[1], 0x5410u), lo1 = prmt(p[2], p[3], 0x5410u);
+    const uint32_t hi0 = prmt(p[0], p[1], 0x7632u), hi1 = prmt(p[2], p[3], 0x7632u);
+    p[0] = lo0;
+    p[1] = lo1;
+    p[2] = hi0;
+    p[3] = hi1;
+}
 // 4 packed words (32 codes along K) -> 16 registers of 16-bit pairs in natural k order.
 template <bool BF16, bool INTER>
-__device__ __forceinline__ void convert32(const uint4 &v, const ZeroScale<BF16> &zs, uint32_t (&out)[16]) {
+__device__ __forceinline__ void convert32(const uint4 &v, const ShortConvert<BF16> &conv, uint32_t (&out)[16]) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         uint32_t p[4];
-        dequant8<BF16>(w[j], zs, p);  // p[i] = (nibble i, nibble i+4)
-        if (INTER) {                  // nibble order c0 c2 c4 c6 c1 c3 c5 c7: pairs are already (c0,c1)(c2,c3)..
-            out[4 * j + 0] = p[0];
-            out[4 * j + 1] = p[1];
-            out[4 * j + 2] = p[2];
-            out[4 * j + 3] = p[3];
-        } else {
-            out[4 * j + 0] = prmt(p[0], p[1], 0x5410u);
-            out[4 * j + 1] = prmt(p[2], p[3], 0x5410u);
-            out[4 * j + 2] = prmt(p[0], p[1], 0x7632u);
-            out[4 * j + 3] = prmt(p[2], p[3], 0x7632u);
-        }
+        conv(w[j], p);            // p[i] = (nibble i, nibble i+4)
+        if (!INTER) reorder8(p);  // nibble order c0 c2 c4 c6 c1 c3 c5 c7: pairs are already (c0,c1)(c2,c3)..
+#pragma unroll
+        for (int i = 0; i < 4; ++i) out[4 * j + i] = p[i];
     }
 }
 
@@ -412,7 +423,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             if (!__all_sync(0xffffffffu, ready)) break;
             tc_fence_after();
             // zero and scale of (this row, this k-block's group) from the stage's slivers
-            ZeroScale<BF16> zs;
+            ShortConvert<BF16> conv;
             {
                 const uint32_t szb = sz_stage(s);
                 uint32_t sbits;
@@ -425,7 +436,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 } else if (p.zero_mode == QF_ZERO_I8) {
                     asm volatile("ld.shared.s8 %0, [%1];" : "=r"(z) : "r"(szb + 256u + row));
                 }
-                zs.set(z, sbits);
+                conv.set(z, sbits);
             }
             const uint32_t wbase = w_stage(s) + row_off;
             const uint32_t a_col = BN + a * C::A_COLS;
@@ -433,8 +444,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             for (int c = 0; c < C::W_ROW_BYTES / 16; ++c) {
                 const uint4 v = lds128(wbase + (((uint32_t)c ^ sw) << 4));
                 uint32_t out[16];
-                convert32<BF16, INTER>(v, zs, out);
+                convert32<BF16, INTER>(v, conv, out);
                 tmem_st16(lane_taddr + a_col + c * 16, out);
+            }
+            if (BF16 && conv.wide) {
+                // once more in the other form. Behind the ordinary path and rolled up: as a branch in front of it, or unrolled,
+                // it cost that path its schedule or its registers (32 bf16 layers at 16 rows: 1688 and 1819 us)
+                tmem_wait_st();
+#pragma unroll 1
+                for (int j = 0; j < C::W_ROW_BYTES / 4; ++j) {
+                    uint32_t q[4];
+                    dequant8<BF16>(lds32(wbase + ((((uint32_t)j >> 2) ^ sw) << 4) + ((uint32_t)j & 3u) * 4u), conv.zs, q);
+                    if (!INTER) reorder8(q);
+                    tmem_st4(lane_taddr + a_col + j * 4, q);
+                }
             }
             tmem_wait_st();
             tc_fence_before();
