@@ -48,6 +48,7 @@ struct GemmCfg {
     static constexpr int A_COLS = BK / 2;                        // 32-bit TMEM columns per A buffer
     static constexpr int TMEM_COLS = (BN + NA * A_COLS) <= 256 ? 256 : 512;
     static constexpr int CTAS_PER_SM = BN <= 64 ? 2 : 1;
+    static_assert(BN * 512 <= STAGES * STAGE_BYTES, "the epilogue stages the fp32 tile in the pipeline's memory");
     static constexpr int SZ_BYTES = 512;                          // per stage: 256 B scales + up to 128 B zeros
     static constexpr int SMEM_BYTES =
         STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + STAGES * SZ_BYTES;
@@ -78,34 +79,87 @@ struct GemmParams {
     int epilogue;          // qf_epilogue (plain instantiations only)
 };
 
-__device__ __forceinline__ float gemm_load_out(const void *R, int out_dtype, int64_t idx) {
-    if (out_dtype == QF_F32) return reinterpret_cast<const float *>(R)[idx];
-    if (out_dtype == QF_F16) return __half2float(reinterpret_cast<const __half *>(R)[idx]);
-    return __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(R)[idx]);
-}
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.f + expf(-gate)) * up; }
-// Four finished outputs of batch row m, weight rows n..n+3 (n a multiple of 4), with the plain or residual epilogue.
-__device__ __forceinline__ void gemm_store4(const GemmParams &p, int64_t m, int64_t n, float4 a) {
-    const int64_t o = m * p.N + n;
-    if (p.epilogue == QF_EPI_RESIDUAL_ADD) {
-        a.x += gemm_load_out(p.residual, p.out_dtype, o);
-        a.y += gemm_load_out(p.residual, p.out_dtype, o + 1);
-        a.z += gemm_load_out(p.residual, p.out_dtype, o + 2);
-        a.w += gemm_load_out(p.residual, p.out_dtype, o + 3);
+// CNT (4 or 8) consecutive elements of the output type, as vectors: element offsets are multiples of CNT, the base is 16-byte
+// aligned and rows are multiples of 128 bytes long.
+template <int CNT>
+__device__ __forceinline__ void store_vec(void *Y, int out_dtype, int64_t o, const float (&v)[CNT]) {
+    if (out_dtype == QF_F32) {
+        float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(Y) + o);
+#pragma unroll
+        for (int i = 0; i < CNT / 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        return;
     }
-    store_out(p.Y, p.out_dtype, o, a.x);
-    store_out(p.Y, p.out_dtype, o + 1, a.y);
-    store_out(p.Y, p.out_dtype, o + 2, a.z);
-    store_out(p.Y, p.out_dtype, o + 3, a.w);
+    uint32_t r[CNT / 2];
+#pragma unroll
+    for (int i = 0; i < CNT / 2; ++i) {
+        if (out_dtype == QF_F16) {
+            const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+            r[i] = *reinterpret_cast<const uint32_t *>(&h);
+        } else {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            r[i] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+    }
+    uint16_t *dst = reinterpret_cast<uint16_t *>(Y) + o;
+    if constexpr (CNT == 8) *reinterpret_cast<uint4 *>(dst) = make_uint4(r[0], r[1], r[2], r[3]);
+    else *reinterpret_cast<uint2 *>(dst) = make_uint2(r[0], r[1]);
 }
-// QF_EPI_SILU_MUL: weight rows n..n+3 (n % 16 < 8) are gate rows, n+8.. the matching up rows; output column
+template <int CNT>
+__device__ __forceinline__ void add_residual(const void *R, int out_dtype, int64_t o, float (&v)[CNT]) {
+    if (out_dtype == QF_F32) {
+        const float4 *src = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(R) + o);
+#pragma unroll
+        for (int i = 0; i < CNT / 4; ++i) {
+            const float4 a = src[i];
+            v[4 * i] += a.x;
+            v[4 * i + 1] += a.y;
+            v[4 * i + 2] += a.z;
+            v[4 * i + 3] += a.w;
+        }
+        return;
+    }
+    uint32_t r[CNT / 2];
+    const uint16_t *src = reinterpret_cast<const uint16_t *>(R) + o;
+    if constexpr (CNT == 8) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(src);
+        r[0] = a.x, r[1] = a.y, r[2] = a.z, r[3] = a.w;
+    } else {
+        const uint2 a = *reinterpret_cast<const uint2 *>(src);
+        r[0] = a.x, r[1] = a.y;
+    }
+#pragma unroll
+    for (int i = 0; i < CNT / 2; ++i) {
+        const float2 f = out_dtype == QF_F16 ? __half22float2(*reinterpret_cast<const __half2 *>(&r[i]))
+                                             : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&r[i]));
+        v[2 * i] += f.x;
+        v[2 * i + 1] += f.y;
+    }
+}
+// CNT finished outputs of batch row m, weight rows n.. (n a multiple of CNT), with the plain or residual epilogue.
+template <int CNT>
+__device__ __forceinline__ void gemm_store(const GemmParams &p, int64_t m, int64_t n, float (&v)[CNT]) {
+    const int64_t o = m * p.N + n;
+    if (p.epilogue == QF_EPI_RESIDUAL_ADD) add_residual<CNT>(p.residual, p.out_dtype, o, v);
+    store_vec<CNT>(p.Y, p.out_dtype, o, v);
+}
+// QF_EPI_SILU_MUL: weight rows n.. (n % 16 < 8) are gate rows, n+8.. the matching up rows; output column
 // (n / 16) * 8 + n % 8 of Y[M, N/2].
+template <int CNT>
+__device__ __forceinline__ void gemm_store_silu(const GemmParams &p, int64_t m, int64_t n, const float (&g)[CNT],
+                                                const float (&u)[CNT]) {
+    float v[CNT];
+#pragma unroll
+    for (int i = 0; i < CNT; ++i) v[i] = silu_mul(g[i], u[i]);
+    store_vec<CNT>(p.Y, p.out_dtype, m * (p.N >> 1) + (n >> 4) * 8 + (n & 7), v);
+}
+__device__ __forceinline__ void gemm_store4(const GemmParams &p, int64_t m, int64_t n, float4 a) {
+    float v[4] = {a.x, a.y, a.z, a.w};
+    gemm_store<4>(p, m, n, v);
+}
 __device__ __forceinline__ void gemm_store4_silu(const GemmParams &p, int64_t m, int64_t n, float4 g, float4 u) {
-    const int64_t o = m * (p.N >> 1) + (n >> 4) * 8 + (n & 7);
-    store_out(p.Y, p.out_dtype, o, silu_mul(g.x, u.x));
-    store_out(p.Y, p.out_dtype, o + 1, silu_mul(g.y, u.y));
-    store_out(p.Y, p.out_dtype, o + 2, silu_mul(g.z, u.z));
-    store_out(p.Y, p.out_dtype, o + 3, silu_mul(g.w, u.w));
+    const float gv[4] = {g.x, g.y, g.z, g.w}, uv[4] = {u.x, u.y, u.z, u.w};
+    gemm_store_silu<4>(p, m, n, gv, uv);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -191,6 +245,15 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t smem_addr) {
     return d;
 }
 
+template <int CNT>
+__device__ __forceinline__ void lds_f4(uint32_t addr, float (&v)[4 * CNT]) {
+#pragma unroll
+    for (int i = 0; i < CNT; ++i)
+        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                     : "=f"(v[4 * i]), "=f"(v[4 * i + 1]), "=f"(v[4 * i + 2]), "=f"(v[4 * i + 3])
+                     : "r"(addr + 16u * i)
+                     : "memory");
+}
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
@@ -474,39 +537,35 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             // this rank has finished and advanced the epoch
             unsigned ar_epoch = 0u;
             if constexpr (EXCH) ar_epoch = exch_read_epoch(ar);
+            // TMEM -> fp32 tile [batch row][weight row] in the (now idle) pipeline stages, from where whole output rows
+            // leave as 16-byte stores. Written straight from TMEM, one element per thread and store with the epilogue chosen per
+            // element, a 128 x 256 tile took 23 700 cycles, a third of the whole K = 4096 tile (M = 2048, 8192 x 28672: 897 ->
+            // 777 us; M = 777, 4096 x 4096: 35.6 -> 28.9 us; 64 x 14336 x 4096: 17.3 -> 15.9 us).
+            // Split-K partial tiles that meet in global memory and exchanged tiles go there directly.
             const int cols_per_wg = p.bn >> 1;
             const int64_t Mp = (int64_t)gridDim.x * p.bn;
+            const bool to_partial = p.split_k > 1 && !(CLUSTER_OK && p.cluster_reduce);
+            float *part = p.partial + ((int64_t)split * Mp + m0) * p.N + n;
 #pragma unroll 1
             for (int c8 = 0; c8 < cols_per_wg >> 3; ++c8) {
                 const int col = wg * cols_per_wg + c8 * 8;
                 uint32_t r[8];
                 tmem_ld8(lane_taddr + col, r);
                 tmem_wait_ld();
+                if (to_partial) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int64_t m = m0 + col + j;
-                    const float v = __uint_as_float(r[j]);
-                    if (p.split_k == 1) {
-                        if constexpr (EXCH) {
-                            if (m < p.M) exch_push(ar, ar_epoch, (size_t)(m * p.N + n), v);
-                        } else if (p.epilogue == QF_EPI_SILU_MUL) {
-                            // lanes 0-7 and 16-23 of a warp hold gate rows, the lanes 8 above them the up rows
-                            const float up = __shfl_xor_sync(0xffffffffu, v, 8);
-                            if (m < p.M && (row & 8) == 0)
-                                store_out(p.Y, p.out_dtype, m * (p.N >> 1) + (n >> 4) * 8 + (n & 7), silu_mul(v, up));
-                        } else if (m < p.M) {
-                            const float res =
-                                p.epilogue == QF_EPI_RESIDUAL_ADD ? gemm_load_out(p.residual, p.out_dtype, m * p.N + n) : 0.f;
-                            store_out(p.Y, p.out_dtype, m * p.N + n, v + res);
-                        }
-                    } else if (CLUSTER_OK && p.cluster_reduce) {
-                        // partial tile [batch row][weight row] fp32 in the (now idle) pipeline stages
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem_base + (uint32_t)((col + j) * 128 + row) * 4u),
-                                     "f"(v)
-                                     : "memory");
-                    } else {
-                        __stcg(p.partial + ((int64_t)split * Mp + m) * p.N + n, v);
+                    for (int j = 0; j < 8; ++j) __stcg(part + (int64_t)(col + j) * p.N, __uint_as_float(r[j]));
+                } else if constexpr (EXCH) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int64_t m = m0 + col + j;
+                        if (m < p.M) exch_push(ar, ar_epoch, (size_t)(m * p.N + n), __uint_as_float(r[j]));
                     }
+                } else {
+                    const uint32_t dst = smem_base + (uint32_t)(col * 128 + row) * 4u;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + j * 512u), "r"(r[j]) : "memory");
                 }
             }
         }
@@ -582,6 +641,25 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         if (tid == 0) atomicExch(p.status, QF_ERR_TIMEOUT);
         __syncthreads();
     } else {
+        if (!EXCH && p.split_k == 1) {
+            const int rows = (int)min((int64_t)p.bn, p.M - m0);
+            if (p.epilogue == QF_EPI_SILU_MUL) {
+                for (int u = tid; u < rows * 8; u += GEMM_THREADS) {
+                    const uint32_t a = smem_base + (uint32_t)u * 64u;  // 8 gate rows, then their 8 up rows
+                    float v[16];
+                    lds_f4<4>(a, v);
+                    const float g[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
+                    const float up[8] = {v[8], v[9], v[10], v[11], v[12], v[13], v[14], v[15]};
+                    gemm_store_silu<8>(p, m0 + (u >> 3), n0 + (u & 7) * 16, g, up);
+                }
+            } else {
+                for (int u = tid; u < rows * 16; u += GEMM_THREADS) {
+                    float v[8];
+                    lds_f4<2>(smem_base + (uint32_t)u * 32u, v);
+                    gemm_store<8>(p, m0 + (u >> 4), n0 + (u & 15) * 8, v);
+                }
+            }
+        }
         bool final_cta = true;  // this CTA holds (or has pushed) the finished tile
         unsigned ar_epoch = 0u;
         if constexpr (EXCH) ar_epoch = exch_read_epoch(ar);
