@@ -161,6 +161,7 @@ struct Plan {
     bool slab;           // QF_LAYOUT_GEMV_SLAB weights: the streaming GEMV kernel
     int m_tiles;         // GEMV: ceil(M/8); GEMM: batch tiles
     int bn;              // GEMM: batch tile width (MMA N)
+    bool pair;           // GEMM: two CTAs share a batch tile (cta_group::2)
     size_t ws_partial_bytes;
     size_t ws_counter_bytes;
 };
@@ -213,7 +214,7 @@ int launch_gemm(qf_ctx *ctx, const qf_linear_desc *d, const Plan &p, const void 
 int launch_prepack(qf_ctx *ctx, const void *in, void *out, int64_t n_words, int to_canonical, cudaStream_t s);
 int launch_prepack_tiled(qf_ctx *ctx, const void *in, void *out, int64_t N, int64_t K, int to_canonical,
                          cudaStream_t s);
-int gemm_block_k(int bn);
+int gemm_block_k(int bn, bool pair);
 int launch_gemv_ar(qf_ctx *ctx, const qf_linear_desc *d, const Plan &p, const void *X, const void *qw,
                    const void *scales, const void *zeros, void *Y, void *ws, cudaStream_t s, const ArParams &ar);
 int launch_gemm_ar(qf_ctx *ctx, const qf_linear_desc *d, const Plan &p, const void *X, const void *qw,

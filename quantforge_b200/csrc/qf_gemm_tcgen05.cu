@@ -35,15 +35,17 @@ namespace qf {
 // ---------------------------------------------------------------------------------------------
 // configuration per batch-tile width
 // ---------------------------------------------------------------------------------------------
-template <int BN>
+// PAIR: two CTAs (weight tiles 2i and 2i + 1 of one batch tile) run their MMAs as one of 256 weight rows.
+template <int BN, bool PAIR = false>
 struct GemmCfg {
-    static constexpr int BK = (BN <= 128) ? 128 : 64;           // codes per k-block
+    static constexpr int BK = (BN <= 128 || PAIR) ? 128 : 64;   // codes per k-block
+    static constexpr int X_ROWS = PAIR ? BN / 2 : BN;            // batch rows a CTA stages (at most)
     static constexpr int W_ROW_BYTES = BK / 2;                   // 64 or 32
     static constexpr int W_STAGE_BYTES = 128 * W_ROW_BYTES;      // 8 KB or 4 KB
-    static constexpr int X_BOX_BYTES = BN * 128;                 // one 64-element box
+    static constexpr int X_BOX_BYTES = X_ROWS * 128;             // one 64-element box
     static constexpr int X_STAGE_BYTES = X_BOX_BYTES * (BK / 64);
     static constexpr int STAGE_BYTES = W_STAGE_BYTES + X_STAGE_BYTES;
-    static constexpr int STAGES = BN == 16 ? 8 : BN == 32 ? 6 : BN == 64 ? 4 : 5;
+    static constexpr int STAGES = BN == 16 || (PAIR && BN == 128) ? 8 : BN == 32 ? 6 : BN == 64 ? 4 : 5;
     static constexpr int NA = BN <= 64 ? 3 : 4;                  // A operand buffers in TMEM
     static constexpr int A_COLS = BK / 2;                        // 32-bit TMEM columns per A buffer
     static constexpr int TMEM_COLS = (BN + NA * A_COLS) <= 256 ? 256 : 512;
@@ -175,15 +177,26 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
+// The forms of one CTA and of a CTA pair (PAIR). All tcgen05 operations of one kernel that name a CTA group name the same one.
+template <bool PAIR>
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
-                 : "memory");
+    if constexpr (PAIR)
+        asm volatile(
+            "tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n\t"
+            "tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::"r"(dst_smem), "r"(ncols)
+            : "memory");
+    else
+        asm volatile(
+            "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n\t"
+            "tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::"r"(dst_smem), "r"(ncols)
+            : "memory");
 }
-__device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
+template <bool PAIR>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    if constexpr (PAIR)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    else
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -209,15 +222,37 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "memory");
 }
 
-// D[tmem] (+)= A[tmem] . B[smem desc]
+// D[tmem] (+)= A[tmem] . B[smem desc]. PAIR: 128 rows of D and A in either CTA's TMEM, half of B's rows in either CTA's
+// shared memory.
+template <bool PAIR>
 __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if constexpr (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Arrive on a barrier of any block of the cluster (address from dsmem_addr). No wider release than the default: what it announces
+// lies in TMEM (ordered by the tcgen05 fences) and in shared memory written by the copy engine; with .release.cluster and an
+// acquire fence behind the wait, both of which wait for the block's earlier memory accesses, M = 2048, 8192 x 28672 took
+// 1190 us.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // One lane of a fully active warp (the same lane every time within a kernel).
 __device__ __forceinline__ bool elect_one() {
@@ -229,9 +264,16 @@ __device__ __forceinline__ bool elect_one() {
         : "=r"(pred));
     return pred != 0;
 }
-// Arrives on the mbarrier once all MMAs issued so far by this thread have completed.
+// Arrives on the mbarrier (of a pair: at this address in both CTAs) once all MMAs issued so far by this thread have completed.
+template <bool PAIR>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    if constexpr (PAIR)
+        asm volatile(
+            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+            "h"((uint16_t)3)
+            : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // K-major shared-memory operand descriptor, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
@@ -300,11 +342,18 @@ __device__ __forceinline__ void convert32(const uint4 &v, const ShortConvert<BF1
 // ---------------------------------------------------------------------------------------------
 // EXCH: finished tiles are exchanged across GPUs (sum or gather) before Y is written; `ar` then is an ArParams.
 // The plain instantiations take an empty struct instead, so their parameter block and code stay what they were.
-template <bool BF16, int BN, bool INTER, bool EXCH>
-__global__ void __launch_bounds__(GEMM_THREADS, GemmCfg<BN>::CTAS_PER_SM)
+// PAIR: the grid runs in clusters of two blocks along x (weight tiles 2i, 2i + 1). A block stages half of the batch tile's
+// rows and its own weights; its converters report to the first block, whose MMA warp issues cta_group::2 MMAs of 256
+// weight rows for both and signals completion to both. With one CTA per MMA a k-block of 64 codes and 256 rows moves 72 KB
+// through a block's shared memory (36 KB in, 32 KB to the tensor core, 4 KB of codes to the converters), 562 cycles at
+// 128 bytes a cycle and more than the 512 the MMAs take; in a pair it is 40 KB. M = 2048, 8192 x 28672: 777 -> 738 us;
+// M = 777, 4096 x 4096: 28.9 -> 27.5 us.
+template <bool BF16, int BN, bool INTER, bool EXCH, bool PAIR>
+__global__ void __launch_bounds__(GEMM_THREADS, GemmCfg<BN, PAIR>::CTAS_PER_SM)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
             const GemmParams p, const typename ExchArg<EXCH>::type ar) {
-    using C = GemmCfg<BN>;
+    using C = GemmCfg<BN, PAIR>;
+    static_assert(!(PAIR && EXCH), "the exchange serves the narrow tiles");
     constexpr int BK = C::BK;
     constexpr int STAGES = C::STAGES;
     constexpr int NA = C::NA;
@@ -329,8 +378,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
-    const int m_tile = blockIdx.x;
-    const int n_tile = blockIdx.y;
+    const int m_tiles = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+    const int m_tile = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x;
+    const int n_tile = PAIR ? (int)blockIdx.y * 2 + ((int)blockIdx.x & 1) : (int)blockIdx.y;
     const int split = blockIdx.z;
     const int kb0 = split * p.kblocks_per_split;
     const int kb1 = min(kb0 + p.kblocks_per_split, p.kblocks);
@@ -342,10 +392,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         s_abort = 0;
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full_bar(s), 1);
-            mbar_init(empty_bar(s), 128 + 1);
+            mbar_init(empty_bar(s), PAIR ? 4 + 1 : 128 + 1);  // pair: one arrival per warp of a converter group
         }
         for (int a = 0; a < NA; ++a) {
-            mbar_init(afull_bar(a), 128);
+            mbar_init(afull_bar(a), PAIR ? 2 * 4 : 128);      // of either block
             mbar_init(aempty_bar(a), 1);
         }
         mbar_init(dfull_bar, 1);
@@ -356,23 +406,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         tma_prefetch_desc(&tmap_x);
     }
     if (warp == 9) {
-        tmem_alloc(smem_u32(&s_tmem_base), C::TMEM_COLS);
-        tmem_relinquish();
+        tmem_alloc<PAIR>(smem_u32(&s_tmem_base), C::TMEM_COLS);
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();  // the other block's barriers exist
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
     volatile int *abort_flag = &s_abort;
     griddep_launch_dependents();  // the next kernel may begin its own set-up and weight prefetch
 
+    const uint32_t rank = PAIR ? cluster_rank() : 0u;
     int producer_issued = 0;  // meaningful in the elected producer lane only
     if (warp == 8) {
         // ------------------------------ TMA producer ------------------------------
         // The whole warp runs the loop (uniform control flow); one elected lane issues the copies.
         const bool leader = elect_one();
         const uint32_t zbytes = p.zero_mode == QF_ZERO_U4 ? 64u : p.zero_mode == QF_ZERO_I8 ? 128u : 0u;
-        const uint32_t tx_bytes = C::W_STAGE_BYTES + (uint32_t)(BK / 64) * (uint32_t)p.bn * 128u + 256u + zbytes;
+        const int x_rows = PAIR ? p.bn >> 1 : p.bn;  // this block's share of the batch tile
+        const int x_row0 = (int)m0 + (int)rank * x_rows;
+        const uint32_t tx_bytes = C::W_STAGE_BYTES + (uint32_t)(BK / 64) * (uint32_t)x_rows * 128u + 256u + zbytes;
         const int group_kb = p.group_size / BK;  // k-blocks per quantisation group (>= 1)
         const int gi = kb0 / group_kb;
         const uint8_t *sc_ptr = (const uint8_t *)(p.scales + n0) + (size_t)gi * p.N * 2;
@@ -405,7 +458,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             const int kb = kb0 + it;
 #pragma unroll
             for (int b = 0; b < BK / 64; ++b)
-                tma_load_2d(x_stage(s) + b * C::X_BOX_BYTES, &tmap_x, full_bar(s), kb * BK + b * 64, (int)m0);
+                tma_load_2d(x_stage(s) + b * C::X_BOX_BYTES, &tmap_x, full_bar(s), kb * BK + b * 64, x_row0);
             producer_issued = it + 1;
         };
         // First pass over the ring: weights, scales and zeros do not depend on the previous kernel of the stream,
@@ -432,13 +485,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         }
     } else if (warp == 9) {
         // ------------------------------ MMA issuer ------------------------------
-        // One thread runs the loop. It waits once per k-block: the converters reported after they had seen the stage's copies
-        // (weights and X share a barrier) arrive.
+        // One thread (of a pair: of the first block) runs the loop. It waits once per k-block: the converters reported after
+        // they had seen the stage's copies (weights and X share a barrier) arrive.
         // (As a whole warp with two waits and a vote on each, a k-block took about 100 cycles more of this warp and of the issue
         // slots that the converters need: a 6-layer step at 9 rows 594 -> 582 us, 32 layers at 16 rows 1604 -> 1596 us.)
-        if (elect_one()) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = (1u << 4) | ((BF16 ? 1u : 0u) << 7) | ((BF16 ? 1u : 0u) << 10) |
-                                   ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+                                   ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)((PAIR ? 256 : 128) >> 4) << 24);
             const uint64_t desc0 = make_b_desc(x_stage(0));
             int s = 0, a = 0, it = 0;
             uint32_t aph = 0;
@@ -447,20 +500,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 tc_fence_after();
                 const uint32_t a_tmem = tmem_base + BN + a * C::A_COLS;
                 const uint64_t desc = desc0 + (uint32_t)s * (uint32_t)(C::STAGE_BYTES >> 4);
-                umma_ts(tmem_base, a_tmem, desc, idesc, it > 0 ? 1u : 0u);
+                umma_ts<PAIR>(tmem_base, a_tmem, desc, idesc, it > 0 ? 1u : 0u);
 #pragma unroll
                 for (int kk = 1; kk < BK / 16; ++kk)
-                    umma_ts(tmem_base, a_tmem + kk * 8, desc + (uint32_t)(((kk >> 2) * C::X_BOX_BYTES + (kk & 3) * 32) >> 4),
-                            idesc, 1u);
-                umma_commit(empty_bar(s));
-                umma_commit(aempty_bar(a));
+                    umma_ts<PAIR>(tmem_base, a_tmem + kk * 8,
+                                  desc + (uint32_t)(((kk >> 2) * C::X_BOX_BYTES + (kk & 3) * 32) >> 4), idesc, 1u);
+                umma_commit<PAIR>(empty_bar(s));
+                umma_commit<PAIR>(aempty_bar(a));
                 if (++s == STAGES) s = 0;
                 if (++a == NA) {
                     a = 0;
                     aph ^= 1;
                 }
             }
-            if (it == nkb) umma_commit(dfull_bar);
+            if (it == nkb) umma_commit<PAIR>(dfull_bar);
         }
         __syncwarp();
     } else {
@@ -522,9 +575,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             }
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(afull_bar(a));
             fence_proxy_async_shared();  // this thread's reads of the stage, before the copy engine refills it
-            mbar_arrive(empty_bar(s));
+            if constexpr (PAIR) {
+                __syncwarp();
+                if (lane == 0) {
+                    // at the first block's barrier; it also says that this block's half of X has arrived
+                    mbar_arrive_cluster(dsmem_addr(afull_bar(a), 0u));
+                    mbar_arrive(empty_bar(s));
+                }
+            } else {
+                mbar_arrive(afull_bar(a));
+                mbar_arrive(empty_bar(s));
+            }
         }
 
         // ------------------------------ epilogue ------------------------------
@@ -541,7 +603,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             // 777 us; M = 777, 4096 x 4096: 35.6 -> 28.9 us; 64 x 14336 x 4096: 17.3 -> 15.9 us).
             // Split-K partial tiles that meet in global memory and exchanged tiles go there directly.
             const int cols_per_wg = p.bn >> 1;
-            const int64_t Mp = (int64_t)gridDim.x * p.bn;
+            const int64_t Mp = (int64_t)m_tiles * p.bn;
             const bool to_partial = p.split_k > 1 && !(CLUSTER_OK && p.cluster_reduce);
             float *part = p.partial + ((int64_t)split * Mp + m0) * p.N + n;
 #pragma unroll 1
@@ -666,7 +728,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             __threadfence();
             __syncthreads();
             if (tid == 0) {
-                int *cnt = p.counters + (int64_t)n_tile * gridDim.x + m_tile;
+                int *cnt = p.counters + (int64_t)n_tile * m_tiles + m_tile;
                 const int prev = atomicAdd(cnt, 1);
                 s_is_last = (prev == p.split_k - 1);
                 if (s_is_last) *cnt = 0;
@@ -677,7 +739,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 __threadfence();
                 // Each thread owns 4 consecutive output columns (one 16-byte load per split) and keeps 4 splits in
                 // flight, so the reduction is not a chain of dependent L2 round trips.
-                const int64_t Mp = (int64_t)gridDim.x * p.bn;
+                const int64_t Mp = (int64_t)m_tiles * p.bn;
                 const size_t split_stride = (size_t)Mp * p.N;
                 for (int u = tid; u < 32 * p.bn; u += GEMM_THREADS) {
                     const int nl = (u & 31) * 4;
@@ -730,9 +792,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             if (tid == 0) exch_block_done(ar, ar_epoch, gridDim.x * gridDim.y, s_abort != 0);
         }
     }
+    // a pair leaves together: MMAs read and signal both blocks, and both give back their TMEM
+    if constexpr (PAIR) cluster_sync_all();
     if (warp == 9) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, C::TMEM_COLS);
+        tmem_dealloc<PAIR>(tmem_base, C::TMEM_COLS);
     }
 }
 
@@ -809,17 +873,23 @@ static int get_tensor_map(qf_ctx *ctx, CUtensorMap *out, const void *ptr, int ki
 // Instantiation (widest batch tile) that serves a batch tile of bn rows.
 static int gemm_tile_of(int bn) { return bn <= 16 ? 16 : bn <= 32 ? 32 : bn <= 64 ? 64 : bn <= 128 ? 128 : 256; }
 
+constexpr bool gemm_has_pair(int bn) { return bn >= 128; }
 constexpr bool gemm_has_exchange(int bn) { return bn <= 64; }  // the cross-GPU exchange serves decode batches only
 
 template <bool BF16, int BN>
 static cudaError_t gemm_set_attr() {
     const int bytes = GemmCfg<BN>::SMEM_BYTES;
     const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, false>, attr, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, true, false>, attr, bytes);
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, false, false>, attr, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, true, false, false>, attr, bytes);
     if constexpr (gemm_has_exchange(BN)) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, true>, attr, bytes);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, true, true>, attr, bytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, true, false>, attr, bytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, true, true, false>, attr, bytes);
+    }
+    if constexpr (gemm_has_pair(BN)) {
+        const int pair_bytes = GemmCfg<BN, true>::SMEM_BYTES;
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, false, true>, attr, pair_bytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, true, false, true>, attr, pair_bytes);
     }
     return e;
 }
@@ -843,30 +913,31 @@ int gemm_init(qf_ctx *ctx) {
     return QF_OK;
 }
 
-template <bool BF16, int BN>
+template <bool BF16, int BN, bool PAIR>
 static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan, const void *X, const void *qw,
                           GemmParams &p, cudaStream_t s, const ArParams *ar) {
-    using C = GemmCfg<BN>;
+    using C = GemmCfg<BN, PAIR>;
     CUtensorMap tw, tx;
     const bool tiled = d->weight_layout == QF_LAYOUT_TILED;
     int st = get_tensor_map(ctx, &tw, qw, 0, tiled ? 64 : (uint64_t)d->K / 2,
                             tiled ? (uint64_t)d->N * (uint64_t)(d->K / 128) : (uint64_t)d->N, C::W_ROW_BYTES, 128,
                             C::BK == 128 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     if (st != QF_OK) return st;
-    st = get_tensor_map(ctx, &tx, X, 1, (uint64_t)d->K, (uint64_t)d->M, 64, (uint32_t)plan.bn,
-                        CU_TENSOR_MAP_SWIZZLE_128B);
+    st = get_tensor_map(ctx, &tx, X, 1, (uint64_t)d->K, (uint64_t)d->M, 64,
+                        (uint32_t)(PAIR ? plan.bn / 2 : plan.bn), CU_TENSOR_MAP_SWIZZLE_128B);
     if (st != QF_OK) return st;
     p.bn = plan.bn;
     p.kblocks = (int)(d->K / C::BK);
     p.kblocks_per_split = plan.chunks_per_split;
-    dim3 grid((unsigned)plan.m_tiles, (unsigned)(d->N / 128), (unsigned)plan.split_k);
+    // a pair's blocks differ in x: the dimension along which cta_group::2 pairs them
+    dim3 grid((unsigned)plan.m_tiles * (PAIR ? 2u : 1u), (unsigned)(d->N / 128) / (PAIR ? 2u : 1u), (unsigned)plan.split_k);
     const dim3 blk(GEMM_THREADS);
     cudaError_t le;
     if (ar) {
-        if constexpr (gemm_has_exchange(BN)) {
-            le = p.interleaved ? launch_kernel(gemm_kernel<BF16, BN, true, true>, grid, blk, C::SMEM_BYTES, s,
+        if constexpr (gemm_has_exchange(BN) && !PAIR) {
+            le = p.interleaved ? launch_kernel(gemm_kernel<BF16, BN, true, true, false>, grid, blk, C::SMEM_BYTES, s,
                                                pdl_enabled(), tw, tx, p, *ar)
-                               : launch_kernel(gemm_kernel<BF16, BN, false, true>, grid, blk, C::SMEM_BYTES, s,
+                               : launch_kernel(gemm_kernel<BF16, BN, false, true, false>, grid, blk, C::SMEM_BYTES, s,
                                                pdl_enabled(), tw, tx, p, *ar);
         } else {
             return fail(ctx, QF_ERR_UNSUPPORTED, "the in-kernel exchange serves M <= 64");
@@ -877,16 +948,16 @@ static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan
         // multiple of the cluster size; a launch that no longer fits in one wave loses more than the on-chip
         // reduction gains (measured: 32 x 8, 80 x 3, 112 x 2 blocks fit; 48 x 6 = 288 of the 296 slots do not).
         unsigned cluster_z = 1;
-        if (BN <= 64 && plan.split_k >= 2 && plan.split_k <= 8 && cluster_reduce_enabled()) {
+        if (BN <= 64 && !PAIR && plan.split_k >= 2 && plan.split_k <= 8 && cluster_reduce_enabled()) {
             if ((int64_t)grid.x * grid.y * grid.z <= kClusterMaxBlocks) {
                 p.cluster_reduce = 1;
                 cluster_z = (unsigned)plan.split_k;
             }
         }
-        le = p.interleaved ? launch_kernel_cluster(gemm_kernel<BF16, BN, true, false>, grid, blk, C::SMEM_BYTES, s,
-                                             pdl_enabled(), dim3(1, 1, cluster_z), tw, tx, p, NoExchange{})
-                           : launch_kernel_cluster(gemm_kernel<BF16, BN, false, false>, grid, blk, C::SMEM_BYTES, s,
-                                             pdl_enabled(), dim3(1, 1, cluster_z), tw, tx, p, NoExchange{});
+        le = p.interleaved ? launch_kernel_cluster(gemm_kernel<BF16, BN, true, false, PAIR>, grid, blk, C::SMEM_BYTES, s,
+                                             pdl_enabled(), dim3(PAIR ? 2 : 1, 1, cluster_z), tw, tx, p, NoExchange{})
+                           : launch_kernel_cluster(gemm_kernel<BF16, BN, false, false, PAIR>, grid, blk, C::SMEM_BYTES, s,
+                                             pdl_enabled(), dim3(PAIR ? 2 : 1, 1, cluster_z), tw, tx, p, NoExchange{});
     }
     g_launch_count.fetch_add(1);
     QF_CUDA_TRY(ctx, le);
@@ -898,16 +969,20 @@ template <bool BF16>
 static int gemm_launch_dt(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan, const void *X, const void *qw,
                           GemmParams &p, cudaStream_t s, const ArParams *ar) {
     switch (gemm_tile_of(plan.bn)) {
-        case 16: return gemm_launch_bn<BF16, 16>(ctx, d, plan, X, qw, p, s, ar);
-        case 32: return gemm_launch_bn<BF16, 32>(ctx, d, plan, X, qw, p, s, ar);
-        case 64: return gemm_launch_bn<BF16, 64>(ctx, d, plan, X, qw, p, s, ar);
-        case 128: return gemm_launch_bn<BF16, 128>(ctx, d, plan, X, qw, p, s, ar);
-        case 256: return gemm_launch_bn<BF16, 256>(ctx, d, plan, X, qw, p, s, ar);
+        case 16: return gemm_launch_bn<BF16, 16, false>(ctx, d, plan, X, qw, p, s, ar);
+        case 32: return gemm_launch_bn<BF16, 32, false>(ctx, d, plan, X, qw, p, s, ar);
+        case 64: return gemm_launch_bn<BF16, 64, false>(ctx, d, plan, X, qw, p, s, ar);
+        case 128:
+            return plan.pair ? gemm_launch_bn<BF16, 128, true>(ctx, d, plan, X, qw, p, s, ar)
+                             : gemm_launch_bn<BF16, 128, false>(ctx, d, plan, X, qw, p, s, ar);
+        case 256:
+            return plan.pair ? gemm_launch_bn<BF16, 256, true>(ctx, d, plan, X, qw, p, s, ar)
+                             : gemm_launch_bn<BF16, 256, false>(ctx, d, plan, X, qw, p, s, ar);
         default: return fail(ctx, QF_ERR_BAD_ARG, "bad batch tile");
     }
 }
 
-int gemm_block_k(int bn) { return bn <= 128 ? 128 : 64; }
+int gemm_block_k(int bn, bool pair) { return bn <= 128 || pair ? 128 : 64; }
 
 static int launch_gemm_impl(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan, const void *X, const void *qw,
                             const void *scales, const void *zeros, void *Y, const void *residual, void *ws,
