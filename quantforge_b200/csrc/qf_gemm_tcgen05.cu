@@ -12,15 +12,15 @@
 //                    converts them with lop3 / packed 16-bit arithmetic (zero and scale of its own
 //                    row and group held in registers), and writes the 16-bit operand straight into
 //                    TMEM lane t with tcgen05.st.  The same threads run the epilogue
-//                    (tcgen05.ld -> convert -> global store, or split-K partials).
+//                    (tcgen05.ld -> fp32 tile in shared memory -> whole output rows, or split-K partials).
 //   warp 8         : TMA producer (one elected thread): packed-weight tile and X tile per stage.
 //   warp 9         : TMEM allocation and, one elected thread, tcgen05.mma issue: A from TMEM,
 //                    B (= X tile, K-major, 128-byte swizzle) from shared memory, fp32 accumulate in TMEM.
 // Every mbarrier wait is bounded: on expiry the CTA raises an abort flag, records QF_ERR_TIMEOUT in
 // the context's status word, drains its own TMA copies, frees its TMEM and returns.
-// Every CTA loads its own tiles (plain TMA loads). Split-K over 2..8 blocks runs as a thread-block cluster whose
+// Every CTA loads its own tiles (plain TMA loads). Wide tiles run as CTA pairs, see gemm_kernel. Split-K over 2..8 blocks runs as a thread-block cluster whose
 // blocks sum their partial tiles through distributed shared memory; other splits use global partial tiles and an
-// arrival counter. Both cluster barriers are passed by every block, aborted or not.
+// arrival counter. All cluster barriers are passed by every block, aborted or not.
 #include <cuda.h>
 
 #include <cstdlib>
