@@ -17,6 +17,35 @@ bool pdl_enabled() {
     return on;
 }
 
+// The node that a stream in capture depends on, where it is a single one.
+static bool capture_tail(cudaStream_t s, unsigned long long *id, cudaGraphNode_t *node) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo_v3(s, &status, id, nullptr, &deps, &edges, &n) != cudaSuccess) {
+        cudaGetLastError();  // the launch says what is wrong with the stream
+        return false;
+    }
+    if (status != cudaStreamCaptureStatusActive || n != 1) return false;
+    *node = deps[0];
+    return true;
+}
+
+// The linear that this thread captured last; the id of a capture is not used again.
+static thread_local unsigned long long t_capture_id = 0;
+static thread_local cudaGraphNode_t t_capture_node = nullptr;
+
+bool follows_linear(cudaStream_t s) {
+    unsigned long long id = 0;
+    cudaGraphNode_t node = nullptr;
+    return capture_tail(s, &id, &node) && node == t_capture_node && id == t_capture_id;
+}
+
+void note_linear(cudaStream_t s) {
+    if (!capture_tail(s, &t_capture_id, &t_capture_node)) t_capture_node = nullptr;
+}
+
 bool cluster_reduce_enabled() {
     static const bool on = [] {
         const char *e = std::getenv("QF_CLUSTER_REDUCE");

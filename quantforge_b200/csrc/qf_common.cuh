@@ -53,9 +53,19 @@ extern std::atomic<long long> g_launch_count;
 
 // Programmatic dependent launch (PDL): a kernel launched with it may start while the previous kernel in the
 // stream is still draining; it must execute griddep_wait() before touching anything that kernel wrote.
-// The linear kernels use the head start for what does not depend on the previous kernel: weight streams,
-// converter constants, barrier and TMEM set-up. QF_PDL=0 in the environment turns it off.
+// The linear kernels use the head start for barrier and TMEM set-up and for their first weights. Where the previous
+// kernel may be the one that wrote those (a prepack, a copy, a cast), they are only prefetched into L2, which is where its
+// writes arrive, and read behind the wait; the next kernel is let in behind the wait as well.
+// Captured behind a linear of this library (follows_linear) the first weights are loaded at once: whatever wrote them
+// precedes the first linear of that row, which let its successor in only when that work was complete. (Called eagerly, the
+// difference is 1 % and less for the slab and tcgen05 kernels, 9.2 -> 10.0 us for M = 3, 3968 x 5136 per channel.)
+// QF_PDL=0 in the environment turns it off.
 bool pdl_enabled();
+// Graph capture: the only node that the next launch on `s` would depend on is the linear that this thread captured last.
+// Outside a capture nobody knows what the stream ran last: false.
+bool follows_linear(cudaStream_t s);
+// After a linear's launch on `s`: remembers its node for follows_linear.
+void note_linear(cudaStream_t s);
 bool cluster_reduce_enabled();
 // Largest launch of the tcgen05 kernel (2 blocks per SM) that runs as one wave of thread-block clusters: clusters
 // are placed inside one GPC, which leaves block slots unused where the GPC's slot count is not a multiple of the
@@ -250,6 +260,10 @@ int launch_repack_kn(qf_ctx *ctx, const void *w_kn, int packed_along_n, int64_t 
 
 // PDL: wait until the previous kernel of the stream has completed and its writes are visible (no-op without PDL).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Asks for `bytes` (a multiple of 16, 16-byte aligned) in L2; reads nothing.
+__device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // PDL: allow the next kernel of the stream to start its own independent prologue.
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 

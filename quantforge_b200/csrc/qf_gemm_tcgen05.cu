@@ -79,6 +79,7 @@ struct GemmParams {
                            //    tiles through distributed shared memory (no global partials, no counters)
     const void *residual;  // QF_EPI_RESIDUAL_ADD: R[M, N] in out_dtype
     int epilogue;          // qf_epilogue (plain instantiations only)
+    int early;             // follows_linear: weights, scales and zeros may be read before the dependency wait
 };
 
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.f + expf(-gate)) * up; }
@@ -172,6 +173,9 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
         : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int c0, int c1) {  // into L2; reads nothing
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
@@ -414,7 +418,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
     volatile int *abort_flag = &s_abort;
-    griddep_launch_dependents();  // the next kernel may begin its own set-up and weight prefetch
+    if (p.early) griddep_launch_dependents();  // the next kernel may begin its own set-up and weight stream
 
     const uint32_t rank = PAIR ? cluster_rank() : 0u;
     int producer_issued = 0;  // meaningful in the elected producer lane only
@@ -435,17 +439,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         const int w_row0 = p.tiled ? n_tile * (int)(p.K >> 7) * 128 : (int)n0;
         // issue_w is called for it = 0, 1, 2, ... in order: the sliver pointers advance incrementally
         int g_rem = kb0 % group_kb;
+        // tile-major weights: rows of 64 bytes, the 128 rows of (n_tile, 128-code block) adjacent
+        auto w_col = [&](int kb) { return !p.tiled ? kb * C::W_ROW_BYTES : (BK == 128) ? 0 : (kb & 1) * 32; };
+        auto w_row = [&](int kb) { return !p.tiled ? w_row0 : w_row0 + ((kb * BK) >> 7) * 128; };
         auto issue_w = [&](int it, int s) {
             const int kb = kb0 + it;
             const uint32_t fb = full_bar(s);
             mbar_arrive_expect_tx(fb, tx_bytes);
-            if (p.tiled) {
-                // tile-major weights: rows of 64 bytes, the 128 rows of (n_tile, 128-code block) adjacent
-                const int kb128 = (kb * BK) >> 7;
-                tma_load_2d(w_stage(s), &tmap_w, fb, (BK == 128) ? 0 : (kb & 1) * 32, w_row0 + kb128 * 128);
-            } else {
-                tma_load_2d(w_stage(s), &tmap_w, fb, kb * C::W_ROW_BYTES, w_row0);
-            }
+            tma_load_2d(w_stage(s), &tmap_w, fb, w_col(kb), w_row(kb));
             bulk_load(sz_stage(s), sc_ptr, 256u, fb);
             if (zbytes) bulk_load(sz_stage(s) + 256u, z_ptr, zbytes, fb);
             if (++g_rem == group_kb) {
@@ -461,14 +462,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 tma_load_2d(x_stage(s) + b * C::X_BOX_BYTES, &tmap_x, full_bar(s), kb * BK + b * 64, x_row0);
             producer_issued = it + 1;
         };
-        // First pass over the ring: weights, scales and zeros do not depend on the previous kernel of the stream,
-        // so they are requested before the dependency wait; the activations after it.
+        // First pass over the ring. Behind a linear (follows_linear), weights, scales and zeros are requested before the
+        // dependency wait and the activations after it; otherwise they go to L2 before the wait, and everything is requested
+        // after it, stage by stage (weights of all stages first: 64 x 14336 x 4096 16.3 us instead of 15.9).
         const int npre = min(STAGES, nkb);
-        if (leader)
-            for (int it = 0; it < npre; ++it) issue_w(it, it);
+        if (leader) {
+            for (int it = 0; it < npre; ++it) {
+                if (p.early) {
+                    issue_w(it, it);
+                } else {
+                    const int dg = (kb0 + it) / group_kb - gi;  // groups behind the first one
+                    tma_prefetch_2d(&tmap_w, w_col(kb0 + it), w_row(kb0 + it));
+                    l2_prefetch(sc_ptr + (size_t)dg * p.N * 2, 256u);
+                    if (zbytes) l2_prefetch(z_ptr + (size_t)dg * z_row, zbytes);
+                }
+            }
+        }
         griddep_wait();
-        if (leader)
-            for (int it = 0; it < npre; ++it) issue_x(it, it);
+        if (!p.early) griddep_launch_dependents();
+        if (leader) {
+            for (int it = 0; it < npre; ++it) {
+                if (!p.early) issue_w(it, it);
+                issue_x(it, it);
+            }
+        }
         int s = npre % STAGES;
         uint32_t ph = npre == STAGES ? 1u : 0u;
         for (int it = npre; it < nkb; ++it) {
@@ -962,6 +979,7 @@ static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan
     g_launch_count.fetch_add(1);
     QF_CUDA_TRY(ctx, le);
     QF_CUDA_TRY(ctx, cudaGetLastError());
+    note_linear(s);
     return QF_OK;
 }
 
@@ -1007,6 +1025,7 @@ static int launch_gemm_impl(qf_ctx *ctx, const qf_linear_desc *d, const Plan &pl
     p.interleaved = d->weight_layout != QF_LAYOUT_CANONICAL;
     p.tiled = d->weight_layout == QF_LAYOUT_TILED;
     p.cluster_reduce = 0;
+    p.early = follows_linear(s) ? 1 : 0;
     if (d->act_dtype == QF_BF16) return gemm_launch_dt<true>(ctx, d, plan, X, qw, p, s, ar);
     return gemm_launch_dt<false>(ctx, d, plan, X, qw, p, s, ar);
 }

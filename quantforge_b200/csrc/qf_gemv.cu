@@ -49,6 +49,7 @@ struct GemvParams {
     int m_pad;          // rows of X staged per batch tile: 1, 2, 4 or 8
     int cluster_reduce; // 1: the split_k blocks of a column block form a thread-block cluster (rank = split) and
                         //    sum their partial outputs through distributed shared memory
+    int early;          // follows_linear: weights, scales and zeros may be read before the dependency wait
 };
 
 // dynamic shared memory: ring | constants table [chunks][64 rows] uint2 | staged X [chunks][4][m_pad][4] uint4
@@ -112,9 +113,14 @@ __device__ __forceinline__ void gemv_body(const GemvParams &p, const typename Ex
     const uint32_t table = (uint32_t)__cvta_generic_to_shared(smem_raw) + GEMV_RING_BYTES;     // [chunk][64] uint2
     const uint32_t xs = table + (uint32_t)p.chunks_per_split * GEMV_ROWS_PER_BLOCK * 8u;       // [chunk][4][m_pad][4]
 
-    // 1. weight stream: fill the ring before anything else
+    // 1. weight stream: fill the ring before anything else (behind a linear: before the dependency wait, see follows_linear;
+    //    an L2 prefetch in front of the wait measured nothing here)
     const uint32_t *ra = p.qw + row_a * (p.K >> 3) + (int64_t)c0 * 16 + t * 4;
     const uint32_t *rb = ra + 8 * (p.K >> 3);
+    if (!p.early) {
+        griddep_wait();
+        griddep_launch_dependents();
+    }
 #pragma unroll
     for (int i = 0; i < GEMV_DEPTH; ++i) {
         if (warp_active && i < nch) {
@@ -125,46 +131,72 @@ __device__ __forceinline__ void gemv_body(const GemvParams &p, const typename Ex
     }
 
     // 2. converter constants of this block's (chunk, row) pairs
-    for (int e = tid; e < nch * GEMV_ROWS_PER_BLOCK; e += GEMV_THREADS) {
-        const int r = e & (GEMV_ROWS_PER_BLOCK - 1);
-        const int cl = e >> 6;
-        const int64_t n = n_blk + r;
-        uint2 ent = make_uint2(0u, 0u);
-        if (n < p.N) {
+    const int n_consts = nch * GEMV_ROWS_PER_BLOCK;
+    auto load_consts = [&](int e, int &z, uint32_t &scale) {
+        const int64_t n = n_blk + (e & (GEMV_ROWS_PER_BLOCK - 1));
+        z = 0, scale = 0u;
+        if (e < n_consts && n < p.N) {
+            const int cl = e >> 6;
             const int64_t gi = p.group_chunks == 1 ? (c0 + cl) : (c0 + cl) / p.group_chunks;
-            ZeroScale<BF16> zs;
-            zs.set(load_zero<ZMODE>(p.zeros, p.zero_const, gi, n, p.N), __ldg(p.scales + gi * p.N + n));
-            ent = make_uint2(zs.zsub, zs.s2);
+            z = load_zero<ZMODE>(p.zeros, p.zero_const, gi, n, p.N);
+            scale = __ldg(p.scales + gi * p.N + n);
         }
-        asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(table + (uint32_t)e * 8u), "r"(ent.x), "r"(ent.y));
-    }
-
-    // Everything above is independent of the previous kernel in the stream; the activations are not.
-    griddep_launch_dependents();
-    griddep_wait();
+    };
+    auto put_consts = [&](int e, int z, uint32_t scale) {
+        ZeroScale<BF16> zs;
+        zs.set(z, scale);
+        if (e < n_consts)
+            asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(table + (uint32_t)e * 8u), "r"(zs.zsub), "r"(zs.s2));
+    };
+    // 3. activations of this K range in fragment order, zero rows beyond M. 16-byte pieces: (m) x (t*4 + j)
+    constexpr int units_per_chunk = m_pad * 16;
+    const int n_x = nch * units_per_chunk;
+    auto load_x = [&](int u) {
+        const int64_t m = (int64_t)mt * 8 + (u >> 4) % m_pad;
+        return u < n_x && m < p.M ? *reinterpret_cast<const uint4 *>(p.X + m * p.K + (int64_t)(c0 + u / units_per_chunk) * 128 +
+                                                                     (u & 15) * 8)
+                                  : make_uint4(0u, 0u, 0u, 0u);
+    };
+    auto put_x = [&](int u, const uint4 &v) {
+        const int piece = u & 15;  // = t*4 + j : 16-byte piece of the chunk's 256-byte row segment
+        const int m = (u >> 4) % m_pad, cl = u / units_per_chunk;
+        const int tt = piece >> 2, j = piece & 3;
+        const uint32_t dst = xs + (uint32_t)((((cl * 4 + j) * m_pad + m) * 4 + tt) * 16);
+        if (u < n_x)  // (e0, e4) (e1, e5) (e2, e6) (e3, e7)
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(prmt(v.x, v.z, 0x5410u)),
+                         "r"(prmt(v.x, v.z, 0x7632u)), "r"(prmt(v.y, v.w, 0x5410u)), "r"(prmt(v.y, v.w, 0x7632u)));
+    };
     unsigned ar_epoch = 0;
-    if constexpr (AR) ar_epoch = exch_read_epoch(ar);
-
-    // 3. activations of this K range in fragment order, zero rows beyond M
-    {
-        const int units_per_chunk = m_pad * 16;  // 16-byte pieces: (m) x (t*4 + j)
-        const int64_t m_base = (int64_t)mt * 8;
-        for (int u = tid; u < nch * units_per_chunk; u += GEMV_THREADS) {
-            const int piece = u & 15;  // = t*4 + j : 16-byte piece of the chunk's 256-byte row segment
-            const int m = (u >> 4) % m_pad;
-            const int cl = u / units_per_chunk;
-            uint4 r = make_uint4(0u, 0u, 0u, 0u);
-            if (m_base + m < p.M) {
-                const uint4 v = *reinterpret_cast<const uint4 *>(p.X + (m_base + m) * p.K + (int64_t)(c0 + cl) * 128 +
-                                                                 piece * 8);
-                r.x = prmt(v.x, v.z, 0x5410u);  // (e0, e4)
-                r.y = prmt(v.x, v.z, 0x7632u);  // (e1, e5)
-                r.z = prmt(v.y, v.w, 0x5410u);  // (e2, e6)
-                r.w = prmt(v.y, v.w, 0x7632u);  // (e3, e7)
-            }
-            const int tt = piece >> 2, j = piece & 3;
-            const uint32_t dst = xs + (uint32_t)((((cl * 4 + j) * m_pad + m) * 4 + tt) * 16);
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w));
+    if (p.early) {
+        // everything above and the constants are independent of the previous kernel of the stream; the activations are not
+        for (int e = tid; e < n_consts; e += GEMV_THREADS) {
+            int z;
+            uint32_t scale;
+            load_consts(e, z, scale);
+            put_consts(e, z, scale);
+        }
+        griddep_launch_dependents();
+        griddep_wait();
+        if constexpr (AR) ar_epoch = exch_read_epoch(ar);
+        for (int u = tid; u < n_x; u += GEMV_THREADS) put_x(u, load_x(u));
+    } else {
+        // constants and activations in one go, B loads of either in flight (one after the other they cost a round trip to L2
+        // more: M = 3, 3968 x 5136 per channel, called eagerly, 10.3 us instead of 10.0; 9.2 with both and the weights read ahead
+        // of the wait, which nothing but a linear in front makes safe)
+        if constexpr (AR) ar_epoch = exch_read_epoch(ar);
+        constexpr int B = 4;
+        for (int i = tid; i < max(n_consts, n_x); i += B * GEMV_THREADS) {
+            int z[B];
+            uint32_t scale[B];
+            uint4 x[B];
+#pragma unroll
+            for (int q = 0; q < B; ++q) x[q] = load_x(i + q * GEMV_THREADS);
+#pragma unroll
+            for (int q = 0; q < B; ++q) load_consts(i + q * GEMV_THREADS, z[q], scale[q]);
+#pragma unroll
+            for (int q = 0; q < B; ++q) put_x(i + q * GEMV_THREADS, x[q]);
+#pragma unroll
+            for (int q = 0; q < B; ++q) put_consts(i + q * GEMV_THREADS, z[q], scale[q]);
         }
     }
     __syncthreads();
@@ -446,12 +478,14 @@ static int launch_gemv_impl(qf_ctx *ctx, const qf_linear_desc *d, const Plan &pl
               (unsigned)plan.m_tiles);
     const int64_t m_in_tile = d->M < 8 ? d->M : 8;
     p.m_pad = m_in_tile <= 1 ? 1 : m_in_tile <= 2 ? 2 : m_in_tile <= 4 ? 4 : 8;
+    p.early = follows_linear(s) ? 1 : 0;
     const size_t smem = gemv_smem_bytes(plan.chunks_per_split, p.m_pad);
     const cudaError_t le = d->act_dtype == QF_BF16 ? gemv_dispatch<true>(d->zero_mode, grid, smem, s, p, ar)
                                                    : gemv_dispatch<false>(d->zero_mode, grid, smem, s, p, ar);
     g_launch_count.fetch_add(1);
     QF_CUDA_TRY(ctx, le);
     QF_CUDA_TRY(ctx, cudaGetLastError());
+    note_linear(s);
     return QF_OK;
 }
 

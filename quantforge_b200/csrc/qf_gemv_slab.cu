@@ -12,9 +12,9 @@
 // Inside a block (160 threads):
 //   warp 4      producer: one cp.async.bulk per PAIR of consecutive units (8704 contiguous bytes of the blob) into a
 //               ring of shared-memory stages (full / empty mbarriers), plus one 512-byte bulk copy per batch row for
-//               the pair's slices of X (two of 256 bytes where the pair straddles a row block). All weight copies of
-//               the first pass over the ring are issued BEFORE the programmatic-dependent-launch wait (weights do
-//               not depend on the previous kernel of the stream), the activation copies after it.
+//               the pair's slices of X (two of 256 bytes where the pair straddles a row block). The weight copies of
+//               the first pass over the ring are issued BEFORE the programmatic-dependent-launch wait where the previous
+//               kernel is a linear (SlabParams::early) and prefetched into L2 otherwise, the activation copies after it.
 //   warps 0-3   consumers: warp w owns rows 16w..16w+15 of the unit. Per unit and lane: 2 x 16 B of codes and two
 //               constants words from shared memory -> lop3 / packed 16-bit arithmetic -> A fragments of
 //               m16n8k16 tensor-core MMAs; B fragments are 16-byte reads of the natural-order activation slice
@@ -59,6 +59,7 @@ struct SlabParams {
     int m_pad;                  // batch rows a stage has room for: 1, 2, 4, 8, 16 or 32
     int out_dtype;
     int epilogue;
+    int early;                  // follows_linear: weights, scales and zeros may be read before the dependency wait
     int stream_only;            // measurement aid: consumers release every stage unread (see launch_gemv_slab_impl)
 };
 
@@ -243,7 +244,7 @@ __device__ __forceinline__ void gemv_slab_body(const SlabParams &p, const typena
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    griddep_launch_dependents();  // the next kernel of the stream may start its own weight prefetch
+    if (p.early) griddep_launch_dependents();  // the next kernel of the stream may start its own weight stream
 
     if (warp == 4) {
         // ------------------------------ producer ------------------------------
@@ -270,16 +271,25 @@ __device__ __forceinline__ void gemv_slab_body(const SlabParams &p, const typena
                 if (nu == 2) bulk_load(dst + 256u, row, 256u, full_bar(s));  // first chunk of the next row block
             }
         };
-        if (lane == 0)
-            for (int ip = 0; ip < npre; ++ip) issue_w(ip, ip);
+        if (lane == 0) {
+            for (int ip = 0; ip < npre; ++ip) {
+                if (p.early) issue_w(ip, ip);
+                else l2_prefetch(src + (size_t)ip * (2 * SLAB_UNIT_BYTES), (uint32_t)pair_units(ip) * (uint32_t)SLAB_UNIT_BYTES);
+            }
+        }
         __syncwarp();
         griddep_wait();  // the activations are the previous kernel's output
+        if (!p.early) griddep_launch_dependents();
         int c = (int)(u0 % p.chunks);
         auto advance_c = [&]() {
             c += 2;
             while (c >= p.chunks) c -= p.chunks;
         };
         for (int ip = 0; ip < npre; ++ip) {
+            if (!p.early) {
+                if (lane == 0) issue_w(ip, ip);
+                __syncwarp();
+            }
             if (lane < M) issue_x(ip, ip, c);
             advance_c();
         }
@@ -785,6 +795,7 @@ static int launch_gemv_slab_impl(qf_ctx *ctx, const qf_linear_desc *d, const Pla
     // a given shape under the same launch sequence (graph, programmatic dependent launch) as the real kernel.
     const char *so = std::getenv("QF_SLAB_STREAM_ONLY");
     p.stream_only = (so && so[0] == '1') ? 1 : 0;
+    p.early = follows_linear(s) ? 1 : 0;
     const dim3 grid((unsigned)plan.split_k), blk(SLAB_THREADS);
     const size_t smem = slab_smem_bytes(p.depth, p.m_pad);
     const bool pdl = pdl_enabled();
@@ -826,6 +837,7 @@ static int launch_gemv_slab_impl(qf_ctx *ctx, const qf_linear_desc *d, const Pla
     g_launch_count.fetch_add(1);
     QF_CUDA_TRY(ctx, le);
     QF_CUDA_TRY(ctx, cudaGetLastError());
+    note_linear(s);
     return QF_OK;
 }
 
