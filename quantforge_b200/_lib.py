@@ -122,6 +122,7 @@ def load_host():
         loader = importlib.machinery.ExtensionFileLoader("_qf_host", HOST_PATH)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_qf_host", loader))
         loader.exec_module(module)
+        module.set_error(QuantForgeError)
         _host = module
     return _host
 

@@ -72,6 +72,7 @@ bool cluster_reduce_enabled();
 // cluster size (measured: 32 x 8, 80 x 3, 112 x 2 blocks fit; 48 x 6 = 288 of the 296 slots do not).
 constexpr int kClusterMaxBlocks = 256;
 
+// A launch's status is what the call itself returns: the runtime's last error may be that of an earlier call.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                  bool pdl, Args &&...args) {
@@ -144,7 +145,9 @@ inline int fail(qf_ctx *ctx, int status, const std::string &msg) {
     return status;
 }
 
+// The error is reported here and not left behind as the runtime's last one.
 inline int cuda_fail(qf_ctx *ctx, cudaError_t e, const char *what) {
+    cudaGetLastError();
     return fail(ctx, QF_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -155,6 +158,13 @@ inline int check_current_device(qf_ctx *ctx) {
     if (dev != ctx->device)
         return fail(ctx, QF_ERR_BAD_ARG, "the current CUDA device (" + std::to_string(dev) +
                                              ") is not the context's device (" + std::to_string(ctx->device) + ")");
+    return QF_OK;
+}
+
+// The end of a launcher: counts the launch, or reports why there was none.
+inline int launched(qf_ctx *ctx, cudaError_t e, const char *what) {
+    if (e != cudaSuccess) return cuda_fail(ctx, e, what);
+    g_launch_count.fetch_add(1);
     return QF_OK;
 }
 

@@ -976,11 +976,8 @@ static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan
                            : launch_kernel_cluster(gemm_kernel<BF16, BN, false, false, PAIR>, grid, blk, C::SMEM_BYTES, s,
                                              pdl_enabled(), dim3(PAIR ? 2 : 1, 1, cluster_z), tw, tx, p, NoExchange{});
     }
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, le);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
     note_linear(s);
-    return QF_OK;
+    return launched(ctx, le, "GEMM");
 }
 
 template <bool BF16>

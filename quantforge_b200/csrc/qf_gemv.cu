@@ -482,11 +482,8 @@ static int launch_gemv_impl(qf_ctx *ctx, const qf_linear_desc *d, const Plan &pl
     const size_t smem = gemv_smem_bytes(plan.chunks_per_split, p.m_pad);
     const cudaError_t le = d->act_dtype == QF_BF16 ? gemv_dispatch<true>(d->zero_mode, grid, smem, s, p, ar)
                                                    : gemv_dispatch<false>(d->zero_mode, grid, smem, s, p, ar);
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, le);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
     note_linear(s);
-    return QF_OK;
+    return launched(ctx, le, "GEMV");
 }
 
 int launch_gemv(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan, const void *X, const void *qw,

@@ -642,37 +642,30 @@ __global__ void __launch_bounds__(256) slab_unpack_kernel(const uint8_t *__restr
 }
 
 template <bool BF16>
-static void slab_prepack_dispatch(const qf_linear_desc *d, unsigned units, cudaStream_t s, const uint32_t *qw,
-                                  const uint16_t *sc, const void *z, uint8_t *blob) {
+static cudaError_t slab_prepack_dispatch(const qf_linear_desc *d, unsigned units, cudaStream_t s, const uint32_t *qw,
+                                         const uint16_t *sc, const void *z, uint8_t *blob) {
     const int chunks = (int)(d->K / 128), gc = d->group_size / 128;
-    if (d->zero_mode == QF_ZERO_CONST)
-        slab_prepack_kernel<BF16, QF_ZERO_CONST><<<units, 256, 0, s>>>(qw, sc, z, d->zero_const, blob, d->N, chunks, gc);
-    else if (d->zero_mode == QF_ZERO_U4)
-        slab_prepack_kernel<BF16, QF_ZERO_U4><<<units, 256, 0, s>>>(qw, sc, z, d->zero_const, blob, d->N, chunks, gc);
-    else
-        slab_prepack_kernel<BF16, QF_ZERO_I8><<<units, 256, 0, s>>>(qw, sc, z, d->zero_const, blob, d->N, chunks, gc);
+    auto *fn = d->zero_mode == QF_ZERO_CONST ? slab_prepack_kernel<BF16, QF_ZERO_CONST>
+               : d->zero_mode == QF_ZERO_U4  ? slab_prepack_kernel<BF16, QF_ZERO_U4>
+                                             : slab_prepack_kernel<BF16, QF_ZERO_I8>;
+    return launch_kernel(fn, dim3(units), dim3(256), 0, s, false, qw, sc, z, d->zero_const, blob, d->N, chunks, gc);
 }
 
 int launch_slab_prepack(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const void *scales, const void *zeros,
                         void *blob, cudaStream_t s) {
     const int64_t units = (d->N / 64) * (d->K / 128);
     if (units > INT32_MAX) return fail(ctx, QF_ERR_UNSUPPORTED, "matrix too large");
-    if (d->act_dtype == QF_BF16)
-        slab_prepack_dispatch<true>(d, (unsigned)units, s, (const uint32_t *)qw, (const uint16_t *)scales, zeros, (uint8_t *)blob);
-    else
-        slab_prepack_dispatch<false>(d, (unsigned)units, s, (const uint32_t *)qw, (const uint16_t *)scales, zeros, (uint8_t *)blob);
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    auto *fn = d->act_dtype == QF_BF16 ? slab_prepack_dispatch<true> : slab_prepack_dispatch<false>;
+    return launched(ctx, fn(d, (unsigned)units, s, (const uint32_t *)qw, (const uint16_t *)scales, zeros, (uint8_t *)blob),
+                    "slab prepack");
 }
 
 int launch_slab_unpack(qf_ctx *ctx, int64_t N, int64_t K, const void *blob, void *qw, cudaStream_t s) {
     const int64_t units = (N / 64) * (K / 128);
     if (units > INT32_MAX) return fail(ctx, QF_ERR_UNSUPPORTED, "matrix too large");
-    slab_unpack_kernel<<<(unsigned)units, 256, 0, s>>>((const uint8_t *)blob, (uint32_t *)qw, (int)(K / 128));
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, launch_kernel(slab_unpack_kernel, dim3((unsigned)units), dim3(256), 0, s, false, (const uint8_t *)blob,
+                                       (uint32_t *)qw, (int)(K / 128)),
+                    "slab unpack");
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -834,11 +827,8 @@ static int launch_gemv_slab_impl(qf_ctx *ctx, const qf_linear_desc *d, const Pla
              : mt == 2 ? launch_kernel(gemv_slab_kernel<false, 2>, grid, blk, smem, s, pdl, p)
                        : launch_kernel(gemv_slab_kernel<false, 4>, grid, blk, smem, s, pdl, p);
     }
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, le);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
     note_linear(s);
-    return QF_OK;
+    return launched(ctx, le, "slab GEMV");
 }
 
 int launch_gemv_slab(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan, const void *X, const void *blob, void *Y,

@@ -3,6 +3,7 @@
 // interpreter. Only the ordinary case is handled here: CUDA tensors of one device, contiguous, right shapes and types,
 // a workspace that this stream already has. Whatever differs - an argument in error included - returns None, and
 // ops.py takes the call from the start: it makes the copies and allocations that are needed, and raises what it has to.
+// None means that nothing was enqueued: a status that says otherwise is raised here.
 //
 // Why: the interpreter needed 15 to 17 us per linear (attribute reads, two foreign calls, a device context manager,
 // ctypes conversions), more than the kernels of small layers take on the GPU.
@@ -56,6 +57,21 @@ bool find_workspace(int device, cudaStream_t stream, size_t need, void **ptr, si
             return true;
         }
     return false;
+}
+
+PyObject *g_error = nullptr;  // QuantForgeError(status, name, message)
+
+// What a call of the C ABI that did not succeed becomes. Its checks come before any launch, and ops.py may start over after
+// them; anything else is an error of CUDA.
+PyObject *failed(int status, int device) {
+    if (status == QF_ERR_BAD_ARG || status == QF_ERR_UNSUPPORTED || status == QF_ERR_WORKSPACE) Py_RETURN_NONE;
+    PyObject *e = PyObject_CallFunction(g_error ? g_error : PyExc_RuntimeError, "iss", status, qf_status_string(status),
+                                        qf_last_error(g_ctx[device]));
+    if (e) {
+        PyErr_SetObject((PyObject *)Py_TYPE(e), e);
+        Py_DECREF(e);
+    }
+    return nullptr;
 }
 
 int type_code(ScalarType t) {
@@ -175,14 +191,14 @@ PyObject *finish(qf_linear_desc *d, int device, const Tensor &x, const void *qw,
     if (out_o != Py_None) {
         const Tensor *y = cuda_tensor(out_o, &device);
         if (!y || !shape_is(*y, d->M, cols) || y->scalar_type() != out_type) Py_RETURN_NONE;
-        if (qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y->data_ptr(), res, ws, ws_bytes, stream) != QF_OK)
-            Py_RETURN_NONE;
+        const int st = qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y->data_ptr(), res, ws, ws_bytes, stream);
+        if (st != QF_OK) return failed(st, device);
         Py_INCREF(out_o);
         return out_o;
     }
     Tensor y = empty({d->M, cols}, out_type, device);
-    if (qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y.data_ptr(), res, ws, ws_bytes, stream) != QF_OK)
-        Py_RETURN_NONE;
+    const int st = qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y.data_ptr(), res, ws, ws_bytes, stream);
+    if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(y));
 }
 
@@ -272,8 +288,8 @@ PyObject *unpack_impl(PyObject *const *a) {
     const int64_t cols = shape.back();
     shape.back() = cols * 2;
     Tensor out = empty(shape, at::kChar, device);
-    if (qf_unpack_int4(g_ctx[device], p->const_data_ptr(), out.data_ptr(), p->numel() / cols, cols, stream_of(device)) != QF_OK)
-        Py_RETURN_NONE;
+    const int st = qf_unpack_int4(g_ctx[device], p->const_data_ptr(), out.data_ptr(), p->numel() / cols, cols, stream_of(device));
+    if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -292,7 +308,8 @@ PyObject *dequant_impl(PyObject *const *a) {
     if (d.zero_mode == QF_ZERO_CONST) d.zero_const = (int32_t)zero_const;
     d.out_dtype = d.act_dtype;
     Tensor out = empty({d.N, d.K}, act, device);
-    if (qf_dequant_w4(g_ctx[device], &d, qw, sc, z, out.data_ptr(), stream_of(device)) != QF_OK) Py_RETURN_NONE;
+    const int st = qf_dequant_w4(g_ctx[device], &d, qw, sc, z, out.data_ptr(), stream_of(device));
+    if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -305,7 +322,8 @@ PyObject *pack_impl(PyObject *const *a) {
     c10::SmallVector<int64_t, 5> shape(c->sizes().begin(), c->sizes().end());
     shape.back() /= 2;
     Tensor out = empty(shape, at::kChar, device);
-    if (qf_pack_int4(g_ctx[device], c->const_data_ptr(), out.data_ptr(), out.numel(), stream_of(device)) != QF_OK) Py_RETURN_NONE;
+    const int st = qf_pack_int4(g_ctx[device], c->const_data_ptr(), out.data_ptr(), out.numel(), stream_of(device));
+    if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -316,8 +334,8 @@ PyObject *pack_zeros_impl(PyObject *const *a) {
     if (!z || z->dim() != 2 || z->scalar_type() != at::kChar || z->numel() == 0 || z->size(1) % 8 != 0 || !ready(device))
         Py_RETURN_NONE;
     Tensor out = empty({z->size(0), z->size(1) / 8}, at::kInt, device);
-    if (qf_pack_int4(g_ctx[device], z->const_data_ptr(), out.data_ptr(), z->numel() / 2, stream_of(device)) != QF_OK)
-        Py_RETURN_NONE;
+    const int st = qf_pack_int4(g_ctx[device], z->const_data_ptr(), out.data_ptr(), z->numel() / 2, stream_of(device));
+    if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -335,9 +353,10 @@ PyObject *quantize_impl(PyObject *const *a) {
     const bool sym = a[2] == Py_True;
     Tensor codes = empty({N, K}, at::kChar, device), scales = empty({K / group, N}, st, device), zeros;
     if (!sym) zeros = empty({K / group, N}, at::kChar, device);
-    if (qf_quantize_w4(g_ctx[device], w->const_data_ptr(), type_code(w->scalar_type()), N, K, (int)group, sym, codes.data_ptr(),
-                       scales.data_ptr(), type_code(st), sym ? nullptr : zeros.data_ptr(), stream_of(device)) != QF_OK)
-        Py_RETURN_NONE;
+    const int status = qf_quantize_w4(g_ctx[device], w->const_data_ptr(), type_code(w->scalar_type()), N, K, (int)group, sym,
+                                      codes.data_ptr(), scales.data_ptr(), type_code(st), sym ? nullptr : zeros.data_ptr(),
+                                      stream_of(device));
+    if (status != QF_OK) return failed(status, device);
     PyObject *c = THPVariable_Wrap(std::move(codes)), *s = THPVariable_Wrap(std::move(scales));
     PyObject *z = sym ? Py_NewRef(Py_None) : THPVariable_Wrap(std::move(zeros));
     return Py_BuildValue("(NNN)", c, s, z);
@@ -361,7 +380,8 @@ PyObject *prepack_slab_impl(PyObject *const *a) {
     const size_t bytes = qf_prepack_bytes(QF_LAYOUT_GEMV_SLAB, d.N, d.K);
     if (bytes == 0) Py_RETURN_NONE;
     Tensor blob = empty({(int64_t)bytes}, at::kByte, device);
-    if (qf_prepack_gemv_slab(g_ctx[device], &d, qw, sc, z, blob.data_ptr(), stream_of(device)) != QF_OK) Py_RETURN_NONE;
+    const int st = qf_prepack_gemv_slab(g_ctx[device], &d, qw, sc, z, blob.data_ptr(), stream_of(device));
+    if (st != QF_OK) return failed(st, device);
     return Py_BuildValue("(NLLi)", THPVariable_Wrap(std::move(blob)), (long long)d.N, (long long)d.K, (int)d.zero_mode);
 }
 
@@ -380,7 +400,7 @@ PyObject *prepack_impl(PyObject *const *a) {
                                              stream_of(device))
                        : qf_prepack_w4(g_ctx[device], q->const_data_ptr(), out.data_ptr(), (int64_t)q->nbytes() / 4, back,
                                        stream_of(device));
-    if (st != QF_OK) Py_RETURN_NONE;
+    if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -405,6 +425,13 @@ PyObject *set_ctx_impl(PyObject *const *a) {
     Py_RETURN_NONE;
 }
 
+// set_error(class): what `failed` raises
+PyObject *set_error_impl(PyObject *const *a) {
+    Py_INCREF(a[0]);
+    Py_XSETREF(g_error, a[0]);
+    Py_RETURN_NONE;
+}
+
 // add_workspace(device, stream, pointer, bytes)
 PyObject *add_workspace_impl(PyObject *const *a) {
     long long device, stream, ptr, bytes;
@@ -419,6 +446,7 @@ PyMethodDef methods[] = {
     QF_FAST("pack", pack_impl, 1),       QF_FAST("pack_zeros", pack_zeros_impl, 1), QF_FAST("quantize", quantize_impl, 4),
     QF_FAST("prepack_slab", prepack_slab_impl, 5), QF_FAST("prepack", prepack_impl, 3),
     QF_FAST("dequant", dequant_impl, 5), QF_FAST("set_ctx", set_ctx_impl, 2), QF_FAST("add_workspace", add_workspace_impl, 4),
+    QF_FAST("set_error", set_error_impl, 1),
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_qf_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -241,16 +241,15 @@ __global__ void __launch_bounds__(256) quantize_group_kernel(const void *__restr
 }
 
 template <int DT, bool SYM>
-static void quantize_launch(const void *w, int64_t N, int64_t K, int group, uint32_t *codes, uint16_t *scales,
-                            int scale_dtype, int8_t *zeros, cudaStream_t s) {
+static cudaError_t quantize_launch(const void *w, int64_t N, int64_t K, int group, uint32_t *codes, uint16_t *scales,
+                                   int scale_dtype, int8_t *zeros, cudaStream_t s) {
     if (group == 128 && (N + 31) / 32 <= 65535) {
         const dim3 grid((unsigned)((K / 128 + 3) / 4), (unsigned)((N + 31) / 32));
-        quantize128_kernel<DT, SYM><<<grid, 256, 0, s>>>(w, N, K, codes, scales, scale_dtype, zeros);
-    } else {
-        const int threads = group >= 1024 ? 256 : group >= 512 ? 128 : group >= 256 ? 64 : 32;
-        quantize_group_kernel<DT, SYM><<<(unsigned)(N * (K / group)), threads, 0, s>>>(w, N, K, group, codes, scales,
-                                                                                     scale_dtype, zeros);
+        return launch_kernel(quantize128_kernel<DT, SYM>, grid, dim3(256), 0, s, false, w, N, K, codes, scales, scale_dtype, zeros);
     }
+    const int threads = group >= 1024 ? 256 : group >= 512 ? 128 : group >= 256 ? 64 : 32;
+    return launch_kernel(quantize_group_kernel<DT, SYM>, dim3((unsigned)(N * (K / group))), dim3(threads), 0, s, false, w, N, K,
+                         group, codes, scales, scale_dtype, zeros);
 }
 
 int launch_quantize(qf_ctx *ctx, const void *w, int dtype, int64_t N, int64_t K, int group, bool symmetric, void *codes,
@@ -258,10 +257,7 @@ int launch_quantize(qf_ctx *ctx, const void *w, int dtype, int64_t N, int64_t K,
     auto *fn = dtype == QF_F16    ? (symmetric ? quantize_launch<QF_F16, true> : quantize_launch<QF_F16, false>)
                : dtype == QF_BF16 ? (symmetric ? quantize_launch<QF_BF16, true> : quantize_launch<QF_BF16, false>)
                                   : (symmetric ? quantize_launch<QF_F32, true> : quantize_launch<QF_F32, false>);
-    fn(w, N, K, group, (uint32_t *)codes, (uint16_t *)scales, scale_dtype, (int8_t *)zeros, s);
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, fn(w, N, K, group, (uint32_t *)codes, (uint16_t *)scales, scale_dtype, (int8_t *)zeros, s), "quantize");
 }
 
 }  // namespace qf

@@ -80,21 +80,20 @@ __global__ void __launch_bounds__(256) unpack_byte_kernel(const uint8_t *__restr
 int launch_unpack(qf_ctx *ctx, const void *packed, void *out, int64_t rows, int64_t packed_cols, cudaStream_t s) {
     const int64_t n_bytes = rows * packed_cols;
     if (n_bytes == 0) return QF_OK;
+    cudaError_t e;
     if ((uintptr_t)packed % 16 == 0 && (uintptr_t)out % 32 == 0) {
         const int64_t n_vec = n_bytes / 16;
         int64_t blocks = (n_vec + 256 * UNPACK_STEPS - 1) / (256 * UNPACK_STEPS);
         if (blocks < 1) blocks = 1;
-        unpack_vec_kernel<<<(unsigned)blocks, 256, 0, s>>>((const uint8_t *)packed, (uint8_t *)out, n_vec,
-                                                          (int)(n_bytes % 16));
+        e = launch_kernel(unpack_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)packed,
+                          (uint8_t *)out, n_vec, (int)(n_bytes % 16));
     } else {
         int64_t blocks = (n_bytes + 255) / 256;
         if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-        unpack_byte_kernel<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<const uint8_t *>(packed),
-                                                           reinterpret_cast<uint8_t *>(out), n_bytes);
+        e = launch_kernel(unpack_byte_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)packed,
+                          (uint8_t *)out, n_bytes);
     }
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, e, "unpack");
 }
 
 // The inverse: out[i] = (codes[2i] & 15) | (codes[2i + 1] & 15) << 4. 16 codes in, 8 bytes out per step.
@@ -125,10 +124,9 @@ int launch_pack(qf_ctx *ctx, const void *codes, void *out, int64_t n_bytes, cuda
     const int64_t n_vec = n_bytes / 8;
     int64_t blocks = (n_vec + 256 * UNPACK_STEPS - 1) / (256 * UNPACK_STEPS);
     if (blocks < 1) blocks = 1;
-    pack_vec_kernel<<<(unsigned)blocks, 256, 0, s>>>((const uint8_t *)codes, (uint8_t *)out, n_vec, (int)(n_bytes % 8));
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, launch_kernel(pack_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)codes,
+                                       (uint8_t *)out, n_vec, (int)(n_bytes % 8)),
+                    "pack");
 }
 
 // Nibble permutation inside each word: qf_prepack_w4.
@@ -144,10 +142,9 @@ __global__ void __launch_bounds__(256) prepack_kernel(const uint32_t *__restrict
 int launch_prepack(qf_ctx *ctx, const void *in, void *out, int64_t n_words, int to_canonical, cudaStream_t s) {
     int64_t blocks = (n_words + 255) / 256;
     if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-    prepack_kernel<<<(unsigned)blocks, 256, 0, s>>>((const uint32_t *)in, (uint32_t *)out, n_words, to_canonical);
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, launch_kernel(prepack_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint32_t *)in,
+                                       (uint32_t *)out, n_words, to_canonical),
+                    "prepack");
 }
 
 // canonical word (n, j) <-> tiled word ((nt * KB + kb) * 128 + r) * 16 + w, n = nt*128 + r, j = kb*16 + w.
@@ -175,10 +172,9 @@ int launch_prepack_tiled(qf_ctx *ctx, const void *in, void *out, int64_t N, int6
                          cudaStream_t s) {
     const int64_t tiles = (N / 128) * (K / 128);
     if (tiles > INT32_MAX) return fail(ctx, QF_ERR_UNSUPPORTED, "matrix too large");
-    prepack_tiled_kernel<<<(unsigned)tiles, 256, 0, s>>>((const uint4 *)in, (uint4 *)out, (int)(K / 128), to_canonical);
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, launch_kernel(prepack_tiled_kernel, dim3((unsigned)tiles), dim3(256), 0, s, false, (const uint4 *)in,
+                                       (uint4 *)out, (int)(K / 128), to_canonical),
+                    "tiled prepack");
 }
 
 // W[K, N] (one code per byte, or two per byte along N) -> canonical qweight [N, K/8] words. One thread per output
@@ -213,10 +209,9 @@ int launch_repack_kn(qf_ctx *ctx, const void *w_kn, int packed_along_n, int64_t 
     const int64_t total = N * (K / 8);
     int64_t blocks = (total + 255) / 256;
     if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-    repack_kn_kernel<<<(unsigned)blocks, 256, 0, s>>>((const uint8_t *)w_kn, packed_along_n, K, N, (uint32_t *)out);
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, launch_kernel(repack_kn_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)w_kn,
+                                       packed_along_n, K, N, (uint32_t *)out),
+                    "repack");
 }
 
 // A block converts 32 rows x 512 codes: a warp covers 512 codes of a row, a thread two neighbouring words of it (8 bytes
@@ -268,14 +263,12 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *__restrict
 }
 
 template <bool BF16, bool WIDE>
-static void dequant_dispatch(int zmode, dim3 grid, cudaStream_t s, const uint32_t *qw, const uint16_t *sc, const void *z,
-                             int zc, uint4 *out, int64_t N, int words_per_row, int group_words) {
-    if (zmode == QF_ZERO_CONST)
-        dequant_kernel<BF16, QF_ZERO_CONST, WIDE><<<grid, 256, 0, s>>>(qw, sc, z, zc, out, N, words_per_row, group_words);
-    else if (zmode == QF_ZERO_U4)
-        dequant_kernel<BF16, QF_ZERO_U4, WIDE><<<grid, 256, 0, s>>>(qw, sc, z, zc, out, N, words_per_row, group_words);
-    else
-        dequant_kernel<BF16, QF_ZERO_I8, WIDE><<<grid, 256, 0, s>>>(qw, sc, z, zc, out, N, words_per_row, group_words);
+static cudaError_t dequant_dispatch(int zmode, dim3 grid, cudaStream_t s, const uint32_t *qw, const uint16_t *sc, const void *z,
+                                    int zc, uint4 *out, int64_t N, int words_per_row, int group_words) {
+    auto *fn = zmode == QF_ZERO_CONST ? dequant_kernel<BF16, QF_ZERO_CONST, WIDE>
+               : zmode == QF_ZERO_U4  ? dequant_kernel<BF16, QF_ZERO_U4, WIDE>
+                                      : dequant_kernel<BF16, QF_ZERO_I8, WIDE>;
+    return launch_kernel(fn, grid, dim3(256), 0, s, false, qw, sc, z, zc, out, N, words_per_row, group_words);
 }
 
 int launch_dequant(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const void *scales, const void *zeros,
@@ -288,11 +281,9 @@ int launch_dequant(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const v
     const bool wide = (uintptr_t)w_out % 32 == 0;
     auto *fn = d->act_dtype == QF_BF16 ? (wide ? dequant_dispatch<true, true> : dequant_dispatch<true, false>)
                                        : (wide ? dequant_dispatch<false, true> : dequant_dispatch<false, false>);
-    fn(d->zero_mode, grid, s, (const uint32_t *)qw, (const uint16_t *)scales, zeros, d->zero_const, (uint4 *)w_out, d->N,
-       (int)words, d->group_size / 8);
-    g_launch_count.fetch_add(1);
-    QF_CUDA_TRY(ctx, cudaGetLastError());
-    return QF_OK;
+    return launched(ctx, fn(d->zero_mode, grid, s, (const uint32_t *)qw, (const uint16_t *)scales, zeros, d->zero_const,
+                            (uint4 *)w_out, d->N, (int)words, d->group_size / 8),
+                    "dequant");
 }
 
 }  // namespace qf
