@@ -5,6 +5,10 @@
 // ops.py takes the call from the start: it makes the copies and allocations that are needed, and raises what it has to.
 // None means that nothing was enqueued: a status that says otherwise is raised here.
 //
+// The interpreter lock is held while Python objects are read and released around allocation and launch, both of which can
+// block (a full launch queue, a free of cached memory): other Python threads go on meanwhile, as around a foreign call. The
+// caller's references keep the arguments alive.
+//
 // Why: the interpreter needed 15 to 17 us per linear (attribute reads, two foreign calls, a device context manager,
 // ctypes conversions), more than the kernels of small layers take on the GPU.
 #define PY_SSIZE_T_CLEAN
@@ -58,6 +62,18 @@ bool find_workspace(int device, cudaStream_t stream, size_t need, void **ptr, si
         }
     return false;
 }
+
+// Other Python threads run while this exists.
+class Unlocked {
+  public:
+    Unlocked() : state_(PyEval_SaveThread()) {}
+    ~Unlocked() { PyEval_RestoreThread(state_); }
+    Unlocked(const Unlocked &) = delete;
+    Unlocked &operator=(const Unlocked &) = delete;
+
+  private:
+    PyThreadState *state_;
+};
 
 PyObject *g_error = nullptr;  // QuantForgeError(status, name, message)
 
@@ -188,17 +204,20 @@ PyObject *finish(qf_linear_desc *d, int device, const Tensor &x, const void *qw,
     void *ws;
     size_t ws_bytes;
     if (!find_workspace(device, stream, qf_w4a16_workspace_bytes(d), &ws, &ws_bytes)) Py_RETURN_NONE;
+    Tensor y;
     if (out_o != Py_None) {
-        const Tensor *y = cuda_tensor(out_o, &device);
-        if (!y || !shape_is(*y, d->M, cols) || y->scalar_type() != out_type) Py_RETURN_NONE;
-        const int st = qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y->data_ptr(), res, ws, ws_bytes, stream);
-        if (st != QF_OK) return failed(st, device);
-        Py_INCREF(out_o);
-        return out_o;
+        const Tensor *o = cuda_tensor(out_o, &device);
+        if (!o || !shape_is(*o, d->M, cols) || o->scalar_type() != out_type) Py_RETURN_NONE;
+        y = *o;
     }
-    Tensor y = empty({d->M, cols}, out_type, device);
-    const int st = qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y.data_ptr(), res, ws, ws_bytes, stream);
+    int st;
+    {
+        Unlocked u;
+        if (!y.defined()) y = empty({d->M, cols}, out_type, device);
+        st = qf_w4a16_linear_fused(g_ctx[device], d, x.const_data_ptr(), qw, sc, z, y.data_ptr(), res, ws, ws_bytes, stream);
+    }
     if (st != QF_OK) return failed(st, device);
+    if (out_o != Py_None) return Py_NewRef(out_o);
     return THPVariable_Wrap(std::move(y));
 }
 
@@ -219,6 +238,7 @@ PyObject *linear_impl(PyObject *const *a) {
     d.split_k = (int32_t)split_k;
     d.epilogue = (int32_t)epilogue;
     const void *qw, *sc = nullptr, *z = nullptr;
+    Tensor blob;
     if (THPVariable_Check(a[1])) {
         ScalarType act;
         if (!as_int(a[4], &group) || !as_int(a[5], &zero_const) || !as_int(a[7], &path) || !as_int(a[10], &layout)) Py_RETURN_NONE;
@@ -235,10 +255,11 @@ PyObject *linear_impl(PyObject *const *a) {
             PyErr_Clear();
             Py_RETURN_NONE;
         }
-        const Tensor *blob = cuda_tensor(blob_o, &device);
-        qw = blob ? blob->const_data_ptr() : nullptr;  // the object keeps the tensor alive for the call
-        const size_t have = blob ? (size_t)blob->nbytes() : 0;
+        const Tensor *t = cuda_tensor(blob_o, &device);
+        if (t) blob = *t;  // another thread may give the object another blob
         Py_DECREF(blob_o);
+        qw = blob.defined() ? blob.const_data_ptr() : nullptr;
+        const size_t have = blob.defined() ? (size_t)blob.nbytes() : 0;
         PyObject *act_o = PyObject_GetAttr(a[1], s_act);
         if (!act_o) PyErr_Clear();
         const bool act_ok = act_o && THPDtype_Check(act_o) && ((THPDtype *)act_o)->scalar_type == x->scalar_type();
@@ -287,8 +308,13 @@ PyObject *unpack_impl(PyObject *const *a) {
     c10::SmallVector<int64_t, 5> shape(p->sizes().begin(), p->sizes().end());
     const int64_t cols = shape.back();
     shape.back() = cols * 2;
-    Tensor out = empty(shape, at::kChar, device);
-    const int st = qf_unpack_int4(g_ctx[device], p->const_data_ptr(), out.data_ptr(), p->numel() / cols, cols, stream_of(device));
+    Tensor out;
+    int st;
+    {
+        Unlocked u;
+        out = empty(shape, at::kChar, device);
+        st = qf_unpack_int4(g_ctx[device], p->const_data_ptr(), out.data_ptr(), p->numel() / cols, cols, stream_of(device));
+    }
     if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
@@ -307,8 +333,13 @@ PyObject *dequant_impl(PyObject *const *a) {
     if (!read_weights(a[0], a[1], a[2], &device, &d, -1, &qw, &sc, &z, &act) || !ready(device)) Py_RETURN_NONE;
     if (d.zero_mode == QF_ZERO_CONST) d.zero_const = (int32_t)zero_const;
     d.out_dtype = d.act_dtype;
-    Tensor out = empty({d.N, d.K}, act, device);
-    const int st = qf_dequant_w4(g_ctx[device], &d, qw, sc, z, out.data_ptr(), stream_of(device));
+    Tensor out;
+    int st;
+    {
+        Unlocked u;
+        out = empty({d.N, d.K}, act, device);
+        st = qf_dequant_w4(g_ctx[device], &d, qw, sc, z, out.data_ptr(), stream_of(device));
+    }
     if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
@@ -321,8 +352,13 @@ PyObject *pack_impl(PyObject *const *a) {
         Py_RETURN_NONE;
     c10::SmallVector<int64_t, 5> shape(c->sizes().begin(), c->sizes().end());
     shape.back() /= 2;
-    Tensor out = empty(shape, at::kChar, device);
-    const int st = qf_pack_int4(g_ctx[device], c->const_data_ptr(), out.data_ptr(), out.numel(), stream_of(device));
+    Tensor out;
+    int st;
+    {
+        Unlocked u;
+        out = empty(shape, at::kChar, device);
+        st = qf_pack_int4(g_ctx[device], c->const_data_ptr(), out.data_ptr(), out.numel(), stream_of(device));
+    }
     if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
@@ -333,8 +369,13 @@ PyObject *pack_zeros_impl(PyObject *const *a) {
     const Tensor *z = cuda_tensor(a[0], &device);
     if (!z || z->dim() != 2 || z->scalar_type() != at::kChar || z->numel() == 0 || z->size(1) % 8 != 0 || !ready(device))
         Py_RETURN_NONE;
-    Tensor out = empty({z->size(0), z->size(1) / 8}, at::kInt, device);
-    const int st = qf_pack_int4(g_ctx[device], z->const_data_ptr(), out.data_ptr(), z->numel() / 2, stream_of(device));
+    Tensor out;
+    int st;
+    {
+        Unlocked u;
+        out = empty({z->size(0), z->size(1) / 8}, at::kInt, device);
+        st = qf_pack_int4(g_ctx[device], z->const_data_ptr(), out.data_ptr(), z->numel() / 2, stream_of(device));
+    }
     if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }
@@ -351,11 +392,17 @@ PyObject *quantize_impl(PyObject *const *a) {
     const int64_t N = w->size(0), K = w->size(1);
     if ((st != at::kHalf && st != at::kBFloat16) || group <= 0 || group > INT32_MAX || K % group != 0) Py_RETURN_NONE;
     const bool sym = a[2] == Py_True;
-    Tensor codes = empty({N, K}, at::kChar, device), scales = empty({K / group, N}, st, device), zeros;
-    if (!sym) zeros = empty({K / group, N}, at::kChar, device);
-    const int status = qf_quantize_w4(g_ctx[device], w->const_data_ptr(), type_code(w->scalar_type()), N, K, (int)group, sym,
-                                      codes.data_ptr(), scales.data_ptr(), type_code(st), sym ? nullptr : zeros.data_ptr(),
-                                      stream_of(device));
+    Tensor codes, scales, zeros;
+    int status;
+    {
+        Unlocked u;
+        codes = empty({N, K}, at::kChar, device);
+        scales = empty({K / group, N}, st, device);
+        if (!sym) zeros = empty({K / group, N}, at::kChar, device);
+        status = qf_quantize_w4(g_ctx[device], w->const_data_ptr(), type_code(w->scalar_type()), N, K, (int)group, sym,
+                                codes.data_ptr(), scales.data_ptr(), type_code(st), sym ? nullptr : zeros.data_ptr(),
+                                stream_of(device));
+    }
     if (status != QF_OK) return failed(status, device);
     PyObject *c = THPVariable_Wrap(std::move(codes)), *s = THPVariable_Wrap(std::move(scales));
     PyObject *z = sym ? Py_NewRef(Py_None) : THPVariable_Wrap(std::move(zeros));
@@ -379,8 +426,13 @@ PyObject *prepack_slab_impl(PyObject *const *a) {
     d.weight_layout = QF_LAYOUT_GEMV_SLAB;
     const size_t bytes = qf_prepack_bytes(QF_LAYOUT_GEMV_SLAB, d.N, d.K);
     if (bytes == 0) Py_RETURN_NONE;
-    Tensor blob = empty({(int64_t)bytes}, at::kByte, device);
-    const int st = qf_prepack_gemv_slab(g_ctx[device], &d, qw, sc, z, blob.data_ptr(), stream_of(device));
+    Tensor blob;
+    int st;
+    {
+        Unlocked u;
+        blob = empty({(int64_t)bytes}, at::kByte, device);
+        st = qf_prepack_gemv_slab(g_ctx[device], &d, qw, sc, z, blob.data_ptr(), stream_of(device));
+    }
     if (st != QF_OK) return failed(st, device);
     return Py_BuildValue("(NLLi)", THPVariable_Wrap(std::move(blob)), (long long)d.N, (long long)d.K, (int)d.zero_mode);
 }
@@ -393,13 +445,18 @@ PyObject *prepack_impl(PyObject *const *a) {
     if (!q || q->dim() != 2 || q->numel() == 0 || !PyBool_Check(a[1]) || !as_int(a[2], &layout) || !ready(device)) Py_RETURN_NONE;
     const int64_t per = is_byte(q->scalar_type()) ? 2 : q->scalar_type() == at::kInt ? 8 : 0;
     if (per == 0 || (int64_t)q->nbytes() % 4 != 0) Py_RETURN_NONE;
-    Tensor out = empty(q->sizes(), q->scalar_type(), device);
     const int back = a[1] == Py_True ? 1 : 0;
-    const int st = layout == QF_LAYOUT_TILED
-                       ? qf_prepack_w4_tiled(g_ctx[device], q->const_data_ptr(), out.data_ptr(), q->size(0), q->size(1) * per, back,
-                                             stream_of(device))
-                       : qf_prepack_w4(g_ctx[device], q->const_data_ptr(), out.data_ptr(), (int64_t)q->nbytes() / 4, back,
-                                       stream_of(device));
+    Tensor out;
+    int st;
+    {
+        Unlocked u;
+        out = empty(q->sizes(), q->scalar_type(), device);
+        if (layout == QF_LAYOUT_TILED)
+            st = qf_prepack_w4_tiled(g_ctx[device], q->const_data_ptr(), out.data_ptr(), q->size(0), q->size(1) * per, back,
+                                     stream_of(device));
+        else
+            st = qf_prepack_w4(g_ctx[device], q->const_data_ptr(), out.data_ptr(), (int64_t)q->nbytes() / 4, back, stream_of(device));
+    }
     if (st != QF_OK) return failed(st, device);
     return THPVariable_Wrap(std::move(out));
 }

@@ -4,6 +4,8 @@ import os
 import shutil
 import subprocess
 import sys
+import threading
+import time
 
 import pytest
 import torch
@@ -123,3 +125,32 @@ def test_an_earlier_error_is_not_the_next_launch_s():
         got = fn()
         assert qf.launch_count() - before == 1, name
         assert torch.equal(got, want[name]), name
+
+
+def test_other_threads_run_while_a_launch_blocks():
+    """A busy stream and more launches than its queue holds: the launching thread waits in the driver, the others do not."""
+    qw = torch.randint(-128, 128, (4, 64), dtype=torch.int8, device="cuda")
+    qf.unpack_int4(qw)
+    torch.cuda.synchronize()
+    longest, stop = 0.0, threading.Event()
+
+    def tick():
+        nonlocal longest
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            longest, last = max(longest, now - last), now
+
+    t = threading.Thread(target=tick)
+    t.start()
+    torch.cuda._sleep(1_000_000_000)  # about half a second
+    t0 = time.perf_counter()
+    for _ in range(4000):
+        qf.unpack_int4(qw)
+    blocked = time.perf_counter() - t0
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert blocked > 0.3, "the queue did not fill"
+    assert longest < 0.15, (longest, blocked)
