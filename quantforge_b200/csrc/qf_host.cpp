@@ -14,7 +14,11 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -109,6 +113,16 @@ const Tensor *cuda_tensor(PyObject *o, int *device) {
 }
 
 bool shape_is(const Tensor &t, int64_t a, int64_t b) { return t.dim() == 2 && t.size(0) == a && t.size(1) == b; }
+
+// The layout helpers (pack, pack_zeros, quantize) are tensor programs in ops.py, which autograd, tracing and function transforms
+// see operator by operator. Whether any of them watches this call on `t`.
+bool watched(PyObject *o, const Tensor &t) {
+    const c10::DispatchKeySet in = c10::impl::tls_local_dispatch_key_set().included_;
+    return !THPVariable_CheckExact(o) || in.has(c10::DispatchKey::Python) || in.has(c10::DispatchKey::Tracer) ||
+           in.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) || in.has(c10::DispatchKey::Functionalize) ||
+           at::impl::torch_function_mode_enabled() || (t.requires_grad() && c10::GradMode::is_enabled()) ||
+           t._fw_grad(0).defined();
+}
 
 // The device must be the current one and must have a context.
 bool ready(int device) {
@@ -348,7 +362,7 @@ PyObject *dequant_impl(PyObject *const *a) {
 PyObject *pack_impl(PyObject *const *a) {
     int device = -1;
     const Tensor *c = cuda_tensor(a[0], &device);
-    if (!c || c->dim() < 1 || c->scalar_type() != at::kChar || c->numel() == 0 || c->sizes().back() % 2 != 0 || !ready(device))
+    if (!c || watched(a[0], *c) || c->dim() < 1 || c->scalar_type() != at::kChar || c->numel() == 0 || c->sizes().back() % 2 != 0 || !ready(device))
         Py_RETURN_NONE;
     c10::SmallVector<int64_t, 5> shape(c->sizes().begin(), c->sizes().end());
     shape.back() /= 2;
@@ -367,7 +381,7 @@ PyObject *pack_impl(PyObject *const *a) {
 PyObject *pack_zeros_impl(PyObject *const *a) {
     int device = -1;
     const Tensor *z = cuda_tensor(a[0], &device);
-    if (!z || z->dim() != 2 || z->scalar_type() != at::kChar || z->numel() == 0 || z->size(1) % 8 != 0 || !ready(device))
+    if (!z || watched(a[0], *z) || z->dim() != 2 || z->scalar_type() != at::kChar || z->numel() == 0 || z->size(1) % 8 != 0 || !ready(device))
         Py_RETURN_NONE;
     Tensor out;
     int st;
@@ -385,7 +399,7 @@ PyObject *quantize_impl(PyObject *const *a) {
     int device = -1;
     const Tensor *w = cuda_tensor(a[0], &device);
     long long group;
-    if (!w || w->dim() != 2 || w->numel() == 0 || type_code(w->scalar_type()) < 0 || !as_int(a[1], &group) || !PyBool_Check(a[2]) ||
+    if (!w || watched(a[0], *w) || w->dim() != 2 || w->numel() == 0 || type_code(w->scalar_type()) < 0 || !as_int(a[1], &group) || !PyBool_Check(a[2]) ||
         !THPDtype_Check(a[3]) || !ready(device))
         Py_RETURN_NONE;
     const ScalarType st = ((THPDtype *)a[3])->scalar_type;

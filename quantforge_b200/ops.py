@@ -77,7 +77,7 @@ def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 def _offer(fn, t: torch.Tensor, *args):
     """fn(t, *args) of the native host path for a layout helper that also works without it: None where it does not
-    apply. A device's first such call creates its context."""
+    apply, which includes autograd, tracing and function transforms. A device's first such call creates its context."""
     out = fn(t, *args)
     if out is None and (t.device.index if t.device.index is not None else torch.cuda.current_device()) not in _ctxs:
         try:
@@ -102,7 +102,7 @@ def pack_int4(weights: torch.Tensor) -> torch.Tensor:
         raise TypeError("pack_int4 expects an int8 tensor of codes")
     if weights.shape[-1] % 2 != 0:
         raise ValueError("last dim must be even")
-    if weights.is_cuda:
+    if weights.is_cuda and not torch.compiler.is_compiling():
         packed = _offer((_fast or _native()).pack, weights)
         if packed is not None:
             return packed
@@ -116,7 +116,7 @@ def pack_zeros_u4(zeros: torch.Tensor) -> torch.Tensor:
     G, N = zeros.shape
     if N % 8 != 0:
         raise ValueError("N must be a multiple of 8")
-    if zeros.is_cuda:
+    if zeros.is_cuda and not torch.compiler.is_compiling():
         packed = _offer((_fast or _native()).pack_zeros, zeros)
         if packed is not None:
             return packed

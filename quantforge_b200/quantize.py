@@ -35,7 +35,7 @@ def quantize_w4(weight: torch.Tensor, group_size: int = 128, symmetric: bool = F
         raise ValueError("K must be a multiple of group_size")
     if scale_dtype is None:
         scale_dtype = weight.dtype if weight.dtype in (torch.float16, torch.bfloat16) else torch.float16
-    if weight.is_cuda:
+    if weight.is_cuda and not torch.compiler.is_compiling():
         made = ops._offer(ops._native().quantize, weight, group_size, bool(symmetric), scale_dtype)
         if made is not None:
             return made
