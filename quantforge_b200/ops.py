@@ -77,9 +77,11 @@ def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 def _offer(fn, t: torch.Tensor, *args):
     """fn(t, *args) of the native host path for a layout helper that also works without it: None where it does not
-    apply, which includes autograd, tracing and function transforms. A device's first such call creates its context."""
+    apply, which includes autograd, tracing and function transforms. A device's first such call creates its context, but not
+    in the middle of a graph capture: the allocations it makes would end that."""
     out = fn(t, *args)
-    if out is None and (t.device.index if t.device.index is not None else torch.cuda.current_device()) not in _ctxs:
+    if out is None and (t.device.index if t.device.index is not None else torch.cuda.current_device()) not in _ctxs and \
+            not torch.cuda.is_current_stream_capturing():
         try:
             _ctx(t.device)
         except QuantForgeError:  # not a device this library runs on

@@ -100,3 +100,30 @@ def test_subclasses_and_modes_see_the_operators():
     with Count() as mode:
         assert torch.equal(qf.pack_int4(codes), want)
     assert mode.n > 2
+
+
+def test_first_call_of_a_process_inside_a_capture():
+    """Without a context yet the helpers are recorded as tensor programs."""
+    import subprocess
+    import sys
+    code = """
+import torch
+import quantforge_b200 as qf
+from quantforge_b200.quantize import quantize_w4
+codes = torch.randint(0, 16, (8, 64), dtype=torch.int8, device="cuda")
+w = torch.randn(8, 256, device="cuda")
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    got = [qf.pack_int4(codes), qf.pack_zeros_u4(codes), *quantize_w4(w, 128)]
+codes.copy_(15 - codes)
+w.neg_()
+g.replay()
+torch.cuda.synchronize()
+assert qf.launch_count() == 0
+want = [qf.pack_int4(codes), qf.pack_zeros_u4(codes), *quantize_w4(w, 128)]
+assert qf.launch_count() == 3
+assert all(torch.equal(a, b) for a, b in zip(got, want))
+"""
+    p = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
