@@ -9,10 +9,16 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import os
+import sysconfig
+import warnings
+
+import torch
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libquantforge_rt.so")
-HOST_PATH = os.path.join(HERE, "lib", "_qf_host.so")  # native host path of the operators (csrc/qf_host.cpp)
+# Native host path of the operators (csrc/qf_host.cpp). It is bound to one interpreter and one torch: its name says which, so
+# that a copy built for others is neither loaded nor taken for this one.
+HOST_PATH = os.path.join(HERE, "lib", f"_qf_host.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
 
 QF_OK = 0
 QF_F16, QF_BF16, QF_F32 = 0, 1, 2
@@ -109,20 +115,30 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+class _NoHost:
+    """In place of the native host path where it is not there: handles nothing, so that ops.py does."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 _host = None
 
 
 def load_host():
-    """Load the native host path of the operators, or raise."""
+    """The native host path of the operators. Without it (not built for this interpreter and torch, or not loadable here) the
+    operators take the Python statements behind it, which need 10 to 15 us more per call."""
     global _host
     if _host is None:
-        load()
-        if not os.path.exists(HOST_PATH):
-            raise ImportError(f"{HOST_PATH} is missing: build it with `python -m quantforge_b200.build`.")
-        loader = importlib.machinery.ExtensionFileLoader("_qf_host", HOST_PATH)
-        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_qf_host", loader))
-        loader.exec_module(module)
-        module.set_error(QuantForgeError)
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("_qf_host", HOST_PATH)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_qf_host", loader))
+            loader.exec_module(module)
+            module.set_error(QuantForgeError)
+        except ImportError as e:
+            warnings.warn(f"the native host path is not available ({e}): calls take longer; "
+                          "build it with `python -m quantforge_b200.build`", RuntimeWarning, stacklevel=2)
+            module = _NoHost()
         _host = module
     return _host
 

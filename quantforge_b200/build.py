@@ -1,5 +1,5 @@
-"""Builds libquantforge_rt.so (CUDA kernels + C ABI) for sm_100a with nvcc, and _qf_host.so (the native host path of
-the Python operators, a CPython extension over torch's C++ API) with g++, in-tree.
+"""Builds libquantforge_rt.so (CUDA kernels + C ABI) for sm_100a with nvcc, and _qf_host.<interpreter>.torch-<version>.so
+(the native host path of the Python operators, a CPython extension over torch's C++ API) with g++, in-tree.
 
     python -m quantforge_b200.build [--force] [--verbose]
 
@@ -80,11 +80,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 HOST_SRC = os.path.join(CSRC, "qf_host.cpp")
-HOST_PATH = os.path.join(LIB_DIR, "_qf_host.so")
 
 
 def build_host(force: bool = False) -> str:
-    """Builds the native host path (part of build(): it links against libquantforge_rt.so)."""
+    """Builds the native host path for this interpreter and torch (part of build(): it links against libquantforge_rt.so)."""
+    from ._lib import HOST_PATH
     if not force and not _older(HOST_PATH, [HOST_SRC, os.path.join(ROOT, "include", "quantforge_rt.h")]):
         return HOST_PATH
     import torch

@@ -84,7 +84,7 @@ def _offer(fn, t: torch.Tensor, *args):
             not torch.cuda.is_current_stream_capturing():
         try:
             _ctx(t.device)
-        except QuantForgeError:  # not a device this library runs on
+        except (QuantForgeError, ImportError):  # not a device this library runs on, or the library is not built
             return None
         out = fn(t, *args)
     return out
