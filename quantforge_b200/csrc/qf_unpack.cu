@@ -34,11 +34,12 @@ __device__ __forceinline__ void unpack_word(uint32_t w, uint32_t &o0, uint32_t &
     o1 = prmt(lo, hi, 0x7362u);
 }
 
-// 16 input bytes per step, four steps in flight per thread, one 32-byte store each. The up to 15 bytes behind the last
-// whole step are unpacked by the first threads of block 0.
+// 16 input bytes per step, four steps in flight per thread, one 32-byte store each (two of 16 bytes where the output is only
+// aligned to that: WIDE is false; 64 MB in 47.3 instead of 43.0 us, a byte per thread 70.6). The up to 15 bytes behind the last whole step are unpacked by the first threads of block 0.
 // Four loads per thread before the first store, and whole-sector stores, are what the memory system needs: one load and
 // two 16-byte stores 32 bytes apart ran at 4.5 TB/s (28672 x 4096 bytes in 77.4 us).
 constexpr int UNPACK_STEPS = 4;
+template <bool WIDE>
 __global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out,
                                                          int64_t n_vec, int tail) {
     const int64_t first = (int64_t)blockIdx.x * (256 * UNPACK_STEPS) + threadIdx.x;
@@ -54,7 +55,13 @@ __global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *__restri
         unpack_word(v[j].y, a.z, a.w);
         unpack_word(v[j].z, b.x, b.y);
         unpack_word(v[j].w, b.z, b.w);
-        st_stream32(out + (first + j * 256) * 32, a, b);
+        uint8_t *dst = out + (first + j * 256) * 32;
+        if (WIDE) {
+            st_stream32(dst, a, b);
+        } else {
+            reinterpret_cast<uint4 *>(dst)[0] = a;
+            reinterpret_cast<uint4 *>(dst)[1] = b;
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x < tail) {
         const int64_t i = n_vec * 16 + threadIdx.x;
@@ -64,7 +71,7 @@ __global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *__restri
     }
 }
 
-// Any alignment: one byte per thread.
+// Any alignment (of the output: 2): one byte per thread.
 __global__ void __launch_bounds__(256) unpack_byte_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out,
                                                           int64_t n_bytes) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -81,12 +88,13 @@ int launch_unpack(qf_ctx *ctx, const void *packed, void *out, int64_t rows, int6
     const int64_t n_bytes = rows * packed_cols;
     if (n_bytes == 0) return QF_OK;
     cudaError_t e;
-    if ((uintptr_t)packed % 16 == 0 && (uintptr_t)out % 32 == 0) {
+    if ((uintptr_t)packed % 16 == 0 && (uintptr_t)out % 16 == 0) {
         const int64_t n_vec = n_bytes / 16;
         int64_t blocks = (n_vec + 256 * UNPACK_STEPS - 1) / (256 * UNPACK_STEPS);
         if (blocks < 1) blocks = 1;
-        e = launch_kernel(unpack_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)packed,
-                          (uint8_t *)out, n_vec, (int)(n_bytes % 16));
+        auto *fn = (uintptr_t)out % 32 == 0 ? unpack_vec_kernel<true> : unpack_vec_kernel<false>;
+        e = launch_kernel(fn, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)packed, (uint8_t *)out, n_vec,
+                          (int)(n_bytes % 16));
     } else {
         int64_t blocks = (n_bytes + 255) / 256;
         if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
