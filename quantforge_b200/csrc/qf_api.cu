@@ -1,4 +1,5 @@
 // C ABI of the runtime (include/quantforge_rt.h): argument checks, planning, dispatch.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -178,53 +179,72 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
         // of 16, 32, 64, 128 or 256 rows ran M = 777 as 1024 rows; 777 x 4096 x 4096 f16, canonical: 38.5 -> 35.1 us.)
         p->m_tiles = d->M > 256 ? (int)((d->M + 255) / 256) : 1;
         const int64_t rows = d->M > p->m_tiles ? (d->M + p->m_tiles - 1) / p->m_tiles : 1;
-        // Above 64 rows two neighbouring weight tiles share one batch tile, whose width is then a multiple of 32. A pair's start
-        // and end cost about 0.9 us more per tile and every 1024 codes give back 0.4 us: K = 8192 781 -> 737 us, 4096 28.5 ->
-        // 27.2 us, but M = 1462, 1024 x 49408 188 -> 195 us.
-        p->pair = rows > 64 && d->N % 256 == 0 && d->K > 2048;
-        const int step = p->pair ? 32 : 16;
-        const int bn = (int)((rows + step - 1) / step * step);
-        const int bk = gemm_block_k(bn, p->pair);
-        const int kblocks = (int)(d->K / bk);
-        p->bn = bn;
         const int64_t tiles = (int64_t)p->m_tiles * (d->N / 128);
-        int split;
-        if (d->split_k > 0) {
-            split = d->split_k;
-        } else {
-            const int64_t slots = (int64_t)kSmCount * (bn <= 64 ? 2 : 1);  // two narrow CTAs fit one SM
-            split = (int)(slots / tiles);
-            if (split < 1) split = 1;
-            // narrow tiles: at most 8 splits, the size of a portable thread-block cluster; 8 splits summed on chip
-            // beat 16 or 32 summed through global memory (measured, 8 tiles, K = 8192: 9.3 -> 6.9 us at M = 16,
-            // 17.7 -> 9.6 us at M = 64)
-            if (bn <= 64 && split > 8) split = 8;
-        }
-        if (split > kblocks) split = kblocks;
-        int kbps = (kblocks + split - 1) / split;
-        const int min_kbps = d->split_k > 0 ? 1 : (kblocks < 4 ? kblocks : 4);
-        if (kbps < min_kbps) kbps = min_kbps;
-        split = (kblocks + kbps - 1) / kbps;
-        if (d->split_k == 0 && split > 2 && kblocks % split != 0) {
-            // a slightly smaller split that divides K evenly beats an uneven one: fewer partial tiles to write and
-            // sum and no short last split (measured on K = 14336: 8 x 14 k-blocks is 3-7 % faster than 8 x 13 + 8)
-            for (int s2 = split - 1; s2 >= split - 2 && s2 >= 2; --s2)
-                if (kblocks % s2 == 0 && (kblocks / s2) * 20 <= kbps * 23) {
-                    split = s2;
-                    kbps = kblocks / s2;
-                    break;
-                }
-        }
-        if (d->split_k == 0 && bn <= 64 && split >= 2 && split <= 8 && tiles * split > kClusterMaxBlocks &&
-            kClusterMaxBlocks / tiles >= 2) {
-            // A launch of more than kClusterMaxBlocks blocks cannot run as one wave of thread-block clusters and
-            // would sum its partial tiles through global memory; fewer, longer splits that keep the on-chip
-            // reduction are faster (measured, 48 tiles: 6 splits 10.0 / 15.8 us at M = 16 / 64, 5 splits 9.1 / 11.9).
-            split = (int)(kClusterMaxBlocks / tiles);
-            kbps = (kblocks + split - 1) / split;
+        auto width = [&](int step) { return (int)((rows + step - 1) / step * step); };
+        // Splits of K for batch tiles of bn rows in k-blocks of bk codes, and k-blocks per split.
+        auto splits = [&](int bn, int bk, int *kbps_out) {
+            const int kblocks = (int)(d->K / bk);
+            int split;
+            if (d->split_k > 0) {
+                split = d->split_k;
+            } else {
+                const int64_t slots = (int64_t)kSmCount * (bn <= 64 ? 2 : 1);  // two narrow CTAs fit one SM
+                split = (int)(slots / tiles);
+                if (split < 1) split = 1;
+                // narrow tiles: at most 8 splits, the size of a portable thread-block cluster; 8 splits summed on chip
+                // beat 16 or 32 summed through global memory (measured, 8 tiles, K = 8192: 9.3 -> 6.9 us at M = 16,
+                // 17.7 -> 9.6 us at M = 64)
+                if (bn <= 64 && split > 8) split = 8;
+            }
+            if (split > kblocks) split = kblocks;
+            int kbps = (kblocks + split - 1) / split;
+            // at least 512 codes a block (with 256, K = 4096, N = 1024 took 38.7 us instead of 30.3 at M = 256)
+            const int min_kbps = d->split_k > 0 ? 1 : std::min(kblocks, 512 / bk);
+            if (kbps < min_kbps) kbps = min_kbps;
             split = (kblocks + kbps - 1) / kbps;
+            if (d->split_k == 0 && split > 2 && kblocks % split != 0) {
+                // a slightly smaller split that divides K evenly beats an uneven one: fewer partial tiles to write and
+                // sum and no short last split (measured on K = 14336: 8 x 14 k-blocks is 3-7 % faster than 8 x 13 + 8)
+                for (int s2 = split - 1; s2 >= split - 2 && s2 >= 2; --s2)
+                    if (kblocks % s2 == 0 && (kblocks / s2) * 20 <= kbps * 23) {
+                        split = s2;
+                        kbps = kblocks / s2;
+                        break;
+                    }
+            }
+            if (d->split_k == 0 && bn <= 64 && split >= 2 && split <= 8 && tiles * split > kClusterMaxBlocks &&
+                kClusterMaxBlocks / tiles >= 2) {
+                // A launch of more than kClusterMaxBlocks blocks cannot run as one wave of thread-block clusters and
+                // would sum its partial tiles through global memory; fewer, longer splits that keep the on-chip
+                // reduction are faster (measured, 48 tiles: 6 splits 10.0 / 15.8 us at M = 16 / 64, 5 splits 9.1 / 11.9).
+                split = (int)(kClusterMaxBlocks / tiles);
+                kbps = (kblocks + split - 1) / split;
+                split = (kblocks + kbps - 1) / kbps;
+            }
+            if (tiles > kMaxCounters) split = 1, kbps = kblocks;
+            *kbps_out = kbps;
+            return split;
+        };
+        // Above 64 rows two neighbouring weight tiles can share one batch tile, whose width is then a multiple of 32. The start
+        // and end of a pair cost about a microsecond, and what it gives back grows with the codes a block runs through (K over
+        // the split) and depends on the width: up to 128 rows either form works on 128 codes at a time and a pair only loads
+        // less of X; above, a block alone works on 64, which tells most where the MMAs of 64 codes are short. Measured for
+        // M 72 to 1462, N 1024 to 28672, K 1536 to 28672, pair against alone, mean over the shapes of each range of codes:
+        //   width     512     1024    1536    2048    3072    4096    6144    8192    more
+        //   <= 128   -5.4 %  -6.8   -12.6    -3.8    -7.2    +0.7    -4.2    +4.0    +8.6
+        //   <= 192   -2.1    -0.4    +0.5    +7.4   +12.0   +14.8   +17.3   +20.3   +19.8
+        //   wider    -2.2    -1.8    -5.5    -1.3    +1.2    +2.6    +4.8    +7.1    +7.3
+        int kbps = 1, split = 1;
+        p->pair = false;
+        if (rows > 64 && d->N % 256 == 0) {
+            split = splits(width(32), gemm_block_k(width(32), true), &kbps);
+            const int64_t codes = (int64_t)kbps * gemm_block_k(width(32), true);
+            // (1536 codes at widths up to 192: 3 to 8 % gained, but 6 to 25 % lost where they are all of K and N = 14336)
+            p->pair = d->K >= 2048 && codes >= (width(32) <= 128 ? 7168 : width(32) <= 192 ? 1536 : 2176);
         }
-        if (tiles > kMaxCounters) split = 1, kbps = kblocks;
+        const int bn = width(p->pair ? 32 : 16);
+        if (!p->pair) split = splits(bn, gemm_block_k(bn, false), &kbps);
+        p->bn = bn;
         p->split_k = split;
         p->chunks_per_split = kbps;
         if (split > 1) {

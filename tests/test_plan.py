@@ -60,3 +60,41 @@ def test_splits_stay_within_one_wave_of_clusters():
     assert _plan(16, 8192, 1024, 1) == (_lib.QF_PATH_GEMM, 8)     # 8 tiles: not 16 splits through global memory
     assert _plan(16, 8192, 10240, 1) == (_lib.QF_PATH_GEMM, 3)    # 80 tiles
     assert _plan(16, 4096, 18944, 1) == (_lib.QF_PATH_GEMM, 2)    # 148 tiles: two splits fill every slot
+
+
+def _tile_rows(M, K, N, split_k=0):
+    """Batch tile width of a split tcgen05 launch, from its scratch: counters, then split x tiles x width x N floats."""
+    d = _lib.LinearDesc(M=M, N=N, K=K, group_size=128, act_dtype=_lib.QF_BF16, out_dtype=_lib.QF_BF16,
+                        zero_mode=_lib.QF_ZERO_U4, zero_const=8, path=_lib.QF_PATH_GEMM, split_k=split_k, weight_layout=2)
+    split = _plan(M, K, N, 2, _lib.QF_PATH_GEMM, split_k)[1]
+    assert split > 1
+    floats = (_lib.load().qf_w4a16_workspace_bytes(ctypes.byref(d)) - 16384 * 4) // 4
+    tiles = (M + 255) // 256
+    assert floats % (split * tiles * N) == 0
+    return floats // (split * tiles * N)
+
+
+@pytest.mark.parametrize("M,K,N,split_k,want", [
+    # a multiple of 32: a pair of blocks; of 16 only: single blocks
+    (72, 4096, 1024, 0, 80),       # 512 codes a block
+    (72, 14336, 4096, 0, 80),      # 3584
+    (72, 28672, 4096, 0, 96),      # 7168
+    (72, 14336, 4096, 2, 96),
+    (140, 4096, 4096, 0, 144),     # 1024
+    (140, 8192, 4096, 0, 160),     # 2048
+    (140, 6144, 4096, 0, 160),     # 1536
+    (140, 8192, 4096, 8, 144),
+    (200, 8192, 1024, 0, 208),     # 512
+    (200, 8192, 4096, 0, 208),     # 2048
+    (200, 14336, 4096, 0, 224),    # 3584
+    (1030, 6144, 1024, 0, 208),    # five tiles of 206 rows, 2048 codes
+    (200, 14336, 4224, 0, 208),    # N no multiple of 256
+])
+def test_pairs_where_a_block_runs_through_enough_codes(M, K, N, split_k, want):
+    assert _tile_rows(M, K, N, split_k) == want
+
+
+@pytest.mark.parametrize("M", [16, 72, 140, 256])
+def test_blocks_take_512_codes_at_least(M):
+    for K in (512, 1024, 2048, 4096):
+        assert K // _plan(M, K, 1024, 2, _lib.QF_PATH_GEMM)[1] >= 512
