@@ -55,7 +55,6 @@ bool cluster_reduce_enabled() {
     return on;
 }
 
-static constexpr int kSmCount = 148;  // planning constant: the library targets B200 only
 // The split-K arrival counters occupy a FIXED region at the start of the workspace, so that a
 // workspace reused by linears of different shapes never exposes stale partial sums as counters.
 static constexpr int kMaxCounters = 16384;

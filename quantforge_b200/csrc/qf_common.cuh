@@ -51,6 +51,8 @@ namespace qf {
 
 extern std::atomic<long long> g_launch_count;
 
+constexpr int kSmCount = 148;  // planning constant: the library targets B200 only
+
 // Programmatic dependent launch (PDL): a kernel launched with it may start while the previous kernel in the
 // stream is still draining; it must execute griddep_wait() before touching anything that kernel wrote.
 // The linear kernels use the head start for barrier and TMEM set-up and for their first weights. Where the previous
@@ -58,7 +60,7 @@ extern std::atomic<long long> g_launch_count;
 // writes arrive, and read behind the wait; the next kernel is let in behind the wait as well.
 // Captured behind a linear of this library (follows_linear) the first weights are loaded at once: whatever wrote them
 // precedes the first linear of that row, which let its successor in only when that work was complete. (Called eagerly, the
-// difference is 1 % and less for the slab and tcgen05 kernels, 9.2 -> 10.0 us for M = 3, 3968 x 5136 per channel.)
+// difference is 1 % and less in the slab and tcgen05 kernels, 9.2 -> 10.0 us for M = 3, 3968 x 5136 per channel.)
 // QF_PDL=0 in the environment turns it off.
 bool pdl_enabled();
 // Graph capture: the only node that the next launch on `s` would depend on is the linear that this thread captured last.
