@@ -226,6 +226,7 @@ int launch_repack_kn(qf_ctx *ctx, const void *w_kn, int packed_along_n, int64_t 
 // in, one 32-byte store out), in four rows, all four loads in flight. The words of a thread lie in one quantisation group, so
 // there is one scale and one zero per row; neighbouring rows' scales share sectors, which the block's rows find in L1.
 // One word per thread with a 64-bit division to find its row ran at 3.2 TB/s (14336 x 4096 bf16 in 45.6 us).
+// Grid: blocks of rows in x, blocks of columns in y and, where K has more than 65535 of them, in z.
 constexpr int DEQUANT_ROWS = 4;
 template <bool BF16, int ZMODE, bool WIDE>
 __global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *__restrict__ qw,
@@ -233,10 +234,10 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *__restrict
                                                       const void *__restrict__ zeros, int zero_const,
                                                       uint4 *__restrict__ w_out, int64_t N, int words_per_row,
                                                       int group_words) {
-    const int j = (int)(blockIdx.y * 64 + (threadIdx.x & 31) * 2);
+    const int64_t j = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * 64 + (threadIdx.x & 31) * 2;
     if (j >= words_per_row) return;
     const int64_t n0 = (int64_t)blockIdx.x * (8 * DEQUANT_ROWS) + (threadIdx.x >> 5);
-    const int64_t gi = j / group_words;
+    const int64_t gi = (int)j / group_words;
     uint2 w[DEQUANT_ROWS];
     ZeroScale<BF16> zs[DEQUANT_ROWS];
 #pragma unroll
@@ -284,8 +285,9 @@ int launch_dequant(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const v
     if (d->N == 0) return QF_OK;
     const int64_t words = d->K / 8;
     const int64_t cols = (words + 63) / 64;
-    if (cols > 65535) return fail(ctx, QF_ERR_UNSUPPORTED, "K too large");
-    const dim3 grid((unsigned)((d->N + 8 * DEQUANT_ROWS - 1) / (8 * DEQUANT_ROWS)), (unsigned)cols);
+    const int64_t planes = (cols + 65534) / 65535;
+    const dim3 grid((unsigned)((d->N + 8 * DEQUANT_ROWS - 1) / (8 * DEQUANT_ROWS)), (unsigned)((cols + planes - 1) / planes),
+                    (unsigned)planes);
     const bool wide = (uintptr_t)w_out % 32 == 0;
     auto *fn = d->act_dtype == QF_BF16 ? (wide ? dequant_dispatch<true, true> : dequant_dispatch<true, false>)
                                        : (wide ? dequant_dispatch<false, true> : dequant_dispatch<false, false>);

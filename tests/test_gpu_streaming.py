@@ -98,3 +98,16 @@ def test_unpack_of_sixteen_byte_aligned_outputs_is_no_byte_loop():
 
     aligned, half = ms(buf[:2 * n]), ms(buf[16:])
     assert half < 1.35 * aligned
+
+
+def test_dequant_of_very_long_rows():
+    """More than 65535 blocks of columns (33.5 million codes a row)."""
+    import quantforge_b200 as qf
+    N, K, group = 16, 512 * 65537, 512 * 65537
+    g = torch.Generator(device="cuda").manual_seed(0)
+    qw = torch.randint(-128, 128, (N, K // 2), dtype=torch.int8, device="cuda", generator=g)
+    sc = (torch.rand(1, N, device="cuda", generator=g) * 0.01 + 0.001).half()
+    got = qf.dequant_w4(qw, sc, None, group)
+    for n in range(N):
+        codes = torch.stack([qw[n] & 15, (qw[n] >> 4) & 15], dim=-1).flatten()
+        assert torch.equal(got[n], (codes - 8).half() * sc[0, n])  # a difference that is exact and one rounding
