@@ -132,6 +132,8 @@ const char *qf_last_error(const qf_ctx *ctx);
  * python/quantforge/baseline.py:34-49 `unpack_int4`).
  * packed int8[rows, packed_cols] -> out int8[rows, 2*packed_cols]:
  * out[r, 2i] = b & 0xF, out[r, 2i+1] = (b >>logical 4) & 0xF.  Bit-exact.
+ * Alignment: `packed` any, `out` 2 bytes. With `packed` and `out` 16-byte aligned whole vectors are moved (`out` to 32 bytes:
+ * 10 % faster still), otherwise a byte per thread (1.6 times the time).
  */
 int qf_unpack_int4(qf_ctx *ctx, const void *packed_i8, void *out_i8, int64_t rows, int64_t packed_cols, void *stream);
 
@@ -145,7 +147,7 @@ int qf_pack_int4(qf_ctx *ctx, const void *codes_i8, void *out_i8, int64_t n_byte
 /*
  * Group-wise quantisation of weight[N, K] (qf_dtype `dtype`, 16-byte aligned): codes int8[N, K] in 0..15, scales [G, N] in
  * `scale_dtype` (QF_F16 or QF_BF16), zeros int8[G, N] in 0..15 (not written when `symmetric`: the zero is the constant 8).
- * group_size: a multiple of 4 that divides K. The arithmetic is fp32: scale = (max - min) / 15 or max|w| / 7, at least
+ * group_size: a multiple of 4 that divides K. The arithmetic is fp32: scale = (max - min) * (1/15) or max|w| * (1/7), at least
  * 2^-14, rounded to scale_dtype before the codes are chosen. No reference counterpart (it starts from codes).
  */
 int qf_quantize_w4(qf_ctx *ctx, const void *weight, int dtype, int64_t N, int64_t K, int group_size, int symmetric,
@@ -188,7 +190,7 @@ int qf_w4a16_linear_fused(qf_ctx *ctx, const qf_linear_desc *desc, const void *X
  * `count` linears enqueued back to back on `stream` by one call (the linears of a decoder layer: q/k/v as one
  * concatenated linear, o with the residual, gate/up with SiLU * mul, down with the residual). Entry i uses
  * descs[i], X[i], qweight[i], scales[i], qzeros[i] (may be NULL), Y[i], residual[i] (`residual` itself may be
- * NULL). Consecutive kernels are chained with programmatic dependent launch, so entry i+1 may read what entry i
+ * NULL). Consecutive kernels are chained with programmatic dependent launch; entry i+1 may read what entry i
  * wrote. `workspace` must hold the largest qf_w4a16_workspace_bytes over the entries. Stops at the first entry
  * that fails and returns its status (earlier entries stay enqueued).
  */

@@ -1,12 +1,14 @@
 // Group-wise INT4 quantisation of a 16- or 32-bit weight [N, K]: codes, scales and zero points in one pass.
 //
-// The arithmetic is the statement of quantforge_b200/quantize.py in fp32, step for step, so that codes, scales and zeros
-// are the same bits whichever of the two computes them:
+// The arithmetic is the statement of quantforge_b200/quantize.py in fp32, step for step as torch computes it on CUDA, so that
+// codes, scales and zeros are the same bits as that gives on the same device:
 //   asymmetric  scale = round16(max((wmax - wmin) * (1/15), 2^-14)), zero = clamp(rint(-wmin / scale), 0, 15)
 //   symmetric   scale = round16(max(wabs * (1/7), 2^-14)),           zero = 8
 //   code = clamp(rint(w / scale) + zero, 0, 15)
-// Bound by HBM: 2 bytes in and 1 byte out per weight (the codes are one byte each, the packing is a separate call). As
-// elementwise passes over fp32 copies it took 300 us at 4096 x 4096.
+// On the CPU torch divides by 15 and 7; a scale there can be the next 16-bit number (about one in 10^4 f16 scales of fp32
+// weights), and with it some codes.
+// 2 bytes in and 1 byte out per 16-bit weight (the codes are one byte each, the packing is a separate call): 7.7 us for
+// 4096 x 4096 at the copy rate. It takes 14.7 us, bound by issue slots; as elementwise passes over fp32 copies it took 300 us.
 #include "qf_common.cuh"
 
 namespace qf {

@@ -4,8 +4,10 @@
     qweight = pack_int4(codes)                      # int8 [N, K/2], the canonical layout of the runtime
     qzeros  = pack_zeros_u4(zeros)                  # int32 [G, N/8]   (asymmetric only)
 
-Layout helpers (any device); nothing here is on the inference hot path. Plain torch ops on the CPU, one kernel per call on
-CUDA tensors (csrc/qf_quantize.cu, the same fp32 arithmetic step for step). The packing rule is the
+Layout helpers (any device); nothing here is on the inference hot path. Plain torch ops on the CPU and wherever autograd or a
+tracer watches, one kernel per call on CUDA tensors (csrc/qf_quantize.cu), with the bits that torch gives on CUDA. There a
+division by 15 or 7 is a product with the reciprocal; on the CPU it is a division, so that about one f16 scale of fp32 weights
+in 10^4 is the next 16-bit number. The packing rule is the
 reference's `pack_int4` (python/quantforge/baseline.py:17-31); quantisation itself has no counterpart in the reference,
 which starts from already-quantised codes.
 """

@@ -11,7 +11,8 @@ import pytest
 import torch
 
 import quantforge_b200 as qf
-from quantforge_b200 import _lib
+from quantforge_b200 import _lib, ops
+from quantforge_b200.quantize import quantize_w4
 
 pytestmark = pytest.mark.gpu
 
@@ -154,3 +155,188 @@ def test_other_threads_run_while_a_launch_blocks():
     torch.cuda.synchronize()
     assert blocked > 0.3, "the queue did not fill"
     assert longest < 0.15, (longest, blocked)
+
+
+def _tensors(act=torch.float16, M=3, N=256, K=512, group=128):
+    g = torch.Generator(device="cuda").manual_seed(N + K + M)
+    t = {"x": torch.randn(M, K, device="cuda", generator=g).to(act), "M": M, "N": N, "K": K, "group": group,
+         "qw": torch.randint(-128, 128, (N, K // 2), dtype=torch.int8, device="cuda", generator=g),
+         "sc": (torch.rand(K // group, N, device="cuda", generator=g) * 0.01 + 0.001).to(act),
+         "z": torch.randint(0, 16, (K // group, N), dtype=torch.int8, device="cuda", generator=g)}
+    t["u4"] = qf.pack_zeros_u4(t["z"])
+    t["res"] = torch.randn(M, N, device="cuda", generator=g).to(act)
+    return t
+
+
+class Passing(_lib._NoHost):
+    """Answers nothing, but hears of contexts and workspaces."""
+    set_ctx, add_workspace = staticmethod(_lib.load_host().set_ctx), staticmethod(_lib.load_host().add_workspace)
+
+
+@pytest.fixture
+def python_path(monkeypatch):
+    """Runs a call on the Python statements alone."""
+    def run(fn):
+        with monkeypatch.context() as m:
+            m.setattr(ops, "_fast", Passing())
+            return fn()
+    return run
+
+
+class Seen:
+    """The native host path, noting for each call whether it answered."""
+
+    def __init__(self):
+        self.host, self.log = _lib.load_host(), []
+
+    def __getattr__(self, name):
+        def call(*args):
+            out = getattr(self.host, name)(*args)
+            self.log.append((name, out is not None))
+            return out
+        return call
+
+
+@pytest.fixture
+def seen(monkeypatch):
+    s = Seen()
+    monkeypatch.setattr(ops, "_fast", s)
+    return s
+
+
+L, I, T = qf.QF_LAYOUT_CANONICAL, qf.QF_LAYOUT_INTERLEAVED, qf.QF_LAYOUT_TILED
+ORDINARY = {
+    "canonical u4": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"]),
+    "canonical i8": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["z"]),
+    "canonical const": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], None, zero_const=7),
+    "uint8 weights": lambda t: qf.w4a16_linear(t["x"], t["qw"].view(torch.uint8), t["sc"], t["u4"]),
+    "int32 weights": lambda t: qf.w4a16_linear(t["x"], t["qw"].view(torch.int32), t["sc"], t["u4"]),
+    "fp32 out": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], out_dtype=torch.float32),
+    "split": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], split_k=2),
+    "residual": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], residual=t["res"], epilogue=qf.QF_EPI_RESIDUAL_ADD),
+    "silu": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], epilogue=qf.QF_EPI_SILU_MUL),
+    "slab": lambda t: qf.w4a16_linear(t["x"], qf.prepack_gemv_slab(t["qw"], t["sc"], t["u4"])),
+    "layer": lambda t: qf.W4A16Linear(t["qw"], t["sc"], t["u4"], prepack=True)(t["x"]),
+    "parameter": lambda t: qf.w4a16_linear(torch.nn.Parameter(t["x"]), t["qw"], t["sc"], t["u4"]),
+    "gemv": lambda t: qf.gemv_int4(t["x"], t["qw"], t["sc"][0].contiguous(), t["z"][0].contiguous()),
+    "unpack": lambda t: qf.unpack_int4(t["qw"]),
+    "unpack 3d": lambda t: qf.unpack_int4(t["qw"].view(2, -1, t["K"] // 2)),
+    "pack": lambda t: qf.pack_int4(t["z"]),
+    "pack_zeros": lambda t: qf.pack_zeros_u4(t["z"]),
+    "quantize": lambda t: torch.cat([a.float().flatten() for a in quantize_w4(t["x"], 128)]),
+    "dequant": lambda t: qf.dequant_w4(t["qw"], t["sc"], t["u4"]),
+    "prepack": lambda t: qf.prepack_w4(t["qw"]),
+    "prepack tiled": lambda t: qf.prepack_w4(t["qw"], layout=T),
+    "prepack back": lambda t: qf.prepack_w4(t["qw"], to_canonical=True, layout=T),
+    "prepack slab": lambda t: qf.prepack_gemv_slab(t["qw"], t["sc"], t["z"]).blob,
+}
+# answered by ops.py: a copy to make, or a form that only it reads
+PASSED_ON = {
+    "x not contiguous": lambda t: qf.w4a16_linear(t["x"].t().contiguous().t(), t["qw"], t["sc"], t["u4"]),
+    "weights not contiguous": lambda t: qf.w4a16_linear(t["x"], t["qw"].t().contiguous().t(), t["sc"], t["u4"]),
+    "scales not contiguous": lambda t: qf.dequant_w4(t["qw"], t["sc"].t().contiguous().t(), t["u4"]),
+    "gemv, zero points of uint8": lambda t: qf.gemv_int4(t["x"], t["qw"], t["sc"][0].contiguous(), t["z"][0].view(torch.uint8)),
+    "no rows": lambda t: qf.w4a16_linear(t["x"][:0], t["qw"], t["sc"], t["u4"]),
+    "zero_const as a float": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], None, zero_const=8.0),
+    "codes not contiguous": lambda t: qf.pack_int4(t["z"].t().contiguous().t()),
+    "codes not aligned": lambda t: qf.pack_int4(t["z"].flatten()[1:-1]),
+    "quantise to fp32 scales": lambda t: quantize_w4(t["x"], 128, True, torch.float32)[1],
+    "quantise odd groups": lambda t: quantize_w4(t["x"][:, :510], 510)[1],
+    "nothing to unpack": lambda t: qf.unpack_int4(t["qw"][:0]),
+}
+REFUSED = {
+    "x of another type": lambda t: qf.w4a16_linear(t["x"].float(), t["qw"], t["sc"], t["u4"]),
+    "x too short": lambda t: qf.w4a16_linear(t["x"][:, :256].contiguous(), t["qw"], t["sc"], t["u4"]),
+    "x of three dimensions": lambda t: qf.w4a16_linear(t["x"][None], t["qw"], t["sc"], t["u4"]),
+    "x misaligned": lambda t: qf.w4a16_linear(torch.cat([t["x"].flatten()] * 2)[1:1 + t["x"].numel()].view(t["x"].shape), t["qw"], t["sc"], t["u4"]),
+    "x on the CPU": lambda t: qf.w4a16_linear(t["x"].cpu(), t["qw"], t["sc"], t["u4"]),
+    "zeros of another shape": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["z"][:1].contiguous()),
+    "zeros of another type": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["z"].short()),
+    "group of 0": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], group_size=0),
+    "residual missing": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], epilogue=qf.QF_EPI_RESIDUAL_ADD),
+    "residual of another type": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], residual=t["res"].float(),
+                                                          epilogue=qf.QF_EPI_RESIDUAL_ADD),
+    "out of another shape": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], out=t["res"][:1]),
+    "zero_const out of range": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], None, zero_const=300),
+    "layout unknown": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], weight_layout=9),
+    "negative split": lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], split_k=-1),
+    "slab of too many rows": lambda t: qf.w4a16_linear(t["x"].repeat(20, 1), qf.prepack_gemv_slab(t["qw"], t["sc"], t["u4"])),
+    "unpack floats": lambda t: qf.unpack_int4(t["x"]),
+    "pack floats": lambda t: qf.pack_int4(t["x"]),
+}
+
+
+@pytest.mark.parametrize("act", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("name", list(ORDINARY))
+def test_ordinary_calls_are_answered_natively_and_alike(seen, python_path, name, act):
+    t = _tensors(act)
+    want = python_path(lambda: ORDINARY[name](t))  # also makes context and workspace
+    seen.log.clear()
+    got = ORDINARY[name](t)
+    assert seen.log and all(ok for _, ok in seen.log), seen.log
+    assert got.dtype == want.dtype and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("name", list(PASSED_ON))
+def test_other_calls_are_passed_on(seen, python_path, name):
+    t = _tensors()
+    want = python_path(lambda: PASSED_ON[name](t))
+    seen.log.clear()
+    got = PASSED_ON[name](t)
+    assert any(not ok for _, ok in seen.log), seen.log
+    assert got.shape == want.shape and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("name", list(REFUSED))
+def test_calls_in_error_are_refused_alike(python_path, name):
+    t = _tensors()
+    qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"])
+    errors = []
+    for run in (lambda fn: fn(), python_path):
+        with pytest.raises(Exception) as e:
+            run(lambda: REFUSED[name](t))
+        errors.append((type(e.value), str(e.value)))
+    assert errors[0] == errors[1]
+
+
+def test_results_go_where_the_caller_says(python_path):
+    t = _tensors()
+    want = python_path(lambda: ORDINARY["residual"](t))
+    y = t["res"].clone()  # out is the residual
+    got = qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], residual=y, out=y, epilogue=qf.QF_EPI_RESIDUAL_ADD)
+    assert got is y and torch.equal(y, want)
+
+
+def test_streams_and_growing_workspaces(seen, python_path):
+    """A stream's first call that needs scratch is passed on and makes it; later ones that fit are answered natively. Results on
+    two streams at once are those of one."""
+    small, large = _tensors(M=16, N=1024, K=4096), _tensors(M=64, N=8192, K=4096)
+    call = lambda t: qf.w4a16_linear(t["x"], t["qw"], t["sc"], t["u4"], split_k=16)  # noqa: E731
+    want = [python_path(lambda t=t: call(t)) for t in (small, large)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for s in streams:
+        with torch.cuda.stream(s):
+            for t in (small, small, large, large, small):
+                seen.log.clear()
+                call(t)
+    got = []
+    for i in range(6):
+        for s in streams:
+            with torch.cuda.stream(s):
+                seen.log.clear()
+                got.append((i % 2, call((small, large)[i % 2])))
+                assert seen.log == [("linear", True)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[k]) for k, y in got)
+    fresh = torch.cuda.Stream()
+    while fresh.cuda_stream in {k[1] for k in ops._workspaces}:  # torch hands its streams out in turn
+        fresh = torch.cuda.Stream()
+    with torch.cuda.stream(fresh):
+        answered = []
+        for t in (small, small, large, large, small):
+            seen.log.clear()
+            call(t)
+            answered.append(seen.log[0][1])
+    assert answered[0] is False and answered[1] is True and answered[3] is True and answered[4] is True
+    torch.cuda.synchronize()

@@ -13,8 +13,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("symmetric", [False, True])
 def test_quantise_kernel_is_the_torch_statement(N, K, group, dtype, symmetric):
-    """A transposed view takes the torch statement on the same device; codes, scales and zeros must be the same bits.
+    """A weight that requires grad takes the torch statement on the same device; codes, scales and zeros must be the same bits.
     Half of the rows hold small integers, whose quotients meet the rounding boundary exactly."""
+    import quantforge_b200 as qf
     from quantforge_b200.quantize import quantize_w4
     gen = torch.Generator(device="cuda").manual_seed(N + K)
     w = torch.randn(N, K, device="cuda", generator=gen) * 0.05
@@ -23,9 +24,28 @@ def test_quantise_kernel_is_the_torch_statement(N, K, group, dtype, symmetric):
     if N > 3:
         w[3, :group] = 0
     got = quantize_w4(w, group, symmetric)
-    want = quantize_w4(w.t().contiguous().t(), group, symmetric)
+    before = qf.launch_count()
+    want = quantize_w4(w.clone().requires_grad_(), group, symmetric)
+    assert qf.launch_count() == before
     for a, b in zip(got, want):
         assert (a is None and b is None) or (a.dtype == b.dtype and torch.equal(a, b))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_quantise_kernel_and_cpu(dtype, symmetric):
+    """The CPU divides where CUDA multiplies with the reciprocal: scales are the same 16-bit number or its neighbour, and
+    under the same scale codes and zeros are the same."""
+    from quantforge_b200.quantize import quantize_w4
+    w = (torch.randn(512, 4096, generator=torch.Generator().manual_seed(5)) * 0.05).to(dtype)
+    codes, scales, zeros = quantize_w4(w.cuda(), 128, symmetric)
+    c, s, z = quantize_w4(w, 128, symmetric)
+    ulps = (scales.cpu().view(torch.int16).int() - s.view(torch.int16).int()).abs()
+    assert ulps.max() <= 1 and (ulps > 0).float().mean() < 2e-3
+    same = ulps == 0
+    assert zeros is None or torch.equal(zeros.cpu()[same], z[same])
+    rows = same.t().repeat_interleave(128, dim=1)
+    assert torch.equal(codes.cpu()[rows], c[rows])
 
 
 @pytest.mark.parametrize("shape", [(1, 2), (3, 10), (5, 48), (33, 998), (4096, 2048), (2, 3, 64)])
