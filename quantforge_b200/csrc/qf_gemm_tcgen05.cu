@@ -18,9 +18,9 @@
 //                    B (= X tile, K-major, 128-byte swizzle) from shared memory, fp32 accumulate in TMEM.
 // Every mbarrier wait is bounded: on expiry the CTA raises an abort flag, records QF_ERR_TIMEOUT in
 // the context's status word, drains its own TMA copies, frees its TMEM and returns.
-// Every CTA loads its own tiles (plain TMA loads). Wide tiles run as CTA pairs, see gemm_kernel. Split-K over 2..8 blocks runs as a thread-block cluster whose
-// blocks sum their partial tiles through distributed shared memory; other splits use global partial tiles and an
-// arrival counter. All cluster barriers are passed by every block, aborted or not.
+// Every CTA loads its own tiles (plain TMA loads). Wide tiles run as CTA pairs, see gemm_kernel. Split-K of narrow tiles over
+// 2..8 blocks runs as a thread-block cluster whose blocks sum their partial tiles through distributed shared memory; other
+// splits use global partial tiles and an arrival counter. All cluster barriers are passed by every block, aborted or not.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -309,13 +309,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
     return v;
-}
-
-__device__ __forceinline__ int load_zero_rt(const void *zeros, int zmode, int zconst, int64_t gi, int64_t n,
-                                            int64_t N) {
-    if (zmode == QF_ZERO_CONST) return zconst;
-    if (zmode == QF_ZERO_U4) return load_zero<QF_ZERO_U4>(zeros, zconst, gi, n, N);
-    return load_zero<QF_ZERO_I8>(zeros, zconst, gi, n, N);
 }
 
 // (c0,c4)(c1,c5)(c2,c6)(c3,c7) -> (c0,c1)(c2,c3)(c4,c5)(c6,c7)
