@@ -601,21 +601,22 @@ gemv_slab_exch_kernel(const SlabParams p, const ArParams ar) {
 // it will own, and 64 threads the unit's constants. One 32-bit division per thread finds the place; one output word per thread
 // with 64-bit divisions took 13.9 us for 4096 x 4096.
 template <bool BF16, int ZMODE>
-__global__ void __launch_bounds__(256) slab_prepack_kernel(const uint32_t *__restrict__ qw,
-                                                           const uint16_t *__restrict__ scales,
-                                                           const void *__restrict__ zeros, int zero_const,
-                                                           uint8_t *__restrict__ blob, int64_t N, int chunks,
+__global__ void __launch_bounds__(256) slab_prepack_kernel(const uint32_t *qw,
+                                                           const uint16_t *scales,
+                                                           const void *zeros, int zero_const,
+                                                           uint8_t *blob, int64_t N, int chunks,
                                                            int group_chunks) {
+    griddep_begin();
     const int b = (int)(blockIdx.x / (unsigned)chunks), c = (int)(blockIdx.x % (unsigned)chunks);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint8_t *unit = blob + (size_t)blockIdx.x * SLAB_UNIT_BYTES;
     const int64_t row = (int64_t)b * 64 + w * 8 + (lane >> 2);
     const uint32_t *src = qw + (row * chunks + c) * 16 + (lane & 3);
     uint4 v;
-    v.x = interleave_word(__ldg(src));
-    v.y = interleave_word(__ldg(src + 4));
-    v.z = interleave_word(__ldg(src + 8));
-    v.w = interleave_word(__ldg(src + 12));
+    v.x = interleave_word(src[0]);
+    v.y = interleave_word(src[4]);
+    v.z = interleave_word(src[8]);
+    v.w = interleave_word(src[12]);
     *reinterpret_cast<uint4 *>(unit + (w >> 1) * SLAB_TILE_BYTES + (w & 1) * 512 + lane * 16) = v;
     if (threadIdx.x < 64) {
         const int r = threadIdx.x;
@@ -624,12 +625,13 @@ __global__ void __launch_bounds__(256) slab_prepack_kernel(const uint32_t *__res
         const int z = load_zero<ZMODE>(zeros, zero_const, gi, n, N);
         const uint32_t zsub = BF16 ? int_to_bf16_bits(128 + z) : int_to_f16_bits(1024 + z);
         *reinterpret_cast<uint32_t *>(unit + (r >> 4) * SLAB_TILE_BYTES + 1024 + (r & 15) * 4) =
-            (zsub & 0xffffu) | ((uint32_t)__ldg(scales + gi * N + n) << 16);
+            (zsub & 0xffffu) | ((uint32_t)scales[gi * N + n] << 16);
     }
 }
 
-__global__ void __launch_bounds__(256) slab_unpack_kernel(const uint8_t *__restrict__ blob, uint32_t *__restrict__ qw,
+__global__ void __launch_bounds__(256) slab_unpack_kernel(const uint8_t *blob, uint32_t *qw,
                                                           int chunks) {
+    griddep_begin();
     const int b = (int)(blockIdx.x / (unsigned)chunks), c = (int)(blockIdx.x % (unsigned)chunks);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint8_t *unit = blob + (size_t)blockIdx.x * SLAB_UNIT_BYTES;
@@ -648,7 +650,7 @@ static cudaError_t slab_prepack_dispatch(const qf_linear_desc *d, unsigned units
     auto *fn = d->zero_mode == QF_ZERO_CONST ? slab_prepack_kernel<BF16, QF_ZERO_CONST>
                : d->zero_mode == QF_ZERO_U4  ? slab_prepack_kernel<BF16, QF_ZERO_U4>
                                              : slab_prepack_kernel<BF16, QF_ZERO_I8>;
-    return launch_kernel(fn, dim3(units), dim3(256), 0, s, false, qw, sc, z, d->zero_const, blob, d->N, chunks, gc);
+    return launch_kernel(fn, dim3(units), dim3(256), 0, s, pdl_enabled(), qw, sc, z, d->zero_const, blob, d->N, chunks, gc);
 }
 
 int launch_slab_prepack(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const void *scales, const void *zeros,
@@ -663,7 +665,7 @@ int launch_slab_prepack(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, co
 int launch_slab_unpack(qf_ctx *ctx, int64_t N, int64_t K, const void *blob, void *qw, cudaStream_t s) {
     const int64_t units = (N / 64) * (K / 128);
     if (units > INT32_MAX) return fail(ctx, QF_ERR_UNSUPPORTED, "matrix too large");
-    return launched(ctx, launch_kernel(slab_unpack_kernel, dim3((unsigned)units), dim3(256), 0, s, false, (const uint8_t *)blob,
+    return launched(ctx, launch_kernel(slab_unpack_kernel, dim3((unsigned)units), dim3(256), 0, s, pdl_enabled(), (const uint8_t *)blob,
                                        (uint32_t *)qw, (int)(K / 128)),
                     "slab unpack");
 }

@@ -16,10 +16,10 @@ namespace qf {
 template <int DT>
 __device__ __forceinline__ void load4(const void *w, int64_t i, float (&v)[4]) {  // i: a multiple of 4
     if constexpr (DT == QF_F32) {
-        const float4 f = __ldg(reinterpret_cast<const float4 *>(w) + (i >> 2));
+        const float4 f = *(reinterpret_cast<const float4 *>(w) + (i >> 2));
         v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
     } else {
-        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(w) + (i >> 2));
+        const uint2 u = *(reinterpret_cast<const uint2 *>(w) + (i >> 2));
         const uint32_t h[4] = {u.x & 0xffffu, u.x >> 16, u.y & 0xffffu, u.y >> 16};
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -126,9 +126,10 @@ __device__ __forceinline__ void codes16(const float (&v)[16], float wmax, const 
 // 32 rows of four groups, so that scales and zeros [G, N] leave as whole sectors. With a group per warp the kernel was bound
 // by issue slots (25.2 us for 4096 x 4096 bf16 instead of the 7.7 its bytes take).
 template <int DT, bool SYM>
-__global__ void __launch_bounds__(256) quantize128_kernel(const void *__restrict__ w, int64_t N, int64_t K,
-                                                          uint32_t *__restrict__ codes, uint16_t *__restrict__ scales,
-                                                          int scale_dtype, int8_t *__restrict__ zeros) {
+__global__ void __launch_bounds__(256) quantize128_kernel(const void *w, int64_t N, int64_t K,
+                                                          uint32_t *codes, uint16_t *scales,
+                                                          int scale_dtype, int8_t *zeros) {
+    griddep_begin();
     __shared__ uint16_t s_scale[4][32];
     __shared__ int8_t s_zero[4][32];
     constexpr int VEC = DT == QF_F32 ? 4 : 8;  // values of a 16-byte load
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(256) quantize128_kernel(const void *__restrict
         for (int l = 0; l < LOADS; ++l) {
             uint4 u = make_uint4(0u, 0u, 0u, 0u);
             if (live)  // neighbouring lanes take neighbouring 16-byte pieces
-                u = __ldg(reinterpret_cast<const uint4 *>(w) + (n * K + gi * 128) / VEC + l * 8 + t);
+                u = *(reinterpret_cast<const uint4 *>(w) + (n * K + gi * 128) / VEC + l * 8 + t);
             const uint32_t x[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -208,9 +209,10 @@ __global__ void __launch_bounds__(256) quantize128_kernel(const void *__restrict
 // Any group size that is a multiple of 4: a block per (row, group), two passes over the group (the second one reads it
 // from L1 or L2).
 template <int DT, bool SYM>
-__global__ void __launch_bounds__(256) quantize_group_kernel(const void *__restrict__ w, int64_t N, int64_t K, int group,
-                                                             uint32_t *__restrict__ codes, uint16_t *__restrict__ scales,
-                                                             int scale_dtype, int8_t *__restrict__ zeros) {
+__global__ void __launch_bounds__(256) quantize_group_kernel(const void *w, int64_t N, int64_t K, int group,
+                                                             uint32_t *codes, uint16_t *scales,
+                                                             int scale_dtype, int8_t *zeros) {
+    griddep_begin();
     __shared__ float s_lo[8], s_hi[8];
     const int64_t G = K / group;
     const int64_t n = blockIdx.x / G, gi = blockIdx.x % G;
@@ -247,10 +249,10 @@ static cudaError_t quantize_launch(const void *w, int64_t N, int64_t K, int grou
                                    int scale_dtype, int8_t *zeros, cudaStream_t s) {
     if (group == 128 && (N + 31) / 32 <= 65535) {
         const dim3 grid((unsigned)((K / 128 + 3) / 4), (unsigned)((N + 31) / 32));
-        return launch_kernel(quantize128_kernel<DT, SYM>, grid, dim3(256), 0, s, false, w, N, K, codes, scales, scale_dtype, zeros);
+        return launch_kernel(quantize128_kernel<DT, SYM>, grid, dim3(256), 0, s, pdl_enabled(), w, N, K, codes, scales, scale_dtype, zeros);
     }
     const int threads = group >= 1024 ? 256 : group >= 512 ? 128 : group >= 256 ? 64 : 32;
-    return launch_kernel(quantize_group_kernel<DT, SYM>, dim3((unsigned)(N * (K / group))), dim3(threads), 0, s, false, w, N, K,
+    return launch_kernel(quantize_group_kernel<DT, SYM>, dim3((unsigned)(N * (K / group))), dim3(threads), 0, s, pdl_enabled(), w, N, K,
                          group, codes, scales, scale_dtype, zeros);
 }
 

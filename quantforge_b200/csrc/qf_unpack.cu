@@ -8,14 +8,14 @@ namespace qf {
 
 __device__ __forceinline__ uint4 ld_stream16(const void *p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint2 ld_stream8(const void *p) {
     uint2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
     return v;
 }
 // 32 bytes with one store instruction (a whole sector per thread): 32-byte aligned addresses only.
@@ -40,8 +40,9 @@ __device__ __forceinline__ void unpack_word(uint32_t w, uint32_t &o0, uint32_t &
 // two 16-byte stores 32 bytes apart ran at 4.5 TB/s (28672 x 4096 bytes in 77.4 us).
 constexpr int UNPACK_STEPS = 4;
 template <bool WIDE>
-__global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out,
+__global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *in, uint8_t *out,
                                                          int64_t n_vec, int tail) {
+    griddep_begin();
     const int64_t first = (int64_t)blockIdx.x * (256 * UNPACK_STEPS) + threadIdx.x;
     uint4 v[UNPACK_STEPS];
 #pragma unroll
@@ -72,8 +73,9 @@ __global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *__restri
 }
 
 // Any alignment (of the output: 2): one byte per thread.
-__global__ void __launch_bounds__(256) unpack_byte_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out,
+__global__ void __launch_bounds__(256) unpack_byte_kernel(const uint8_t *in, uint8_t *out,
                                                           int64_t n_bytes) {
+    griddep_begin();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_bytes; i += stride) {
         const uint8_t b = in[i];
@@ -93,12 +95,12 @@ int launch_unpack(qf_ctx *ctx, const void *packed, void *out, int64_t rows, int6
         int64_t blocks = (n_vec + 256 * UNPACK_STEPS - 1) / (256 * UNPACK_STEPS);
         if (blocks < 1) blocks = 1;
         auto *fn = (uintptr_t)out % 32 == 0 ? unpack_vec_kernel<true> : unpack_vec_kernel<false>;
-        e = launch_kernel(fn, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)packed, (uint8_t *)out, n_vec,
+        e = launch_kernel(fn, dim3((unsigned)blocks), dim3(256), 0, s, pdl_enabled(), (const uint8_t *)packed, (uint8_t *)out, n_vec,
                           (int)(n_bytes % 16));
     } else {
         int64_t blocks = (n_bytes + 255) / 256;
         if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-        e = launch_kernel(unpack_byte_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)packed,
+        e = launch_kernel(unpack_byte_kernel, dim3((unsigned)blocks), dim3(256), 0, s, pdl_enabled(), (const uint8_t *)packed,
                           (uint8_t *)out, n_bytes);
     }
     return launched(ctx, e, "unpack");
@@ -111,8 +113,9 @@ __device__ __forceinline__ uint32_t pack_words(uint32_t lo, uint32_t hi) {
     hi &= 0x0f0f0f0fu;
     return prmt(lo | (lo >> 4), hi | (hi >> 4), 0x6420u);
 }
-__global__ void __launch_bounds__(256) pack_vec_kernel(const uint8_t *__restrict__ codes, uint8_t *__restrict__ out,
+__global__ void __launch_bounds__(256) pack_vec_kernel(const uint8_t *codes, uint8_t *out,
                                                        int64_t n_vec, int tail) {
+    griddep_begin();
     const int64_t first = (int64_t)blockIdx.x * (256 * UNPACK_STEPS) + threadIdx.x;
     uint4 v[UNPACK_STEPS];
 #pragma unroll
@@ -132,14 +135,15 @@ int launch_pack(qf_ctx *ctx, const void *codes, void *out, int64_t n_bytes, cuda
     const int64_t n_vec = n_bytes / 8;
     int64_t blocks = (n_vec + 256 * UNPACK_STEPS - 1) / (256 * UNPACK_STEPS);
     if (blocks < 1) blocks = 1;
-    return launched(ctx, launch_kernel(pack_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)codes,
+    return launched(ctx, launch_kernel(pack_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, s, pdl_enabled(), (const uint8_t *)codes,
                                        (uint8_t *)out, n_vec, (int)(n_bytes % 8)),
                     "pack");
 }
 
 // Nibble permutation inside each word: qf_prepack_w4.
-__global__ void __launch_bounds__(256) prepack_kernel(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
+__global__ void __launch_bounds__(256) prepack_kernel(const uint32_t *in, uint32_t *out,
                                                       int64_t n_words, int to_canonical) {
+    griddep_begin();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += stride) {
         const uint32_t w = in[i];
@@ -150,7 +154,7 @@ __global__ void __launch_bounds__(256) prepack_kernel(const uint32_t *__restrict
 int launch_prepack(qf_ctx *ctx, const void *in, void *out, int64_t n_words, int to_canonical, cudaStream_t s) {
     int64_t blocks = (n_words + 255) / 256;
     if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-    return launched(ctx, launch_kernel(prepack_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint32_t *)in,
+    return launched(ctx, launch_kernel(prepack_kernel, dim3((unsigned)blocks), dim3(256), 0, s, pdl_enabled(), (const uint32_t *)in,
                                        (uint32_t *)out, n_words, to_canonical),
                     "prepack");
 }
@@ -158,21 +162,29 @@ int launch_prepack(qf_ctx *ctx, const void *in, void *out, int64_t n_words, int 
 // canonical word (n, j) <-> tiled word ((nt * KB + kb) * 128 + r) * 16 + w, n = nt*128 + r, j = kb*16 + w.
 // A block moves one tile (8 KB, contiguous on the tiled side): two 16-byte pieces per thread, four threads to the 64
 // bytes of a row.
-__global__ void __launch_bounds__(256) prepack_tiled_kernel(const uint4 *__restrict__ in, uint4 *__restrict__ out,
+__global__ void __launch_bounds__(256) prepack_tiled_kernel(const uint4 *in, uint4 *out,
                                                             int KB, int to_canonical) {
+    griddep_begin();
     const int nt = (int)(blockIdx.x / (unsigned)KB), kb = (int)(blockIdx.x % (unsigned)KB);
     const int64_t tile = (int64_t)blockIdx.x * 512;
     const int64_t canon0 = ((int64_t)nt * 128 * KB + kb) * 4;
+    int64_t canon[2];
+    uint4 piece[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int i = h * 256 + (int)threadIdx.x;
-        const int64_t canon = canon0 + (int64_t)(i >> 2) * KB * 4 + (i & 3);
-        uint4 v = in[to_canonical ? tile + i : canon];
+        canon[h] = canon0 + (int64_t)(i >> 2) * KB * 4 + (i & 3);
+        piece[h] = in[to_canonical ? tile + i : canon[h]];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = h * 256 + (int)threadIdx.x;
+        uint4 v = piece[h];
         if (to_canonical)
             v = make_uint4(deinterleave_word(v.x), deinterleave_word(v.y), deinterleave_word(v.z), deinterleave_word(v.w));
         else
             v = make_uint4(interleave_word(v.x), interleave_word(v.y), interleave_word(v.z), interleave_word(v.w));
-        out[to_canonical ? canon : tile + i] = v;
+        out[to_canonical ? canon[h] : tile + i] = v;
     }
 }
 
@@ -180,15 +192,16 @@ int launch_prepack_tiled(qf_ctx *ctx, const void *in, void *out, int64_t N, int6
                          cudaStream_t s) {
     const int64_t tiles = (N / 128) * (K / 128);
     if (tiles > INT32_MAX) return fail(ctx, QF_ERR_UNSUPPORTED, "matrix too large");
-    return launched(ctx, launch_kernel(prepack_tiled_kernel, dim3((unsigned)tiles), dim3(256), 0, s, false, (const uint4 *)in,
+    return launched(ctx, launch_kernel(prepack_tiled_kernel, dim3((unsigned)tiles), dim3(256), 0, s, pdl_enabled(), (const uint4 *)in,
                                        (uint4 *)out, (int)(K / 128), to_canonical),
                     "tiled prepack");
 }
 
 // W[K, N] (one code per byte, or two per byte along N) -> canonical qweight [N, K/8] words. One thread per output
 // word; consecutive threads take consecutive n, so the reads are coalesced (the 4-byte writes are not: one-time op).
-__global__ void __launch_bounds__(256) repack_kn_kernel(const uint8_t *__restrict__ w_kn, int packed_along_n,
-                                                        int64_t K, int64_t N, uint32_t *__restrict__ out) {
+__global__ void __launch_bounds__(256) repack_kn_kernel(const uint8_t *w_kn, int packed_along_n,
+                                                        int64_t K, int64_t N, uint32_t *out) {
+    griddep_begin();
     const int64_t words_per_row = K >> 3;
     const int64_t total = N * words_per_row;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -217,7 +230,7 @@ int launch_repack_kn(qf_ctx *ctx, const void *w_kn, int packed_along_n, int64_t 
     const int64_t total = N * (K / 8);
     int64_t blocks = (total + 255) / 256;
     if (blocks > (int64_t)ctx->sm_count * 16) blocks = (int64_t)ctx->sm_count * 16;
-    return launched(ctx, launch_kernel(repack_kn_kernel, dim3((unsigned)blocks), dim3(256), 0, s, false, (const uint8_t *)w_kn,
+    return launched(ctx, launch_kernel(repack_kn_kernel, dim3((unsigned)blocks), dim3(256), 0, s, pdl_enabled(), (const uint8_t *)w_kn,
                                        packed_along_n, K, N, (uint32_t *)out),
                     "repack");
 }
@@ -229,11 +242,12 @@ int launch_repack_kn(qf_ctx *ctx, const void *w_kn, int packed_along_n, int64_t 
 // Grid: blocks of rows in x, blocks of columns in y and, where K has more than 65535 of them, in z.
 constexpr int DEQUANT_ROWS = 4;
 template <bool BF16, int ZMODE, bool WIDE>
-__global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *__restrict__ qw,
-                                                      const uint16_t *__restrict__ scales,
-                                                      const void *__restrict__ zeros, int zero_const,
-                                                      uint4 *__restrict__ w_out, int64_t N, int words_per_row,
+__global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *qw,
+                                                      const uint16_t *scales,
+                                                      const void *zeros, int zero_const,
+                                                      uint4 *w_out, int64_t N, int words_per_row,
                                                       int group_words) {
+    griddep_begin();
     const int64_t j = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * 64 + (threadIdx.x & 31) * 2;
     if (j >= words_per_row) return;
     const int64_t n0 = (int64_t)blockIdx.x * (8 * DEQUANT_ROWS) + (threadIdx.x >> 5);
@@ -246,7 +260,7 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *__restrict
 #pragma unroll
     for (int r = 0; r < DEQUANT_ROWS; ++r) {
         const int64_t n = n0 + 8 * r;
-        if (n < N) zs[r].set(load_zero<ZMODE>(zeros, zero_const, gi, n, N), __ldg(scales + gi * N + n));
+        if (n < N) zs[r].set(load_zero<ZMODE>(zeros, zero_const, gi, n, N), scales[gi * N + n]);
     }
 #pragma unroll
     for (int r = 0; r < DEQUANT_ROWS; ++r) {
@@ -277,7 +291,7 @@ static cudaError_t dequant_dispatch(int zmode, dim3 grid, cudaStream_t s, const 
     auto *fn = zmode == QF_ZERO_CONST ? dequant_kernel<BF16, QF_ZERO_CONST, WIDE>
                : zmode == QF_ZERO_U4  ? dequant_kernel<BF16, QF_ZERO_U4, WIDE>
                                       : dequant_kernel<BF16, QF_ZERO_I8, WIDE>;
-    return launch_kernel(fn, grid, dim3(256), 0, s, false, qw, sc, z, zc, out, N, words_per_row, group_words);
+    return launch_kernel(fn, grid, dim3(256), 0, s, pdl_enabled(), qw, sc, z, zc, out, N, words_per_row, group_words);
 }
 
 int launch_dequant(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const void *scales, const void *zeros,
