@@ -8,7 +8,7 @@
 // On the CPU torch divides by 15 and 7; a scale there can be the next 16-bit number (about one in 10^4 f16 scales of fp32
 // weights), and with it some codes.
 // 2 bytes in and 1 byte out per 16-bit weight (the codes are one byte each, the packing is a separate call): 7.7 us for
-// 4096 x 4096 at the copy rate. It takes 14.7 us, bound by issue slots; as elementwise passes over fp32 copies it took 300 us.
+// 4096 x 4096 at the copy rate. It takes 13.7 us, bound by issue slots; as elementwise passes over fp32 copies it took 300 us.
 #include "qf_common.cuh"
 
 namespace qf {
@@ -84,7 +84,13 @@ __device__ __forceinline__ GroupParams group_params(float lo, float hi, int scal
         g.scale = __half2float(h);
     }
     g.rcp = 1.0f / g.scale;
-    g.zero = SYM ? 8.0f : fminf(fmaxf(rintf(-lo / g.scale), 0.0f), 15.0f);
+    if (SYM) {
+        g.zero = 8.0f;
+    } else {
+        float z = rintf(-lo * g.rcp);
+        if (!(fabsf(fmaf(-lo, g.rcp, -z)) < 0.4999f && fabsf(z) < 256.0f)) z = rintf(-lo / g.scale);  // as code_exact
+        g.zero = fminf(fmaxf(z, 0.0f), 15.0f);
+    }
     return g;
 }
 
@@ -96,21 +102,41 @@ constexpr float kRound = 12582912.0f;
 __device__ __forceinline__ uint32_t code_exact(float w, const GroupParams &g) {
     return (uint32_t)(int)fminf(fmaxf(rintf(w / g.scale) + g.zero, 0.0f), 15.0f);
 }
-__device__ __forceinline__ float rounded(float w, const GroupParams &g, float &off) {
-    const float t = w * g.rcp;
-    const float m = t + kRound;
-    off = fmaxf(off, fabsf(t - (m - kRound)));
-    return m;
+// Two fp32 values in a 64-bit register: one instruction works on both.
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
-// Four codes, one per byte; `wmax`: the largest magnitude in the group. Zero point and clamp are applied to two 16-bit
-// values at a time.
+__device__ __forceinline__ void split_f32x2(uint64_t v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// Four codes, one per byte; `wmax`: the largest magnitude in the group. Products and roundings are made for two values at a
+// time in fp32, zero point and clamp for two in 16 bits.
 __device__ __forceinline__ uint32_t codes4(const float *v, float wmax, const GroupParams &g) {
+    const uint64_t rcp = f32x2(g.rcp, g.rcp), round = f32x2(kRound, kRound), minus = f32x2(-1.0f, -1.0f);
     float off = 0.f;
-    const uint32_t m0 = __float_as_uint(rounded(v[0], g, off)), m1 = __float_as_uint(rounded(v[1], g, off)),
-                   m2 = __float_as_uint(rounded(v[2], g, off)), m3 = __float_as_uint(rounded(v[3], g, off));
+    uint32_t m[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint64_t w = f32x2(v[2 * h], v[2 * h + 1]);
+        const uint64_t r = fma_f32x2(w, rcp, round);
+        const uint64_t d = fma_f32x2(w, rcp, fma_f32x2(r, minus, round));  // distance from the integer
+        float a, b;
+        split_f32x2(d, a, b);
+        off = fmaxf(off, fmaxf(fabsf(a), fabsf(b)));
+        split_f32x2(r, a, b);
+        m[2 * h] = __float_as_uint(a);
+        m[2 * h + 1] = __float_as_uint(b);
+    }
     const uint32_t zero = dup16((uint32_t)(int)g.zero);
-    const uint32_t a = __viaddmin_s16x2_relu(prmt(m0, m1, 0x5410u), zero, 0x000f000fu);
-    const uint32_t b = __viaddmin_s16x2_relu(prmt(m2, m3, 0x5410u), zero, 0x000f000fu);
+    const uint32_t a = __viaddmin_s16x2_relu(prmt(m[0], m[1], 0x5410u), zero, 0x000f000fu);
+    const uint32_t b = __viaddmin_s16x2_relu(prmt(m[2], m[3], 0x5410u), zero, 0x000f000fu);
     uint32_t c = prmt(a, b, 0x6420u);
     if (!(off < 0.4999f && wmax * g.rcp < 256.0f))
         c = code_exact(v[0], g) | code_exact(v[1], g) << 8 | code_exact(v[2], g) << 16 | code_exact(v[3], g) << 24;
@@ -123,69 +149,80 @@ __device__ __forceinline__ void codes16(const float (&v)[16], float wmax, const 
 
 // Groups of 128: eight lanes hold a group in registers, sixteen values each, so a warp works on four neighbouring groups of
 // a row (1 KB in for 16-bit weights) and the scale's divisions and roundings are paid once per 512 weights. A block covers
-// 32 rows of four groups, so that scales and zeros [G, N] leave as whole sectors. With a group per warp the kernel was bound
-// by issue slots (25.2 us for 4096 x 4096 bf16 instead of the 7.7 its bytes take).
+// 16 rows of four groups, so that scales [G, N] leave as whole sectors; all its loads are in flight before the first is used.
+// (32 rows with half of the loads ahead: 1.7 waves for 4096 x 4096. Alone, on weights not in L2, bf16 asymmetric / f16 symmetric:
+// 15.9 / 12.2 -> 13.7 / 10.1 us, 14336 x 4096 47.1 / 36.0 -> 40.8 / 31.3; all bytes at the copy rate 7.7 and 27.) Five blocks of
+// 48 registers per SM for 16-bit weights; fp32 ones need the registers (four blocks 13.3 us, five 14.4).
+// With a group per warp the kernel was bound by issue slots (25.2 us for 4096 x 4096 bf16).
+constexpr int QUANT_PASSES = 2;  // rows a warp works on
 template <int DT, bool SYM>
-__global__ void __launch_bounds__(256) quantize128_kernel(const void *w, int64_t N, int64_t K,
-                                                          uint32_t *codes, uint16_t *scales,
-                                                          int scale_dtype, int8_t *zeros) {
+__global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(const void *w, int64_t N, int64_t K, uint32_t *codes,
+                                                          uint16_t *scales, int scale_dtype, int8_t *zeros) {
     griddep_begin();
-    __shared__ uint16_t s_scale[4][32];
-    __shared__ int8_t s_zero[4][32];
+    constexpr int ROWS = 8 * QUANT_PASSES;
+    __shared__ uint16_t s_scale[4][ROWS];
+    __shared__ int8_t s_zero[4][ROWS];
     constexpr int VEC = DT == QF_F32 ? 4 : 8;  // values of a 16-byte load
     constexpr int LOADS = 16 / VEC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int q = lane >> 3, t = lane & 7;  // group of the warp's four, lane of the group
     const int64_t G = K >> 7;
     const int64_t gi = (int64_t)blockIdx.x * 4 + q;
-    const int64_t n0 = (int64_t)blockIdx.y * 32;
+    const int64_t n0 = (int64_t)blockIdx.y * ROWS;
     const bool have = gi < G;
-#pragma unroll 2
-    for (int pass = 0; pass < 4; ++pass) {
+    const int64_t first = (n0 + warp) * K + gi * 128;  // of the row of pass 0; a pass is 8 rows
+    uint4 u[QUANT_PASSES][LOADS];
+#pragma unroll
+    for (int pass = 0; pass < QUANT_PASSES; ++pass)
+#pragma unroll
+        for (int l = 0; l < LOADS; ++l) {
+            u[pass][l] = make_uint4(0u, 0u, 0u, 0u);
+            if (have && n0 + pass * 8 + warp < N)  // neighbouring lanes take neighbouring 16-byte pieces
+                u[pass][l] = reinterpret_cast<const uint4 *>(w)[(first + pass * 8 * K) / VEC + l * 8 + t];
+        }
+#pragma unroll
+    for (int pass = 0; pass < QUANT_PASSES; ++pass) {
         const int row = pass * 8 + warp;
-        const int64_t n = n0 + row;
-        const bool live = have && n < N;
-        float v[16];
+        float v[16], lo, hi;
         uint32_t lo2 = 0, hi2 = 0;  // 16-bit types: running minimum and maximum of two values at a time
 #pragma unroll
         for (int l = 0; l < LOADS; ++l) {
-            uint4 u = make_uint4(0u, 0u, 0u, 0u);
-            if (live)  // neighbouring lanes take neighbouring 16-byte pieces
-                u = *(reinterpret_cast<const uint4 *>(w) + (n * K + gi * 128) / VEC + l * 8 + t);
-            const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+            const uint32_t x[4] = {u[pass][l].x, u[pass][l].y, u[pass][l].z, u[pass][l].w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                if constexpr (DT != QF_F32) {
-                    lo2 = l + k == 0 ? x[0] : min2_nan<DT>(lo2, x[k]);
-                    hi2 = l + k == 0 ? x[0] : max2_nan<DT>(hi2, x[k]);
-                }
                 if constexpr (DT == QF_F32) {
                     v[l * 4 + k] = __uint_as_float(x[k]);
                 } else {
+                    lo2 = l + k == 0 ? x[0] : min2_nan<DT>(lo2, x[k]);
+                    hi2 = l + k == 0 ? x[0] : max2_nan<DT>(hi2, x[k]);
                     v[l * 8 + 2 * k] = low_half<DT>(x[k]);
                     v[l * 8 + 2 * k + 1] = high_half<DT>(x[k]);
                 }
             }
         }
-        float lo, hi;
         if constexpr (DT == QF_F32) {
             lo = hi = v[0];
 #pragma unroll
             for (int k = 1; k < 16; ++k) lo = min_nan(lo, v[k]), hi = max_nan(hi, v[k]);
-        } else {
-            lo = min_nan(low_half<DT>(lo2), high_half<DT>(lo2));
-            hi = max_nan(low_half<DT>(hi2), high_half<DT>(hi2));
-        }
 #pragma unroll
-        for (int o = 4; o; o >>= 1) {
-            lo = min_nan(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-            hi = max_nan(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            for (int o = 4; o; o >>= 1) {
+                lo = min_nan(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                hi = max_nan(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            }
+        } else {
+            // (minimum, -maximum) in one word: the minimum of such words, over the halves and over the lanes, is both
+            hi2 ^= 0x80008000u;
+            uint32_t e = min2_nan<DT>(prmt(lo2, hi2, 0x5410u), prmt(lo2, hi2, 0x7632u));
+#pragma unroll
+            for (int o = 4; o; o >>= 1) e = min2_nan<DT>(e, __shfl_xor_sync(0xffffffffu, e, o));
+            lo = low_half<DT>(e);
+            hi = -high_half<DT>(e);
         }
         const GroupParams g = group_params<SYM>(lo, hi, scale_dtype);
         uint32_t c[4];
         codes16(v, fmaxf(fabsf(lo), fabsf(hi)), g, c);
-        if (live) {
-            uint32_t *dst = codes + (n * K + gi * 128) / 4;
+        if (have && n0 + row < N) {
+            uint32_t *dst = codes + (first + pass * 8 * K) / 4;
 #pragma unroll
             for (int l = 0; l < LOADS; ++l) {
                 if constexpr (VEC == 8) reinterpret_cast<uint2 *>(dst)[l * 8 + t] = make_uint2(c[2 * l], c[2 * l + 1]);
@@ -200,7 +237,7 @@ __global__ void __launch_bounds__(256) quantize128_kernel(const void *w, int64_t
     __syncthreads();
     const int64_t n = n0 + lane;
     const int64_t go = (int64_t)blockIdx.x * 4 + warp;
-    if (warp < 4 && go < G && n < N) {
+    if (warp < 4 && lane < ROWS && go < G && n < N) {
         scales[go * N + n] = s_scale[warp][lane];
         if (!SYM) zeros[go * N + n] = s_zero[warp][lane];
     }
@@ -247,8 +284,9 @@ __global__ void __launch_bounds__(256) quantize_group_kernel(const void *w, int6
 template <int DT, bool SYM>
 static cudaError_t quantize_launch(const void *w, int64_t N, int64_t K, int group, uint32_t *codes, uint16_t *scales,
                                    int scale_dtype, int8_t *zeros, cudaStream_t s) {
-    if (group == 128 && (N + 31) / 32 <= 65535) {
-        const dim3 grid((unsigned)((K / 128 + 3) / 4), (unsigned)((N + 31) / 32));
+    constexpr int ROWS = 8 * QUANT_PASSES;
+    if (group == 128 && (N + ROWS - 1) / ROWS <= 65535) {
+        const dim3 grid((unsigned)((K / 128 + 3) / 4), (unsigned)((N + ROWS - 1) / ROWS));
         return launch_kernel(quantize128_kernel<DT, SYM>, grid, dim3(256), 0, s, pdl_enabled(), w, N, K, codes, scales, scale_dtype, zeros);
     }
     const int threads = group >= 1024 ? 256 : group >= 512 ? 128 : group >= 256 ? 64 : 32;
