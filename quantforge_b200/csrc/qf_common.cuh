@@ -41,6 +41,8 @@ struct qf_ctx {
     HostSlot host_slot[2];
     int host_next = 0;
     cudaStream_t copy_stream = nullptr;
+    // Activations of calls with small page-locked host buffers, fetched by a kernel of the caller's stream.
+    void *mapped_x = nullptr;
     std::vector<void *> retired;  // outgrown staging buffers
     // device status word written by kernels whose bounded waits expire (tcgen05 path)
     int *dev_status = nullptr;
@@ -224,6 +226,7 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why);
 
 // kernels (defined in their own translation units)
 int launch_unpack(qf_ctx *ctx, const void *packed, void *out, int64_t rows, int64_t packed_cols, cudaStream_t s);
+int launch_fetch(qf_ctx *ctx, const void *src, void *dst, int64_t bytes, cudaStream_t s);
 int launch_pack(qf_ctx *ctx, const void *codes, void *out, int64_t n_bytes, cudaStream_t s);
 int launch_quantize(qf_ctx *ctx, const void *w, int dtype, int64_t N, int64_t K, int group, bool symmetric, void *codes,
                     void *scales, int scale_dtype, void *zeros, cudaStream_t s);
