@@ -139,7 +139,7 @@ __device__ __forceinline__ void gemv_body(const GemvParams &p, const typename Ex
             const int cl = e >> 6;
             const int64_t gi = p.group_chunks == 1 ? (c0 + cl) : (c0 + cl) / p.group_chunks;
             z = load_zero<ZMODE>(p.zeros, p.zero_const, gi, n, p.N);
-            scale = __ldg(p.scales + gi * p.N + n);
+            scale = p.scales[gi * p.N + n];  // an ordinary load: the block may have started beside the kernel that wrote them
         }
     };
     auto put_consts = [&](int e, int z, uint32_t scale) {
