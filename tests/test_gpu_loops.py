@@ -1,0 +1,64 @@
+"""The streaming kernels that loop: unpack of bytes at odd addresses and the interleaved prepack, at sizes around a pass of their
+loops, and that several of their loads are in flight at a time."""
+import pytest
+import torch
+
+import quantforge_b200 as qf
+
+pytestmark = pytest.mark.gpu
+
+PASS = 148 * 16 * 256  # elements that the largest grid takes in one step of the loop; the kernels take four steps a pass
+
+
+def best_ms(fn, reps=7):
+    fn()
+    best = 1e9
+    for _ in range(reps):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        fn()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, PASS - 1, PASS + 1, 3 * PASS + 5, 4 * PASS, 4 * PASS + 1, 9 * PASS + 77])
+def test_unpack_of_bytes(n):
+    packed = torch.randint(-128, 128, (n + 1,), dtype=torch.int8, device="cuda")[1:]
+    want = torch.stack([packed & 15, (packed >> 4) & 15], dim=-1).flatten()
+    assert torch.equal(qf.unpack_int4(packed), want)
+
+
+def _in_place(words, to_canonical):
+    from quantforge_b200 import _lib, ops
+    assert _lib.load().qf_prepack_w4(ops._ctx(words.device), words.data_ptr(), words.data_ptr(), words.numel(), to_canonical,
+                                     torch.cuda.current_stream().cuda_stream) == 0
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, PASS - 1, PASS + 1, 3 * PASS + 5, 4 * PASS, 4 * PASS + 1, 9 * PASS + 77])
+def test_interleaved_prepack(n):
+    """The even nibbles of a word in its low half, the odd ones in its high half; and back, also in place."""
+    words = torch.randint(-2 ** 31, 2 ** 31 - 1, (1, n), dtype=torch.int32, device="cuda")
+    want = torch.zeros(1, n, dtype=torch.int64, device="cuda")
+    for j in range(8):
+        want |= ((words.long() >> 4 * j) & 15) << (4 * (j // 2) + 16 * (j % 2))
+    out = qf.prepack_w4(words)
+    assert torch.equal(out.long() & 0xffffffff, want)
+    assert torch.equal(qf.prepack_w4(out, to_canonical=True), words)
+    _in_place(words, 0)
+    assert torch.equal(words, out)
+    _in_place(words, 1)
+    assert torch.equal(qf.prepack_w4(words), out)
+
+
+def test_loops_keep_several_loads_in_flight():
+    """A byte at a time takes 1.6 times the time of whole vectors and the interleaved prepack 1.2 times that of the tiled one;
+    with one load in flight per thread it is 3.6 and 1.8 times."""
+    n = 64 << 20
+    flat = torch.randint(-128, 128, (n + 16,), dtype=torch.int8, device="cuda")
+    odd, even = best_ms(lambda: qf.unpack_int4(flat[1:n + 1])), best_ms(lambda: qf.unpack_int4(flat[:n]))
+    assert odd < 2.1 * even
+    w = torch.randint(-128, 128, (28672, 4096), dtype=torch.int8, device="cuda")
+    inter, tiled = best_ms(lambda: qf.prepack_w4(w)), best_ms(lambda: qf.prepack_w4(w, layout=qf.QF_LAYOUT_TILED))
+    assert inter < 1.45 * tiled
