@@ -244,12 +244,15 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(
 }
 
 // Any group size that is a multiple of 4: a block per (row, group), two passes over the group (the second one reads it
-// from L1 or L2).
+// from L1 or L2). Only blocks of 256 threads let the next kernel in early: the GPU takes one such signal a nanosecond, and there is
+// one per block, so that in smaller blocks they were all the time (4096 x 4096 bf16 in groups of 64: 270.8 us instead of 137.6,
+// of 256: 68.4 instead of 37.0, of 512: 36.8 instead of 36.3; in groups of 4096 22.7 with the signal, 22.9 without).
 template <int DT, bool SYM>
 __global__ void __launch_bounds__(256) quantize_group_kernel(const void *w, int64_t N, int64_t K, int group,
                                                              uint32_t *codes, uint16_t *scales,
                                                              int scale_dtype, int8_t *zeros) {
-    griddep_begin();
+    if (blockDim.x == 256) griddep_launch_dependents();
+    griddep_wait();
     __shared__ float s_lo[8], s_hi[8];
     const int64_t G = K / group;
     const int64_t n = blockIdx.x / G, gi = blockIdx.x % G;

@@ -1,9 +1,10 @@
-"""The streaming kernels that loop: unpack of bytes at odd addresses and the interleaved prepack, at sizes around a pass of their
-loops, and that several of their loads are in flight at a time."""
+"""The streaming kernels that loop (unpack of bytes at odd addresses, the interleaved prepack) at sizes around a pass of their
+loops, and what keeps them and the quantise kernels at speed: loads in flight, signals to the next kernel, the right kernel."""
 import pytest
 import torch
 
 import quantforge_b200 as qf
+from quantforge_b200.quantize import quantize_w4
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +63,12 @@ def test_loops_keep_several_loads_in_flight():
     w = torch.randint(-128, 128, (28672, 4096), dtype=torch.int8, device="cuda")
     inter, tiled = best_ms(lambda: qf.prepack_w4(w)), best_ms(lambda: qf.prepack_w4(w, layout=qf.QF_LAYOUT_TILED))
     assert inter < 1.45 * tiled
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_small_groups_are_not_bound_by_their_blocks_signals(symmetric):
+    """Groups of 256, a block of 64 threads each, take about the time of groups of 1024 in blocks of 256; 1.8 times that when
+    every block signals the next kernel."""
+    w = (torch.randn(4096, 14336, device="cuda") * 0.02).to(torch.bfloat16)
+    small, large = (best_ms(lambda: quantize_w4(w, g, symmetric)) for g in (256, 1024))
+    assert small < 1.35 * large
