@@ -72,3 +72,24 @@ def test_small_groups_are_not_bound_by_their_blocks_signals(symmetric):
     w = (torch.randn(4096, 14336, device="cuda") * 0.02).to(torch.bfloat16)
     small, large = (best_ms(lambda: quantize_w4(w, g, symmetric)) for g in (256, 1024))
     assert small < 1.35 * large
+
+
+@pytest.mark.parametrize("N", [65535 * 16 - 1, 65535 * 16 + 1, 2 * 65535 * 16 + 33])
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_quantise_more_than_65535_blocks_of_rows(N, symmetric):
+    """The rows of a tall matrix, in groups of 128, are the rows of its parts."""
+    w = torch.randn(N, 128, device="cuda").mul_(0.02).to(torch.bfloat16)
+    codes, scales, zeros = quantize_w4(w, 128, symmetric)
+    for a, b in ((0, 500000), (500000, 65535 * 16 - 40), (65535 * 16 - 40, N)):
+        for c0 in range(a, b, 1000000):
+            c1 = min(b, c0 + 1000000)
+            c, s, z = quantize_w4(w[c0:c1], 128, symmetric)
+            assert torch.equal(codes[c0:c1], c) and torch.equal(scales[:, c0:c1], s)
+            assert symmetric or torch.equal(zeros[:, c0:c1], z)
+
+
+def test_tall_matrices_take_the_same_kernel():
+    """1.1 million rows take about as long a row as 1.0 million; a block per group took three times that."""
+    w = torch.randn(1100000, 128, device="cuda").mul_(0.02).to(torch.bfloat16)
+    tall, lower = best_ms(lambda: quantize_w4(w, 128)), best_ms(lambda: quantize_w4(w[:1000000], 128))
+    assert tall < 1.3 * lower
