@@ -212,7 +212,8 @@ int qf_w4a16_linear_host(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_
  * The same without the final wait: the copies and the kernel are enqueued on `stream` and the call returns.
  * Y_host holds the result once the caller has synchronised `stream`; X_host must stay unchanged until then.
  * Use page-locked host buffers (with pageable ones the copies block the host anyway): up to 2 MB each, 16-byte aligned, kernels
- * on `stream` read and write them in place. Otherwise (and in a graph capture) they are copied. Calls on one stream may be
+ * on `stream` read and write them in place. Otherwise they are copied. A capturing stream is refused (QF_ERR_UNSUPPORTED), and a
+ * call that is refused enqueues nothing. Calls on one stream may be
  * issued back to back: the context keeps two staging slots and copies the activations of a call on a stream of its
  * own, so that they cross PCIe while the previous call's kernel runs; results return on `stream`. The slot written by
  * call i+2 holds Y of call i until that call's copy back has been enqueued on `stream`, which stream order guarantees.

@@ -277,6 +277,39 @@ static int check_linear_args(qf_ctx *ctx, const qf_linear_desc *d, const void *X
     return QF_OK;
 }
 
+// Everything that a linear's launch relies on, and its plan. M == 0 needs no tensors.
+static int check_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, const void *qweight, const void *scales,
+                        const void *qzeros_or_null, const void *Y, const void *residual, const void *workspace,
+                        size_t workspace_bytes, Plan *plan) {
+    std::string why;
+    int st = make_plan(desc, plan, &why);
+    if (st != QF_OK) return fail(ctx, st, why);
+    if (desc->M == 0) return QF_OK;
+    st = check_linear_args(ctx, desc, X, qweight, scales, qzeros_or_null, Y);
+    if (st != QF_OK) return st;
+    st = check_current_device(ctx);
+    if (st != QF_OK) return st;
+    if (desc->epilogue == QF_EPI_RESIDUAL_ADD && (!residual || !aligned16(residual)))
+        return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_RESIDUAL_ADD needs a 16-byte aligned residual tensor");
+    if (desc->epilogue == QF_EPI_SILU_MUL && desc->N % 16 != 0)
+        return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_SILU_MUL needs N (gate and up rows together) to be a multiple of 16");
+    const size_t need = plan->ws_partial_bytes + plan->ws_counter_bytes;
+    if (need > 0) {
+        if (!workspace || workspace_bytes < need)
+            return fail(ctx, QF_ERR_WORKSPACE, "workspace smaller than qf_w4a16_workspace_bytes(desc)");
+        if (!aligned16(workspace)) return fail(ctx, QF_ERR_BAD_ARG, "workspace must be 16-byte aligned");
+    }
+    return QF_OK;
+}
+
+static int launch_linear(qf_ctx *ctx, const qf_linear_desc *desc, const Plan &plan, const void *X, const void *qweight,
+                         const void *scales, const void *qzeros_or_null, void *Y, const void *residual, void *workspace,
+                         cudaStream_t s) {
+    if (plan.slab) return launch_gemv_slab(ctx, desc, plan, X, qweight, Y, residual, workspace, s);
+    if (plan.path == QF_PATH_GEMV) return launch_gemv(ctx, desc, plan, X, qweight, scales, qzeros_or_null, Y, workspace, s);
+    return launch_gemm(ctx, desc, plan, X, qweight, scales, qzeros_or_null, Y, residual, workspace, s);
+}
+
 }  // namespace qf
 
 using namespace qf;
@@ -431,30 +464,9 @@ int qf_w4a16_linear_fused(qf_ctx *ctx, const qf_linear_desc *desc, const void *X
                           void *workspace, size_t workspace_bytes, void *stream) {
     if (!ctx) return QF_ERR_BAD_ARG;
     Plan plan;
-    std::string why;
-    int st = make_plan(desc, &plan, &why);
-    if (st != QF_OK) return fail(ctx, st, why);
-    if (desc->M == 0) return QF_OK;
-    st = check_linear_args(ctx, desc, X, qweight, scales, qzeros_or_null, Y);
-    if (st != QF_OK) return st;
-    st = check_current_device(ctx);
-    if (st != QF_OK) return st;
-    if (desc->epilogue == QF_EPI_RESIDUAL_ADD && (!residual || !aligned16(residual)))
-        return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_RESIDUAL_ADD needs a 16-byte aligned residual tensor");
-    if (desc->epilogue == QF_EPI_SILU_MUL && desc->N % 16 != 0)
-        return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_SILU_MUL needs N (gate and up rows together) to be a multiple of 16");
-    const size_t need = plan.ws_partial_bytes + plan.ws_counter_bytes;
-    if (need > 0) {
-        if (!workspace || workspace_bytes < need)
-            return fail(ctx, QF_ERR_WORKSPACE, "workspace smaller than qf_w4a16_workspace_bytes(desc)");
-        if (!aligned16(workspace)) return fail(ctx, QF_ERR_BAD_ARG, "workspace must be 16-byte aligned");
-    }
-    if (plan.slab)
-        return launch_gemv_slab(ctx, desc, plan, X, qweight, Y, residual, workspace, (cudaStream_t)stream);
-    if (plan.path == QF_PATH_GEMV)
-        return launch_gemv(ctx, desc, plan, X, qweight, scales, qzeros_or_null, Y, workspace, (cudaStream_t)stream);
-    return launch_gemm(ctx, desc, plan, X, qweight, scales, qzeros_or_null, Y, residual, workspace,
-                       (cudaStream_t)stream);
+    const int st = check_linear(ctx, desc, X, qweight, scales, qzeros_or_null, Y, residual, workspace, workspace_bytes, &plan);
+    if (st != QF_OK || desc->M == 0) return st;
+    return launch_linear(ctx, desc, plan, X, qweight, scales, qzeros_or_null, Y, residual, workspace, (cudaStream_t)stream);
 }
 
 int qf_w4a16_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, const void *qweight, const void *scales,
@@ -615,22 +627,28 @@ int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const vo
     if (!desc) return fail(ctx, QF_ERR_BAD_ARG, "desc is null");
     if (!X_host || !Y_host) return fail(ctx, QF_ERR_BAD_ARG, "null host pointer");
     if (desc->M == 0) return QF_OK;
-    if (desc->M < 0 || desc->N <= 0 || desc->K <= 0) return fail(ctx, QF_ERR_BAD_ARG, "bad shape");
-    int st = check_current_device(ctx);
+    if (desc->epilogue == QF_EPI_RESIDUAL_ADD)
+        return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_RESIDUAL_ADD takes its residual through qf_w4a16_linear_fused");
+    // Everything is checked before anything is allocated or enqueued. The linear's X and Y will be staging buffers or mapped
+    // addresses, aligned like this one.
+    alignas(16) static const char aligned[16] = {};
+    Plan plan;
+    int st = check_linear(ctx, desc, aligned, qweight, scales, qzeros_or_null, aligned, nullptr, workspace, workspace_bytes, &plan);
     if (st != QF_OK) return st;
+    cudaStream_t s = (cudaStream_t)stream;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();  // the launch says what is wrong with the stream
+    if (capture != cudaStreamCaptureStatusNone)
+        return fail(ctx, QF_ERR_UNSUPPORTED, "linears on host buffers cannot be captured");
     const size_t xb = (size_t)desc->M * desc->K * 2;
     const int64_t out_cols = desc->epilogue == QF_EPI_SILU_MUL ? desc->N / 2 : desc->N;
     const size_t yb = (size_t)desc->M * out_cols * (desc->out_dtype == QF_F32 ? 4 : 2);
-    if (xb <= kMappedX && yb <= kMappedY) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        void *x = nullptr, *y = nullptr;
-        if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
-            (x = mapped_host(X_host, xb)) != nullptr && (y = mapped_host(Y_host, yb)) != nullptr) {
-            if (!ctx->mapped_x) QF_CUDA_TRY(ctx, cudaMalloc(&ctx->mapped_x, kMappedX));
-            st = launch_fetch(ctx, x, ctx->mapped_x, (int64_t)xb, (cudaStream_t)stream);
-            if (st != QF_OK) return st;
-            return qf_w4a16_linear(ctx, desc, ctx->mapped_x, qweight, scales, qzeros_or_null, y, workspace, workspace_bytes, stream);
-        }
+    void *x = nullptr, *y = nullptr;
+    if (xb <= kMappedX && yb <= kMappedY && (x = mapped_host(X_host, xb)) != nullptr && (y = mapped_host(Y_host, yb)) != nullptr) {
+        if (!ctx->mapped_x) QF_CUDA_TRY(ctx, cudaMalloc(&ctx->mapped_x, kMappedX));
+        st = launch_fetch(ctx, x, ctx->mapped_x, (int64_t)xb, s);
+        if (st != QF_OK) return st;
+        return launch_linear(ctx, desc, plan, ctx->mapped_x, qweight, scales, qzeros_or_null, y, nullptr, workspace, s);
     }
     if (!ctx->copy_stream) {
         QF_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
@@ -645,13 +663,12 @@ int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const vo
     if (st != QF_OK) return st;
     st = grow(ctx, &sl.y, &sl.y_bytes, yb);
     if (st != QF_OK) return st;
-    cudaStream_t s = (cudaStream_t)stream;
     // activations: on the copy stream, as soon as the slot's previous kernel (two calls ago) has read its own
     QF_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->copy_stream, sl.kernel_done, 0));  // no-op before the first record
     QF_CUDA_TRY(ctx, cudaMemcpyAsync(sl.x, X_host, xb, cudaMemcpyHostToDevice, ctx->copy_stream));
     QF_CUDA_TRY(ctx, cudaEventRecord(sl.copied_in, ctx->copy_stream));
     QF_CUDA_TRY(ctx, cudaStreamWaitEvent(s, sl.copied_in, 0));
-    st = qf_w4a16_linear(ctx, desc, sl.x, qweight, scales, qzeros_or_null, sl.y, workspace, workspace_bytes, stream);
+    st = launch_linear(ctx, desc, plan, sl.x, qweight, scales, qzeros_or_null, sl.y, nullptr, workspace, s);
     if (st != QF_OK) return st;
     QF_CUDA_TRY(ctx, cudaEventRecord(sl.kernel_done, s));
     // the result goes back on the caller's stream: synchronising it is all the caller has to do

@@ -1,0 +1,86 @@
+"""What the linears on host buffers promise beside the result: nothing enqueued by a call that is refused, and order between calls
+of several streams, threads and buffers."""
+import ctypes
+
+import pytest
+import torch
+
+import quantforge_b200 as qf
+from quantforge_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(N, K, dtype=torch.float16, prepack=False, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    qw = torch.randint(-128, 128, (N, K // 2), dtype=torch.int8, device="cuda", generator=gen)
+    sc = (torch.randn(K // 128, N, device="cuda", generator=gen).abs() * 0.003).clamp_min(2.0 ** -14).to(dtype)
+    z = torch.randint(0, 16, (K // 128, N), dtype=torch.int8, device="cuda", generator=gen)
+    return qf.W4A16Linear(qw, sc, qf.pack_zeros_u4(z), prepack=prepack)
+
+
+def _c_call(d, x, qw, sc, z, y, ws, ws_bytes):
+    lib, ctx = _lib.load(), ops._ctx(qw.device)
+    st = lib.qf_w4a16_linear_host_async(ctx, ctypes.byref(d), x.data_ptr(), qw.data_ptr(), sc.data_ptr(), z.data_ptr(), y.data_ptr(),
+                                        ws.data_ptr() if ws is not None else 0, ws_bytes, torch.cuda.current_stream().cuda_stream)
+    return _lib.status_name(st)
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+def test_a_refused_call_enqueues_nothing(pinned):
+    lin = _layer(4096, 4096)
+    x, y = torch.randn(2, 4096).half(), torch.zeros(2, 4096, dtype=torch.float16)
+    if pinned:
+        x, y = x.pin_memory(), y.pin_memory()
+    lin.forward_host(x, y)
+    torch.cuda.synchronize()
+    y.zero_()
+
+    def desc(M=2, N=4096, K=4096):
+        return ops._make_desc(M, N, K, 128, torch.float16, torch.float16, lin.zeros, 8, 0, 0)
+
+    need = qf.workspace_bytes(desc())
+    assert need > 0
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    args = (x, lin.qweight, lin.scales, lin.zeros, y)
+    before = qf.launch_count()
+    assert _c_call(desc(), *args, ws, need - 1) == "QF_ERR_WORKSPACE"
+    assert _c_call(desc(), *args, None, 0) == "QF_ERR_WORKSPACE"
+    assert _c_call(desc(M=1, K=4), *args, ws, need) == "QF_ERR_BAD_ARG"  # eight bytes of activations
+    assert _c_call(desc(K=4096 - 64), *args, ws, need) == "QF_ERR_BAD_ARG"
+    d = desc()
+    d.epilogue = _lib.QF_EPI_RESIDUAL_ADD
+    assert _c_call(d, *args, ws, need) == "QF_ERR_BAD_ARG"
+    d = desc()
+    d.reserved[0] = 1
+    assert _c_call(d, *args, ws, need) == "QF_ERR_BAD_ARG"
+    torch.cuda.synchronize()
+    assert qf.launch_count() == before and not y.any()
+    assert _c_call(desc(), *args, ws, need) == "QF_OK"
+    torch.cuda.synchronize()
+    assert torch.equal(y, lin(x.cuda()).cpu())
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+def test_a_capture_refuses_and_goes_on(pinned):
+    """Host buffers are not part of a graph; the call says so and leaves the capture as it was."""
+    lin = _layer(512, 512)
+    x, y = torch.randn(2, 512).half(), torch.zeros(2, 512, dtype=torch.float16)
+    if pinned:
+        x, y = x.pin_memory(), y.pin_memory()
+    xd = x.cuda()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        lin.forward_host(x, y)
+        lin(xd)
+    want = y.clone()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        with pytest.raises(_lib.QuantForgeError):
+            lin.forward_host(x, y, wait=False)
+        out = lin(xd)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out.cpu(), want)
