@@ -622,9 +622,10 @@ class W4A16Linear:
     def forward_host(self, x_host: torch.Tensor, out_host: torch.Tensor, wait: bool = True) -> torch.Tensor:
         """Host activations in, host result out (both contiguous, ideally pinned), on the current stream of the
         weights' device, which must be the current device. Descriptor, workspace and weight pointers are prepared
-        once per (batch, dtypes), so that a serving loop pays for little more than the C call.
+        once per (batch, dtypes, stream), so that a serving loop pays for little more than the C call.
         wait=False: returns after enqueueing; out_host is valid once the stream has been synchronised."""
-        key = (x_host.shape[0], x_host.dtype, out_host.dtype)
+        stream = torch.cuda.current_stream(self.qweight.device).cuda_stream
+        key = (x_host.shape[0], x_host.dtype, out_host.dtype, stream)  # a workspace belongs to its stream
         prep = self._host_prep.get(key)
         if prep is None:
             if x_host.is_cuda or out_host.is_cuda:
@@ -638,13 +639,12 @@ class W4A16Linear:
             lib = _lib.load()
             prep = (d, ctypes.byref(d), _ctx(dev), _ptr(self.qweight), _ptr(self.scales), _ptr(self.zeros), _ptr(ws),
                     ws.numel() if ws is not None else 0, ws, (M, N), lib.qf_w4a16_linear_host,
-                    lib.qf_w4a16_linear_host_async, dev)
+                    lib.qf_w4a16_linear_host_async)
             self._host_prep[key] = prep
-        d, dref, ctx, pw, ps, pz, pws, wsn, _ws, shape, fn_wait, fn_async, dev = prep
+        d, dref, ctx, pw, ps, pz, pws, wsn, _ws, shape, fn_wait, fn_async = prep
         if tuple(out_host.shape) != shape or not out_host.is_contiguous() or not x_host.is_contiguous():
             raise ValueError("x_host and out_host must be contiguous and out_host of shape [M, N]")
-        st = (fn_wait if wait else fn_async)(ctx, dref, x_host.data_ptr(), pw, ps, pz, out_host.data_ptr(), pws, wsn,
-                                             torch.cuda.current_stream(dev).cuda_stream)
+        st = (fn_wait if wait else fn_async)(ctx, dref, x_host.data_ptr(), pw, ps, pz, out_host.data_ptr(), pws, wsn, stream)
         if st != 0:
             _check(st, ctx)
         return out_host

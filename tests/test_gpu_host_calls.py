@@ -84,3 +84,29 @@ def test_a_capture_refuses_and_goes_on(pinned):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out.cpu(), want)
+
+
+def test_each_stream_has_its_own_workspace(monkeypatch):
+    """A layer that was called on one stream and then on another passes each call the scratch of the stream it runs on: split sums
+    of device calls on the first stream may be under way."""
+    lin = _layer(4096, 4096)
+    x, y = torch.randn(2, 4096).half().pin_memory(), torch.empty(2, 4096, dtype=torch.float16, pin_memory=True)
+    real, passed = _lib.load().qf_w4a16_linear_host, []
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(_LIB, name)
+
+        def qf_w4a16_linear_host(self, *args):
+            passed.append((args[-1], args[7].value))
+            return real(*args)
+
+    _LIB = _lib.load()
+    monkeypatch.setattr(_lib, "load", Lib)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for s in streams * 2:
+        with torch.cuda.stream(s):
+            lin.forward_host(x, y)
+    assert len({stream for stream, _ in passed}) == 3 and len({ws for _, ws in passed}) == 3
+    for stream, ws in passed:
+        assert ws in {b.data_ptr() for b in ops._workspaces[(0, stream)]}
