@@ -622,10 +622,10 @@ class W4A16Linear:
     def forward_host(self, x_host: torch.Tensor, out_host: torch.Tensor, wait: bool = True) -> torch.Tensor:
         """Host activations in, host result out (both contiguous, ideally pinned), on the current stream of the
         weights' device, which must be the current device. Descriptor, workspace and weight pointers are prepared
-        once per (batch, dtypes, stream), so that a serving loop pays for little more than the C call.
+        once per (shape, dtypes, stream), so that a serving loop pays for little more than the C call.
         wait=False: returns after enqueueing; out_host is valid once the stream has been synchronised."""
         stream = torch.cuda.current_stream(self.qweight.device).cuda_stream
-        key = (x_host.shape[0], x_host.dtype, out_host.dtype, stream)  # a workspace belongs to its stream
+        key = (x_host.shape, x_host.dtype, out_host.dtype, stream)  # a workspace belongs to its stream
         prep = self._host_prep.get(key)
         if prep is None:
             if x_host.is_cuda or out_host.is_cuda:

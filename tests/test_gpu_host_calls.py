@@ -110,3 +110,11 @@ def test_each_stream_has_its_own_workspace(monkeypatch):
     assert len({stream for stream, _ in passed}) == 3 and len({ws for _, ws in passed}) == 3
     for stream, ws in passed:
         assert ws in {b.data_ptr() for b in ops._workspaces[(0, stream)]}
+
+
+def test_activations_of_another_width_are_refused():
+    lin = _layer(512, 512)
+    y = torch.empty(2, 512, dtype=torch.float16, pin_memory=True)
+    lin.forward_host(torch.randn(2, 512).half().pin_memory(), y)
+    with pytest.raises(ValueError):
+        lin.forward_host(torch.randn(2, 256).half().pin_memory(), y)
