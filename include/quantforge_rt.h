@@ -120,7 +120,8 @@ typedef struct qf_linear_desc {
 int qf_version(void);
 const char *qf_status_string(int status);
 
-/* One context per device. Owns only small caches (tensor maps, staging buffers of the *_host calls). */
+/* One context per device (and one per stream for *_host calls on several streams). Owns only small caches (tensor maps, staging
+ * buffers of the *_host calls). */
 int qf_ctx_create(qf_ctx **out, int device);
 int qf_ctx_destroy(qf_ctx *ctx);
 /* Message of the last error recorded on this context (never NULL). */
@@ -217,7 +218,8 @@ int qf_w4a16_linear_host(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_
  * issued back to back: the context keeps two staging slots and copies the activations of a call on a stream of its
  * own, so that they cross PCIe while the previous call's kernel runs; results return on `stream`. The slot written by
  * call i+2 holds Y of call i until that call's copy back has been enqueued on `stream`, which stream order guarantees.
- * Calls on different streams of one context must not overlap. Staging grows on first use of a larger shape
+ * Threads may call on one context and one stream at the same time. Calls on different streams of one context must not
+ * overlap: a stream that runs beside another needs a context of its own. Staging grows on first use of a larger shape
  * (a device allocation); outgrown buffers are released with the context.
  */
 int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_host, const void *qweight,

@@ -21,6 +21,7 @@ LIB_PATH = os.path.join(HERE, "lib", "libquantforge_rt.so")
 HOST_PATH = os.path.join(HERE, "lib", f"_qf_host.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
 
 QF_OK = 0
+QF_ERR_UNSUPPORTED = -2
 QF_F16, QF_BF16, QF_F32 = 0, 1, 2
 QF_ZERO_CONST, QF_ZERO_U4, QF_ZERO_I8 = 0, 1, 2
 QF_PATH_AUTO, QF_PATH_GEMV, QF_PATH_GEMM = 0, 1, 2

@@ -344,13 +344,13 @@ int qf_ctx_create(qf_ctx **out, int device) {
     qf_ctx *ctx = new (std::nothrow) qf_ctx();
     if (!ctx) return QF_ERR_CUDA;
     ctx->device = device;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) {
+    int major = 0;
+    if (cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess) {
         delete ctx;
         return QF_ERR_CUDA;
     }
-    ctx->sm_count = prop.multiProcessorCount;
-    if (prop.major != 10) {
+    if (major != 10) {
         delete ctx;
         return QF_ERR_UNSUPPORTED;  // built for sm_100a only
     }
@@ -624,6 +624,7 @@ int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const vo
                          const void *scales, const void *qzeros_or_null, void *Y_host, void *workspace,
                          size_t workspace_bytes, void *stream) {
     if (!ctx) return QF_ERR_BAD_ARG;
+    std::lock_guard<std::mutex> lock(ctx->host_mutex);
     if (!desc) return fail(ctx, QF_ERR_BAD_ARG, "desc is null");
     if (!X_host || !Y_host) return fail(ctx, QF_ERR_BAD_ARG, "null host pointer");
     if (desc->M == 0) return QF_OK;

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -26,10 +27,12 @@ struct qf_ctx {
     int device = 0;
     int sm_count = 148;
     std::string last_error;
-    // Staging for the *_host entry points: two slots used in turn, so that the activations of call i+1 cross PCIe (on
-    // the context's own copy stream) while the kernel of call i runs. Buffers only ever grow; a buffer that became
-    // too small is kept until the context is destroyed (kernels enqueued earlier may still use it, and freeing
-    // would synchronise the device in the middle of a hot call).
+    // Staging for the *_host entry points. Their calls on one context run in stream order (one stream, or streams that do not
+    // overlap); a thread holds the mutex while it enqueues one, so that no other call comes between its fetch and its linear.
+    // Two slots used in turn, so that the activations of call i+1 cross PCIe (on the context's own copy stream) while the
+    // kernel of call i runs. Buffers only ever grow; a buffer that became too small is kept until the context is destroyed
+    // (kernels enqueued earlier may still use it, and freeing would synchronise the device in the middle of a hot call).
+    std::mutex host_mutex;
     struct HostSlot {
         void *x = nullptr;
         size_t x_bytes = 0;
@@ -41,7 +44,8 @@ struct qf_ctx {
     HostSlot host_slot[2];
     int host_next = 0;
     cudaStream_t copy_stream = nullptr;
-    // Activations of calls with small page-locked host buffers, fetched by a kernel of the caller's stream.
+    // Activations of calls with small page-locked host buffers, fetched by a kernel of the caller's stream behind all that the
+    // stream ran before, the last linear that read them here included.
     void *mapped_x = nullptr;
     std::vector<void *> retired;  // outgrown staging buffers
     // device status word written by kernels whose bounded waits expire (tcgen05 path)

@@ -12,6 +12,7 @@ The hot operators first offer the call to the native host path (csrc/qf_host.cpp
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import Optional
 
 import torch
@@ -23,6 +24,8 @@ from ._lib import (QF_BF16, QF_EPI_NONE, QF_EPI_RESIDUAL_ADD, QF_EPI_SILU_MUL, Q
 
 _DT = {torch.float16: QF_F16, torch.bfloat16: QF_BF16, torch.float32: QF_F32}
 _ctxs: dict[int, ctypes.c_void_p] = {}
+_host_ctxs: dict[tuple[int, int], ctypes.c_void_p] = {}  # by device and stream
+_host_lock = threading.Lock()
 _workspaces: dict[tuple[int, int], list] = {}
 _fast = None  # the native host path, loaded on first use
 
@@ -34,19 +37,41 @@ def _native():
     return _fast
 
 
+def _new_ctx(idx: int) -> ctypes.c_void_p:
+    lib = _lib.load()
+    h = ctypes.c_void_p()
+    with torch.cuda.device(idx):
+        st = lib.qf_ctx_create(ctypes.byref(h), idx)
+    if st != 0:
+        raise QuantForgeError(st, _lib.status_name(st), f"qf_ctx_create(device={idx}) failed")
+    return h
+
+
 def _ctx(device: torch.device) -> ctypes.c_void_p:
     """The runtime context of `device` (created on first use; the caller's current device is left as it is)."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
     if idx not in _ctxs:
-        lib = _lib.load()
-        h = ctypes.c_void_p()
-        with torch.cuda.device(idx):
-            st = lib.qf_ctx_create(ctypes.byref(h), idx)
-        if st != 0:
-            raise QuantForgeError(st, _lib.status_name(st), f"qf_ctx_create(device={idx}) failed")
+        h = _new_ctx(idx)
         _ctxs[idx] = h
         _native().set_ctx(idx, h.value)
     return _ctxs[idx]
+
+
+def _host_ctx(device: torch.device, stream: int) -> ctypes.c_void_p:
+    """The context that holds the staging of host-buffer calls on `stream` of `device`. One per stream: calls on different
+    streams run side by side, and a context's staging is for one after the other."""
+    key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
+    h = _host_ctxs.get(key)
+    if h is None:
+        with torch.cuda.device(key[0]):
+            if torch.cuda.is_current_stream_capturing():  # the allocations of a new context would end the capture
+                raise QuantForgeError(_lib.QF_ERR_UNSUPPORTED, _lib.status_name(_lib.QF_ERR_UNSUPPORTED),
+                                      "linears on host buffers cannot be captured")
+        with _host_lock:
+            h = _host_ctxs.get(key)
+            if h is None:
+                h = _host_ctxs[key] = _new_ctx(key[0])
+    return h
 
 
 def _check(st: int, ctx) -> None:
@@ -491,8 +516,8 @@ def w4a16_linear_host(x_host: torch.Tensor, qweight: torch.Tensor, scales: torch
                       wait: bool = True) -> torch.Tensor:
     """Same linear with activations and result in HOST memory (pinned for speed); weights stay on the GPU.
 
-    wait=False enqueues the copies and the kernel on the current stream and returns at once: out_host is valid
-    after the stream has been synchronised (pinned buffers; x_host must not change until then)."""
+    wait=False enqueues the work on the current stream and returns at once: out_host is valid after the stream has been
+    synchronised (pinned buffers; x_host must not change until then). Streams and threads may call side by side."""
     if x_host.is_cuda:
         raise ValueError("x_host must be a CPU tensor")
     dev = _need_cuda(qweight, scales, zeros)
@@ -502,7 +527,7 @@ def w4a16_linear_host(x_host: torch.Tensor, qweight: torch.Tensor, scales: torch
     if out_host is None:
         out_host = torch.empty((M, N), dtype=out_dtype, pin_memory=True)
     d = _make_desc(M, N, K, group_size, x_host.dtype, out_dtype, zeros, zero_const, path, 0, weight_layout)
-    ctx = _ctx(dev)
+    ctx = _host_ctx(dev, torch.cuda.current_stream(dev).cuda_stream)
     with torch.cuda.device(dev):
         ws = _workspace(dev, workspace_bytes(d))
         fn = _lib.load().qf_w4a16_linear_host if wait else _lib.load().qf_w4a16_linear_host_async
@@ -565,16 +590,22 @@ def prepack_w4(qweight: torch.Tensor, to_canonical: bool = False, layout: int = 
     return out
 
 
+def _all_ctxs(dev: torch.device) -> list:
+    idx = dev.index if dev.index is not None else torch.cuda.current_device()
+    return [_ctx(dev)] + [c for (i, _), c in list(_host_ctxs.items()) if i == idx]
+
+
 def device_status(device: Optional[torch.device] = None) -> int:
-    """Sticky device-side status of the context (0, or QF_ERR_TIMEOUT after a bounded wait expired). Synchronises."""
+    """Sticky device-side status of the device's contexts (0, or QF_ERR_TIMEOUT after a bounded wait expired). Synchronises."""
     dev = device or torch.device("cuda", torch.cuda.current_device())
     torch.cuda.synchronize(dev)
-    return int(_lib.load().qf_ctx_status(_ctx(dev)))
+    return next((st for st in (int(_lib.load().qf_ctx_status(c)) for c in _all_ctxs(dev)) if st != 0), 0)
 
 
 def clear_device_status(device: Optional[torch.device] = None) -> None:
     dev = device or torch.device("cuda", torch.cuda.current_device())
-    _lib.load().qf_ctx_clear_status(_ctx(dev))
+    for c in _all_ctxs(dev):
+        _lib.load().qf_ctx_clear_status(c)
 
 
 def gemv_int4(x: torch.Tensor, w_packed: torch.Tensor, scale: torch.Tensor, zero_point: torch.Tensor) -> torch.Tensor:
@@ -623,7 +654,8 @@ class W4A16Linear:
         """Host activations in, host result out (both contiguous, ideally pinned), on the current stream of the
         weights' device, which must be the current device. Descriptor, workspace and weight pointers are prepared
         once per (shape, dtypes, stream), so that a serving loop pays for little more than the C call.
-        wait=False: returns after enqueueing; out_host is valid once the stream has been synchronised."""
+        wait=False: returns after enqueueing; out_host is valid once the stream has been synchronised. Streams and threads
+        may call side by side."""
         stream = torch.cuda.current_stream(self.qweight.device).cuda_stream
         key = (x_host.shape, x_host.dtype, out_host.dtype, stream)  # a workspace belongs to its stream
         prep = self._host_prep.get(key)
@@ -634,10 +666,11 @@ class W4A16Linear:
             M, N, K = _check_linear_tensors(x_host, self.qweight, self.scales, self.zeros, self.group_size)
             d = _make_desc(M, N, K, self.group_size, x_host.dtype, out_host.dtype, self.zeros, self.zero_const,
                            QF_PATH_AUTO, 0, self.weight_layout)
+            ctx = _host_ctx(dev, stream)
             with torch.cuda.device(dev):
                 ws = _workspace(dev, workspace_bytes(d))
             lib = _lib.load()
-            prep = (d, ctypes.byref(d), _ctx(dev), _ptr(self.qweight), _ptr(self.scales), _ptr(self.zeros), _ptr(ws),
+            prep = (d, ctypes.byref(d), ctx, _ptr(self.qweight), _ptr(self.scales), _ptr(self.zeros), _ptr(ws),
                     ws.numel() if ws is not None else 0, ws, (M, N), lib.qf_w4a16_linear_host,
                     lib.qf_w4a16_linear_host_async)
             self._host_prep[key] = prep

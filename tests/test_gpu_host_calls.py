@@ -1,6 +1,7 @@
 """What the linears on host buffers promise beside the result: nothing enqueued by a call that is refused, and order between calls
 of several streams, threads and buffers."""
 import ctypes
+import threading
 
 import pytest
 import torch
@@ -118,3 +119,86 @@ def test_activations_of_another_width_are_refused():
     lin.forward_host(torch.randn(2, 512).half().pin_memory(), y)
     with pytest.raises(ValueError):
         lin.forward_host(torch.randn(2, 256).half().pin_memory(), y)
+
+
+def _calls(lin, K, N, rows, pinned, seed):
+    """(activations, result, device call's result) of calls on `lin`, one per entry of `rows`."""
+    gen = torch.Generator().manual_seed(seed)
+    out = []
+    for m in rows:
+        x, y = torch.randn(m, K, generator=gen).half(), torch.empty(m, N, dtype=torch.float16)
+        out.append((x.pin_memory(), y.pin_memory()) if pinned else (x, y))
+    want = [lin(x.cuda()).cpu() for x, _ in out]
+    torch.cuda.synchronize()
+    return [(x, y, w) for (x, y), w in zip(out, want)]
+
+
+# few rows: fetched by a kernel; 1100 rows of 1024: copied; a mixture of both
+ROWS = {"fetched": [2, 16, 1, 64, 33, 5], "copied": [1100, 1300, 1024 + 9], "mixed": [2, 1100, 64, 1100, 7, 40]}
+
+
+@pytest.mark.parametrize("kind", sorted(ROWS))
+@pytest.mark.parametrize("order", ["abab", "aabb", "abbaab"])
+def test_streams_side_by_side(kind, order):
+    """One thread, two streams, a layer for each, no wait between the calls: everybody gets its own rows."""
+    K = N = 1024
+    lins = {c: _layer(N, K, prepack=True, seed=i) for i, c in enumerate("ab")}
+    streams = {c: torch.cuda.Stream() for c in "ab"}
+    calls = {c: _calls(lins[c], K, N, ROWS[kind] * 4, True, i) for i, c in enumerate("ab")}
+    todo = {c: list(calls[c]) for c in "ab"}
+    while todo["a"] or todo["b"]:
+        for c in order:
+            if todo[c]:
+                x, y, _ = todo[c].pop(0)
+                with torch.cuda.stream(streams[c]):
+                    lins[c].forward_host(x, y, wait=False)
+    torch.cuda.synchronize()
+    for c in "ab":
+        for _, y, want in calls[c]:
+            assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("kind", sorted(ROWS))
+@pytest.mark.parametrize("wait", [True, False])
+@pytest.mark.parametrize("own_streams", [False, True])
+def test_threads_side_by_side(kind, wait, own_streams):
+    """Four threads with a layer each, on streams of their own or all on the same one."""
+    K = N = 1024
+    lins = [_layer(N, K, prepack=True, seed=i) for i in range(4)]
+    calls = [_calls(lin, K, N, ROWS[kind] * 6, True, i) for i, lin in enumerate(lins)]
+    start, errors = threading.Barrier(4), []
+
+    def work(i):
+        try:
+            start.wait()
+            with torch.cuda.stream(torch.cuda.Stream() if own_streams else torch.cuda.default_stream()):
+                for x, y, _ in calls[i]:
+                    lins[i].forward_host(x, y, wait=wait)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    for per_layer in calls:
+        for _, y, want in per_layer:
+            assert torch.equal(y, want)
+
+
+def test_one_staging_for_each_stream():
+    """Calls on two streams go through contexts of their own, found again by the next call on the stream."""
+    lin = _layer(512, 512)
+    x, y = torch.randn(2, 512).half().pin_memory(), torch.empty(2, 512, dtype=torch.float16, pin_memory=True)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for s in streams * 2:
+        with torch.cuda.stream(s):
+            lin.forward_host(x, y)
+            qf.w4a16_linear_host(x, lin.qweight, lin.scales, lin.zeros, out_host=y)
+    ctxs = [ops._host_ctxs[(0, s.cuda_stream)].value for s in streams]
+    assert len(set(ctxs)) == 2 and ops._ctx(lin.qweight.device).value not in ctxs
+    assert {prep[2].value for prep in lin._host_prep.values()} == set(ctxs)
+    assert qf.device_status() == 0
