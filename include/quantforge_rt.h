@@ -211,7 +211,9 @@ int qf_w4a16_linear_host(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_
                          size_t workspace_bytes, void *stream);
 /*
  * The same without the final wait: the copies and the kernel are enqueued on `stream` and the call returns.
- * Y_host holds the result once the caller has synchronised `stream`; X_host must stay unchanged until then.
+ * Y_host holds the result once the caller has synchronised `stream`; X_host must stay unchanged until then. X_host is read
+ * beside earlier work of the stream: it holds its values when the call is made, or is (part of) the Y_host of an earlier call on
+ * the same context, which is waited for; other work that writes it has to be waited for by the caller.
  * Use page-locked host buffers (with pageable ones the copies block the host anyway): up to 2 MB each, 16-byte aligned, kernels
  * on `stream` read and write them in place. Otherwise they are copied. A capturing stream is refused (QF_ERR_UNSUPPORTED), and a
  * call that is refused enqueues nothing. Calls on one stream may be

@@ -377,6 +377,7 @@ int qf_ctx_destroy(qf_ctx *ctx) {
     }
     if (ctx->mapped_x) cudaFree(ctx->mapped_x);
     for (void *q : ctx->retired) cudaFree(q);
+    if (ctx->order) cudaEventDestroy(ctx->order);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->host_status) cudaFreeHost(ctx->host_status);
     delete ctx;
@@ -620,9 +621,39 @@ static void *mapped_host(const void *p, size_t bytes) {
     return (void *)(uintptr_t)dev;
 }
 
-int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_host, const void *qweight,
-                         const void *scales, const void *qzeros_or_null, void *Y_host, void *workspace,
-                         size_t workspace_bytes, void *stream) {
+// Puts the copy stream behind all that `s` holds so far: no result is pending for its copies any more.
+static int order_copies(qf_ctx *ctx, cudaStream_t s) {
+    if (ctx->copy_stream) {
+        QF_CUDA_TRY(ctx, cudaEventRecord(ctx->order, s));
+        QF_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->order, 0));
+    }
+    ctx->n_pending = 0;
+    return QF_OK;
+}
+
+static bool pending(const qf_ctx *ctx, const qf_ctx::HostRange &x) {
+    for (int i = 0; i < ctx->n_pending; ++i)
+        if (x.meets(ctx->pending_y[i])) return true;
+    return false;
+}
+
+// After a call has been enqueued; one that waits leaves nothing pending.
+static int note_result(qf_ctx *ctx, const qf_ctx::HostRange &y, bool waits, cudaStream_t s) {
+    ctx->last_y = waits ? qf_ctx::HostRange{0, 0} : y;
+    if (waits) return QF_OK;
+    for (int i = 0; i < ctx->n_pending; ++i)
+        if (ctx->pending_y[i].begin <= y.begin && y.end <= ctx->pending_y[i].end) return QF_OK;
+    if (ctx->n_pending == qf_ctx::kMaxPending) {
+        const int st = order_copies(ctx, s);
+        if (st != QF_OK) return st;
+    }
+    ctx->pending_y[ctx->n_pending++] = y;
+    return QF_OK;
+}
+
+static int enqueue_host_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_host, const void *qweight,
+                               const void *scales, const void *qzeros_or_null, void *Y_host, void *workspace,
+                               size_t workspace_bytes, void *stream, bool waits) {
     if (!ctx) return QF_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lock(ctx->host_mutex);
     if (!desc) return fail(ctx, QF_ERR_BAD_ARG, "desc is null");
@@ -644,19 +675,27 @@ int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const vo
     const size_t xb = (size_t)desc->M * desc->K * 2;
     const int64_t out_cols = desc->epilogue == QF_EPI_SILU_MUL ? desc->N / 2 : desc->N;
     const size_t yb = (size_t)desc->M * out_cols * (desc->out_dtype == QF_F32 ? 4 : 2);
+    const qf_ctx::HostRange x_range = {(uintptr_t)X_host, (uintptr_t)X_host + xb}, y_range = {(uintptr_t)Y_host, (uintptr_t)Y_host + yb};
     void *x = nullptr, *y = nullptr;
     if (xb <= kMappedX && yb <= kMappedY && (x = mapped_host(X_host, xb)) != nullptr && (y = mapped_host(Y_host, yb)) != nullptr) {
         if (!ctx->mapped_x) QF_CUDA_TRY(ctx, cudaMalloc(&ctx->mapped_x, kMappedX));
-        st = launch_fetch(ctx, x, ctx->mapped_x, (int64_t)xb, s);
+        st = launch_fetch(ctx, x, ctx->mapped_x, (int64_t)xb, x_range.meets(ctx->last_y), s);
         if (st != QF_OK) return st;
-        return launch_linear(ctx, desc, plan, ctx->mapped_x, qweight, scales, qzeros_or_null, y, nullptr, workspace, s);
+        st = launch_linear(ctx, desc, plan, ctx->mapped_x, qweight, scales, qzeros_or_null, y, nullptr, workspace, s);
+        return st != QF_OK ? st : note_result(ctx, y_range, waits, s);
     }
-    if (!ctx->copy_stream) {
+    const bool first = !ctx->copy_stream;
+    if (first) {
+        QF_CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->order, cudaEventDisableTiming));
         QF_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
         for (auto &sl : ctx->host_slot) {
             QF_CUDA_TRY(ctx, cudaEventCreateWithFlags(&sl.copied_in, cudaEventDisableTiming));
             QF_CUDA_TRY(ctx, cudaEventCreateWithFlags(&sl.kernel_done, cudaEventDisableTiming));
         }
+    }
+    if (first || pending(ctx, x_range)) {
+        st = order_copies(ctx, s);
+        if (st != QF_OK) return st;
     }
     qf_ctx::HostSlot &sl = ctx->host_slot[ctx->host_next];
     ctx->host_next ^= 1;
@@ -674,14 +713,21 @@ int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const vo
     QF_CUDA_TRY(ctx, cudaEventRecord(sl.kernel_done, s));
     // the result goes back on the caller's stream: synchronising it is all the caller has to do
     QF_CUDA_TRY(ctx, cudaMemcpyAsync(Y_host, sl.y, yb, cudaMemcpyDeviceToHost, s));
-    return QF_OK;
+    return note_result(ctx, y_range, waits, s);
+}
+
+int qf_w4a16_linear_host_async(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_host, const void *qweight,
+                         const void *scales, const void *qzeros_or_null, void *Y_host, void *workspace,
+                         size_t workspace_bytes, void *stream) {
+    return enqueue_host_linear(ctx, desc, X_host, qweight, scales, qzeros_or_null, Y_host, workspace, workspace_bytes, stream,
+                               false);
 }
 
 int qf_w4a16_linear_host(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_host, const void *qweight,
                          const void *scales, const void *qzeros_or_null, void *Y_host, void *workspace,
                          size_t workspace_bytes, void *stream) {
-    const int st = qf_w4a16_linear_host_async(ctx, desc, X_host, qweight, scales, qzeros_or_null, Y_host, workspace,
-                                              workspace_bytes, stream);
+    const int st = enqueue_host_linear(ctx, desc, X_host, qweight, scales, qzeros_or_null, Y_host, workspace, workspace_bytes,
+                                       stream, true);
     if (st != QF_OK) return st;
     QF_CUDA_TRY(ctx, cudaStreamSynchronize((cudaStream_t)stream));
     return QF_OK;

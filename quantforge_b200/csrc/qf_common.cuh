@@ -44,6 +44,18 @@ struct qf_ctx {
     HostSlot host_slot[2];
     int host_next = 0;
     cudaStream_t copy_stream = nullptr;
+    // Results of calls that did not wait may still be on their way to the host when a later call takes one as its activations. The
+    // copy stream may run before any of those that have come since it was last put behind the caller's stream; a fetch, which is
+    // on the caller's stream, only beside the last one: a linear lets its successor in when all before it is complete.
+    struct HostRange {
+        uintptr_t begin, end;
+        bool meets(const HostRange &o) const { return begin < o.end && o.begin < end; }
+    };
+    static constexpr int kMaxPending = 16;
+    HostRange pending_y[kMaxPending];
+    int n_pending = 0;
+    HostRange last_y = {0, 0};
+    cudaEvent_t order = nullptr;
     // Activations of calls with small page-locked host buffers, fetched by a kernel of the caller's stream behind all that the
     // stream ran before, the last linear that read them here included.
     void *mapped_x = nullptr;
@@ -230,7 +242,7 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why);
 
 // kernels (defined in their own translation units)
 int launch_unpack(qf_ctx *ctx, const void *packed, void *out, int64_t rows, int64_t packed_cols, cudaStream_t s);
-int launch_fetch(qf_ctx *ctx, const void *src, void *dst, int64_t bytes, cudaStream_t s);
+int launch_fetch(qf_ctx *ctx, const void *src, void *dst, int64_t bytes, bool behind, cudaStream_t s);
 int launch_pack(qf_ctx *ctx, const void *codes, void *out, int64_t n_bytes, cudaStream_t s);
 int launch_quantize(qf_ctx *ctx, const void *w, int dtype, int64_t N, int64_t K, int group, bool symmetric, void *codes,
                     void *scales, int scale_dtype, void *zeros, cudaStream_t s);

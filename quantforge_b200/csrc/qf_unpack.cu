@@ -128,22 +128,23 @@ int launch_unpack(qf_ctx *ctx, const void *packed, void *out, int64_t rows, int6
 }
 
 // Mapped host memory to device memory, 16 bytes per thread. Bound by the round trip over PCIe for a few rows of activations, then
-// by its bandwidth. The source is the caller's and stays as it is until the stream has been synchronised, so its way begins
-// before earlier work of the stream has ended; the destination is written behind the wait. (14336 -> 4096, 8 rows, calls back to
-// back: 17.4 us; 30.7 with the read behind the wait.)
-__global__ void __launch_bounds__(256) fetch_kernel(const uint4 *src, uint4 *dst, int64_t n_vec) {
+// by its bandwidth. The source is the caller's and final when the call is made, so its way begins before earlier work of the stream
+// has ended; the destination is written behind the wait. (14336 -> 4096, 8 rows, calls back to back: 17.4 us; 30.7 with the read
+// behind the wait.) Where it is the result of an earlier call (`behind`), the linear that writes it may be running: read behind the wait.
+__global__ void __launch_bounds__(256) fetch_kernel(const uint4 *src, uint4 *dst, int64_t n_vec, int behind) {
     griddep_launch_dependents();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (behind) griddep_wait();
     if (i < n_vec) v = ld_stream16(src + i);
-    griddep_wait();
+    if (!behind) griddep_wait();
     if (i < n_vec) dst[i] = v;
 }
 
-int launch_fetch(qf_ctx *ctx, const void *src, void *dst, int64_t bytes, cudaStream_t s) {
+int launch_fetch(qf_ctx *ctx, const void *src, void *dst, int64_t bytes, bool behind, cudaStream_t s) {
     const int64_t n_vec = bytes / 16;
     return launched(ctx, launch_kernel(fetch_kernel, dim3((unsigned)((n_vec + 255) / 256)), dim3(256), 0, s, pdl_enabled(),
-                                       (const uint4 *)src, (uint4 *)dst, n_vec),
+                                       (const uint4 *)src, (uint4 *)dst, n_vec, behind ? 1 : 0),
                     "fetch");
 }
 

@@ -517,7 +517,8 @@ def w4a16_linear_host(x_host: torch.Tensor, qweight: torch.Tensor, scales: torch
     """Same linear with activations and result in HOST memory (pinned for speed); weights stay on the GPU.
 
     wait=False enqueues the work on the current stream and returns at once: out_host is valid after the stream has been
-    synchronised (pinned buffers; x_host must not change until then). Streams and threads may call side by side."""
+    synchronised (pinned buffers; x_host must not change until then). x_host holds its values when the call is made or is the
+    out_host of an earlier call on the stream. Streams and threads may call side by side."""
     if x_host.is_cuda:
         raise ValueError("x_host must be a CPU tensor")
     dev = _need_cuda(qweight, scales, zeros)
@@ -654,8 +655,8 @@ class W4A16Linear:
         """Host activations in, host result out (both contiguous, ideally pinned), on the current stream of the
         weights' device, which must be the current device. Descriptor, workspace and weight pointers are prepared
         once per (shape, dtypes, stream), so that a serving loop pays for little more than the C call.
-        wait=False: returns after enqueueing; out_host is valid once the stream has been synchronised. Streams and threads
-        may call side by side."""
+        wait=False: returns after enqueueing; out_host is valid once the stream has been synchronised. x_host holds its values
+        when the call is made or is the out_host of an earlier call on the stream. Streams and threads may call side by side."""
         stream = torch.cuda.current_stream(self.qweight.device).cuda_stream
         key = (x_host.shape, x_host.dtype, out_host.dtype, stream)  # a workspace belongs to its stream
         prep = self._host_prep.get(key)

@@ -202,3 +202,39 @@ def test_one_staging_for_each_stream():
     assert len(set(ctxs)) == 2 and ops._ctx(lin.qweight.device).value not in ctxs
     assert {prep[2].value for prep in lin._host_prep.values()} == set(ctxs)
     assert qf.device_status() == 0
+
+
+# rows of the chain's layers; "mixed": the second layer takes a part of what the first one wrote
+@pytest.mark.parametrize("rows", [(4, 4, 4), (64, 64, 64), (1100, 1100, 1100), (1100, 1000, 17), (40, 1100, 1100)])
+@pytest.mark.parametrize("in_front", [False, True])
+def test_the_result_of_one_call_is_the_activations_of_the_next(rows, in_front):
+    """Without a wait in between, page-locked: fetched, copied, and from one to the other. Behind work that keeps the GPU busy, and
+    with more results pending than the context keeps a list of."""
+    K = N = 1024
+    lins = [_layer(N, K, prepack=True, seed=i) for i in range(3)]
+    big = max(rows)
+    busy = _layer(8192, 8192, prepack=True, seed=9)
+    gen = torch.Generator().manual_seed(sum(rows))
+    runs = []
+    for _ in range(7):
+        bufs = [torch.zeros(big, N, dtype=torch.float16, pin_memory=True) for _ in range(4)]
+        bufs[0].copy_(torch.randn(big, K, generator=gen))
+        want = [bufs[0].clone()] + [b.clone() for b in bufs[1:]]
+        for i, m in enumerate(rows):
+            want[i + 1][:m] = lins[i](want[i][:m].cuda()).cpu()
+        runs.append((bufs, want))
+    xb = torch.randn(256, 8192, device="cuda").half()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for bufs, _ in runs:
+            for b in bufs[1:]:
+                b.zero_()
+        for bufs, _ in runs:
+            if in_front:
+                busy(xb)
+            for i, m in enumerate(rows):
+                lins[i].forward_host(bufs[i][:m], bufs[i + 1][:m], wait=False)
+        torch.cuda.synchronize()
+        for bufs, want in runs:
+            for i, m in enumerate(rows):
+                assert torch.equal(bufs[i + 1][:m], want[i + 1][:m])
