@@ -579,13 +579,22 @@ int qf_w4a16_gemv_static_scratch(qf_ctx *ctx, const qf_linear_desc *desc, const 
 
 // Page-locked host buffers up to these sizes: a kernel of the caller's stream fetches the activations and the linear writes its
 // result to the host, two launches one behind the other instead of two copies, a second stream and three events. The copy
-// engine moves larger ones, on a stream of its own. Measured, waiting for each call / calls back to back, before -> now:
-//   2 rows 4096 -> 14336 (16 and 57 KB)       39.1 -> 35.7 us / 25.1 -> 16.5
-//   64 rows 512 -> 512 (64 and 64 KB)         35.4 -> 27.7    / 18.2 -> 10.8
-//   64 rows 4096 -> 14336 (0.5 and 1.8 MB)    90.8 -> 77.3    / 75.9 -> 49.7
-//   64 rows 14336 -> 4096 (1.8 and 0.5 MB)    85.1 -> 77.2    / 53.0 -> 50.6
+// engine moves larger ones, on a stream of its own. Measured on weights not in L2, waiting for each call / calls back to back,
+// copied -> fetched:
+//   2 rows 4096 -> 14336 (16 and 57 KB)       48.3 -> 40.3 us / 36.1 -> 24.3
+//   64 rows 512 -> 512 (64 and 64 KB)         35.0 -> 25.0    / 17.2 -> 10.2
+//   16 rows 4096 -> 4112 fp32 (128, 257 KB)   49.1 -> 38.5    / 27.6 -> 19.9  (GEMV kernel: four bytes a thread)
+//   64 rows 4096 -> 14336 (0.5 and 1.8 MB)    87.0 -> 75.6    / 68.5 -> 49.9
+//   256 rows 4096 -> 4096 (2 and 2 MB)         135 -> 113     / 89.6 -> 80.8
+//   64 rows 14336 -> 4096 (1.8 and 0.5 MB)    85.9 -> 77.0    / 56.4 -> 57.7
+//   73 rows 14336 -> 512 (2 and 0.07 MB)      90.9 -> 81.8    / 46.4 -> 57.1  (long K, small result: the one loss seen below 2 MB)
 //   128 rows 4096 -> 14336 (1 and 3.7 MB)      155 -> 128     /  100 -> 114
-constexpr size_t kMappedX = 2u << 20, kMappedY = 2u << 20;
+// The tcgen05 kernel without a split stores fp32 results as half sectors, 32 bytes a thread in two pieces, which PCIe takes at
+// 15 GB/s; these go to the host up to 192 KB:
+//   64 rows 512 -> 512 fp32 (64 and 128 KB)   35.0 -> 30.0    / 23.0 -> 15.0
+//   128 rows 512 -> 512 fp32 (128, 256 KB)    43.0 -> 45.5    / 23.2 -> 25.2
+//   1000 rows 512 -> 512 fp32 (1 and 2 MB)    93.2 -> 180     / 62.3 -> 156
+constexpr size_t kMappedX = 2u << 20, kMappedY = 2u << 20, kMappedHalfSectors = 192u << 10;
 
 // Staging buffers only grow; the outgrown one is retired, not freed (see qf_ctx::HostSlot).
 static int grow(qf_ctx *ctx, void **buf, size_t *have, size_t need) {
@@ -677,7 +686,9 @@ static int enqueue_host_linear(qf_ctx *ctx, const qf_linear_desc *desc, const vo
     const size_t yb = (size_t)desc->M * out_cols * (desc->out_dtype == QF_F32 ? 4 : 2);
     const qf_ctx::HostRange x_range = {(uintptr_t)X_host, (uintptr_t)X_host + xb}, y_range = {(uintptr_t)Y_host, (uintptr_t)Y_host + yb};
     void *x = nullptr, *y = nullptr;
-    if (xb <= kMappedX && yb <= kMappedY && (x = mapped_host(X_host, xb)) != nullptr && (y = mapped_host(Y_host, yb)) != nullptr) {
+    const bool half_sectors = plan.path == QF_PATH_GEMM && plan.split_k == 1 && desc->out_dtype == QF_F32;
+    if (xb <= kMappedX && yb <= (half_sectors ? kMappedHalfSectors : kMappedY) &&
+        (x = mapped_host(X_host, xb)) != nullptr && (y = mapped_host(Y_host, yb)) != nullptr) {
         if (!ctx->mapped_x) QF_CUDA_TRY(ctx, cudaMalloc(&ctx->mapped_x, kMappedX));
         st = launch_fetch(ctx, x, ctx->mapped_x, (int64_t)xb, x_range.meets(ctx->last_y), s);
         if (st != QF_OK) return st;

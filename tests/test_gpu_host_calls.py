@@ -238,3 +238,32 @@ def test_the_result_of_one_call_is_the_activations_of_the_next(rows, in_front):
         for bufs, want in runs:
             for i, m in enumerate(rows):
                 assert torch.equal(bufs[i + 1][:m], want[i + 1][:m])
+
+
+# M, K, N, tiled weights, fp32 result, way: page-locked and aligned
+WAYS = [(1, 512, 512, False, False, "fetched"), (2, 4096, 4096, False, True, "fetched"), (64, 512, 512, True, False, "fetched"),
+        (256, 4096, 4096, True, False, "fetched"), (257, 4096, 4096, True, False, "copied"), (80, 512, 14336, True, False, "copied"),
+        (64, 4096, 8192, True, True, "fetched"), (64, 4096, 8192 + 128, True, True, "copied"),
+        # fp32 from the tcgen05 kernel: without a split up to 192 KB
+        (96, 512, 512, True, True, "fetched"), (97, 512, 512, True, True, "copied"), (1000, 512, 512, True, True, "copied"),
+        (1000, 512, 512, True, False, "fetched"), (256, 4096, 2048, True, True, "fetched")]
+
+
+@pytest.mark.parametrize("M,K,N,prepack,wide,way", WAYS)
+def test_which_way(M, K, N, prepack, wide, way):
+    """A fetched call is one launch more than a copied one; pageable and unaligned buffers are copied whatever their size."""
+    lin = _layer(N, K, prepack=prepack)
+    out = torch.float32 if wide else torch.float16
+    x = torch.randn(M * K + 8).half()
+    want = lin(x[:M * K].view(M, K).cuda(), out_dtype=out).cpu()
+    xp, yp = x.pin_memory(), torch.empty(M * N + 8, dtype=out, pin_memory=True)
+    xu = torch.empty(M * K + 8, dtype=torch.float16, pin_memory=True)
+    xu[1:1 + M * K] = x[:M * K]
+    y = yp[:M * N].view(M, N)
+    lin.forward_host(xp[:M * K].view(M, K), y)
+    for xh, yh, expected in [(xp[:M * K], yp[:M * N], way), (x[:M * K], yp[:M * N], "copied"), (xp[:M * K], torch.empty(M * N, dtype=out), "copied"),
+                             (xu[1:1 + M * K], yp[:M * N], "copied"), (xp[:M * K], yp[1:1 + M * N], "copied")]:
+        before = qf.launch_count()
+        lin.forward_host(xh.view(M, K), yh.view(M, N))
+        assert qf.launch_count() - before == (2 if expected == "fetched" else 1)
+        assert torch.equal(yh.view(M, N), want)
