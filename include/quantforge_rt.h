@@ -133,8 +133,8 @@ const char *qf_last_error(const qf_ctx *ctx);
  * python/quantforge/baseline.py:34-49 `unpack_int4`).
  * packed int8[rows, packed_cols] -> out int8[rows, 2*packed_cols]:
  * out[r, 2i] = b & 0xF, out[r, 2i+1] = (b >>logical 4) & 0xF.  Bit-exact.
- * Alignment: `packed` any, `out` 2 bytes. With `packed` and `out` 16-byte aligned whole vectors are moved (`out` to 32 bytes:
- * 10 % faster still), otherwise a byte per thread (1.6 times the time).
+ * Alignment: `packed` any, `out` 2 bytes. With `packed` and `out` 16-byte aligned whole vectors are moved, otherwise a byte per thread
+ * (64 MB: 32.7 us with `out` aligned to 32 bytes, 41.3 to 16, 57.2 a byte per thread).
  */
 int qf_unpack_int4(qf_ctx *ctx, const void *packed_i8, void *out_i8, int64_t rows, int64_t packed_cols, void *stream);
 
@@ -202,24 +202,24 @@ int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs,
 
 /*
  * The same linear for callers that hold activations in HOST memory (the reference's Python entry
- * point takes CPU tensors when no GPU is used): copies X_host to the device, runs the kernel,
- * copies Y back and waits.  Weights, scales and zeros stay DEVICE pointers (they are loaded once).
- * Staging buffers live in the context and grow on first use; workspace as above.
+ * point takes CPU tensors when no GPU is used): brings X_host to the device, runs the kernel,
+ * brings Y back and waits, by the ways of the call below.  Weights, scales and zeros stay DEVICE pointers (they are loaded
+ * once).  Staging buffers live in the context and grow on first use; workspace as above.
  */
 int qf_w4a16_linear_host(qf_ctx *ctx, const qf_linear_desc *desc, const void *X_host, const void *qweight,
                          const void *scales, const void *qzeros_or_null, void *Y_host, void *workspace,
                          size_t workspace_bytes, void *stream);
 /*
- * The same without the final wait: the copies and the kernel are enqueued on `stream` and the call returns.
+ * The same without the final wait: the work is enqueued on `stream` and the call returns.
  * Y_host holds the result once the caller has synchronised `stream`; X_host must stay unchanged until then. X_host is read
  * beside earlier work of the stream: it holds its values when the call is made, or is (part of) the Y_host of an earlier call on
  * the same context, which is waited for; other work that writes it has to be waited for by the caller.
- * Use page-locked host buffers (with pageable ones the copies block the host anyway): up to 2 MB each, 16-byte aligned, kernels
- * on `stream` read and write them in place. Otherwise they are copied. A capturing stream is refused (QF_ERR_UNSUPPORTED), and a
- * call that is refused enqueues nothing. Calls on one stream may be
- * issued back to back: the context keeps two staging slots and copies the activations of a call on a stream of its
- * own, so that they cross PCIe while the previous call's kernel runs; results return on `stream`. The slot written by
- * call i+2 holds Y of call i until that call's copy back has been enqueued on `stream`, which stream order guarantees.
+ * Use page-locked host buffers (with pageable ones the copies block the host anyway). Both up to 2 MB (fp32 results of unsplit
+ * tcgen05 tiles: 192 KB) and 16-byte aligned: a kernel on `stream` fetches X_host into the context, where it stays until that
+ * stream's next such call, and the linear stores to Y_host. Otherwise they are copied: the context keeps two staging slots used
+ * in turn and copies the activations on a stream of its own, so that they cross PCIe while the previous call's kernel runs;
+ * results return on `stream`, which orders the copy back of a slot before the slot's next kernel. Calls on one stream may be
+ * issued back to back. A capturing stream is refused (QF_ERR_UNSUPPORTED), and a call that is refused enqueues nothing.
  * Threads may call on one context and one stream at the same time. Calls on different streams of one context must not
  * overlap: a stream that runs beside another needs a context of its own. Staging grows on first use of a larger shape
  * (a device allocation); outgrown buffers are released with the context.

@@ -299,10 +299,13 @@ __device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 // First statement of the streaming kernels (unpack, dequant, quantise, the packs and prepacks): the next kernel's blocks take the
 // slots that this one leaves free, and nothing is read or written before the previous one is complete. What is saved is the way
-// from the end of a kernel to the first blocks of the next, 2 us a launch: unpack 28672 x 4096 56.9 -> 54.6 us, dequant
-// 14336 x 4096 27.9 -> 25.3, quantise, two packs and slab prepack of 4096 x 4096 32.8 -> 25.6. Such a kernel may be running while
-// its inputs are still being written, so it reads them with ordinary loads: the read-only path (ld.global.nc, and what the
-// compiler makes of const __restrict__) promises that nobody writes them during the kernel.
+// from the end of a kernel to the first blocks of the next, 2 us a launch between two kernels of this library (behind others,
+// which signal nothing before they end, nothing is saved): calls back to back, unpack 28672 x 4096 56.9 -> 54.6 us, dequant
+// 14336 x 4096 27.9 -> 25.3, quantise, two packs and slab prepack of 4096 x 4096 32.8 -> 25.6. The GPU takes one block's signal a
+// nanosecond: a kernel of many small blocks does without (quantize_group_kernel). A kernel that starts behind these, the
+// linears included, may be running while its inputs are still being written, so it reads them with ordinary loads: the read-only
+// path (ld.global.nc, and what the compiler makes of const __restrict__) promises that nobody writes them during the kernel. Nor does
+// it say __restrict__ elsewhere, so the compiler moves no load ahead of a store: loops write several loads ahead.
 __device__ __forceinline__ void griddep_begin() {
     griddep_launch_dependents();
     griddep_wait();

@@ -152,7 +152,9 @@ __device__ __forceinline__ void codes16(const float (&v)[16], float wmax, const 
 // 16 rows of four groups, so that scales [G, N] leave as whole sectors; all its loads are in flight before the first is used.
 // (32 rows with half of the loads ahead: 1.7 waves for 4096 x 4096. Alone, on weights not in L2, bf16 asymmetric / f16 symmetric:
 // 15.9 / 12.2 -> 13.7 / 10.1 us, 14336 x 4096 47.1 / 36.0 -> 40.8 / 31.3; all bytes at the copy rate 7.7 and 27.) Five blocks of
-// 48 registers per SM for 16-bit weights; fp32 ones need the registers (four blocks 13.3 us, five 14.4).
+// 48 registers per SM for 16-bit weights, for which the asymmetric forms spill ten bytes; fp32 ones need the registers (four blocks
+// 13.3 us, five 14.4). The steps from 32 rows to this (16 rows, loads ahead, two fp32 values per instruction, extremes in one word,
+// zero point by reciprocal) were measured together only.
 // With a group per warp the kernel was bound by issue slots (25.2 us for 4096 x 4096 bf16).
 constexpr int QUANT_PASSES = 2;  // rows a warp works on
 template <int DT, bool SYM, bool TALL>

@@ -35,7 +35,7 @@ __device__ __forceinline__ void unpack_word(uint32_t w, uint32_t &o0, uint32_t &
 }
 
 // 16 input bytes per step, four steps in flight per thread, one 32-byte store each (two of 16 bytes where the output is only
-// aligned to that: WIDE is false; 64 MB in 47.3 instead of 43.0 us, a byte per thread 70.6). The up to 15 bytes behind the last whole step are unpacked by the first threads of block 0.
+// aligned to that: WIDE is false; 64 MB in 41.3 instead of 32.7 us, a byte per thread 57.2). The up to 15 bytes behind the last whole step are unpacked by the first threads of block 0.
 // Four loads per thread before the first store, and whole-sector stores, are what the memory system needs: one load and
 // two 16-byte stores 32 bytes apart ran at 4.5 TB/s (28672 x 4096 bytes in 77.4 us).
 constexpr int UNPACK_STEPS = 4;

@@ -99,8 +99,8 @@ def test_unpack_at_any_alignment(n, offset, shift):
 
 
 def test_unpack_of_sixteen_byte_aligned_outputs_is_no_byte_loop():
-    """An output that starts in the middle of a 32-byte sector takes the vector kernel too: 1.10 times the time of an aligned
-    one (47.3 against 43.0 us), where a byte per thread takes 1.62 times (70.6 us)."""
+    """An output that starts in the middle of a 32-byte sector takes the vector kernel too: 1.22 times the time of an aligned
+    one (47.3 against 38.7 us), where a byte per thread takes 1.65 times (63.8 us)."""
     n = 64 << 20
     packed = torch.randint(-128, 128, (n,), dtype=torch.int8, device="cuda")
     buf = torch.empty(2 * n + 16, dtype=torch.int8, device="cuda")
