@@ -7,6 +7,7 @@
 #include <cuda.h>
 
 #include "qf_common.cuh"
+#include "qf_stream.cuh"
 
 namespace qf {
 
@@ -64,6 +65,24 @@ static constexpr size_t kCounterBytes = (size_t)kMaxCounters * sizeof(int);
 
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
+// Which of the two kernels that read slab weights runs a linear called by itself. The streaming tcgen05 kernel takes its SMs whole
+// and starts when its predecessor has ended, about 10 us a call that do not depend on the size; per byte it is faster, the more so
+// the more rows. Measured on weights not in L2, calls back to back, us, GEMV -> tcgen05 (blob in MiB):
+//   rows   8.5           13            30, K 4096    30, K 14336   34            59.5          119           238
+//   4      7.5 -> 10.6   8.4 -> 12.3   11.2 -> 14.6  13.5 -> 15.3  12.8 -> 16.5  18.1 -> 21.7  33.3 -> 34.2  57.9 -> 56.3
+//   8      7.6 -> 10.5   8.4 -> 12.5   11.9 -> 16.6  14.2 -> 15.9  13.3 -> 16.5  19.2 -> 22.7  34.9 -> 33.1  61.9 -> 57.6
+//   9      9.5 -> 10.8   10.5 -> 12.5  15.3 -> 16.6  19.7 -> 15.6  17.6 -> 16.6  23.1 -> 22.7  42.5 -> 33.6  75.6 -> 57.6
+//   16     10.3 -> 11.4  12.0 -> 14.5  16.6 -> 17.6  21.2 -> 16.2  19.1 -> 18.3  24.6 -> 23.0  44.6 -> 35.0  83.2 -> 63.8
+//   24     15.9 -> 15.6  16.1 -> 16.5  23.0 -> 19.2  28.7 -> 19.0  27.0 -> 20.7  35.5 -> 26.8  66.3 -> 37.1  129 -> 67.9
+//   32     17.0 -> 16.5  17.9 -> 18.6  24.8 -> 22.7  31.1 -> 20.0  29.0 -> 21.4  37.8 -> 28.7  70.2 -> 38.7  135 -> 69.9
+static bool stream_serves(const qf_linear_desc *d) {
+    const int64_t mib = d->N / 64 * (d->K / 128) * QF_SLAB_UNIT_BYTES >> 20;
+    if (d->M <= 2) return false;
+    if (d->M <= kSlabGemvRows) return mib >= 160;
+    if (d->M <= 16) return mib >= (d->K >= 8192 ? 24 : 33);
+    return mib >= 24;
+}
+
 int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
     auto bad = [&](int st, const char *m) {
         if (why) *why = m;
@@ -92,6 +111,7 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
     for (int i = 0; i < 3; ++i)
         if (d->reserved[i] != 0) return bad(QF_ERR_BAD_ARG, "reserved fields must be zero");
     p->slab = false;
+    p->stream = false;
     p->pair = false;
     if (d->weight_layout == QF_LAYOUT_GEMV_SLAB) {
         if (d->path == QF_PATH_GEMM)
@@ -99,6 +119,17 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
         if (d->N % 64 != 0) return bad(QF_ERR_BAD_ARG, "QF_LAYOUT_GEMV_SLAB needs N to be a multiple of 64");
         if (d->M > QF_SLAB_MAX_M)
             return bad(QF_ERR_UNSUPPORTED, "QF_LAYOUT_GEMV_SLAB serves M <= 32; use a tcgen05 layout for larger batches");
+        if (d->split_k == 0 && d->path == QF_PATH_AUTO && stream_serves(d)) {
+            p->stream = true;
+            p->path = QF_PATH_GEMV;
+            p->split_k = 2 * kSmCount;
+            p->chunks_per_split = 0;
+            p->m_tiles = 1;
+            p->bn = d->M <= 16 ? 16 : 32;
+            p->ws_partial_bytes = stream_workspace_bytes(d->M);
+            p->ws_counter_bytes = kCounterBytes;
+            return QF_OK;
+        }
         int grid = 1, depth = 1;
         slab_geometry(d->M, d->N, d->K, kSmCount, d->split_k, &grid, &depth);
         p->slab = true;
@@ -302,10 +333,27 @@ static int check_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, 
     return QF_OK;
 }
 
+// Slab weights, and nothing in the descriptor that names a kernel.
+static bool slab_any(const qf_linear_desc *d) {
+    return d->weight_layout == QF_LAYOUT_GEMV_SLAB && d->split_k == 0 && d->path == QF_PATH_AUTO;
+}
+
+// Linears that qf_w4a16_linear_batched runs as one launch.
+static bool chains(const qf_linear_desc *d) { return slab_any(d) && d->M > kSlabGemvRows && d->N % 128 == 0; }
+
 static int launch_linear(qf_ctx *ctx, const qf_linear_desc *desc, const Plan &plan, const void *X, const void *qweight,
                          const void *scales, const void *qzeros_or_null, void *Y, const void *residual, void *workspace,
                          cudaStream_t s) {
     if (plan.slab) return launch_gemv_slab(ctx, desc, plan, X, qweight, Y, residual, workspace, s);
+    if (plan.stream) {
+        const int st = launch_stream(ctx, StreamLinear{desc, X, qweight, residual, Y, 1, 0}, workspace, kCounterBytes, s);
+        if (st != kStreamNoRoom) return st;
+        qf_linear_desc d = *desc;
+        d.path = QF_PATH_GEMV;
+        Plan other;  // its workspace is the smaller one
+        if (make_plan(&d, &other, nullptr) != QF_OK) return fail(ctx, QF_ERR_UNSUPPORTED, "no kernel for this linear");
+        return launch_gemv_slab(ctx, desc, other, X, qweight, Y, residual, workspace, s);
+    }
     if (plan.path == QF_PATH_GEMV) return launch_gemv(ctx, desc, plan, X, qweight, scales, qzeros_or_null, Y, workspace, s);
     return launch_gemm(ctx, desc, plan, X, qweight, scales, qzeros_or_null, Y, residual, workspace, s);
 }
@@ -357,6 +405,7 @@ int qf_ctx_create(qf_ctx **out, int device) {
     int st = gemv_init(ctx);
     if (st == QF_OK) st = gemm_init(ctx);
     if (st == QF_OK) st = gemv_slab_init(ctx);
+    if (st == QF_OK) st = stream_init(ctx);
     if (st != QF_OK) {
         delete ctx;
         return st;
@@ -448,7 +497,15 @@ int qf_dequant_w4(qf_ctx *ctx, const qf_linear_desc *desc, const void *qweight, 
 size_t qf_w4a16_workspace_bytes(const qf_linear_desc *desc) {
     Plan plan;
     if (make_plan(desc, &plan, nullptr) != QF_OK) return 0;
-    return plan.ws_partial_bytes + plan.ws_counter_bytes;
+    size_t need = plan.ws_partial_bytes + plan.ws_counter_bytes;
+    if (slab_any(desc)) {
+        // enough for either kernel: an exchanging call on the same descriptor takes the one, a batched call the other
+        qf_linear_desc d = *desc;
+        d.path = QF_PATH_GEMV;
+        if (make_plan(&d, &plan, nullptr) == QF_OK) need = std::max(need, plan.ws_partial_bytes + plan.ws_counter_bytes);
+        need = std::max(need, stream_workspace_bytes(d.M) + kCounterBytes);
+    }
+    return need;
 }
 
 int qf_w4a16_plan(const qf_linear_desc *desc, int32_t *path_out, int32_t *split_k_out) {
@@ -486,7 +543,31 @@ int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs,
     if (count < 0) return fail(ctx, QF_ERR_BAD_ARG, "negative count");
     if (count == 0) return QF_OK;
     if (!descs || !X || !qweight || !Y) return fail(ctx, QF_ERR_BAD_ARG, "null argument array");
+    std::vector<StreamLinear> run;
     for (int i = 0; i < count; ++i) {
+        // linears on slab weights from here on, as far as nothing is wrong with them: one launch
+        run.clear();
+        for (int j = i; j < count && chains(&descs[j]); ++j) {
+            Plan plan;
+            const void *res = residual ? residual[j] : nullptr;
+            if (check_linear(ctx, &descs[j], X[j], qweight[j], nullptr, nullptr, Y[j], res, workspace, workspace_bytes, &plan) != QF_OK ||
+                workspace_bytes < stream_workspace_bytes(descs[j].M) + kCounterBytes)
+                break;
+            // K is cut as the tcgen05 kernel cuts it for the same sizes in its own layouts: the sums are the same bits
+            qf_linear_desc d = descs[j];
+            d.weight_layout = QF_LAYOUT_INTERLEAVED;
+            if (make_plan(&d, &plan, nullptr) != QF_OK || plan.path != QF_PATH_GEMM) break;
+            run.push_back(StreamLinear{&descs[j], X[j], qweight[j], res, Y[j], plan.split_k, plan.chunks_per_split});
+        }
+        const int n = run.size() > 1 ? stream_chain_length(run.data(), (int)run.size()) : 0;
+        if (n > 1) {
+            const int st = launch_stream_chain(ctx, run.data(), n, workspace, kCounterBytes, (cudaStream_t)stream);
+            if (st != QF_OK && st != kStreamNoRoom) return st;
+            if (st == QF_OK) {
+                i += n - 1;
+                continue;
+            }
+        }
         const int st = qf_w4a16_linear_fused(ctx, &descs[i], X[i], qweight[i], scales ? scales[i] : nullptr,
                                              qzeros ? qzeros[i] : nullptr, Y[i], residual ? residual[i] : nullptr,
                                              workspace, workspace_bytes, stream);

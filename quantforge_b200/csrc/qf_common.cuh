@@ -199,6 +199,7 @@ struct Plan {
     int split_k;         // number of K splits (slab GEMV: thread blocks of the launch)
     int chunks_per_split;  // GEMV: 128-code chunks per split; GEMM: k-blocks per split; slab GEMV: ring depth
     bool slab;           // QF_LAYOUT_GEMV_SLAB weights: the streaming GEMV kernel
+    bool stream;         // QF_LAYOUT_GEMV_SLAB weights: the streaming tcgen05 kernel
     int m_tiles;         // GEMV: ceil(M/8); GEMM: batch tiles
     int bn;              // GEMM: batch tile width (MMA N)
     bool pair;           // GEMM: two CTAs share a batch tile (cta_group::2)
@@ -271,6 +272,8 @@ int gemv_slab_init(qf_ctx *ctx);
 // neighbours are kernels of other sizes, a limit of 36 MB measured no better than 16 MB (5.84 vs 5.79 ms per
 // token on two GPUs), so the limit stays where the step-level numbers were taken.
 constexpr long long kSlabSmallBytes = 16ll << 20;
+// Rows up to which the streaming GEMV kernel is the kernel of choice for slab weights.
+constexpr int64_t kSlabGemvRows = 8;
 int slab_m_pad(int64_t M);
 void slab_geometry(int64_t M, int64_t N, int64_t K, int sm_count, int grid_request, int *grid_out, int *depth_out);
 size_t slab_workspace_bytes(int grid, int64_t M);
@@ -441,6 +444,19 @@ struct ShortConvert {
             zq = fma_bf16x2(zs.zsub, 0xbe80be80u, 0x42004200u);  // -(128 + z) / 4 + 32, exact
             s4 = mul_bf16x2(zs.s2, 0x40804080u);
             wide = __any_sync(0xffffffffu, (scale_bits & 0x7fffu) >= 0x7e80u);  // |s| >= 2^126
+        }
+    }
+    // From a constants word of a QF_LAYOUT_GEMV_SLAB tile: zsub in the low half, the scale in the high one. All 32 lanes.
+    __device__ __forceinline__ void set_slab(uint32_t word) {
+        zs.zsub = prmt(word, word, 0x1010u);
+        zs.s2 = prmt(word, word, 0x3232u);
+        if (BF16) {
+            zs.zfma = 0u;
+            zq = fma_bf16x2(zs.zsub, 0xbe80be80u, 0x42004200u);
+            s4 = mul_bf16x2(zs.s2, 0x40804080u);
+            wide = __any_sync(0xffffffffu, (word & 0x7fff0000u) >= 0x7e800000u);
+        } else {
+            zs.zfma = fma_f16x2(zs.zsub, 0xbc00bc00u, 0x63806380u);  // (1024 + z) * -1 + 960 = -(64 + z), exact
         }
     }
     __device__ __forceinline__ void operator()(uint32_t w, uint32_t (&p)[4]) const {

@@ -1,0 +1,843 @@
+// K4: W4A16 linears of up to 32 rows on QF_LAYOUT_GEMV_SLAB weights, converted into tensor memory; one linear, or a chain of them in
+// one launch.
+//
+// Y[M,N] = X[M,K] . W^T as Y^T = W . X^T: the dequantised weights are the A operand of tcgen05 MMAs (128 weight rows x 16 codes an
+// instruction) and live in TMEM only, the activations are B from shared memory. What the streaming GEMV kernel (mma.sync) spends
+// on fragments of X and on the MMAs themselves, which take issue slots and packed-half time from the conversion and grow with the
+// rows, is here one thread's work. Without memory, converters and MMAs alone take 283 cycles per 128 x 128 codes and SM; HBM delivers
+// those in 377; the kernel takes about 450, bound by the issue slots that the conversion and its hand-overs share.
+//
+// Work split. Units of 128 rows x 128 codes. Of a single linear they are numbered row block major, K chunk minor, and stream i of G
+// owns a contiguous range of them (the first r streams one more than the others): every stream moves the same number of bytes
+// whatever the shape is. A chain is a list of phases; the linears of a phase do not depend on each other, a phase needs the results
+// of the earlier ones. There K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same sizes on other
+// layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any other order
+// into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least surprise).
+// The pieces of a phase are dealt to the streams one after the other. Weights are requested as far ahead as the ring of stages allows,
+// across linears and phases; only the activations of a phase wait for the phase before it.
+//
+// A thread block has its SM to itself and runs two streams side by side (one stream's waits are the other's time to convert), each
+// with half of its threads, shared memory and TMEM. (One block per SM because a cooperative launch admits no more of a kernel that
+// allocates TMEM.) Of a stream's sixteen warps:
+//   warps 0-7    two converter groups, alternating units: thread t owns weight row t of the unit, reads its 64 bytes of codes and
+//                its constants from the swizzled stage, converts and writes them to TMEM lane t (tcgen05.st).
+//   one warp     copies of weights: one TMA box per unit, a chunk of two row blocks of the blob as 64-byte lines.
+//   one warp     copies of activations (MMA B tiles, K-major, 128-byte swizzle), and the wait for the phase before.
+//   one warp     one thread issues the MMAs of a unit once its weights and activations are there.
+//   warps 12-15  results: a row block's accumulators go from TMEM to Y, or to the workspace where others have chunks of it too.
+//
+// Row blocks whose K range is shared by several streams (its members): a member leaves its partial sums in a slot of the workspace
+// as 8-byte (value, token) words - no fence, no atomic. The members finish the pairs of batch rows in turn (one member
+// reading ten others' sums of 16 rows would be a dozen trips to L2 in a row): whoever finishes a pair polls all members' words
+// (bounded), adds in their order (deterministic), writes Y and clears the words for the next user of the slots. The next phase starts
+// when this one is finished. As streams wait for one another, the launch is cooperative, and without programmatic dependent launch:
+// it would find no room beside another kernel's blocks.
+//
+// Shared memory takes all but a few KB of the SM's first-level cache, so a spilled register is a trip to L2: the registers are split
+// between the roles such that none is (see setmaxnreg below).
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "qf_stream.cuh"
+#include "qf_tcgen05.cuh"
+
+namespace qf {
+
+constexpr int ST_THREADS = 1024;                             // two streams of sixteen warps
+constexpr int ST_LINES = QF_SLAB_UNIT_BYTES / 64;            // 64-byte lines of a unit of 64 rows
+constexpr int ST_UNIT_BYTES = 2 * QF_SLAB_UNIT_BYTES;        // two row blocks, one chunk
+constexpr int ST_NA = 3;                                     // A operand buffers in TMEM, 64 columns each
+constexpr int ST_TMEM_COLS = 256;                            // of a stream: half an SM's
+
+// NB: the MMA's N, batch rows padded to 16 or 32.
+template <int NB>
+struct StreamCfg {
+    static constexpr int W_STAGES = 8;
+    static constexpr int X_STAGES = NB == 16 ? 8 : 4;
+    static constexpr int X_BOX_BYTES = NB * 128;             // 64 codes
+    static constexpr int X_BYTES = 2 * X_BOX_BYTES;
+    static constexpr int W_OFF = X_STAGES * X_BYTES;
+    static constexpr int BAR_OFF = W_OFF + W_STAGES * ST_UNIT_BYTES;
+    static constexpr int BARS = 2 * W_STAGES + 2 * X_STAGES + 2 * ST_NA + 2 * 2 + 1;
+    static constexpr int STREAM_BYTES = (BAR_OFF + BARS * 8 + 1023) / 1024 * 1024;
+    static_assert(2 * NB + ST_NA * 64 <= ST_TMEM_COLS, "two accumulators and the A operands");
+};
+
+struct StreamEntry {  // one linear
+    void *Y;
+    const void *residual;
+    int N, chunks;   // chunks of 128 codes along K
+    int begin, end;  // its units (or pieces) within the phase
+    int split, per;  // pieces: K is cut into `split` of them, `per` chunks each (the last may be shorter)
+    int x_map;
+    int16_t out_dtype, epilogue;
+};
+struct StreamPhase {
+    int first;    // entry
+    int pieces;   // 0: ranges of units; else how many pieces the phase has
+    int q, r;     // ranges: units of the phase = q * G + r, streams 0..r-1 have q + 1
+    int streams;  // G
+    int active;   // streams that have work
+};
+struct StreamArgs {
+    unsigned long long *slots;  // [kStreamSlots][slot_words] (value | token << 32), zero between launches
+    unsigned *done;             // [phases] result warps that have finished the phase, zero between launches
+    int *status;
+    int slot_words;
+    int M, x_rows;              // x_rows: rows of an X box (M rounded up to 8)
+    int phases, linears;
+};
+template <int CAP>
+struct StreamParams {
+    static constexpr int XCAP = CAP == 1 ? 1 : 16;
+    CUtensorMap w[CAP];
+    CUtensorMap x[XCAP];
+    StreamEntry e[CAP];
+    StreamPhase ph[CAP];
+    StreamArgs a;
+};
+static_assert(sizeof(StreamParams<kStreamMaxLinears>) <= 32764, "kernel parameters");
+// The lists of linears and phases, in shared memory: every role reads the next phase's when it gets there, and from the parameter
+// space that was a miss of the constant cache each time.
+template <int CAP>
+struct StreamTables {
+    StreamEntry e[CAP];
+    StreamPhase ph[CAP];
+};
+template <int NB, int CAP>
+constexpr int stream_smem_bytes() {
+    return 2 * StreamCfg<NB>::STREAM_BYTES + 1024 /*alignment*/ + (int)sizeof(StreamTables<CAP>);
+}
+static_assert(stream_smem_bytes<16, kStreamMaxLinears>() <= 227 << 10 && stream_smem_bytes<32, kStreamMaxLinears>() <= 227 << 10,
+              "shared memory of a block");
+
+// Consecutive chunks of one row block, and who else has chunks of it: `members` of which this one is number `self`. A member's sums go
+// to slot `base` + its number, the first member's to `slot0`.
+struct Segment {
+    int e, b, c, len;
+    int members, self, slot0, base;
+};
+// Units of stream `id` in a phase: how many, and *u0 the first. Pieces: whether it has any.
+__device__ __forceinline__ int stream_range(const StreamPhase &ph, int id, int *u0) {
+    *u0 = id * ph.q + min(id, ph.r);
+    return ph.pieces ? id < ph.pieces : ph.q + (id < ph.r ? 1 : 0);
+}
+// The stream that has unit u.
+__device__ __forceinline__ int stream_of(const StreamPhase &ph, int u) {
+    const int head = ph.r * (ph.q + 1);
+    return u < head ? u / (ph.q + 1) : ph.r + (u - head) / ph.q;
+}
+// Walks a stream's work segment by segment; f returns whether to go on.
+template <int CAP, typename F>
+__device__ __forceinline__ void for_segments(const StreamTables<CAP> &t, int phase, int id, F f) {
+    const StreamPhase ph = t.ph[phase];
+    int u;
+    const int n = stream_range(ph, id, &u);
+    if (n <= 0) return;
+    int e = ph.first;
+    Segment g;
+    if (CAP > 1) {
+        // dealt to the streams forwards and backwards in turn: the next linear's pieces go first to streams that have none or short ones
+        for (int round = 0;; ++round) {
+            const int j = round * ph.streams + (round & 1 ? ph.streams - 1 - id : id);
+            if (j >= ph.pieces) return;
+            while (j >= t.e[e].end) ++e;
+            const int split = t.e[e].split, local = j - t.e[e].begin;
+            g.e = e;
+            g.b = local / split;
+            g.self = local - g.b * split;
+            g.c = g.self * t.e[e].per;
+            g.len = min(t.e[e].per, t.e[e].chunks - g.c);
+            g.members = split;
+            g.base = g.slot0 = j - g.self;
+            if (!f(g)) return;
+        }
+    }
+    const int end = u + n, chunks = t.e[e].chunks;
+    g.e = e;
+    g.b = u / chunks;
+    g.c = u - g.b * chunks;
+    while (true) {
+        g.len = min(chunks - g.c, end - u);
+        const int first = g.c + g.len == chunks && g.c == 0 ? id : stream_of(ph, u - g.c);
+        g.members = (g.len == chunks ? id : stream_of(ph, u - g.c + chunks - 1)) - first + 1;
+        g.self = id - first;
+        g.base = first;
+        g.slot0 = ph.streams + first;  // a stream's last segment may begin a row block, while its first one ends another
+        if (!f(g)) return;
+        u += g.len;
+        if (u == end) return;
+        ++g.b;
+        g.c = 0;
+    }
+}
+
+__device__ __forceinline__ void st_words2(unsigned long long *ptr, unsigned long long a, unsigned long long b) {
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(ptr), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void ld_words2(const unsigned long long *ptr, unsigned long long &a, unsigned long long &b) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(ptr) : "memory");
+}
+__device__ __forceinline__ unsigned long long word_of(uint32_t v) { return (unsigned long long)v | (1ull << 32); }
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *ptr) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
+    return v;
+}
+// Between ordinary accesses to global memory and accesses of the copy engine.
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+__device__ __forceinline__ float load_elem(const void *R, int out_dtype, int64_t idx) {
+    if (out_dtype == QF_F32) return reinterpret_cast<const float *>(R)[idx];
+    if (out_dtype == QF_F16) return __half2float(reinterpret_cast<const __half *>(R)[idx]);
+    return __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(R)[idx]);
+}
+
+// Writes finished sums: PAIRS pairs of batch rows from row m0 on (as far as M goes) of weight row n. All 32 lanes of a warp, which
+// hold 32 consecutive weight rows. The steps of all pairs go side by side: these warps run a chain of dependent instructions
+// otherwise, 450 cycles a pair.
+template <int PAIRS>
+__device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, int m0, const float (&v)[2 * PAIRS]) {
+    const int type = e.out_dtype;
+    if (e.epilogue == QF_EPI_SILU_MUL) {
+        // rows 0..7 of sixteen are gate rows, 8..15 the matching up rows: of a pair the gate lane does the first batch row, the up lane
+        // the second
+        const bool up_lane = n & 8;
+        const int64_t cols = e.N >> 1, col = (n >> 4) * 8 + (n & 7);
+        float gate[PAIRS], up[PAIRS];
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            const float other = __shfl_xor_sync(0xffffffffu, up_lane ? v[2 * i] : v[2 * i + 1], 8);
+            gate[i] = up_lane ? other : v[2 * i];
+            up[i] = up_lane ? v[2 * i + 1] : other;
+        }
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) up[i] = gate[i] / (1.f + expf(-gate[i])) * up[i];
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            const int m = m0 + 2 * i + (up_lane ? 1 : 0);
+            if (m < M) store_out(e.Y, type, m * cols + col, up[i]);
+        }
+        return;
+    }
+    const int64_t o = (int64_t)m0 * e.N + n;
+    float r[2 * PAIRS];
+#pragma unroll
+    for (int i = 0; i < 2 * PAIRS; ++i)
+        r[i] = e.epilogue == QF_EPI_RESIDUAL_ADD && m0 + i < M ? load_elem(e.residual, type, o + (int64_t)i * e.N) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 2 * PAIRS; ++i)
+        if (m0 + i < M) store_out(e.Y, type, o + (int64_t)i * e.N, e.epilogue == QF_EPI_RESIDUAL_ADD ? v[i] + r[i] : v[i]);
+}
+
+__device__ __forceinline__ unsigned long long *slot_of(const StreamArgs &a, const Segment &g, int member) {
+    return a.slots + (size_t)(member == 0 ? g.slot0 : g.base + member) * a.slot_words;
+}
+// Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of eight members are requested
+// at a time. Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us,
+// then 1500 to 1528.)
+__device__ __forceinline__ bool stream_sum(const StreamArgs &a, const Segment &g, int pair, int row, float (&v)[2],
+                                           volatile int *abort_flag) {
+    constexpr int WORDS = 8;
+    v[0] = v[1] = 0.f;
+#pragma unroll 1
+    for (int m0 = 0; m0 < g.members; m0 += WORDS) {
+        unsigned long long *src[WORDS], w[WORDS][2];
+#pragma unroll
+        for (int j = 0; j < WORDS; ++j) src[j] = slot_of(a, g, m0 + j) + (pair * 128 + row) * 2;
+        const long long t0 = clock64();
+        while (true) {
+            bool miss = false;
+#pragma unroll
+            for (int j = 0; j < WORDS; ++j)
+                if (m0 + j < g.members) ld_words2(src[j], w[j][0], w[j][1]);
+#pragma unroll
+            for (int j = 0; j < WORDS; ++j)
+                if (m0 + j < g.members) miss = miss || (uint32_t)(w[j][0] >> 32) != 1u || (uint32_t)(w[j][1] >> 32) != 1u;
+            if (!__any_sync(0xffffffffu, miss)) break;
+            if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles || *abort_flag != 0)) return false;
+        }
+#pragma unroll
+        for (int j = 0; j < WORDS; ++j)
+            if (m0 + j < g.members) {
+                v[0] += __uint_as_float((uint32_t)w[j][0]);
+                v[1] += __uint_as_float((uint32_t)w[j][1]);
+                st_words2(src[j], 0ull, 0ull);
+            }
+    }
+    return true;
+}
+
+// Bounded wait. The thread asks to be suspended for up to 20 us at a time: a warp that waits takes no issue slots, which the
+// converters need.
+__device__ __forceinline__ bool stream_try_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool stream_wait_on(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    const long long t0 = clock64();
+    while (true) {
+        if (stream_try_wait(bar, parity)) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > kWaitCycles) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+}
+
+__device__ __forceinline__ bool stream_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return stream_try_wait(bar, parity) || stream_wait_on(bar, parity, abort_flag);
+}
+
+template <bool BF16, int NB, int CAP>
+__global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_constant__ StreamParams<CAP> p) {
+    using C = StreamCfg<NB>;
+    extern __shared__ uint8_t stream_smem[];
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+
+    const int tid = threadIdx.x & 511;
+    const int half = threadIdx.x >> 9;
+    const int warp = tid >> 5;
+    const int lane = tid & 31;
+    // The single threads of the two streams sit on different schedulers (a warp's is its number mod 4): weights 8 and 10,
+    // activations 9 and 11, MMAs 10 and 8.
+    // roles: 0 converts, 1 weights, 2 activations, 3 MMAs, 4 results, 5 none
+    const int role = warp < 8 ? 0 : warp >= 12 ? 4 : (half == 0 ? 0x5321 : 0x2153) >> (4 * (warp - 8)) & 7;
+    const int id = half * (int)gridDim.x + (int)blockIdx.x;  // of the stream: two streams of a block differ by at most a unit
+    const uint32_t base = ((smem_u32(stream_smem) + 1023u) & ~1023u) + (uint32_t)half * C::STREAM_BYTES;
+    const uint32_t bars = base + C::BAR_OFF;
+    auto x_stage = [&](int s) { return base + (uint32_t)s * C::X_BYTES; };
+    auto w_stage = [&](int s) { return base + C::W_OFF + (uint32_t)s * ST_UNIT_BYTES; };
+    auto wfull = [&](int s) { return bars + 8u * s; };
+    auto wempty = [&](int s) { return bars + 8u * (C::W_STAGES + s); };
+    auto xfull = [&](int s) { return bars + 8u * (2 * C::W_STAGES + s); };
+    auto xempty = [&](int s) { return bars + 8u * (2 * C::W_STAGES + C::X_STAGES + s); };
+    constexpr int AB = 2 * C::W_STAGES + 2 * C::X_STAGES;
+    auto afull = [&](int a) { return bars + 8u * (AB + a); };
+    auto aempty = [&](int a) { return bars + 8u * (AB + ST_NA + a); };
+    auto dfull = [&](int d) { return bars + 8u * (AB + 2 * ST_NA + d); };
+    auto dempty = [&](int d) { return bars + 8u * (AB + 2 * ST_NA + 2 + d); };
+    const uint32_t gate = bars + 8u * (AB + 2 * ST_NA + 4);
+
+    const StreamArgs &a = p.a;
+    StreamTables<CAP> &t = *reinterpret_cast<StreamTables<CAP> *>(
+        stream_smem + ((1024u - (smem_u32(stream_smem) & 1023u)) & 1023u) + 2 * C::STREAM_BYTES);
+    const int phases = CAP == 1 ? 1 : a.phases;
+    volatile int *abort_flag = &s_abort;
+
+    if (tid == 0) {
+        s_abort = 0;
+        for (int s = 0; s < C::W_STAGES; ++s) {
+            mbar_init(wfull(s), 1);
+            mbar_init(wempty(s), 4);  // the warps of the group that converts the unit
+        }
+        for (int s = 0; s < C::X_STAGES; ++s) {
+            mbar_init(xfull(s), 1);
+            mbar_init(xempty(s), 1);
+        }
+        for (int i = 0; i < ST_NA; ++i) {
+            mbar_init(afull(i), 4);
+            mbar_init(aempty(i), 1);
+        }
+        for (int d = 0; d < 2; ++d) {
+            mbar_init(dfull(d), 1);
+            mbar_init(dempty(d), 4);
+        }
+        mbar_init(gate, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 10 && half == 0) tmem_alloc<false>(smem_u32(&s_tmem_base), 2 * ST_TMEM_COLS);
+    if (a.x_rows < NB) {
+        // the rows of the B tiles that no copy writes
+        for (uint32_t o = tid * 16u; o < (uint32_t)C::W_OFF; o += 512u * 16u)
+            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(base + o), "r"(0u) : "memory");
+        fence_proxy_async_shared();
+    }
+    for (int i = threadIdx.x; i < a.linears * (int)(sizeof(StreamEntry) / 4); i += ST_THREADS)
+        reinterpret_cast<uint32_t *>(t.e)[i] = reinterpret_cast<const uint32_t *>(p.e)[i];
+    for (int i = threadIdx.x; i < phases * (int)(sizeof(StreamPhase) / 4); i += ST_THREADS)
+        reinterpret_cast<uint32_t *>(t.ph)[i] = reinterpret_cast<const uint32_t *>(p.ph)[i];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem_base + (uint32_t)half * ST_TMEM_COLS;  // two accumulators of NB columns, then the A operands
+
+    // Registers: 64 a thread at launch; a stream's four warpgroups share them as 2 x 48, 56 and 104. With 64 for all, the result warps
+    // spilled addresses and sums in flight: the linears of 32 layers at 16 rows took 1971 us, with 64, 40 and 88 1557, with this 1495.
+    if (role == 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    else if (role == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    int issued = 0;  // copies of this thread (elected lanes of roles 1 and 2)
+    if (role == 1) {
+        // ------------------------------ weights ------------------------------
+        const bool leader = elect_one();
+        if (leader) {
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int phase = 0; phase < phases && ok; ++phase)
+                for_segments(t, phase, id, [&](const Segment &g) {
+                    if (g.e + 1 < a.linears) tma_prefetch_desc(&p.w[g.e + 1]);
+                    for (int i = 0; i < g.len; ++i) {
+                        if (!stream_wait(wempty(s), ph ^ 1u, abort_flag)) return ok = false;
+                        mbar_arrive_expect_tx(wfull(s), ST_UNIT_BYTES);
+                        tma_load_4d(w_stage(s), &p.w[g.e], wfull(s), 0, 0, g.c + i, 2 * g.b);
+                        ++issued;
+                        if (++s == C::W_STAGES) {
+                            s = 0;
+                            ph ^= 1u;
+                        }
+                    }
+                    return true;
+                });
+        }
+        __syncwarp();
+    } else if (role == 2) {
+        // ------------------------------ activations ------------------------------
+        const bool leader = elect_one();
+        if (leader) {
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            const uint32_t tx = 2u * (uint32_t)a.x_rows * 128u;
+            for (int phase = 0; phase < phases && ok; ++phase) {
+                bool behind = phase > 0;
+                for_segments(t, phase, id, [&](const Segment &g) {
+                    if (behind) {
+                        // all results of the phase before are in memory
+                        const long long t0 = clock64();
+                        while (ld_acquire(a.done + phase - 1) < 4u * (unsigned)t.ph[phase - 1].active) {
+                            if (*abort_flag) return ok = false;
+                            if (clock64() - t0 > kWaitCycles) {
+                                *abort_flag = 1;
+                                return ok = false;
+                            }
+                        }
+                        // they were stored through the generic proxy and are read by the copy engine
+                        fence_proxy_async_all();
+                        mbar_arrive(gate);
+                        // the phase before is complete: nobody waits for the one before that any more
+                        if (id == 0 && phase > 1) a.done[phase - 2] = 0u;
+                        behind = false;
+                    }
+                    const CUtensorMap *map = &p.x[t.e[g.e].x_map];
+                    for (int i = 0; i < g.len; ++i) {
+                        if (!stream_wait(xempty(s), ph ^ 1u, abort_flag)) return ok = false;
+                        mbar_arrive_expect_tx(xfull(s), tx);
+                        tma_load_2d(x_stage(s), map, xfull(s), (g.c + i) * 128, 0);
+                        tma_load_2d(x_stage(s) + C::X_BOX_BYTES, map, xfull(s), (g.c + i) * 128 + 64, 0);
+                        ++issued;
+                        if (++s == C::X_STAGES) {
+                            s = 0;
+                            ph ^= 1u;
+                        }
+                    }
+                    return true;
+                });
+            }
+        }
+        __syncwarp();
+    } else if (role == 3) {
+        // ------------------------------ MMAs ------------------------------
+        if (elect_one()) {
+            const uint32_t idesc = (1u << 4) | ((BF16 ? 1u : 0u) << 7) | ((BF16 ? 1u : 0u) << 10) | ((uint32_t)(NB >> 3) << 17) |
+                                   ((uint32_t)(128 >> 4) << 24);
+            const uint64_t desc0 = make_b_desc(x_stage(0));
+            int i = 0, s = 0, seg = 0;
+            uint32_t aph = 0, xph = 0;
+            bool ok = true;
+            for (int phase = 0; phase < phases && ok; ++phase)
+                for_segments(t, phase, id, [&](const Segment &g) {
+                    const int d = seg & 1;
+                    if (!stream_wait(dempty(d), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) return ok = false;
+                    const uint32_t d_tmem = tmem + d * NB;
+                    for (int k = 0; k < g.len; ++k) {
+                        if (!stream_wait(afull(i), aph, abort_flag) || !stream_wait(xfull(s), xph, abort_flag)) return ok = false;
+                        tc_fence_after();
+                        const uint32_t a_tmem = tmem + 2 * NB + i * 64;
+                        const uint64_t desc = desc0 + (uint32_t)s * (uint32_t)(C::X_BYTES >> 4);
+                        umma_ts<false>(d_tmem, a_tmem, desc, idesc, k > 0 ? 1u : 0u);
+#pragma unroll
+                        for (int kk = 1; kk < 8; ++kk)
+                            umma_ts<false>(d_tmem, a_tmem + kk * 8, desc + (uint32_t)(((kk >> 2) * C::X_BOX_BYTES + (kk & 3) * 32) >> 4),
+                                           idesc, 1u);
+                        umma_commit<false>(aempty(i));
+                        umma_commit<false>(xempty(s));
+                        if (++i == ST_NA) {
+                            i = 0;
+                            aph ^= 1u;
+                        }
+                        if (++s == C::X_STAGES) {
+                            s = 0;
+                            xph ^= 1u;
+                        }
+                    }
+                    umma_commit<false>(dfull(d));
+                    ++seg;
+                    return true;
+                });
+        }
+        __syncwarp();
+    } else if (role == 0) {
+        // ------------------------------ converters ------------------------------
+        int total = 0;
+        for (int q = CAP == 1 ? 0 : lane; q < phases; q += 32) for_segments(t, q, id, [&](const Segment &g) { return total += g.len, true; });
+        if (CAP > 1) total = __reduce_add_sync(0xffffffffu, total);
+        const int row = tid & 127;
+        const uint32_t lane_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * NB;
+        // A tile of the blob is 17 lines of 64 bytes, sixteen rows and their constants; line l of a stage holds its 16-byte piece i
+        // at i ^ (l / 2 % 4).
+        const int tile = (row >> 6) * ST_LINES + ((row & 63) >> 4) * 17;
+        const int line = tile + (row & 15), cline = tile + 16;
+        const uint32_t w_off = (uint32_t)line * 64u + (((uint32_t)(line >> 1) & 3u) << 4);  // its piece 0
+        const uint32_t c_off = (uint32_t)cline * 64u + ((((uint32_t)(row & 15) >> 2) ^ ((uint32_t)(cline >> 1) & 3u)) << 4) +
+                               ((uint32_t)row & 3u) * 4u;
+        int s = warp >> 2, i = warp >> 2;  // stage and A operand buffer of the unit
+        uint32_t wph = 0u, aph = 1u;
+        for (int it = warp >> 2; it < total; it += 2) {
+            bool ready = stream_wait(wfull(s), wph, abort_flag);
+            ready = ready && stream_wait(aempty(i), aph, abort_flag);
+            if (!__all_sync(0xffffffffu, ready)) break;  // the tcgen05.st below is warp-collective
+            tc_fence_after();
+            const uint32_t stage = w_stage(s);
+            ShortConvert<BF16> conv;
+            conv.set_slab(lds32(stage + c_off));
+            // Piece j holds words j, j + 4, j + 8, j + 12 of the row's sixteen; the next piece is on its way while one is converted.
+            // (All four pieces first and stores of 16 columns: 59.6 us on 57344 x 8192, this form 56.6.)
+            const uint32_t piece = stage + w_off;
+            uint32_t col = lane_tmem + i * 64;
+            uint4 v = lds128(piece);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint4 next = j < 3 ? lds128(piece ^ ((uint32_t)(j + 1) << 4)) : v;
+                uint32_t q[4];
+                conv(v.x, q);
+                tmem_st4(col, q);
+                conv(v.y, q);
+                tmem_st4(col + 16, q);
+                conv(v.z, q);
+                tmem_st4(col + 32, q);
+                conv(v.w, q);
+                tmem_st4(col + 48, q);
+                v = next;
+                col += 4;
+            }
+            if (BF16 && conv.wide) {
+                // once more in the form for scales of 2^126 and more (see ShortConvert). It reads everything again: values kept
+                // for it would cost the ordinary path registers (59 -> 63 us on 57344 x 8192)
+                tmem_wait_st();
+                ShortConvert<BF16> again;
+                again.set_slab(lds32(stage + c_off));
+#pragma unroll 1
+                for (int j = 0; j < 16; ++j) {
+                    uint32_t q[4];
+                    dequant8<BF16>(lds32((piece ^ (((uint32_t)j & 3u) << 4)) + ((uint32_t)j & 12u)), again.zs, q);
+                    tmem_st4(lane_tmem + i * 64 + j * 4, q);
+                }
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            fence_proxy_async_shared();  // this thread's reads of the stage, before the copy engine refills it
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(afull(i));
+                mbar_arrive(wempty(s));
+            }
+            if ((s += 2) >= C::W_STAGES) {
+                s -= C::W_STAGES;
+                wph ^= 1u;
+            }
+            if ((i += 2) >= ST_NA) {
+                i -= ST_NA;
+                aph ^= 1u;
+            }
+        }
+    } else if (role == 4) {
+        // ------------------------------ results ------------------------------
+        const int quad = warp & 3;  // TMEM lanes 32 * quad ..
+        const int row = quad * 32 + lane;
+        const uint32_t lane_tmem = tmem + ((uint32_t)(quad * 32) << 16);
+        int seg = 0;
+        uint32_t gph = 0;
+        bool ok = true;
+        for (int phase = 0; phase < phases; ++phase) {
+            int u0;
+            if (stream_range(t.ph[phase], id, &u0) <= 0) continue;
+            if (phase > 0) {
+                ok = __all_sync(0xffffffffu, ok && stream_wait(gate, gph, abort_flag));
+                gph ^= 1u;
+            }
+            for_segments(t, phase, id, [&](const Segment &g) {
+                const int d = seg & 1;
+                const StreamEntry &en = t.e[g.e];
+                const int n = g.b * 128 + row;
+                const bool in = g.b * 128 + quad * 32 < en.N;  // N is a multiple of 64: the last row block may be half
+                unsigned long long *slot = slot_of(a, g, g.self) + row * 2;
+                ok = __all_sync(0xffffffffu, ok && stream_wait(dfull(d), (uint32_t)(seg >> 1) & 1u, abort_flag));
+                if (!ok) return false;
+                ++seg;
+                tc_fence_after();
+#pragma unroll 1
+                for (int m0 = 0; m0 < a.M; m0 += 8) {
+                    uint32_t r[8];
+                    tmem_ld8(lane_tmem + d * NB + m0, r);
+                    tmem_wait_ld();
+                    if (!in) continue;
+                    if (g.members == 1) {
+                        float v[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
+                        stream_emit<4>(en, a.M, n, m0, v);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2)
+                            if (m0 + j < a.M) st_words2(slot + (m0 + j) * 128, word_of(r[j]), word_of(r[j + 1]));
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(dempty(d));
+                return true;
+            });
+            // The members of a shared row block finish its pairs of batch rows in turn.
+            for_segments(t, phase, id, [&](const Segment &g) {
+                const StreamEntry &en = t.e[g.e];
+                if (!ok || g.members == 1 || g.b * 128 + quad * 32 >= en.N) return ok;
+#pragma unroll 1
+                for (int pair = g.members - 1 - g.self; pair < (a.M + 1) >> 1; pair += g.members) {
+                    float v[2];
+                    ok = stream_sum(a, g, pair, row, v, abort_flag);
+                    if (!ok) {
+                        *abort_flag = 1;
+                        return false;
+                    }
+                    stream_emit<1>(en, a.M, g.b * 128 + row, 2 * pair, v);
+                }
+                return true;
+            });
+            if (phases > 1) {
+                __syncwarp();
+                if (lane == 0 && ok) {
+                    if (phase < phases - 1) {
+                        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.done + phase) : "memory");
+                    } else if (atomicAdd(a.done + phase, 1u) + 1u == 4u * (unsigned)t.ph[phase].active) {
+                        a.done[phase - 1] = 0u;
+                        a.done[phase] = 0u;
+                    }
+                }
+            }
+        }
+    }
+
+    // ------------------------------ teardown ------------------------------
+    tc_fence_before();
+    __syncthreads();
+    if (s_abort) {
+        // this block's own copies, before its shared memory goes away
+        int dummy = 0;
+        volatile int *no_abort = &dummy;
+        if (role == 1)
+            for (int it = max(0, issued - C::W_STAGES); it < issued; ++it)
+                stream_wait(wfull(it % C::W_STAGES), (uint32_t)(it / C::W_STAGES) & 1u, no_abort);
+        if (role == 2)
+            for (int it = max(0, issued - C::X_STAGES); it < issued; ++it)
+                stream_wait(xfull(it % C::X_STAGES), (uint32_t)(it / C::X_STAGES) & 1u, no_abort);
+        if (threadIdx.x == 0) atomicExch(a.status, QF_ERR_TIMEOUT);
+        __syncthreads();
+    }
+    if (warp == 10 && half == 0) {
+        tc_fence_after();
+        tmem_dealloc<false>(tmem, 2 * ST_TMEM_COLS);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+template <bool BF16, int NB, int CAP>
+static cudaError_t stream_set_attr() {
+    cudaError_t e = cudaFuncSetAttribute(stream_kernel<BF16, NB, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (stream_smem_bytes<NB, CAP>()));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(stream_kernel<BF16, NB, CAP>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared);
+    return e;
+}
+
+int stream_init(qf_ctx *ctx) {
+    QF_CUDA_TRY(ctx, (stream_set_attr<false, 16, 1>()));
+    QF_CUDA_TRY(ctx, (stream_set_attr<false, 32, 1>()));
+    QF_CUDA_TRY(ctx, (stream_set_attr<true, 16, 1>()));
+    QF_CUDA_TRY(ctx, (stream_set_attr<true, 32, 1>()));
+    QF_CUDA_TRY(ctx, (stream_set_attr<false, 16, kStreamMaxLinears>()));
+    QF_CUDA_TRY(ctx, (stream_set_attr<false, 32, kStreamMaxLinears>()));
+    QF_CUDA_TRY(ctx, (stream_set_attr<true, 16, kStreamMaxLinears>()));
+    QF_CUDA_TRY(ctx, (stream_set_attr<true, 32, kStreamMaxLinears>()));
+    return QF_OK;
+}
+
+static size_t slot_words(int64_t M) { return (size_t)((M + 1) / 2) * 2 * 128; }
+
+size_t stream_workspace_bytes(int64_t M) { return (size_t)kStreamSlots * slot_words(M) * sizeof(unsigned long long); }
+
+template <bool BF16, int NB, int CAP>
+static cudaError_t stream_go(const StreamParams<CAP> &p, int grid, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(ST_THREADS);
+    cfg.dynamicSmemBytes = (stream_smem_bytes<NB, CAP>());
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    return cudaLaunchKernelEx(&cfg, stream_kernel<BF16, NB, CAP>, p);
+}
+
+template <int CAP>
+static cudaError_t stream_dispatch(const StreamParams<CAP> &p, bool bf16, int grid, cudaStream_t s) {
+    if (p.a.M <= 16) return bf16 ? stream_go<true, 16, CAP>(p, grid, s) : stream_go<false, 16, CAP>(p, grid, s);
+    return bf16 ? stream_go<true, 32, CAP>(p, grid, s) : stream_go<false, 32, CAP>(p, grid, s);
+}
+
+namespace {
+struct Range {
+    uintptr_t lo, hi;
+    bool meets(const Range &o) const { return lo < o.hi && o.lo < hi; }
+};
+Range range_of(const void *p, int64_t bytes) { return Range{(uintptr_t)p, (uintptr_t)p + (p ? (uintptr_t)bytes : 0u)}; }
+struct Touched {
+    Range x, r, y;
+};
+Touched touched(const StreamLinear &l) {
+    const qf_linear_desc &d = *l.d;
+    const int64_t cols = d.epilogue == QF_EPI_SILU_MUL ? d.N / 2 : d.N, size = d.out_dtype == QF_F32 ? 4 : 2;
+    return Touched{range_of(l.X, d.M * d.K * 2), range_of(d.epilogue == QF_EPI_RESIDUAL_ADD ? l.residual : nullptr, d.M * cols * size),
+                   range_of(l.Y, d.M * cols * size)};
+}
+int64_t row_blocks(const qf_linear_desc &d) { return (d.N + 127) / 128; }
+}  // namespace
+
+template <int CAP>
+static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s) {
+    StreamParams<CAP> p;
+    const qf_linear_desc &d0 = *l[0].d;
+    p.a.slots = (unsigned long long *)((char *)ws + counter_bytes);
+    p.a.done = (unsigned *)ws;
+    p.a.status = ctx->dev_status;
+    p.a.slot_words = (int)slot_words(d0.M);
+    p.a.M = (int)d0.M;
+    p.a.x_rows = (int)((d0.M + 7) / 8) * 8;
+    const void *x_of[StreamParams<CAP>::XCAP];
+    int64_t x_k[StreamParams<CAP>::XCAP];
+    int maps = 0, phases = 0;
+    int64_t most = 0, work = 0, slots = 0;
+    std::vector<Touched> in_phase;
+    for (int i = 0; i < count; ++i) {
+        const qf_linear_desc &d = *l[i].d;
+        const Touched t = touched(l[i]);
+        const int64_t pieces = row_blocks(d) * l[i].split;
+        bool next = phases == 0;
+        for (const Touched &o : in_phase)
+            next = next || o.y.meets(t.x) || o.y.meets(t.r) || o.y.meets(t.y) || t.y.meets(o.x) || t.y.meets(o.r);
+        if (next || slots + pieces > kStreamSlots) {  // (a piece that is a whole row block needs no slot, but has a number)
+            p.ph[phases++] = StreamPhase{i, 0, 0, 0, 0, 0};
+            work = slots = 0;
+            in_phase.clear();
+        }
+        in_phase.push_back(t);
+        StreamEntry &e = p.e[i];
+        e.Y = l[i].Y;
+        e.residual = l[i].residual;
+        e.N = (int)d.N;
+        e.chunks = (int)(d.K / 128);
+        e.split = l[i].split;
+        e.per = l[i].per;
+        e.begin = (int)work;
+        work += CAP == 1 ? row_blocks(d) * e.chunks : pieces;
+        slots += pieces;
+        e.end = (int)work;
+        e.out_dtype = (int16_t)d.out_dtype;
+        e.epilogue = (int16_t)d.epilogue;
+        p.ph[phases - 1].pieces = (int)work;
+        most = std::max(most, work);
+        int st = get_slab_map(ctx, &p.w[i], l[i].blob, (uint64_t)(d.N / 64), (uint64_t)e.chunks);
+        if (st != QF_OK) return st;
+        e.x_map = 0;
+        while (e.x_map < maps && !(x_of[e.x_map] == l[i].X && x_k[e.x_map] == d.K)) ++e.x_map;
+        if (e.x_map == maps) {
+            x_of[maps] = l[i].X;
+            x_k[maps] = d.K;
+            st = get_tensor_map(ctx, &p.x[maps++], l[i].X, 1, (uint64_t)d.K, (uint64_t)d.M, 64, (uint32_t)p.a.x_rows,
+                                CU_TENSOR_MAP_SWIZZLE_128B);
+            if (st != QF_OK) return st;
+        }
+    }
+    const int grid = (int)std::min<int64_t>(std::min(ctx->sm_count, kSmCount), (most + 1) / 2), streams = 2 * grid;
+    for (int q = 0; q < phases; ++q) {
+        StreamPhase &ph = p.ph[q];
+        ph.streams = streams;
+        ph.active = std::min(ph.pieces, streams);
+        ph.q = ph.pieces / streams;
+        ph.r = ph.pieces % streams;
+        if (CAP == 1) ph.pieces = 0;
+    }
+    p.a.phases = phases;
+    p.a.linears = count;
+    const cudaError_t e = stream_dispatch<CAP>(p, d0.act_dtype == QF_BF16, grid, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return kStreamNoRoom;
+    }
+    return launched(ctx, e, "streaming linear");
+}
+
+int launch_stream(qf_ctx *ctx, const StreamLinear &l, void *ws, size_t counter_bytes, cudaStream_t s) {
+    return stream_launch<1>(ctx, &l, 1, ws, counter_bytes, s);
+}
+
+int launch_stream_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s) {
+    return stream_launch<kStreamMaxLinears>(ctx, l, count, ws, counter_bytes, s);
+}
+
+int stream_chain_length(const StreamLinear *l, int count) {
+    constexpr int XCAP = StreamParams<kStreamMaxLinears>::XCAP;
+    const void *x_of[XCAP];
+    int64_t x_k[XCAP];
+    std::vector<Range> written;
+    int maps = 0, n = 0;
+    for (; n < count && n < kStreamMaxLinears; ++n) {
+        const qf_linear_desc &d = *l[n].d;
+        if (d.M != l[0].d->M || d.act_dtype != l[0].d->act_dtype || row_blocks(d) * l[n].split > (1 << 24)) break;
+        int m = 0;
+        while (m < maps && !(x_of[m] == l[n].X && x_k[m] == d.K)) ++m;
+        if (m == XCAP) break;
+        // weights are read ahead of the phases: they must not be an earlier linear's result
+        const Range w = range_of(l[n].blob, d.N / 64 * (d.K / 128) * QF_SLAB_UNIT_BYTES);
+        bool meets = false;
+        for (const Range &y : written) meets = meets || y.meets(w);
+        if (meets) break;
+        if (m == maps) {
+            x_of[maps] = l[n].X;
+            x_k[maps++] = d.K;
+        }
+        const Range y = touched(l[n]).y;
+        bool known = false;
+        for (const Range &o : written) known = known || (o.lo <= y.lo && y.hi <= o.hi);
+        if (!known) written.push_back(y);
+    }
+    return n;
+}
+
+}  // namespace qf

@@ -1,0 +1,34 @@
+// Host interface of the streaming tcgen05 kernel on QF_LAYOUT_GEMV_SLAB weights (qf_stream.cu).
+#pragma once
+
+#include "qf_common.cuh"
+
+namespace qf {
+
+constexpr int kStreamMaxLinears = 112;  // of one launch: the tensor maps travel as kernel parameters (32 764 bytes)
+
+constexpr int kStreamSlots = 4 * kSmCount;  // two for each of the two streams of an SM
+
+// A checked linear on slab weights. In a chain K is cut into `split` pieces of `per` chunks of 128 codes.
+struct StreamLinear {
+    const qf_linear_desc *d;
+    const void *X, *blob, *residual;
+    void *Y;
+    int split, per;
+};
+
+// Returned by the launches where the current context has fewer SMs than the device (a partition of it), so that the blocks of a
+// cooperative launch do not fit: nothing was launched, and the other kernels serve.
+constexpr int kStreamNoRoom = 1;
+
+int stream_init(qf_ctx *ctx);
+// Bytes behind the counter region of the workspace, for linears of M rows.
+size_t stream_workspace_bytes(int64_t M);
+int launch_stream(qf_ctx *ctx, const StreamLinear &l, void *ws, size_t counter_bytes, cudaStream_t s);
+// How many of the linears from the first on one launch can take: the same rows and activation type, weights that no earlier one
+// writes.
+int stream_chain_length(const StreamLinear *l, int count);
+// Linears of one launch, each seeing the results of the earlier ones.
+int launch_stream_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s);
+
+}  // namespace qf

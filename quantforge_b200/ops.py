@@ -398,6 +398,56 @@ def w4a16_linear(x: torch.Tensor, qweight, scales: Optional[torch.Tensor] = None
     return out
 
 
+CHAIN_LINEARS = 112  # linears that one launch takes (see qf_w4a16_linear_batched)
+
+
+class LinearBatch:
+    """Linears on slab weights that run one after the other, each seeing the results of the earlier ones, enqueued by one call:
+    `calls` is a sequence of (x, SlabWeight, out, epilogue, residual or None) with the meaning they have in `w4a16_linear`. The
+    tensors are kept and read where they are at each `run()`, which may be captured. Linears of 9 to 32 rows go to the GPU as one
+    launch, up to CHAIN_LINEARS of them, with the bits that the tcgen05 kernel gives on other layouts."""
+
+    def __init__(self, calls):
+        calls = list(calls)
+        if not calls:
+            raise ValueError("a batch needs at least one linear")
+        n = len(calls)
+        self._tensors = [(x, w.blob, out, residual) for x, w, out, _, residual in calls]
+        self.device = _need_cuda(*[t for ts in self._tensors for t in ts])
+        self._descs = (LinearDesc * n)()
+        for d, (x, w, out, epilogue, residual) in zip(self._descs, calls):
+            if x.dim() != 2 or x.shape[1] != w.K or not x.is_contiguous() or x.dtype != w.act_dtype:
+                raise ValueError(f"x must be a contiguous [M, {w.K}] tensor of the dtype the slab was built for")
+            shape = (x.shape[0], w.N // 2 if epilogue == QF_EPI_SILU_MUL else w.N)
+            if tuple(out.shape) != shape or out.dtype not in _DT or not out.is_contiguous():
+                raise ValueError(f"out must be a contiguous {list(shape)} tensor")
+            if epilogue == QF_EPI_RESIDUAL_ADD and (residual is None or tuple(residual.shape) != shape or
+                                                    residual.dtype != out.dtype or not residual.is_contiguous()):
+                raise ValueError("QF_EPI_RESIDUAL_ADD needs a contiguous residual of the output's shape and dtype")
+            d.M, d.N, d.K, d.group_size = x.shape[0], w.N, w.K, w.group_size
+            d.act_dtype, d.out_dtype, d.zero_mode, d.zero_const = _DT[x.dtype], _DT[out.dtype], w.zero_mode, w.zero_const
+            d.path, d.weight_layout, d.epilogue = QF_PATH_AUTO, QF_LAYOUT_GEMV_SLAB, epilogue
+        self._arrays = [(ctypes.c_void_p * n)(*[t.data_ptr() if t is not None else 0 for t in col]) for col in zip(*self._tensors)]
+        self._ws_bytes = max(workspace_bytes(d) for d in self._descs)
+
+    @staticmethod
+    def key(calls):
+        """What a batch of these calls is made of: equal keys, the same launch."""
+        return [(x.data_ptr(), x.shape, x.stride(), x.dtype, w.blob.data_ptr(), w.N, w.K, out.data_ptr(), out.shape, out.dtype, epilogue,
+                 None if residual is None else (residual.data_ptr(), residual.shape, residual.dtype))
+                for x, w, out, epilogue, residual in calls]
+
+    def run(self) -> None:
+        dev = self.device
+        ctx = _ctx(dev)
+        x, w, out, residual = self._arrays
+        with torch.cuda.device(dev):
+            ws = _workspace(dev, self._ws_bytes)
+            st = _lib.load().qf_w4a16_linear_batched(ctx, len(self._descs), self._descs, x, w, None, None, out, residual, _ptr(ws),
+                                                     ws.numel() if ws is not None else 0, _stream(dev))
+        _check(st, ctx)
+
+
 class Comm:
     """Exchange buffers of a group of ranks (one process per GPU of one node) for `w4a16_linear_allreduce`.
 

@@ -14,7 +14,8 @@ Modes
   fused_allreduce  (world > 1, batch <= 64) the row-parallel o and down linears sum across ranks inside the kernel
                    over NVLink peer memory instead of being followed by an NCCL all-reduce
 Batches of up to 8 rows read QF_LAYOUT_GEMV_SLAB weights (the streaming GEMV kernel), larger ones the
-interleaved layout of the tcgen05 kernel.
+interleaved layout of the tcgen05 kernel. On one GPU, 9 to 16 rows of large linears read slab weights too and
+run as a chain: one launch for up to 112 linears, the same results bit for bit.
 """
 from __future__ import annotations
 
@@ -30,6 +31,14 @@ LLAMA3_8B = {"hidden": 4096, "kv": 1024, "ffn": 14336, "layers": 32}
 LLAMA3_70B = {"hidden": 8192, "kv": 1024, "ffn": 28672, "layers": 80}
 GROUP = 128
 SLAB_BATCH = 8  # up to here the streaming GEMV kernel is the faster one (measured); beyond, the tcgen05 kernel
+# Batches above SLAB_BATCH run as a chain where a linear has so many bytes of codes on average. Measured, us a step, linear by linear
+# -> chain, 9 / 16 rows:
+#   fused    hidden 4096 (27 MB) 1556 -> 1410 / 1578 -> 1456, 8192 (107 MB) 774 -> 745 / 777 -> 761, 3072 (12 MB) 512 -> 484 / 526 -> 542,
+#            2048 (6 MB) 606 -> 598 / 616 -> 634
+#   unfused  hidden 4096 (16 MB) 2005 -> 1624 / 2036 -> 1719, 3072 (7 MB) 709 -> 536 / 729 -> 587, 8192 (61 MB) 837 -> 766 / 842 -> 775
+# At 24 and 32 rows the fused hidden 4096 takes 1632 -> 1628 and 1644 -> 1717, smaller ones lose up to 25 %.
+CHAIN_BATCH = 16
+CHAIN_BYTES_FUSED, CHAIN_BYTES_UNFUSED = 13_000_000, 6_000_000
 SAMPLE_COLUMNS = 64  # output columns per linear of layer 0 kept on the CPU for `check_parity`
 
 
@@ -43,7 +52,8 @@ class _Linear:
     """One quantised linear of the stack in the layout its kernel reads, plus (layer 0 only) a CPU copy of a few
     weight rows in canonical form for the parity check."""
 
-    def __init__(self, N, K, dtype, dev, gen, batch, exchange: bool, silu: bool = False, sample: bool = False):
+    def __init__(self, N, K, dtype, dev, gen, batch, exchange: bool, silu: bool = False, sample: bool = False,
+                 chain: bool = False):
         self.N, self.K, self.silu = N, K, silu
         G = K // GROUP
         qw = torch.randint(-128, 128, (N, K // 2), dtype=torch.int8, device=dev, generator=gen)
@@ -63,7 +73,7 @@ class _Linear:
         zr = ops.pack_zeros_u4(z8)
         self.slab = None
         self.layout = QF_LAYOUT_CANONICAL
-        if batch <= SLAB_BATCH and N % 64 == 0 and not exchange:
+        if (batch <= SLAB_BATCH or chain) and N % 64 == 0 and not exchange:
             self.slab = ops.prepack_gemv_slab(qw, sc, zr, GROUP)
             self.qw = self.sc = self.zr = None
         else:
@@ -105,10 +115,14 @@ class DecodeLinearStack:
                 raise ValueError("fused_allreduce needs batch <= 64")
             self.comm = ops.Comm(batch * H, device=self.dev, group=group)
         exch = self.comm is not None and not exchange_in_slab_kernel
+        codes = (2 * H * H + 2 * H * KV + 3 * H * F) // 2  # bytes of a layer's codes
+        self.chain = (world == 1 and SLAB_BATCH < batch <= CHAIN_BATCH and H % 128 == 0 and KV % 128 == 0 and F % 128 == 0 and
+                      codes >= (4 * CHAIN_BYTES_FUSED if fuse else 7 * CHAIN_BYTES_UNFUSED))
+        self._batch = None
         self.layers = []
         for li in range(self.L):
             s = li == 0
-            mk = lambda N, K, exchange=False, silu=False: _Linear(N, K, dtype, self.dev, gen, batch, exchange, silu, s)  # noqa: E731
+            mk = lambda N, K, exchange=False, silu=False: _Linear(N, K, dtype, self.dev, gen, batch, exchange, silu, s, self.chain)  # noqa: E731
             if fuse:
                 self.layers.append({
                     "qkv": mk((H + 2 * KV) // world, H),
@@ -159,9 +173,28 @@ class DecodeLinearStack:
 
     def close(self):
         self._graph = None
+        self._batch = None
         if self.comm is not None:
             self.comm.close()
             self.comm = None
+
+    def _chain_calls(self):
+        """The linears of a step as (x, weights, out, epilogue, residual), in the order in which `_layer` calls them."""
+        b, calls, h = self.buf, [], self.buf["h_in"]
+        for ly in self.layers:
+            if self.fuse:
+                add = QF_EPI_RESIDUAL_ADD if self.residual else QF_EPI_NONE
+                up, epi = (b["act"], QF_EPI_SILU_MUL) if self.epilogues else (b["gate_up"], QF_EPI_NONE)
+                calls += [(h, ly["qkv"].slab, b["qkv"], QF_EPI_NONE, None),
+                          (b["attn"], ly["o"].slab, b["o"], add, h if self.residual else None),
+                          (b["o"], ly["gate_up"].slab, up, epi, None),
+                          (b["act"], ly["down"].slab, b["down"], add, b["o"] if self.residual else None)]
+            else:
+                calls += [(h, ly[n].slab, b[n], QF_EPI_NONE, None) for n in ("q", "k", "v")]
+                calls += [(b[x], ly[n].slab, b[n], QF_EPI_NONE, None) for x, n in (("q", "o"), ("o", "gate"), ("o", "up"),
+                                                                                   ("gate", "down"))]
+            h = b["down"]
+        return calls
 
     def _layer(self, ly, h):
         b = self.buf
@@ -185,6 +218,13 @@ class DecodeLinearStack:
 
     def step(self) -> torch.Tensor:
         """One token step through all layers, from buf["h_in"]; returns the last hidden state buffer."""
+        if self.chain:
+            calls = self._chain_calls()
+            key = ops.LinearBatch.key(calls)  # another buffer or weight in the place of one makes another batch
+            if self._batch is None or self._batch[0] != key:
+                self._batch = (key, ops.LinearBatch(calls))
+            self._batch[1].run()
+            return calls[-1][2]
         h = self.buf["h_in"]
         for ly in self.layers:
             h = self._layer(ly, h)
@@ -216,7 +256,8 @@ class DecodeLinearStack:
         return out_host
 
     def launches_per_step(self) -> int:
-        return (4 if self.fuse else 7) * self.L
+        n = (4 if self.fuse else 7) * self.L
+        return -(-n // ops.CHAIN_LINEARS) if self.chain else n
 
     def bytes_per_step(self) -> int:
         """Algorithmic bytes of the whole (unsharded) token step."""
@@ -229,7 +270,7 @@ class DecodeLinearStack:
 
     # ------------------------------------------------------------------------------------------
     def check_parity(self, oracle_linear: Callable, silu_mul: Callable) -> dict:
-        """Runs every linear of layer 0 through the call path `step` uses and compares SAMPLE_COLUMNS output columns
+        """Runs every linear of layer 0 through the call path `step` uses (those of a chain one by one) and compares SAMPLE_COLUMNS output columns
         with `oracle_linear(x, qweight_rows, scales, zeros, group) -> float array [M, rows]` (a CPU restatement the
         caller provides; this package has none). Row-parallel linears are compared after the sum over ranks, with
         the oracle's partial sums added across ranks in float64; every rank must also hold identical bits.
