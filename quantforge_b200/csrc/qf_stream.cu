@@ -9,11 +9,13 @@
 //
 // Work split. Units of 128 rows x 128 codes. Of a single linear they are numbered row block major, K chunk minor, and stream i of G
 // owns a contiguous range of them (the first r streams one more than the others): every stream moves the same number of bytes
-// whatever the shape is. A chain is a list of phases; the linears of a phase do not depend on each other, a phase needs the results
-// of the earlier ones. There K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same sizes on other
+// whatever the shape is. A chain is a list of phases, each of linears that do not depend on each other, and each with the phases that
+// it waits for. What the next step of the chain does not touch (q, k and v beside o) is a phase of its own that holds nothing up: it
+// goes to streams that have nothing to do in that step, or fills the time in which the others hand over (the linears of 32 layers at
+// 16 rows 1459 -> 1355 us). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same sizes on other
 // layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any other order
 // into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least surprise).
-// The pieces of a phase are dealt to the streams one after the other. Weights are requested as far ahead as the ring of stages allows,
+// The pieces of a phase are dealt to the streams forwards and backwards in turn. Weights are requested as far ahead as the ring of stages allows,
 // across linears and phases; only the activations of a phase wait for the phase before it.
 //
 // A thread block has its SM to itself and runs two streams side by side (one stream's waits are the other's time to convert), each
@@ -29,8 +31,7 @@
 // Row blocks whose K range is shared by several streams (its members): a member leaves its partial sums in a slot of the workspace
 // as 8-byte (value, token) words - no fence, no atomic. The members finish the pairs of batch rows in turn (one member
 // reading ten others' sums of 16 rows would be a dozen trips to L2 in a row): whoever finishes a pair polls all members' words
-// (bounded), adds in their order (deterministic), writes Y and clears the words for the next user of the slots. The next phase starts
-// when this one is finished. As streams wait for one another, the launch is cooperative, and without programmatic dependent launch:
+// (bounded), adds in their order (deterministic), writes Y and clears the words for the next user of the slots. As streams wait for one another, the launch is cooperative, and without programmatic dependent launch:
 // it would find no room beside another kernel's blocks.
 //
 // Shared memory takes all but a few KB of the SM's first-level cache, so a spilled register is a trip to L2: the registers are split
@@ -59,7 +60,7 @@ struct StreamCfg {
     static constexpr int X_BYTES = 2 * X_BOX_BYTES;
     static constexpr int W_OFF = X_STAGES * X_BYTES;
     static constexpr int BAR_OFF = W_OFF + W_STAGES * ST_UNIT_BYTES;
-    static constexpr int BARS = 2 * W_STAGES + 2 * X_STAGES + 2 * ST_NA + 2 * 2 + 1;
+    static constexpr int BARS = 2 * W_STAGES + 2 * X_STAGES + 2 * ST_NA + 2 * 2;
     static constexpr int STREAM_BYTES = (BAR_OFF + BARS * 8 + 1023) / 1024 * 1024;
     static_assert(2 * NB + ST_NA * 64 <= ST_TMEM_COLS, "two accumulators and the A operands");
 };
@@ -70,19 +71,22 @@ struct StreamEntry {  // one linear
     int N, chunks;   // chunks of 128 codes along K
     int begin, end;  // its units (or pieces) within the phase
     int split, per;  // pieces: K is cut into `split` of them, `per` chunks each (the last may be shorter)
+    int slot;        // of its first piece, where there are several to a row block
     int x_map;
     int16_t out_dtype, epilogue;
 };
 struct StreamPhase {
-    int first;    // entry
-    int pieces;   // 0: ranges of units; else how many pieces the phase has
-    int q, r;     // ranges: units of the phase = q * G + r, streams 0..r-1 have q + 1
-    int streams;  // G
-    int active;   // streams that have work
+    int first;       // entry
+    int pieces;      // 0: ranges of units; else how many pieces the phase has
+    int q, r;        // ranges: units of the phase = q * G + r, streams 0..r-1 have q + 1
+    int streams;     // ranges: G; pieces: the streams from `home` on that they are dealt to, forwards and backwards in turn
+    int home, flip;  // flip: backwards first
+    int active;      // streams that have work
+    int wait[2];     // phases that are complete before this one reads or writes anything (or -1)
 };
 struct StreamArgs {
     unsigned long long *slots;  // [kStreamSlots][slot_words] (value | token << 32), zero between launches
-    unsigned *done;             // [phases] result warps that have finished the phase, zero between launches
+    unsigned *done;             // [phases] result warps that have finished the phase, [kStreamMaxLinears] all; zero between launches
     int *status;
     int slot_words;
     int M, x_rows;              // x_rows: rows of an X box (M rounded up to 8)
@@ -98,6 +102,7 @@ struct StreamParams {
     StreamArgs a;
 };
 static_assert(sizeof(StreamParams<kStreamMaxLinears>) <= 32764, "kernel parameters");
+static_assert((kStreamMaxLinears + 1) * sizeof(unsigned) <= 65536, "the counter region of the workspace");
 // The lists of linears and phases, in shared memory: every role reads the next phase's when it gets there, and from the parameter
 // space that was a miss of the constant cache each time.
 template <int CAP>
@@ -118,10 +123,21 @@ struct Segment {
     int e, b, c, len;
     int members, self, slot0, base;
 };
-// Units of stream `id` in a phase: how many, and *u0 the first. Pieces: whether it has any.
+// Units of stream `id` in a phase: how many, and *u0 the first.
 __device__ __forceinline__ int stream_range(const StreamPhase &ph, int id, int *u0) {
     *u0 = id * ph.q + min(id, ph.r);
-    return ph.pieces ? id < ph.pieces : ph.q + (id < ph.r ? 1 : 0);
+    return ph.q + (id < ph.r ? 1 : 0);
+}
+// The piece that stream `id` gets in a round of dealing (none: a number from ph.pieces on).
+__device__ __forceinline__ int stream_piece(const StreamPhase &ph, int id, int round) {
+    const int k = id - ph.home;
+    if ((unsigned)k >= (unsigned)ph.streams) return ph.pieces;
+    return round * ph.streams + ((round ^ ph.flip) & 1 ? ph.streams - 1 - k : k);
+}
+template <int CAP>
+__device__ __forceinline__ bool stream_works(const StreamPhase &ph, int id) {
+    int u;
+    return CAP > 1 ? stream_piece(ph, id, 0) < ph.pieces : stream_range(ph, id, &u) > 0;
 }
 // The stream that has unit u.
 __device__ __forceinline__ int stream_of(const StreamPhase &ph, int u) {
@@ -132,15 +148,11 @@ __device__ __forceinline__ int stream_of(const StreamPhase &ph, int u) {
 template <int CAP, typename F>
 __device__ __forceinline__ void for_segments(const StreamTables<CAP> &t, int phase, int id, F f) {
     const StreamPhase ph = t.ph[phase];
-    int u;
-    const int n = stream_range(ph, id, &u);
-    if (n <= 0) return;
     int e = ph.first;
     Segment g;
     if (CAP > 1) {
-        // dealt to the streams forwards and backwards in turn: the next linear's pieces go first to streams that have none or short ones
         for (int round = 0;; ++round) {
-            const int j = round * ph.streams + (round & 1 ? ph.streams - 1 - id : id);
+            const int j = stream_piece(ph, id, round);
             if (j >= ph.pieces) return;
             while (j >= t.e[e].end) ++e;
             const int split = t.e[e].split, local = j - t.e[e].begin;
@@ -150,10 +162,13 @@ __device__ __forceinline__ void for_segments(const StreamTables<CAP> &t, int pha
             g.c = g.self * t.e[e].per;
             g.len = min(t.e[e].per, t.e[e].chunks - g.c);
             g.members = split;
-            g.base = g.slot0 = j - g.self;
+            g.base = g.slot0 = t.e[e].slot + g.b * split;
             if (!f(g)) return;
         }
     }
+    int u;
+    const int n = stream_range(ph, id, &u);
+    if (n == 0) return;
     const int end = u + n, chunks = t.e[e].chunks;
     g.e = e;
     g.b = u / chunks;
@@ -304,6 +319,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
     extern __shared__ uint8_t stream_smem[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
+    __shared__ int s_gates[2];  // of a stream: phases whose waits are over (those that it has work in)
 
     const int tid = threadIdx.x & 511;
     const int half = threadIdx.x >> 9;
@@ -327,7 +343,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
     auto aempty = [&](int a) { return bars + 8u * (AB + ST_NA + a); };
     auto dfull = [&](int d) { return bars + 8u * (AB + 2 * ST_NA + d); };
     auto dempty = [&](int d) { return bars + 8u * (AB + 2 * ST_NA + 2 + d); };
-    const uint32_t gate = bars + 8u * (AB + 2 * ST_NA + 4);
+    volatile int *gates = &s_gates[half];
 
     const StreamArgs &a = p.a;
     StreamTables<CAP> &t = *reinterpret_cast<StreamTables<CAP> *>(
@@ -353,7 +369,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
             mbar_init(dfull(d), 1);
             mbar_init(dempty(d), 4);
         }
-        mbar_init(gate, 1);
+        s_gates[half] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 10 && half == 0) tmem_alloc<false>(smem_u32(&s_tmem_base), 2 * ST_TMEM_COLS);
@@ -373,7 +389,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
     const uint32_t tmem = s_tmem_base + (uint32_t)half * ST_TMEM_COLS;  // two accumulators of NB columns, then the A operands
 
     // Registers: 64 a thread at launch; a stream's four warpgroups share them as 2 x 48, 56 and 104. With 64 for all, the result warps
-    // spilled addresses and sums in flight: the linears of 32 layers at 16 rows took 1971 us, with 64, 40 and 88 1557, with this 1495.
+    // spilled addresses and sums in flight: a first form of the chain took 1971 us for 32 layers at 16 rows, with 64, 40 and 88 1557,
+    // with this 1495.
     if (role == 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     else if (role == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -410,24 +427,29 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
             uint32_t ph = 0;
             bool ok = true;
             const uint32_t tx = 2u * (uint32_t)a.x_rows * 128u;
+            int passed[2] = {-1, -1}, opened = 0;
             for (int phase = 0; phase < phases && ok; ++phase) {
-                bool behind = phase > 0;
+                bool behind = CAP > 1 && (t.ph[phase].wait[0] >= 0 || t.ph[phase].wait[1] >= 0);
                 for_segments(t, phase, id, [&](const Segment &g) {
                     if (behind) {
-                        // all results of the phase before are in memory
-                        const long long t0 = clock64();
-                        while (ld_acquire(a.done + phase - 1) < 4u * (unsigned)t.ph[phase - 1].active) {
-                            if (*abort_flag) return ok = false;
-                            if (clock64() - t0 > kWaitCycles) {
-                                *abort_flag = 1;
-                                return ok = false;
+                        for (int i = 0; i < 2; ++i) {
+                            const int w = t.ph[phase].wait[i];
+                            if (w < 0 || w == passed[i]) continue;
+                            const unsigned want = 4u * (unsigned)t.ph[w].active;
+                            const long long t0 = clock64();
+                            while (ld_acquire(a.done + w) < want) {
+                                if (*abort_flag) return ok = false;
+                                if (clock64() - t0 > kWaitCycles) {
+                                    *abort_flag = 1;
+                                    return ok = false;
+                                }
                             }
+                            passed[i] = w;
                         }
-                        // they were stored through the generic proxy and are read by the copy engine
+                        // the results were stored through the generic proxy and are read by the copy engine
                         fence_proxy_async_all();
-                        mbar_arrive(gate);
-                        // the phase before is complete: nobody waits for the one before that any more
-                        if (id == 0 && phase > 1) a.done[phase - 2] = 0u;
+                        __threadfence_block();
+                        *gates = ++opened;
                         behind = false;
                     }
                     const CUtensorMap *map = &p.x[t.e[g.e].x_map];
@@ -568,14 +590,21 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
         const int row = quad * 32 + lane;
         const uint32_t lane_tmem = tmem + ((uint32_t)(quad * 32) << 16);
         int seg = 0;
-        uint32_t gph = 0;
+        int opened = 0;
         bool ok = true;
         for (int phase = 0; phase < phases; ++phase) {
-            int u0;
-            if (stream_range(t.ph[phase], id, &u0) <= 0) continue;
-            if (phase > 0) {
-                ok = __all_sync(0xffffffffu, ok && stream_wait(gate, gph, abort_flag));
-                gph ^= 1u;
+            if (!stream_works<CAP>(t.ph[phase], id)) continue;
+            if (CAP > 1 && (t.ph[phase].wait[0] >= 0 || t.ph[phase].wait[1] >= 0)) {
+                // idle until then: the results come behind the activations. (Not a barrier's phase: the other side may be two ahead.)
+                ++opened;
+                const long long t0 = clock64();
+                while (ok && *gates < opened) {
+                    __nanosleep(100);
+                    if (*abort_flag) ok = false;
+                    else if (clock64() - t0 > kWaitCycles) *abort_flag = 1;
+                }
+                ok = __all_sync(0xffffffffu, ok);
+                __threadfence_block();
             }
             for_segments(t, phase, id, [&](const Segment &g) {
                 const int d = seg & 1;
@@ -625,16 +654,18 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
                 }
                 return true;
             });
-            if (phases > 1) {
+            if (CAP > 1) {
                 __syncwarp();
-                if (lane == 0 && ok) {
-                    if (phase < phases - 1) {
-                        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.done + phase) : "memory");
-                    } else if (atomicAdd(a.done + phase, 1u) + 1u == 4u * (unsigned)t.ph[phase].active) {
-                        a.done[phase - 1] = 0u;
-                        a.done[phase] = 0u;
-                    }
-                }
+                if (lane == 0 && ok) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.done + phase) : "memory");
+            }
+        }
+        if (CAP > 1 && lane == 0 && ok) {
+            // The last result warp of the launch leaves the counters as they were: behind everybody's last count and wait.
+            unsigned before;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.done + kStreamMaxLinears) : "memory");
+            if (before + 1u == 8u * gridDim.x) {
+                for (int q = 0; q < phases; ++q) a.done[q] = 0u;
+                a.done[kStreamMaxLinears] = 0u;
             }
         }
     }
@@ -719,6 +750,8 @@ struct Range {
 Range range_of(const void *p, int64_t bytes) { return Range{(uintptr_t)p, (uintptr_t)p + (p ? (uintptr_t)bytes : 0u)}; }
 struct Touched {
     Range x, r, y;
+    // Whether this linear has to come behind an earlier one: reads what that writes, writes what that reads or writes.
+    bool after(const Touched &o) const { return o.y.meets(x) || o.y.meets(r) || o.y.meets(y) || y.meets(o.x) || y.meets(o.r); }
 };
 Touched touched(const StreamLinear &l) {
     const qf_linear_desc &d = *l.d;
@@ -741,38 +774,24 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
     p.a.x_rows = (int)((d0.M + 7) / 8) * 8;
     const void *x_of[StreamParams<CAP>::XCAP];
     int64_t x_k[StreamParams<CAP>::XCAP];
-    int maps = 0, phases = 0;
-    int64_t most = 0, work = 0, slots = 0;
-    std::vector<Touched> in_phase;
-    for (int i = 0; i < count; ++i) {
+    int maps = 0, phases = 0, next = 0;
+    // The linear at `i` becomes the next entry, of the phase at hand.
+    auto enter = [&](int i) {
         const qf_linear_desc &d = *l[i].d;
-        const Touched t = touched(l[i]);
-        const int64_t pieces = row_blocks(d) * l[i].split;
-        bool next = phases == 0;
-        for (const Touched &o : in_phase)
-            next = next || o.y.meets(t.x) || o.y.meets(t.r) || o.y.meets(t.y) || t.y.meets(o.x) || t.y.meets(o.r);
-        if (next || slots + pieces > kStreamSlots) {  // (a piece that is a whole row block needs no slot, but has a number)
-            p.ph[phases++] = StreamPhase{i, 0, 0, 0, 0, 0};
-            work = slots = 0;
-            in_phase.clear();
-        }
-        in_phase.push_back(t);
-        StreamEntry &e = p.e[i];
+        StreamPhase &ph = p.ph[phases - 1];
+        StreamEntry &e = p.e[next];
         e.Y = l[i].Y;
         e.residual = l[i].residual;
         e.N = (int)d.N;
         e.chunks = (int)(d.K / 128);
         e.split = l[i].split;
         e.per = l[i].per;
-        e.begin = (int)work;
-        work += CAP == 1 ? row_blocks(d) * e.chunks : pieces;
-        slots += pieces;
-        e.end = (int)work;
+        e.slot = 0;
+        e.begin = ph.pieces;
+        e.end = ph.pieces += (int)row_blocks(d) * (CAP == 1 ? e.chunks : e.split);
         e.out_dtype = (int16_t)d.out_dtype;
         e.epilogue = (int16_t)d.epilogue;
-        p.ph[phases - 1].pieces = (int)work;
-        most = std::max(most, work);
-        int st = get_slab_map(ctx, &p.w[i], l[i].blob, (uint64_t)(d.N / 64), (uint64_t)e.chunks);
+        int st = get_slab_map(ctx, &p.w[next++], l[i].blob, (uint64_t)(d.N / 64), (uint64_t)e.chunks);
         if (st != QF_OK) return st;
         e.x_map = 0;
         while (e.x_map < maps && !(x_of[e.x_map] == l[i].X && x_k[e.x_map] == d.K)) ++e.x_map;
@@ -781,17 +800,96 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
             x_k[maps] = d.K;
             st = get_tensor_map(ctx, &p.x[maps++], l[i].X, 1, (uint64_t)d.K, (uint64_t)d.M, 64, (uint32_t)p.a.x_rows,
                                 CU_TENSOR_MAP_SWIZZLE_128B);
-            if (st != QF_OK) return st;
         }
-    }
-    const int grid = (int)std::min<int64_t>(std::min(ctx->sm_count, kSmCount), (most + 1) / 2), streams = 2 * grid;
-    for (int q = 0; q < phases; ++q) {
-        StreamPhase &ph = p.ph[q];
-        ph.streams = streams;
-        ph.active = std::min(ph.pieces, streams);
-        ph.q = ph.pieces / streams;
-        ph.r = ph.pieces % streams;
-        if (CAP == 1) ph.pieces = 0;
+        return st;
+    };
+    const int sms = std::min(ctx->sm_count, kSmCount);
+    int grid = 1;
+    if (CAP == 1) {
+        p.ph[phases++] = StreamPhase{0, 0, 0, 0, 0, 0, 0, 0, {-1, -1}};
+        const int st = enter(0);
+        if (st != QF_OK) return st;
+        StreamPhase &ph = p.ph[0];
+        grid = std::min(sms, (ph.pieces + 1) / 2);
+        ph.streams = 2 * grid;
+        ph.q = ph.pieces / ph.streams;
+        ph.r = ph.pieces % ph.streams;
+        ph.pieces = 0;
+    } else {
+        // Steps: linears that do not touch each other's results, each step behind the one before. Of a step only what the next one
+        // touches holds that up; the rest ("late") is a phase of its own, which the step after the next waits for.
+        grid = sms;
+        const int streams = 2 * grid;
+        std::vector<Touched> all;
+        std::vector<int> step_of;
+        auto slots_of = [&](int i) { return l[i].split > 1 ? row_blocks(*l[i].d) * l[i].split : 0; };
+        int steps = 0;
+        int64_t slots = 0;
+        for (int i = 0; i < count; ++i) {
+            all.push_back(touched(l[i]));
+            bool fresh = steps == 0 || slots + slots_of(i) > kStreamSlots;
+            for (int o = i; !fresh && o-- > 0 && step_of[o] == steps - 1;) fresh = all[i].after(all[o]);
+            if (fresh) {
+                ++steps;
+                slots = 0;
+            }
+            slots += slots_of(i);
+            step_of.push_back(steps - 1);
+        }
+        int last = -1, late_before = -1, late = -1;  // phases: of the step before; late ones two steps back and one
+        for (int q = 0, i0 = 0; q < steps; ++q) {
+            int i1 = i0, i2;
+            while (i1 < count && step_of[i1] == q) ++i1;
+            for (i2 = i1; i2 < count && step_of[i2] == q + 1;) ++i2;
+            int64_t here = 0, there = 0;
+            for (int i = i0; i < i1; ++i) here += slots_of(i);
+            for (int i = i1; i < i2; ++i) there += slots_of(i);
+            std::vector<char> waits(i1 - i0, i1 == i2 || here + there > kStreamSlots);
+            bool any = false;
+            for (int i = i0; i < i1; ++i) {
+                for (int o = i1; o < i2; ++o) waits[i - i0] = waits[i - i0] || all[o].after(all[i]);
+                any = any || waits[i - i0];
+            }
+            if (!any) waits.assign(i1 - i0, 1);
+            // slots: from the lower end and the upper one in turn, so that a late phase and the next step have their own
+            int slot = q & 1 ? kStreamSlots - (int)here : 0;
+            const int wait0 = last, wait1 = late_before;
+            late_before = late;
+            late = -1;
+            for (int part = 0; part < 2; ++part) {
+                if (part == 1 && std::find(waits.begin(), waits.end(), 0) == waits.end()) continue;  // nothing is late
+                StreamPhase &ph = p.ph[phases++];
+                ph = StreamPhase{next, 0, 0, 0, streams, 0, 0, 0, {wait0, wait1}};
+                for (int i = i0; i < i1; ++i)
+                    if ((waits[i - i0] != 0) == (part == 0)) {
+                        const int st = enter(i);
+                        if (st != QF_OK) return st;
+                        p.e[next - 1].slot = slot;
+                        slot += (int)slots_of(i);
+                    }
+                if (part == 0) {
+                    last = phases - 1;
+                } else {
+                    late = phases - 1;
+                    // to the streams that have nothing in the next step, if they can do it in that time; else to all, those first
+                    // that had nothing in this one
+                    int64_t pieces = 0, longest = 0, work = 0;
+                    for (int i = i1; i < i2; ++i) {
+                        pieces += row_blocks(*l[i].d) * l[i].split;
+                        longest = std::max<int64_t>(longest, l[i].per);
+                    }
+                    for (int e = ph.first; e < next; ++e) work += (int64_t)(p.e[e].end - p.e[e].begin) * p.e[e].per;
+                    if (pieces < streams && work <= longest * (streams - pieces)) {
+                        ph.home = (int)pieces;
+                        ph.streams = streams - (int)pieces;
+                    } else {
+                        ph.flip = 1;
+                    }
+                }
+                ph.active = std::min(ph.pieces, ph.streams);
+            }
+            i0 = i1;
+        }
     }
     p.a.phases = phases;
     p.a.linears = count;

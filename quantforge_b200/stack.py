@@ -14,7 +14,7 @@ Modes
   fused_allreduce  (world > 1, batch <= 64) the row-parallel o and down linears sum across ranks inside the kernel
                    over NVLink peer memory instead of being followed by an NCCL all-reduce
 Batches of up to 8 rows read QF_LAYOUT_GEMV_SLAB weights (the streaming GEMV kernel), larger ones the
-interleaved layout of the tcgen05 kernel. On one GPU, 9 to 16 rows of large linears read slab weights too and
+interleaved layout of the tcgen05 kernel. On one GPU, 9 to 32 rows of large linears read slab weights too and
 run as a chain: one launch for up to 112 linears, the same results bit for bit.
 """
 from __future__ import annotations
@@ -31,14 +31,24 @@ LLAMA3_8B = {"hidden": 4096, "kv": 1024, "ffn": 14336, "layers": 32}
 LLAMA3_70B = {"hidden": 8192, "kv": 1024, "ffn": 28672, "layers": 80}
 GROUP = 128
 SLAB_BATCH = 8  # up to here the streaming GEMV kernel is the faster one (measured); beyond, the tcgen05 kernel
-# Batches above SLAB_BATCH run as a chain where a linear has so many bytes of codes on average. Measured, us a step, linear by linear
-# -> chain, 9 / 16 rows:
-#   fused    hidden 4096 (27 MB) 1556 -> 1410 / 1578 -> 1456, 8192 (107 MB) 774 -> 745 / 777 -> 761, 3072 (12 MB) 512 -> 484 / 526 -> 542,
-#            2048 (6 MB) 606 -> 598 / 616 -> 634
-#   unfused  hidden 4096 (16 MB) 2005 -> 1624 / 2036 -> 1719, 3072 (7 MB) 709 -> 536 / 729 -> 587, 8192 (61 MB) 837 -> 766 / 842 -> 775
-# At 24 and 32 rows the fused hidden 4096 takes 1632 -> 1628 and 1644 -> 1717, smaller ones lose up to 25 %.
-CHAIN_BATCH = 16
-CHAIN_BYTES_FUSED, CHAIN_BYTES_UNFUSED = 13_000_000, 6_000_000
+CHAIN_BATCH = 32
+
+
+def _chain_bytes(batch: int, fuse: bool) -> float:
+    """Mean bytes of codes of a linear from which batches above SLAB_BATCH run as a chain. Measured, us a step, linear by linear ->
+    chain, at 9 / 16 / 24 / 32 rows (16 layers where not said):
+      fused    1.5 MB (hidden 1024)   324 -> 319 / 323 -> 379 / 367 -> 452 / 368 -> 539
+               5.6 MB (2048)          407 -> 384 / 411 -> 406 / 451 -> 485 / 460 -> 550
+               12 MB (3072, 2048)     517 -> 457 / 525 -> 503 / 562 -> 564 / 572 -> 632,  519 -> 477 / 526 -> 483 / 564 -> 548 / 570 -> 590
+               27 MB (4096, 32 layers) 1556 -> 1333 / 1578 -> 1355 / 1607 -> 1511 / 1624 -> 1581
+               107 MB (8192, 6 layers) 774 -> 704 / 777 -> 714 / 798 -> 752 / 802 -> 786
+      unfused  0.8 MB (1024) 521 -> 398 / 521 -> 464 / 570 -> 551 / 571 -> 637,  3.2 MB (2048) 592 -> 440 / 600 -> 464 / 648 -> 534 / 652 -> 593
+               16 MB (4096, 32 layers) 2028 -> 1597 / 2032 -> 1751 / 2131 -> 1973 / 2147 -> 2153"""
+    if not fuse:
+        return 2e6
+    return 5e6 if batch <= 16 else 13e6 if batch <= 24 else 24e6
+
+
 SAMPLE_COLUMNS = 64  # output columns per linear of layer 0 kept on the CPU for `check_parity`
 
 
@@ -117,7 +127,7 @@ class DecodeLinearStack:
         exch = self.comm is not None and not exchange_in_slab_kernel
         codes = (2 * H * H + 2 * H * KV + 3 * H * F) // 2  # bytes of a layer's codes
         self.chain = (world == 1 and SLAB_BATCH < batch <= CHAIN_BATCH and H % 128 == 0 and KV % 128 == 0 and F % 128 == 0 and
-                      codes >= (4 * CHAIN_BYTES_FUSED if fuse else 7 * CHAIN_BYTES_UNFUSED))
+                      codes >= (4 if fuse else 7) * _chain_bytes(batch, fuse))
         self._batch = None
         self.layers = []
         for li in range(self.L):

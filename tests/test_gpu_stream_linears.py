@@ -92,7 +92,8 @@ def _one_by_one(calls):
 
 @pytest.mark.parametrize("M,hidden,kv,ffn,layers,dtype", [
     (9, 1024, 512, 2816, 3, torch.bfloat16), (16, 1152, 128, 1280, 2, torch.float16), (13, 4096, 1024, 14336, 2, torch.bfloat16),
-    (17, 1024, 256, 5632, 2, torch.float16), (32, 2048, 512, 2048, 2, torch.bfloat16), (10, 256, 128, 256, 30, torch.bfloat16)])
+    (17, 1024, 256, 5632, 2, torch.float16), (32, 2048, 512, 2048, 2, torch.bfloat16), (10, 256, 128, 256, 30, torch.bfloat16),
+    (9, 256, 128, 18944, 2, torch.float16), (24, 4096, 1024, 14336, 2, torch.bfloat16)])
 def test_chain_is_the_tcgen05_kernel_bit_for_bit(M, hidden, kv, ffn, layers, dtype):
     made = _layers(hidden, kv, ffn, layers, dtype)
     want, got = _buffers(M, hidden, kv, ffn, dtype), _buffers(M, hidden, kv, ffn, dtype)

@@ -41,19 +41,20 @@ def test_ranges(blocks, chunks, streams):
                 slots.add(slot)
 
 
-@pytest.mark.parametrize("pieces,streams", [(1, 2), (5, 10), (296, 296), (297, 296), (496, 296), (1000, 148), (592, 296)])
-def test_pieces_are_dealt_once(pieces, streams):
-    dealt = []
+@pytest.mark.parametrize("flip", [0, 1])
+@pytest.mark.parametrize("pieces,streams", [(1, 2), (5, 10), (296, 296), (297, 296), (496, 296), (1000, 148), (592, 296), (240, 72)])
+def test_pieces_are_dealt_once(pieces, streams, flip):
+    dealt, working = [], 0
     for s in range(streams):
         k = 0
         while True:
-            j = k * streams + (streams - 1 - s if k & 1 else s)
+            j = k * streams + (streams - 1 - s if (k ^ flip) & 1 else s)
             if j >= pieces:
                 break
             dealt.append(j)
             k += 1
-        assert (s < pieces) == (k > 0)
-    assert sorted(dealt) == list(range(pieces))
+        working += k > 0
+    assert sorted(dealt) == list(range(pieces)) and working == min(pieces, streams)
 
 
 def test_a_walk_that_ends_early_misses_nothing():
