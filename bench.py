@@ -553,7 +553,10 @@ def run_stack_workload(env, args):
     if rank == 0:
         gbs = nbytes / (ms * 1e-3) / 1e9
         per_launch_us = ms * 1e3 / launches_per_step
-        kernel = ("qf::gemv_slab_kernel" if args.batch <= 8 else "qf::stream_kernel (tcgen05, the step in few launches)" if st.chain
+        one_by_one = (4 if fuse else 7) * st.L
+        kernel = ("qf::gemv_slab_kernel" if args.batch <= 8 and st.launches_per_step() == one_by_one else
+                  "qf::slab_chain_kernel (the step in few launches)" if args.batch <= 8 else
+                  "qf::stream_kernel (tcgen05, the step in few launches)" if st.chain
                   else "qf::gemm_kernel (tcgen05)")
         if in_kernel and args.batch <= 8:
             kernel += " + qf::gemv_slab_exch_kernel (row-parallel linears)"

@@ -194,15 +194,20 @@ int qf_w4a16_linear_fused(qf_ctx *ctx, const qf_linear_desc *desc, const void *X
  * NULL). Consecutive kernels are chained with programmatic dependent launch; entry i+1 may read what entry i
  * wrote. `workspace` must hold the largest qf_w4a16_workspace_bytes over the entries. Stops at the first entry
  * that fails and returns its status (earlier entries stay enqueued).
- * Consecutive entries on QF_LAYOUT_GEMV_SLAB weights that leave path and split_k to the library and have the same M in 9..32, the
- * same act_dtype and N % 128 == 0 run as ONE cooperative launch (at most 112 linears and 16 different X; weights that an earlier
- * entry writes begin a new one): entries that do not touch each other's results run side by side, the others one behind the other,
- * and weights are fetched ahead. Their results are the bits that QF_PATH_GEMM gives for the same linear on the other layouts.
+ * Consecutive entries on QF_LAYOUT_GEMV_SLAB weights that leave path and split_k to the library and have the same M <= 32, the
+ * same act_dtype and, above 8 rows, N % 128 == 0 run as ONE cooperative launch (at most 112 linears and 16 different X; weights that
+ * an earlier entry writes begin a new one): entries that do not touch each other's results run side by side, the others one behind
+ * the other, and weights are fetched ahead. Up to 8 rows that is done where it is the faster way (a rule on the sizes), and the
+ * results are those of the linears launched one by one, bit for bit; above, the bits that QF_PATH_GEMM gives for the same linear on
+ * the other layouts.
  */
 int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs, const void *const *X,
                             const void *const *qweight, const void *const *scales, const void *const *qzeros,
                             void *const *Y, const void *const *residual, void *workspace, size_t workspace_bytes,
                             void *stream);
+/* Kernel launches that this call would make (-1: bad arguments). Nothing is enqueued. */
+int qf_w4a16_batched_launches(qf_ctx *ctx, int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight,
+                              void *const *Y, const void *const *residual, const void *workspace, size_t workspace_bytes);
 
 /*
  * The same linear for callers that hold activations in HOST memory (the reference's Python entry

@@ -58,11 +58,6 @@ bool cluster_reduce_enabled() {
     return on;
 }
 
-// The split-K arrival counters occupy a FIXED region at the start of the workspace, so that a
-// workspace reused by linears of different shapes never exposes stale partial sums as counters.
-static constexpr int kMaxCounters = 16384;
-static constexpr size_t kCounterBytes = (size_t)kMaxCounters * sizeof(int);
-
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
 // Which of the two kernels that read slab weights runs a linear called by itself. The streaming tcgen05 kernel takes its SMs whole
@@ -339,7 +334,41 @@ static bool slab_any(const qf_linear_desc *d) {
 }
 
 // Linears that qf_w4a16_linear_batched runs as one launch.
-static bool chains(const qf_linear_desc *d) { return slab_any(d) && d->M > kSlabGemvRows && d->N % 128 == 0; }
+static bool chains(const qf_linear_desc *d) {
+    // (up to kSlabGemvRows rows with the results of the call for one linear, so only what the streaming GEMV kernel serves there)
+    return slab_any(d) && (d->M <= kSlabGemvRows ? slab_chain_takes(d) && !stream_serves(d) : d->N % 128 == 0);
+}
+// The workspace of that launch.
+static size_t chain_workspace_bytes(int64_t M) {
+    return kCounterBytes + (M <= kSlabGemvRows ? slab_chain_workspace_bytes() : stream_workspace_bytes(M));
+}
+
+// How many of the linears from entry i on one launch could take, those linears, and whether it does or they go one by one. (A linear
+// with which something is wrong goes alone, and its check says what.)
+static int chain_from(qf_ctx *ctx, int i, int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight,
+                      void *const *Y, const void *const *residual, const void *workspace, size_t workspace_bytes,
+                      std::vector<StreamLinear> *run, bool *pays) {
+    run->clear();
+    for (int j = i; j < count && chains(&descs[j]); ++j) {
+        Plan plan;
+        const void *res = residual ? residual[j] : nullptr;
+        if (check_linear(ctx, &descs[j], X[j], qweight[j], nullptr, nullptr, Y[j], res, workspace, workspace_bytes, &plan) != QF_OK ||
+            workspace_bytes < chain_workspace_bytes(descs[j].M))
+            break;
+        if (descs[j].M <= kSlabGemvRows) {
+            run->push_back(StreamLinear{&descs[j], X[j], qweight[j], res, Y[j], 1, 0});
+            continue;
+        }
+        // K is cut as the tcgen05 kernel cuts it for the same sizes in its own layouts: the sums are the same bits
+        qf_linear_desc d = descs[j];
+        d.weight_layout = QF_LAYOUT_INTERLEAVED;
+        if (make_plan(&d, &plan, nullptr) != QF_OK || plan.path != QF_PATH_GEMM) break;
+        run->push_back(StreamLinear{&descs[j], X[j], qweight[j], res, Y[j], plan.split_k, plan.chunks_per_split});
+    }
+    const int n = run->size() > 1 ? stream_chain_length(run->data(), (int)run->size()) : 1;
+    *pays = n > 1 && (descs[i].M > kSlabGemvRows || slab_chain_pays(run->data(), n));
+    return std::max(n, 1);
+}
 
 static int launch_linear(qf_ctx *ctx, const qf_linear_desc *desc, const Plan &plan, const void *X, const void *qweight,
                          const void *scales, const void *qzeros_or_null, void *Y, const void *residual, void *workspace,
@@ -406,6 +435,7 @@ int qf_ctx_create(qf_ctx **out, int device) {
     if (st == QF_OK) st = gemm_init(ctx);
     if (st == QF_OK) st = gemv_slab_init(ctx);
     if (st == QF_OK) st = stream_init(ctx);
+    if (st == QF_OK) st = slab_chain_init(ctx);
     if (st != QF_OK) {
         delete ctx;
         return st;
@@ -503,7 +533,7 @@ size_t qf_w4a16_workspace_bytes(const qf_linear_desc *desc) {
         qf_linear_desc d = *desc;
         d.path = QF_PATH_GEMV;
         if (make_plan(&d, &plan, nullptr) == QF_OK) need = std::max(need, plan.ws_partial_bytes + plan.ws_counter_bytes);
-        need = std::max(need, stream_workspace_bytes(d.M) + kCounterBytes);
+        need = std::max(need, std::max(kCounterBytes + stream_workspace_bytes(d.M), chain_workspace_bytes(d.M)));
     }
     return need;
 }
@@ -544,24 +574,13 @@ int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs,
     if (count == 0) return QF_OK;
     if (!descs || !X || !qweight || !Y) return fail(ctx, QF_ERR_BAD_ARG, "null argument array");
     std::vector<StreamLinear> run;
-    for (int i = 0; i < count; ++i) {
-        // linears on slab weights from here on, as far as nothing is wrong with them: one launch
-        run.clear();
-        for (int j = i; j < count && chains(&descs[j]); ++j) {
-            Plan plan;
-            const void *res = residual ? residual[j] : nullptr;
-            if (check_linear(ctx, &descs[j], X[j], qweight[j], nullptr, nullptr, Y[j], res, workspace, workspace_bytes, &plan) != QF_OK ||
-                workspace_bytes < stream_workspace_bytes(descs[j].M) + kCounterBytes)
-                break;
-            // K is cut as the tcgen05 kernel cuts it for the same sizes in its own layouts: the sums are the same bits
-            qf_linear_desc d = descs[j];
-            d.weight_layout = QF_LAYOUT_INTERLEAVED;
-            if (make_plan(&d, &plan, nullptr) != QF_OK || plan.path != QF_PATH_GEMM) break;
-            run.push_back(StreamLinear{&descs[j], X[j], qweight[j], res, Y[j], plan.split_k, plan.chunks_per_split});
-        }
-        const int n = run.size() > 1 ? stream_chain_length(run.data(), (int)run.size()) : 0;
-        if (n > 1) {
-            const int st = launch_stream_chain(ctx, run.data(), n, workspace, kCounterBytes, (cudaStream_t)stream);
+    for (int i = 0, alone = 0; i < count; ++i) {
+        bool pays = false;
+        const int n = i < alone ? 1 : chain_from(ctx, i, count, descs, X, qweight, Y, residual, workspace, workspace_bytes, &run, &pays);
+        alone = std::max(alone, i + n);
+        if (pays) {
+            const auto launch = descs[i].M <= kSlabGemvRows ? launch_slab_chain : launch_stream_chain;
+            const int st = launch(ctx, run.data(), n, workspace, kCounterBytes, (cudaStream_t)stream);
             if (st != QF_OK && st != kStreamNoRoom) return st;
             if (st == QF_OK) {
                 i += n - 1;
@@ -577,6 +596,19 @@ int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs,
         }
     }
     return QF_OK;
+}
+
+int qf_w4a16_batched_launches(qf_ctx *ctx, int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight,
+                              void *const *Y, const void *const *residual, const void *workspace, size_t workspace_bytes) {
+    if (!ctx || count < 0 || (count > 0 && (!descs || !X || !qweight || !Y))) return -1;
+    std::vector<StreamLinear> run;
+    int launches = 0;
+    for (int i = 0, n; i < count; i += n) {
+        bool pays = false;
+        n = chain_from(ctx, i, count, descs, X, qweight, Y, residual, workspace, workspace_bytes, &run, &pays);
+        launches += pays ? 1 : n;
+    }
+    return launches;
 }
 
 size_t qf_prepack_bytes(int layout, int64_t N, int64_t K) {

@@ -267,6 +267,11 @@ int gemv_init(qf_ctx *ctx);
 int gemm_init(qf_ctx *ctx);
 // streaming GEMV on QF_LAYOUT_GEMV_SLAB weights (qf_gemv_slab.cu)
 int gemv_slab_init(qf_ctx *ctx);
+// The split-K arrival counters occupy a FIXED region at the start of the workspace, so that a
+// workspace reused by linears of different shapes never exposes stale partial sums as counters.
+constexpr int kMaxCounters = 16384;
+constexpr size_t kCounterBytes = (size_t)kMaxCounters * sizeof(int);
+
 // Blobs up to this size run with two thread blocks per SM, larger ones with four (see slab_geometry). Launched
 // alone, matrices up to about 34 MB are faster with two (17 MB: 7.0 vs 8.4 us); inside a decode step, where the
 // neighbours are kernels of other sizes, a limit of 36 MB measured no better than 16 MB (5.84 vs 5.79 ms per

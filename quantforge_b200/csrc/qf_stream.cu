@@ -762,6 +762,51 @@ Touched touched(const StreamLinear &l) {
 int64_t row_blocks(const qf_linear_desc &d) { return (d.N + 127) / 128; }
 }  // namespace
 
+void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t room_step, int64_t room_two, std::vector<int> *order,
+                  std::vector<ChainPhase> *phases) {
+    std::vector<Touched> all;
+    std::vector<int> step_of;
+    int steps = 0;
+    int64_t used = 0;
+    for (int i = 0; i < count; ++i) {
+        all.push_back(touched(l[i]));
+        bool fresh = steps == 0 || used + room[i] > room_step;
+        for (int o = i; !fresh && o-- > 0 && step_of[o] == steps - 1;) fresh = all[i].after(all[o]);
+        if (fresh) {
+            ++steps;
+            used = 0;
+        }
+        used += room[i];
+        step_of.push_back(steps - 1);
+    }
+    int last = -1, late_before = -1, late = -1;  // phases: of the step before; late ones two steps back and one
+    for (int q = 0, i0 = 0, i1, i2; q < steps; ++q, i0 = i1) {
+        for (i1 = i0; i1 < count && step_of[i1] == q;) ++i1;
+        for (i2 = i1; i2 < count && step_of[i2] == q + 1;) ++i2;
+        int64_t here = 0, there = 0;
+        for (int i = i0; i < i1; ++i) here += room[i];
+        for (int i = i1; i < i2; ++i) there += room[i];
+        std::vector<char> waits(i1 - i0, i1 == i2 || here + there > room_two);
+        bool any = false;
+        for (int i = i0; i < i1; ++i) {
+            for (int o = i1; o < i2; ++o) waits[i - i0] = waits[i - i0] || all[o].after(all[i]);
+            any = any || waits[i - i0];
+        }
+        if (!any) waits.assign(i1 - i0, 1);
+        const int wait0 = last, wait1 = late_before;
+        late_before = late;
+        late = -1;
+        for (int part = 0; part < 2; ++part) {
+            ChainPhase c{(int)order->size(), 0, {wait0, wait1}, q, part == 1, here, i1, i2};
+            for (int i = i0; i < i1; ++i)
+                if ((waits[i - i0] != 0) == (part == 0)) order->push_back(i), ++c.count;
+            if (c.count == 0) continue;
+            (part == 0 ? last : late) = (int)phases->size();
+            phases->push_back(c);
+        }
+    }
+}
+
 template <int CAP>
 static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s) {
     StreamParams<CAP> p;
@@ -816,79 +861,43 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
         ph.r = ph.pieces % ph.streams;
         ph.pieces = 0;
     } else {
-        // Steps: linears that do not touch each other's results, each step behind the one before. Of a step only what the next one
-        // touches holds that up; the rest ("late") is a phase of its own, which the step after the next waits for.
         grid = sms;
         const int streams = 2 * grid;
-        std::vector<Touched> all;
-        std::vector<int> step_of;
+        std::vector<int> order;
+        std::vector<ChainPhase> chain;
         auto slots_of = [&](int i) { return l[i].split > 1 ? row_blocks(*l[i].d) * l[i].split : 0; };
-        int steps = 0;
-        int64_t slots = 0;
-        for (int i = 0; i < count; ++i) {
-            all.push_back(touched(l[i]));
-            bool fresh = steps == 0 || slots + slots_of(i) > kStreamSlots;
-            for (int o = i; !fresh && o-- > 0 && step_of[o] == steps - 1;) fresh = all[i].after(all[o]);
-            if (fresh) {
-                ++steps;
-                slots = 0;
-            }
-            slots += slots_of(i);
-            step_of.push_back(steps - 1);
-        }
-        int last = -1, late_before = -1, late = -1;  // phases: of the step before; late ones two steps back and one
-        for (int q = 0, i0 = 0; q < steps; ++q) {
-            int i1 = i0, i2;
-            while (i1 < count && step_of[i1] == q) ++i1;
-            for (i2 = i1; i2 < count && step_of[i2] == q + 1;) ++i2;
-            int64_t here = 0, there = 0;
-            for (int i = i0; i < i1; ++i) here += slots_of(i);
-            for (int i = i1; i < i2; ++i) there += slots_of(i);
-            std::vector<char> waits(i1 - i0, i1 == i2 || here + there > kStreamSlots);
-            bool any = false;
-            for (int i = i0; i < i1; ++i) {
-                for (int o = i1; o < i2; ++o) waits[i - i0] = waits[i - i0] || all[o].after(all[i]);
-                any = any || waits[i - i0];
-            }
-            if (!any) waits.assign(i1 - i0, 1);
+        std::vector<int64_t> slots(count);
+        for (int i = 0; i < count; ++i) slots[i] = slots_of(i);
+        chain_phases(l, count, slots.data(), kStreamSlots, kStreamSlots, &order, &chain);
+        int slot = 0;
+        for (const ChainPhase &c : chain) {
+            StreamPhase &ph = p.ph[phases++];
+            ph = StreamPhase{next, 0, 0, 0, streams, 0, 0, 0, {c.wait[0], c.wait[1]}};
             // slots: from the lower end and the upper one in turn, so that a late phase and the next step have their own
-            int slot = q & 1 ? kStreamSlots - (int)here : 0;
-            const int wait0 = last, wait1 = late_before;
-            late_before = late;
-            late = -1;
-            for (int part = 0; part < 2; ++part) {
-                if (part == 1 && std::find(waits.begin(), waits.end(), 0) == waits.end()) continue;  // nothing is late
-                StreamPhase &ph = p.ph[phases++];
-                ph = StreamPhase{next, 0, 0, 0, streams, 0, 0, 0, {wait0, wait1}};
-                for (int i = i0; i < i1; ++i)
-                    if ((waits[i - i0] != 0) == (part == 0)) {
-                        const int st = enter(i);
-                        if (st != QF_OK) return st;
-                        p.e[next - 1].slot = slot;
-                        slot += (int)slots_of(i);
-                    }
-                if (part == 0) {
-                    last = phases - 1;
-                } else {
-                    late = phases - 1;
-                    // to the streams that have nothing in the next step, if they can do it in that time; else to all, those first
-                    // that had nothing in this one
-                    int64_t pieces = 0, longest = 0, work = 0;
-                    for (int i = i1; i < i2; ++i) {
-                        pieces += row_blocks(*l[i].d) * l[i].split;
-                        longest = std::max<int64_t>(longest, l[i].per);
-                    }
-                    for (int e = ph.first; e < next; ++e) work += (int64_t)(p.e[e].end - p.e[e].begin) * p.e[e].per;
-                    if (pieces < streams && work <= longest * (streams - pieces)) {
-                        ph.home = (int)pieces;
-                        ph.streams = streams - (int)pieces;
-                    } else {
-                        ph.flip = 1;
-                    }
-                }
-                ph.active = std::min(ph.pieces, ph.streams);
+            if (!c.late) slot = c.step & 1 ? kStreamSlots - (int)c.room : 0;
+            for (int k = c.first; k < c.first + c.count; ++k) {
+                const int st = enter(order[k]);
+                if (st != QF_OK) return st;
+                p.e[next - 1].slot = slot;
+                slot += (int)slots[order[k]];
             }
-            i0 = i1;
+            if (c.late) {
+                // to the streams that have nothing in the next step, if they can do it in that time; else to all, those first
+                // that had nothing in this one
+                int64_t pieces = 0, longest = 0, work = 0;
+                for (int i = c.next0; i < c.next1; ++i) {
+                    pieces += row_blocks(*l[i].d) * l[i].split;
+                    longest = std::max<int64_t>(longest, l[i].per);
+                }
+                for (int e = ph.first; e < next; ++e) work += (int64_t)(p.e[e].end - p.e[e].begin) * p.e[e].per;
+                if (pieces < streams && work <= longest * (streams - pieces)) {
+                    ph.home = (int)pieces;
+                    ph.streams = streams - (int)pieces;
+                } else {
+                    ph.flip = 1;
+                }
+            }
+            ph.active = std::min(ph.pieces, ph.streams);
         }
     }
     p.a.phases = phases;

@@ -1,6 +1,8 @@
 // Host interface of the streaming tcgen05 kernel on QF_LAYOUT_GEMV_SLAB weights (qf_stream.cu).
 #pragma once
 
+#include <vector>
+
 #include "qf_common.cuh"
 
 namespace qf {
@@ -17,6 +19,21 @@ struct StreamLinear {
     int split, per;
 };
 
+// Steps of a chain: linears that do not touch each other's results, each step behind the one before. Of a step only what the next
+// one touches holds that up; the rest ("late") is a phase of its own, which the step after the next waits for.
+struct ChainPhase {
+    int first, count;  // of the order
+    int wait[2];       // phases that are complete before this one begins (or -1)
+    int step;
+    bool late;
+    int64_t room;      // of the whole step
+    int next0, next1;  // the linears of the next step
+};
+// room[i]: what linear i needs of something that a step has room_step of, and a step with late linears and the next one together
+// room_two.
+void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t room_step, int64_t room_two, std::vector<int> *order,
+                  std::vector<ChainPhase> *phases);
+
 // Returned by the launches where the current context has fewer SMs than the device (a partition of it), so that the blocks of a
 // cooperative launch do not fit: nothing was launched, and the other kernels serve.
 constexpr int kStreamNoRoom = 1;
@@ -30,5 +47,13 @@ int launch_stream(qf_ctx *ctx, const StreamLinear &l, void *ws, size_t counter_b
 int stream_chain_length(const StreamLinear *l, int count);
 // Linears of one launch, each seeing the results of the earlier ones.
 int launch_stream_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s);
+
+// The same for linears of up to kSlabGemvRows rows, with the arithmetic of the streaming GEMV kernel (qf_slab_chain.cu).
+int slab_chain_init(qf_ctx *ctx);
+bool slab_chain_takes(const qf_linear_desc *d);
+// Whether one launch is the faster way.
+bool slab_chain_pays(const StreamLinear *l, int count);
+size_t slab_chain_workspace_bytes();
+int launch_slab_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s);
 
 }  // namespace qf

@@ -405,7 +405,8 @@ class LinearBatch:
     """Linears on slab weights that run one after the other, each seeing the results of the earlier ones, enqueued by one call:
     `calls` is a sequence of (x, SlabWeight, out, epilogue, residual or None) with the meaning they have in `w4a16_linear`. The
     tensors are kept and read where they are at each `run()`, which may be captured. Linears of 9 to 32 rows go to the GPU as one
-    launch, up to CHAIN_LINEARS of them, with the bits that the tcgen05 kernel gives on other layouts."""
+    launch, up to CHAIN_LINEARS of them, with the bits that the tcgen05 kernel gives on other layouts; so do those of up to 8 rows where
+    it is the faster way, with the bits that they have one by one."""
 
     def __init__(self, calls):
         calls = list(calls)
@@ -436,6 +437,14 @@ class LinearBatch:
         return [(x.data_ptr(), x.shape, x.stride(), x.dtype, w.blob.data_ptr(), w.N, w.K, out.data_ptr(), out.shape, out.dtype, epilogue,
                  None if residual is None else (residual.data_ptr(), residual.shape, residual.dtype))
                 for x, w, out, epilogue, residual in calls]
+
+    def launches(self) -> int:
+        """Kernel launches of a `run()`."""
+        x, w, out, residual = self._arrays
+        with torch.cuda.device(self.device):
+            ws = _workspace(self.device, self._ws_bytes)
+            return _lib.load().qf_w4a16_batched_launches(_ctx(self.device), len(self._descs), self._descs, x, w, out, residual, _ptr(ws),
+                                                         ws.numel() if ws is not None else 0)
 
     def run(self) -> None:
         dev = self.device

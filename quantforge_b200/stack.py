@@ -15,7 +15,7 @@ Modes
                    over NVLink peer memory instead of being followed by an NCCL all-reduce
 Batches of up to 8 rows read QF_LAYOUT_GEMV_SLAB weights (the streaming GEMV kernel), larger ones the
 interleaved layout of the tcgen05 kernel. On one GPU, 9 to 32 rows of large linears read slab weights too and
-run as a chain: one launch for up to 112 linears, the same results bit for bit.
+run as a chain: one launch for up to 112 linears, the same results bit for bit. So do up to 8 rows where that is the faster way.
 """
 from __future__ import annotations
 
@@ -126,8 +126,9 @@ class DecodeLinearStack:
             self.comm = ops.Comm(batch * H, device=self.dev, group=group)
         exch = self.comm is not None and not exchange_in_slab_kernel
         codes = (2 * H * H + 2 * H * KV + 3 * H * F) // 2  # bytes of a layer's codes
-        self.chain = (world == 1 and SLAB_BATCH < batch <= CHAIN_BATCH and H % 128 == 0 and KV % 128 == 0 and F % 128 == 0 and
-                      codes >= (4 if fuse else 7) * _chain_bytes(batch, fuse))
+        # up to SLAB_BATCH rows the batched call decides by itself whether one launch is the faster way
+        self.chain = (world == 1 and batch <= CHAIN_BATCH and H % 128 == 0 and KV % 128 == 0 and F % 128 == 0 and
+                      (batch <= SLAB_BATCH or codes >= (4 if fuse else 7) * _chain_bytes(batch, fuse)))
         self._batch = None
         self.layers = []
         for li in range(self.L):
@@ -206,6 +207,14 @@ class DecodeLinearStack:
             h = b["down"]
         return calls
 
+    def _chained(self):
+        """The batched call of a step and the tensor that holds its result."""
+        calls = self._chain_calls()
+        key = ops.LinearBatch.key(calls)  # another buffer or weight in the place of one makes another batch
+        if self._batch is None or self._batch[0] != key:
+            self._batch = (key, ops.LinearBatch(calls))
+        return self._batch[1], calls[-1][2]
+
     def _layer(self, ly, h):
         b = self.buf
         if self.fuse:
@@ -229,12 +238,9 @@ class DecodeLinearStack:
     def step(self) -> torch.Tensor:
         """One token step through all layers, from buf["h_in"]; returns the last hidden state buffer."""
         if self.chain:
-            calls = self._chain_calls()
-            key = ops.LinearBatch.key(calls)  # another buffer or weight in the place of one makes another batch
-            if self._batch is None or self._batch[0] != key:
-                self._batch = (key, ops.LinearBatch(calls))
-            self._batch[1].run()
-            return calls[-1][2]
+            batch, out = self._chained()
+            batch.run()
+            return out
         h = self.buf["h_in"]
         for ly in self.layers:
             h = self._layer(ly, h)
@@ -266,8 +272,7 @@ class DecodeLinearStack:
         return out_host
 
     def launches_per_step(self) -> int:
-        n = (4 if self.fuse else 7) * self.L
-        return -(-n // ops.CHAIN_LINEARS) if self.chain else n
+        return self._chained()[0].launches() if self.chain else (4 if self.fuse else 7) * self.L
 
     def bytes_per_step(self) -> int:
         """Algorithmic bytes of the whole (unsharded) token step."""
