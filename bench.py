@@ -500,6 +500,7 @@ def run_stack_workload(env, args):
     ms = ms_bracket / args.steps
     nbytes = st.bytes_per_step()
     launches_per_step = st.launches_per_step()
+    chained = launches_per_step < (4 if fuse else 7) * st.L
 
     # ---- end to end: the hidden state comes from pinned host memory and the last hidden state goes back, every step ----
     H = cfg["hidden"]
@@ -553,11 +554,10 @@ def run_stack_workload(env, args):
     if rank == 0:
         gbs = nbytes / (ms * 1e-3) / 1e9
         per_launch_us = ms * 1e3 / launches_per_step
-        one_by_one = (4 if fuse else 7) * st.L
-        kernel = ("qf::gemv_slab_kernel" if args.batch <= 8 and st.launches_per_step() == one_by_one else
-                  "qf::slab_chain_kernel (the step in few launches)" if args.batch <= 8 else
-                  "qf::stream_kernel (tcgen05, the step in few launches)" if st.chain
-                  else "qf::gemm_kernel (tcgen05)")
+        if chained:
+            kernel = "qf::slab_chain_kernel" if args.batch <= 8 else "qf::stream_kernel (tcgen05)"
+        else:
+            kernel = "qf::gemv_slab_kernel" if args.batch <= 8 else "qf::gemm_kernel (tcgen05)"
         if in_kernel and args.batch <= 8:
             kernel += " + qf::gemv_slab_exch_kernel (row-parallel linears)"
         line = {
