@@ -12,7 +12,7 @@
 // What bounds it. The converters, 560 cycles for 128 x 128 weights and SM as in the streaming GEMV kernel, 27 us of the 42 of a layer of
 // 4096 / 14336, and for each phase the way from the last product to the next one's first, about 4 us: partial sums to their owner,
 // results, counter, activations. Linears of a step share that way, which is why layers of seven linears gain the most (x1.1 to x1.45)
-// and those of four 1.06 to 1.2: a token of 32 layers of 4096 / 14336 from and to the host 1426 us -> 1343.
+// and those of four 1.06 to 1.2: a token of 32 layers of 4096 / 14336 from and to the host 1426 us -> 1339.
 //
 // A linear that the streaming GEMV kernel runs with G thread blocks takes G of this launch's blocks (four per SM, all resident: the
 // launch is cooperative); linears of one step take different ones. Roles inside a block, the ring of pairs of units, the sharing of
@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, SC_BLOCKS_PER_SM) slab_chain_ker
                     const unsigned want = (unsigned)p.ph[w].blocks;
                     const long long t0 = clock64();
                     while (!__all_sync(0xffffffffu, lane != 0 || sc_acquire(p.done + w) >= want)) {
+                        __nanosleep(100);  // leaves issue slots and the counter's word to the others (0.5 to 1 % of a step)
                         if (clock64() - t0 > kWaitCycles) *abort_flag = 1;
                         if (__any_sync(0xffffffffu, *abort_flag != 0)) {
                             ok = false;
