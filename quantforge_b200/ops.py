@@ -431,13 +431,6 @@ class LinearBatch:
         self._arrays = [(ctypes.c_void_p * n)(*[t.data_ptr() if t is not None else 0 for t in col]) for col in zip(*self._tensors)]
         self._ws_bytes = max(workspace_bytes(d) for d in self._descs)
 
-    @staticmethod
-    def key(calls):
-        """What a batch of these calls is made of: equal keys, the same launch."""
-        return [(x.data_ptr(), x.shape, x.stride(), x.dtype, w.blob.data_ptr(), w.N, w.K, out.data_ptr(), out.shape, out.dtype, epilogue,
-                 None if residual is None else (residual.data_ptr(), residual.shape, residual.dtype))
-                for x, w, out, epilogue, residual in calls]
-
     def launches(self) -> int:
         """Kernel launches of a `run()`."""
         x, w, out, residual = self._arrays

@@ -209,11 +209,13 @@ class DecodeLinearStack:
 
     def _chained(self):
         """The batched call of a step and the tensor that holds its result."""
-        calls = self._chain_calls()
-        key = ops.LinearBatch.key(calls)  # another buffer or weight in the place of one makes another batch
+        # another buffer or weight in the place of one makes another batch
+        key = ([(t.data_ptr(), t.shape, t.stride(), t.dtype) for t in self.buf.values()],
+               [(ln.slab.blob.data_ptr(), ln.slab.N, ln.slab.K) for ly in self.layers for ln in ly.values()])
         if self._batch is None or self._batch[0] != key:
-            self._batch = (key, ops.LinearBatch(calls))
-        return self._batch[1], calls[-1][2]
+            calls = self._chain_calls()
+            self._batch = (key, ops.LinearBatch(calls), calls[-1][2])
+        return self._batch[1:]
 
     def _layer(self, ly, h):
         b = self.buf
