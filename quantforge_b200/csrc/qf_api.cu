@@ -70,10 +70,11 @@ static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 //   16     10.3 -> 11.4  12.0 -> 14.5  16.6 -> 17.6  21.2 -> 16.2  19.1 -> 18.3  24.6 -> 23.0  44.6 -> 35.0  83.2 -> 63.8
 //   24     15.9 -> 15.6  16.1 -> 16.5  23.0 -> 19.2  28.7 -> 19.0  27.0 -> 20.7  35.5 -> 26.8  66.3 -> 37.1  129 -> 67.9
 //   32     17.0 -> 16.5  17.9 -> 18.6  24.8 -> 22.7  31.1 -> 20.0  29.0 -> 21.4  37.8 -> 28.7  70.2 -> 38.7  135 -> 69.9
+// Up to 8 rows the GEMV kernel serves whatever the size is: what the largest matrices gain waiting for each call is 1 % (4 rows,
+// 57344 x 8192, SiLU * mul: 65.3 -> 64.7), and their sums would be made in another order than those of all smaller ones.
 static bool stream_serves(const qf_linear_desc *d) {
     const int64_t mib = d->N / 64 * (d->K / 128) * QF_SLAB_UNIT_BYTES >> 20;
-    if (d->M <= 2) return false;
-    if (d->M <= kSlabGemvRows) return mib >= 160;
+    if (d->M <= kSlabGemvRows) return false;
     if (d->M <= 16) return mib >= (d->K >= 8192 ? 24 : 33);
     return mib >= 24;
 }
@@ -335,8 +336,7 @@ static bool slab_any(const qf_linear_desc *d) {
 
 // Linears that qf_w4a16_linear_batched runs as one launch.
 static bool chains(const qf_linear_desc *d) {
-    // (up to kSlabGemvRows rows with the results of the call for one linear, so only what the streaming GEMV kernel serves there)
-    return slab_any(d) && (d->M <= kSlabGemvRows ? slab_chain_takes(d) && !stream_serves(d) : d->N % 128 == 0);
+    return slab_any(d) && (d->M <= kSlabGemvRows ? slab_chain_takes(d) : d->N % 128 == 0);
 }
 // The workspace of that launch.
 static size_t chain_workspace_bytes(int64_t M) {

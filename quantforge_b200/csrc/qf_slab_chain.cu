@@ -568,8 +568,10 @@ bool slab_chain_pays(const StreamLinear *l, int count) {
 }
 
 bool slab_chain_takes(const qf_linear_desc *d) {
-    // numbers of units times blocks in 32 bits
-    return d->M <= kSlabGemvRows && (d->N / 64) * (d->K / 128) < (int64_t)UINT32_MAX / (SC_BLOCKS_PER_SM * kSmCount + 1);
+    // From 160 MiB on a linear goes by itself, so that its size does not speak for those around it (slab_chain_pays). That also keeps
+    // units times blocks within 32 bits.
+    static_assert((160ull << 20) / QF_SLAB_UNIT_BYTES * (SC_BLOCKS_PER_SM * kSmCount + 1) <= UINT32_MAX, "share arithmetic");
+    return d->M <= kSlabGemvRows && (d->N / 64) * (d->K / 128) <= (160 << 20) / QF_SLAB_UNIT_BYTES;
 }
 
 }  // namespace qf

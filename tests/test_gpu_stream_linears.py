@@ -29,7 +29,8 @@ def _silu_mul(y):  # rows in eights of gate and up
     return gate / (1 + torch.exp(-gate)) * up
 
 
-# sizes of the rule's region (at least 24 or 33 MiB, 160 MiB up to 8 rows), half row blocks at the end, few and many members a row block
+# sizes of the rule's region (at least 24 or 33 MiB), half row blocks at the end, few and many members a row block; the largest of up to
+# 8 rows, which the streaming GEMV kernel serves
 @pytest.mark.parametrize("M,N,K,dtype,group", [
     (9, 8256, 8192, torch.bfloat16, 128), (16, 2112, 28672, torch.float16, 256), (12, 17408, 4096, torch.float16, 128),
     (17, 6208, 8192, torch.bfloat16, 8192), (25, 24640, 2048, torch.float16, 128), (32, 1792, 28672, torch.bfloat16, 128),

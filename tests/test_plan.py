@@ -98,3 +98,10 @@ def test_pairs_where_a_block_runs_through_enough_codes(M, K, N, split_k, want):
 def test_blocks_take_512_codes_at_least(M):
     for K in (512, 1024, 2048, 4096):
         assert K // _plan(M, K, 1024, 2, _lib.QF_PATH_GEMM)[1] >= 512
+
+
+@pytest.mark.parametrize("K,N", [(128, 64), (4096, 4096), (8192, 28672), (5760, 57344), (8192, 57344), (28672, 11520), (28672, 28672)])
+def test_up_to_8_rows_one_kernel_reads_slab_weights(K, N):
+    # AUTO is the streaming GEMV kernel, which QF_PATH_GEMV names, at any size: one order of sums for all of them
+    for M in range(1, 9):
+        assert _plan(M, K, N, _lib.QF_LAYOUT_GEMV_SLAB) == _plan(M, K, N, _lib.QF_LAYOUT_GEMV_SLAB, _lib.QF_PATH_GEMV)
