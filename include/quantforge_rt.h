@@ -208,6 +208,13 @@ int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs,
 /* Kernel launches that this call would make (-1: bad arguments). Nothing is enqueued. */
 int qf_w4a16_batched_launches(qf_ctx *ctx, int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight,
                               void *const *Y, const void *const *residual, const void *workspace, size_t workspace_bytes);
+/* How this call would run on a B200 (host only: nothing is enqueued, and no pointer is followed). For entry i,
+ * out[QF_BATCHED_PLAN_WORDS * i ..]: the number of its launch (-1: none, M == 0) and, -1 for an entry that goes by itself, its phase in
+ * the launch; the two phases that are complete before it reads or writes anything (-1: none); its first slot of partial sums and their
+ * number; up to 8 rows the place of its first thread block (4 * SM + place on the SM) and the number of its blocks, else -1. */
+#define QF_BATCHED_PLAN_WORDS 8
+int qf_w4a16_batched_plan(int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight, void *const *Y,
+                          const void *const *residual, const void *workspace, size_t workspace_bytes, int32_t *out);
 
 /*
  * The same linear for callers that hold activations in HOST memory (the reference's Python entry

@@ -288,7 +288,6 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
 
 static int check_linear_args(qf_ctx *ctx, const qf_linear_desc *d, const void *X, const void *qw, const void *scales,
                              const void *zeros, const void *Y) {
-    if (!ctx) return QF_ERR_BAD_ARG;
     if (d->weight_layout == QF_LAYOUT_GEMV_SLAB) {
         // the blob carries scales and zeros
         if (!X || !qw || !Y) return fail(ctx, QF_ERR_BAD_ARG, "null tensor pointer");
@@ -304,7 +303,7 @@ static int check_linear_args(qf_ctx *ctx, const qf_linear_desc *d, const void *X
     return QF_OK;
 }
 
-// Everything that a linear's launch relies on, and its plan. M == 0 needs no tensors.
+// Everything that a linear's launch relies on, and its plan. M == 0 needs no tensors. Without a context: all but the current device.
 static int check_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, const void *qweight, const void *scales,
                         const void *qzeros_or_null, const void *Y, const void *residual, const void *workspace,
                         size_t workspace_bytes, Plan *plan) {
@@ -314,7 +313,7 @@ static int check_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, 
     if (desc->M == 0) return QF_OK;
     st = check_linear_args(ctx, desc, X, qweight, scales, qzeros_or_null, Y);
     if (st != QF_OK) return st;
-    st = check_current_device(ctx);
+    if (ctx) st = check_current_device(ctx);
     if (st != QF_OK) return st;
     if (desc->epilogue == QF_EPI_RESIDUAL_ADD && (!residual || !aligned16(residual)))
         return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_RESIDUAL_ADD needs a 16-byte aligned residual tensor");
@@ -334,9 +333,10 @@ static bool slab_any(const qf_linear_desc *d) {
     return d->weight_layout == QF_LAYOUT_GEMV_SLAB && d->split_k == 0 && d->path == QF_PATH_AUTO;
 }
 
-// Linears that qf_w4a16_linear_batched runs as one launch.
+// Linears that qf_w4a16_linear_batched runs as one launch. (One without rows goes alone: it has no launch, and its pointers were not
+// looked at.)
 static bool chains(const qf_linear_desc *d) {
-    return slab_any(d) && (d->M <= kSlabGemvRows ? slab_chain_takes(d) : d->N % 128 == 0);
+    return d->M > 0 && slab_any(d) && (d->M <= kSlabGemvRows ? slab_chain_takes(d) : d->N % 128 == 0);
 }
 // The workspace of that launch.
 static size_t chain_workspace_bytes(int64_t M) {
@@ -606,9 +606,42 @@ int qf_w4a16_batched_launches(qf_ctx *ctx, int count, const qf_linear_desc *desc
     for (int i = 0, n; i < count; i += n) {
         bool pays = false;
         n = chain_from(ctx, i, count, descs, X, qweight, Y, residual, workspace, workspace_bytes, &run, &pays);
-        launches += pays ? 1 : n;
+        if (pays) ++launches;
+        else
+            for (int j = i; j < i + n; ++j) launches += descs[j].M > 0;
     }
     return launches;
+}
+
+int qf_w4a16_batched_plan(int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight, void *const *Y,
+                          const void *const *residual, const void *workspace, size_t workspace_bytes, int32_t *out) {
+    if (count < 0 || (count > 0 && (!descs || !X || !qweight || !Y || !out))) return QF_ERR_BAD_ARG;
+    std::vector<StreamLinear> run;
+    ChainPlan plan;
+    for (int i = 0, n, launch = 0; i < count; i += n) {
+        bool pays = false;
+        n = chain_from(nullptr, i, count, descs, X, qweight, Y, residual, workspace, workspace_bytes, &run, &pays);
+        int32_t *o = out + (size_t)i * QF_BATCHED_PLAN_WORDS;
+        std::fill(o, o + (size_t)n * QF_BATCHED_PLAN_WORDS, -1);
+        const bool gemv = descs[i].M <= kSlabGemvRows;
+        if (!pays || (gemv && !plan_slab_chain(run.data(), n, kSmCount, &plan))) {
+            for (int j = 0; j < n; ++j)
+                if (descs[i + j].M > 0) o[j * QF_BATCHED_PLAN_WORDS] = launch++;
+            continue;
+        }
+        if (!gemv) plan_stream_chain(run.data(), n, 2 * kSmCount, &plan);
+        for (size_t q = 0; q < plan.phases.size(); ++q) {
+            const ChainPhase &c = plan.phases[q];
+            for (int k = c.first; k < c.first + c.count; ++k) {
+                const ChainLinear &x = plan.linears[plan.order[k]];
+                const int32_t words[QF_BATCHED_PLAN_WORDS] = {launch, (int32_t)q, c.wait[0], c.wait[1], x.slot, x.slots,
+                                                              gemv ? kSlabChainPlaces * x.first_sm + x.home : -1, gemv ? x.grid : -1};
+                std::copy(words, words + QF_BATCHED_PLAN_WORDS, o + (size_t)plan.order[k] * QF_BATCHED_PLAN_WORDS);
+            }
+        }
+        ++launch;
+    }
+    return QF_OK;
 }
 
 size_t qf_prepack_bytes(int layout, int64_t N, int64_t K) {

@@ -1,0 +1,168 @@
+// Host side of the chains (qf_w4a16_linear_batched): which linears one launch takes, in which steps, and what each gets of the things
+// that several of them share. Plain C++, no GPU.
+#include <algorithm>
+
+#include "qf_stream.cuh"
+
+namespace qf {
+
+namespace {
+struct Range {
+    uintptr_t lo, hi;
+    bool meets(const Range &o) const { return lo < o.hi && o.lo < hi; }
+};
+Range range_of(const void *p, int64_t bytes) { return Range{(uintptr_t)p, (uintptr_t)p + (p ? (uintptr_t)bytes : 0u)}; }
+struct Touched {
+    Range x, r, y;
+    // Whether this linear has to come behind an earlier one: reads what that writes, writes what that reads or writes.
+    bool after(const Touched &o) const { return o.y.meets(x) || o.y.meets(r) || o.y.meets(y) || y.meets(o.x) || y.meets(o.r); }
+};
+Touched touched(const StreamLinear &l) {
+    const qf_linear_desc &d = *l.d;
+    const int64_t cols = d.epilogue == QF_EPI_SILU_MUL ? d.N / 2 : d.N, size = d.out_dtype == QF_F32 ? 4 : 2;
+    return Touched{range_of(l.X, d.M * d.K * 2), range_of(d.epilogue == QF_EPI_RESIDUAL_ADD ? l.residual : nullptr, d.M * cols * size),
+                   range_of(l.Y, d.M * cols * size)};
+}
+}  // namespace
+
+void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t room_step, int64_t room_two, std::vector<int> *order,
+                  std::vector<ChainPhase> *phases) {
+    std::vector<Touched> all;
+    std::vector<int> step_of;
+    int steps = 0;
+    int64_t used = 0;
+    for (int i = 0; i < count; ++i) {
+        all.push_back(touched(l[i]));
+        bool fresh = steps == 0 || used + room[i] > room_step;
+        for (int o = i; !fresh && o-- > 0 && step_of[o] == steps - 1;) fresh = all[i].after(all[o]);
+        if (fresh) {
+            ++steps;
+            used = 0;
+        }
+        used += room[i];
+        step_of.push_back(steps - 1);
+    }
+    int last = -1, late_before = -1, late = -1;  // phases: of the step before; late ones two steps back and one
+    for (int q = 0, i0 = 0, i1, i2; q < steps; ++q, i0 = i1) {
+        for (i1 = i0; i1 < count && step_of[i1] == q;) ++i1;
+        for (i2 = i1; i2 < count && step_of[i2] == q + 1;) ++i2;
+        int64_t here = 0, there = 0;
+        for (int i = i0; i < i1; ++i) here += room[i];
+        for (int i = i1; i < i2; ++i) there += room[i];
+        std::vector<char> waits(i1 - i0, i1 == i2 || here + there > room_two);
+        bool any = false;
+        for (int i = i0; i < i1; ++i) {
+            for (int o = i1; o < i2; ++o) waits[i - i0] = waits[i - i0] || all[o].after(all[i]);
+            any = any || waits[i - i0];
+        }
+        if (!any) waits.assign(i1 - i0, 1);
+        const int wait0 = last, wait1 = late_before;
+        late_before = late;
+        late = -1;
+        for (int part = 0; part < 2; ++part) {
+            ChainPhase c{(int)order->size(), 0, {wait0, wait1}, q, part == 1, here, i1, i2, 0, 0, 0};
+            for (int i = i0; i < i1; ++i)
+                if ((waits[i - i0] != 0) == (part == 0)) order->push_back(i), ++c.count;
+            if (c.count == 0) continue;
+            (part == 0 ? last : late) = (int)phases->size();
+            phases->push_back(c);
+        }
+    }
+}
+
+void plan_stream_chain(const StreamLinear *l, int count, int streams, ChainPlan *plan) {
+    std::vector<int64_t> slots(count);
+    plan->linears.assign(count, ChainLinear{});
+    for (int i = 0; i < count; ++i) {
+        slots[i] = l[i].split > 1 ? row_blocks(*l[i].d) * l[i].split : 0;
+        plan->linears[i].slots = (int)slots[i];
+    }
+    chain_phases(l, count, slots.data(), kStreamSlots, kStreamSlots, &plan->order, &plan->phases);
+    auto pieces_of = [&](int i) { return row_blocks(*l[i].d) * l[i].split; };
+    int slot = 0;
+    for (ChainPhase &c : plan->phases) {
+        // slots: from the lower end and the upper one in turn, so that a late phase and the next step have their own
+        if (!c.late) slot = c.step & 1 ? kStreamSlots - (int)c.room : 0;
+        for (int k = c.first; k < c.first + c.count; ++k) {
+            plan->linears[plan->order[k]].slot = slot;
+            slot += (int)slots[plan->order[k]];
+        }
+        c.streams = streams;
+        if (c.late) {
+            // to the streams that have nothing in the next step, if they can do it in that time; else to all, those first
+            // that had nothing in this one
+            int64_t pieces = 0, longest = 0, work = 0;
+            for (int i = c.next0; i < c.next1; ++i) {
+                pieces += pieces_of(i);
+                longest = std::max<int64_t>(longest, l[i].per);
+            }
+            for (int k = c.first; k < c.first + c.count; ++k) work += pieces_of(plan->order[k]) * l[plan->order[k]].per;
+            if (pieces < streams && work <= longest * (streams - pieces)) {
+                c.home = (int)pieces;
+                c.streams = streams - (int)pieces;
+            } else {
+                c.flip = 1;
+            }
+        }
+    }
+}
+
+bool plan_slab_chain(const StreamLinear *l, int count, int sms, ChainPlan *plan) {
+    const int blocks = kSlabChainPlaces * sms;
+    std::vector<int64_t> per_sm(count);
+    plan->linears.assign(count, ChainLinear{});
+    for (int i = 0; i < count; ++i) {
+        int depth;
+        ChainLinear &x = plan->linears[i];
+        slab_geometry(l[i].d->M, l[i].d->N, l[i].d->K, kSmCount, 0, &x.grid, &depth);
+        if (x.grid > blocks) return false;
+        x.slots = x.grid;
+        per_sm[i] = x.per_sm = (x.grid + sms - 1) / sms;
+    }
+    chain_phases(l, count, per_sm.data(), kSlabChainPlaces, 2 * kSlabChainPlaces, &plan->order, &plan->phases);
+    int home = 0, first_sm = 0, used = 0;  // places of the step
+    for (const ChainPhase &c : plan->phases) {
+        if (!c.late) used = 0;
+        for (int k = c.first; k < c.first + c.count; ++k) {
+            ChainLinear &x = plan->linears[plan->order[k]];
+            x.home = home;
+            x.first_sm = first_sm;
+            x.slot = (c.step & 1) * blocks + used * sms;
+            // the next linear begins where this one ends: what small ones leave idle is spread, and reads ahead
+            home = (home + x.per_sm) % kSlabChainPlaces;
+            first_sm = (first_sm + (x.grid + x.per_sm - 1) / x.per_sm) % sms;
+            used += x.per_sm;
+        }
+    }
+    return true;
+}
+
+int stream_chain_length(const StreamLinear *l, int count) {
+    const void *x_of[kStreamMaxX];
+    int64_t x_k[kStreamMaxX];
+    std::vector<Range> written;
+    int maps = 0, n = 0;
+    for (; n < count && n < kStreamMaxLinears; ++n) {
+        const qf_linear_desc &d = *l[n].d;
+        if (d.M != l[0].d->M || d.act_dtype != l[0].d->act_dtype || row_blocks(d) * l[n].split > (1 << 24)) break;
+        int m = 0;
+        while (m < maps && !(x_of[m] == l[n].X && x_k[m] == d.K)) ++m;
+        if (m == kStreamMaxX) break;
+        // weights are read ahead of the phases: they must not be an earlier linear's result
+        const Range w = range_of(l[n].blob, d.N / 64 * (d.K / 128) * QF_SLAB_UNIT_BYTES);
+        bool meets = false;
+        for (const Range &y : written) meets = meets || y.meets(w);
+        if (meets) break;
+        if (m == maps) {
+            x_of[maps] = l[n].X;
+            x_k[maps++] = d.K;
+        }
+        const Range y = touched(l[n]).y;
+        bool known = false;
+        for (const Range &o : written) known = known || (o.lo <= y.lo && y.hi <= o.hi);
+        if (!known) written.push_back(y);
+    }
+    return n;
+}
+
+}  // namespace qf

@@ -27,7 +27,7 @@
 
 namespace qf {
 
-constexpr int SC_BLOCKS_PER_SM = 4;
+constexpr int SC_BLOCKS_PER_SM = kSlabChainPlaces;
 constexpr int kSlabChainMax = 112;  // linears of a launch
 // Words of the counter region, all zero between launches: thread blocks that have finished a phase, and everything; thread blocks
 // that an SM has started; places given out among the first, second, ... of the SMs.
@@ -460,26 +460,17 @@ int launch_slab_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, s
     SlabChainParams p;
     const qf_linear_desc &d0 = *l[0].d;
     const int sms = std::min(ctx->sm_count, kSmCount), blocks = SC_BLOCKS_PER_SM * sms;
-    std::vector<int> grids(count);
-    std::vector<int64_t> per_sm(count);
-    for (int i = 0; i < count; ++i) {
-        int depth;
-        slab_geometry(l[i].d->M, l[i].d->N, l[i].d->K, kSmCount, 0, &grids[i], &depth);
-        if (grids[i] > blocks) return kStreamNoRoom;
-        per_sm[i] = (grids[i] + sms - 1) / sms;
-    }
-    std::vector<int> order;
-    std::vector<ChainPhase> chain;
-    chain_phases(l, count, per_sm.data(), SC_BLOCKS_PER_SM, 2 * SC_BLOCKS_PER_SM, &order, &chain);
-    p.phases = (int)chain.size();
-    int next = 0, home = 0, first_sm = 0, used = 0;  // places of the step
+    ChainPlan plan;
+    if (!plan_slab_chain(l, count, sms, &plan)) return kStreamNoRoom;
+    p.phases = (int)plan.phases.size();
+    int next = 0;
     for (int q = 0; q < p.phases; ++q) {
-        const ChainPhase &c = chain[q];
+        const ChainPhase &c = plan.phases[q];
         SlabChainPhase &ph = p.ph[q];
-        if (!c.late) used = 0;
         ph = SlabChainPhase{next, c.count, 0, c.step & 1, {c.wait[0], c.wait[1]}};
         for (int k = c.first; k < c.first + c.count; ++k) {
-            const StreamLinear &x = l[order[k]];
+            const StreamLinear &x = l[plan.order[k]];
+            const ChainLinear &at = plan.linears[plan.order[k]];
             SlabChainEntry &e = p.e[next++];
             e.blob = (const uint8_t *)x.blob;
             e.X = (const uint16_t *)x.X;
@@ -490,18 +481,14 @@ int launch_slab_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, s
             e.K = x.d->K;
             e.chunks = (int)(x.d->K / 128);
             e.units = (unsigned)(x.d->N / 64 * e.chunks);
-            e.grid = (unsigned)grids[order[k]];
-            e.home = home;
+            e.grid = (unsigned)at.grid;
+            e.home = at.home;
             e.out_dtype = x.d->out_dtype;
             e.epilogue = x.d->epilogue;
-            e.per_sm = (int)per_sm[order[k]];
-            e.first_sm = first_sm;
-            e.slot = (unsigned)((c.step & 1) * blocks + used * sms);
-            // the next linear begins where this one ends: what small ones leave idle is spread, and reads ahead
-            home = (home + e.per_sm) % SC_BLOCKS_PER_SM;
-            first_sm = (first_sm + ((int)e.grid + e.per_sm - 1) / e.per_sm) % sms;
-            used += e.per_sm;
-            ph.blocks += (int)e.grid;
+            e.per_sm = at.per_sm;
+            e.first_sm = at.first_sm;
+            e.slot = (unsigned)at.slot;
+            ph.blocks += at.grid;
         }
     }
     p.pairs = (unsigned long long *)((char *)ws + counter_bytes);

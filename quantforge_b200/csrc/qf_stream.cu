@@ -37,7 +37,6 @@
 // Shared memory takes all but a few KB of the SM's first-level cache, so a spilled register is a trip to L2: the registers are split
 // between the roles such that none is (see setmaxnreg below).
 #include <algorithm>
-#include <cstring>
 #include <vector>
 
 #include "qf_stream.cuh"
@@ -94,7 +93,7 @@ struct StreamArgs {
 };
 template <int CAP>
 struct StreamParams {
-    static constexpr int XCAP = CAP == 1 ? 1 : 16;
+    static constexpr int XCAP = CAP == 1 ? 1 : kStreamMaxX;
     CUtensorMap w[CAP];
     CUtensorMap x[XCAP];
     StreamEntry e[CAP];
@@ -742,71 +741,6 @@ static cudaError_t stream_dispatch(const StreamParams<CAP> &p, bool bf16, int gr
     return bf16 ? stream_go<true, 32, CAP>(p, grid, s) : stream_go<false, 32, CAP>(p, grid, s);
 }
 
-namespace {
-struct Range {
-    uintptr_t lo, hi;
-    bool meets(const Range &o) const { return lo < o.hi && o.lo < hi; }
-};
-Range range_of(const void *p, int64_t bytes) { return Range{(uintptr_t)p, (uintptr_t)p + (p ? (uintptr_t)bytes : 0u)}; }
-struct Touched {
-    Range x, r, y;
-    // Whether this linear has to come behind an earlier one: reads what that writes, writes what that reads or writes.
-    bool after(const Touched &o) const { return o.y.meets(x) || o.y.meets(r) || o.y.meets(y) || y.meets(o.x) || y.meets(o.r); }
-};
-Touched touched(const StreamLinear &l) {
-    const qf_linear_desc &d = *l.d;
-    const int64_t cols = d.epilogue == QF_EPI_SILU_MUL ? d.N / 2 : d.N, size = d.out_dtype == QF_F32 ? 4 : 2;
-    return Touched{range_of(l.X, d.M * d.K * 2), range_of(d.epilogue == QF_EPI_RESIDUAL_ADD ? l.residual : nullptr, d.M * cols * size),
-                   range_of(l.Y, d.M * cols * size)};
-}
-int64_t row_blocks(const qf_linear_desc &d) { return (d.N + 127) / 128; }
-}  // namespace
-
-void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t room_step, int64_t room_two, std::vector<int> *order,
-                  std::vector<ChainPhase> *phases) {
-    std::vector<Touched> all;
-    std::vector<int> step_of;
-    int steps = 0;
-    int64_t used = 0;
-    for (int i = 0; i < count; ++i) {
-        all.push_back(touched(l[i]));
-        bool fresh = steps == 0 || used + room[i] > room_step;
-        for (int o = i; !fresh && o-- > 0 && step_of[o] == steps - 1;) fresh = all[i].after(all[o]);
-        if (fresh) {
-            ++steps;
-            used = 0;
-        }
-        used += room[i];
-        step_of.push_back(steps - 1);
-    }
-    int last = -1, late_before = -1, late = -1;  // phases: of the step before; late ones two steps back and one
-    for (int q = 0, i0 = 0, i1, i2; q < steps; ++q, i0 = i1) {
-        for (i1 = i0; i1 < count && step_of[i1] == q;) ++i1;
-        for (i2 = i1; i2 < count && step_of[i2] == q + 1;) ++i2;
-        int64_t here = 0, there = 0;
-        for (int i = i0; i < i1; ++i) here += room[i];
-        for (int i = i1; i < i2; ++i) there += room[i];
-        std::vector<char> waits(i1 - i0, i1 == i2 || here + there > room_two);
-        bool any = false;
-        for (int i = i0; i < i1; ++i) {
-            for (int o = i1; o < i2; ++o) waits[i - i0] = waits[i - i0] || all[o].after(all[i]);
-            any = any || waits[i - i0];
-        }
-        if (!any) waits.assign(i1 - i0, 1);
-        const int wait0 = last, wait1 = late_before;
-        late_before = late;
-        late = -1;
-        for (int part = 0; part < 2; ++part) {
-            ChainPhase c{(int)order->size(), 0, {wait0, wait1}, q, part == 1, here, i1, i2};
-            for (int i = i0; i < i1; ++i)
-                if ((waits[i - i0] != 0) == (part == 0)) order->push_back(i), ++c.count;
-            if (c.count == 0) continue;
-            (part == 0 ? last : late) = (int)phases->size();
-            phases->push_back(c);
-        }
-    }
-}
-
 template <int CAP>
 static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s) {
     StreamParams<CAP> p;
@@ -862,40 +796,15 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
         ph.pieces = 0;
     } else {
         grid = sms;
-        const int streams = 2 * grid;
-        std::vector<int> order;
-        std::vector<ChainPhase> chain;
-        auto slots_of = [&](int i) { return l[i].split > 1 ? row_blocks(*l[i].d) * l[i].split : 0; };
-        std::vector<int64_t> slots(count);
-        for (int i = 0; i < count; ++i) slots[i] = slots_of(i);
-        chain_phases(l, count, slots.data(), kStreamSlots, kStreamSlots, &order, &chain);
-        int slot = 0;
-        for (const ChainPhase &c : chain) {
+        ChainPlan plan;
+        plan_stream_chain(l, count, 2 * grid, &plan);
+        for (const ChainPhase &c : plan.phases) {
             StreamPhase &ph = p.ph[phases++];
-            ph = StreamPhase{next, 0, 0, 0, streams, 0, 0, 0, {c.wait[0], c.wait[1]}};
-            // slots: from the lower end and the upper one in turn, so that a late phase and the next step have their own
-            if (!c.late) slot = c.step & 1 ? kStreamSlots - (int)c.room : 0;
+            ph = StreamPhase{next, 0, 0, 0, c.streams, c.home, c.flip, 0, {c.wait[0], c.wait[1]}};
             for (int k = c.first; k < c.first + c.count; ++k) {
-                const int st = enter(order[k]);
+                const int st = enter(plan.order[k]);
                 if (st != QF_OK) return st;
-                p.e[next - 1].slot = slot;
-                slot += (int)slots[order[k]];
-            }
-            if (c.late) {
-                // to the streams that have nothing in the next step, if they can do it in that time; else to all, those first
-                // that had nothing in this one
-                int64_t pieces = 0, longest = 0, work = 0;
-                for (int i = c.next0; i < c.next1; ++i) {
-                    pieces += row_blocks(*l[i].d) * l[i].split;
-                    longest = std::max<int64_t>(longest, l[i].per);
-                }
-                for (int e = ph.first; e < next; ++e) work += (int64_t)(p.e[e].end - p.e[e].begin) * p.e[e].per;
-                if (pieces < streams && work <= longest * (streams - pieces)) {
-                    ph.home = (int)pieces;
-                    ph.streams = streams - (int)pieces;
-                } else {
-                    ph.flip = 1;
-                }
+                p.e[next - 1].slot = plan.linears[plan.order[k]].slot;
             }
             ph.active = std::min(ph.pieces, ph.streams);
         }
@@ -916,35 +825,6 @@ int launch_stream(qf_ctx *ctx, const StreamLinear &l, void *ws, size_t counter_b
 
 int launch_stream_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s) {
     return stream_launch<kStreamMaxLinears>(ctx, l, count, ws, counter_bytes, s);
-}
-
-int stream_chain_length(const StreamLinear *l, int count) {
-    constexpr int XCAP = StreamParams<kStreamMaxLinears>::XCAP;
-    const void *x_of[XCAP];
-    int64_t x_k[XCAP];
-    std::vector<Range> written;
-    int maps = 0, n = 0;
-    for (; n < count && n < kStreamMaxLinears; ++n) {
-        const qf_linear_desc &d = *l[n].d;
-        if (d.M != l[0].d->M || d.act_dtype != l[0].d->act_dtype || row_blocks(d) * l[n].split > (1 << 24)) break;
-        int m = 0;
-        while (m < maps && !(x_of[m] == l[n].X && x_k[m] == d.K)) ++m;
-        if (m == XCAP) break;
-        // weights are read ahead of the phases: they must not be an earlier linear's result
-        const Range w = range_of(l[n].blob, d.N / 64 * (d.K / 128) * QF_SLAB_UNIT_BYTES);
-        bool meets = false;
-        for (const Range &y : written) meets = meets || y.meets(w);
-        if (meets) break;
-        if (m == maps) {
-            x_of[maps] = l[n].X;
-            x_k[maps++] = d.K;
-        }
-        const Range y = touched(l[n]).y;
-        bool known = false;
-        for (const Range &o : written) known = known || (o.lo <= y.lo && y.hi <= o.hi);
-        if (!known) written.push_back(y);
-    }
-    return n;
 }
 
 }  // namespace qf

@@ -1,4 +1,5 @@
-// Host interface of the streaming tcgen05 kernel on QF_LAYOUT_GEMV_SLAB weights (qf_stream.cu).
+// Host interface of the streaming tcgen05 kernel on QF_LAYOUT_GEMV_SLAB weights (qf_stream.cu), of the chains of up to 8 rows
+// (qf_slab_chain.cu) and of the planner of both (qf_chain_plan.cu).
 #pragma once
 
 #include <vector>
@@ -8,8 +9,9 @@
 namespace qf {
 
 constexpr int kStreamMaxLinears = 112;  // of one launch: the tensor maps travel as kernel parameters (32 764 bytes)
-
+constexpr int kStreamMaxX = 16;         // different activations of one launch, likewise
 constexpr int kStreamSlots = 4 * kSmCount;  // two for each of the two streams of an SM
+constexpr int kSlabChainPlaces = 4;     // thread blocks per SM of a chain of up to kSlabGemvRows rows
 
 // A checked linear on slab weights. In a chain K is cut into `split` pieces of `per` chunks of 128 codes.
 struct StreamLinear {
@@ -28,11 +30,28 @@ struct ChainPhase {
     bool late;
     int64_t room;      // of the whole step
     int next0, next1;  // the linears of the next step
+    int home, streams, flip;  // more than kSlabGemvRows rows: the streams from `home` on that its pieces are dealt to, backwards first
 };
 // room[i]: what linear i needs of something that a step has room_step of, and a step with late linears and the next one together
 // room_two.
 void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t room_step, int64_t room_two, std::vector<int> *order,
                   std::vector<ChainPhase> *phases);
+
+// What a linear of a chain gets.
+struct ChainLinear {
+    int slot, slots;  // of partial sums
+    // up to kSlabGemvRows rows: thread blocks, those of an SM, and where they are (see sc_number in qf_slab_chain.cu)
+    int grid, per_sm, home, first_sm;
+};
+struct ChainPlan {
+    std::vector<int> order;  // the linears, phase by phase
+    std::vector<ChainPhase> phases;
+    std::vector<ChainLinear> linears;
+};
+inline int64_t row_blocks(const qf_linear_desc &d) { return (d.N + 127) / 128; }
+void plan_stream_chain(const StreamLinear *l, int count, int streams, ChainPlan *plan);
+// false: more thread blocks than the SMs have places for.
+bool plan_slab_chain(const StreamLinear *l, int count, int sms, ChainPlan *plan);
 
 // Returned by the launches where the current context has fewer SMs than the device (a partition of it), so that the blocks of a
 // cooperative launch do not fit: nothing was launched, and the other kernels serve.
