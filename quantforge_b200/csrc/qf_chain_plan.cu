@@ -72,7 +72,8 @@ void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t
 
 void plan_stream_chain(const StreamLinear *l, int count, int streams, ChainPlan *plan) {
     std::vector<int64_t> slots(count);
-    plan->linears.assign(count, ChainLinear{});
+    *plan = ChainPlan{};
+    plan->linears.resize(count);
     for (int i = 0; i < count; ++i) {
         slots[i] = l[i].split > 1 ? row_blocks(*l[i].d) * l[i].split : 0;
         plan->linears[i].slots = (int)slots[i];
@@ -110,7 +111,8 @@ void plan_stream_chain(const StreamLinear *l, int count, int streams, ChainPlan 
 bool plan_slab_chain(const StreamLinear *l, int count, int sms, ChainPlan *plan) {
     const int blocks = kSlabChainPlaces * sms;
     std::vector<int64_t> per_sm(count);
-    plan->linears.assign(count, ChainLinear{});
+    *plan = ChainPlan{};
+    plan->linears.resize(count);
     for (int i = 0; i < count; ++i) {
         int depth;
         ChainLinear &x = plan->linears[i];

@@ -1,6 +1,7 @@
 """How a batched call divides its linears into launches and phases (qf_w4a16_batched_plan): host logic, no GPU. Addresses are made up;
 nothing reads them."""
 import ctypes
+import random
 
 import pytest
 
@@ -79,3 +80,82 @@ def test_linears_without_rows(rows):
             calls = layers(rows, 2048, 5632, 4)
             mixed = plan(calls[:14] + [empty] * 3 + calls[14:])
             assert [p["launch"] for p in mixed] == [0] * 14 + [-1] * 3 + [1] * 14
+
+
+def _meet(a, b):
+    return a[0] < b[1] and b[0] < a[1]
+
+
+def _ranges(c):
+    """What a linear reads (activations, residual, weights) and what it writes."""
+    cols = c["N"] // 2 if c["epilogue"] == QF_EPI_SILU_MUL else c["N"]
+    reads = [(c["x"], c["x"] + c["M"] * c["K"] * 2)]
+    if c["epilogue"] == QF_EPI_RESIDUAL_ADD:
+        reads.append((c["residual"], c["residual"] + c["M"] * cols * 2))
+    return reads, (c["w"], c["w"] + blob_bytes(c["N"], c["K"])), (c["y"], c["y"] + c["M"] * cols * 2)
+
+
+def _check(calls, got):
+    """Every pair of linears of a launch of which one touches what the other writes has an order, and so do those that share slots."""
+    launches = {}
+    for c, p in zip(calls, got):
+        launches.setdefault(p["launch"], []).append((c, p))
+    for linears in launches.values():
+        if len(linears) == 1:
+            continue
+        behind = {}  # phase -> all phases that are complete before it begins
+        for _, p in sorted(linears, key=lambda cp: cp[1]["phase"]):
+            if p["phase"] not in behind:
+                waits = [w for w in (p["wait0"], p["wait1"]) if w >= 0]
+                assert all(w < p["phase"] for w in waits)
+                behind[p["phase"]] = set(waits).union(*[behind[w] for w in waits])
+        for j, (cj, pj) in enumerate(linears):
+            rj, wj, yj = _ranges(cj)
+            for ci, pi in linears[:j]:
+                ri, wi, yi = _ranges(ci)
+                assert not _meet(yi, wj)  # weights are fetched ahead of all waits
+                if any(_meet(yi, r) for r in rj + [yj]) or any(_meet(yj, r) for r in ri + [wi]):
+                    assert pi["phase"] in behind[pj["phase"]], (ci, cj)
+                side_by_side = pi["phase"] not in behind[pj["phase"]] and pj["phase"] not in behind[pi["phase"]]
+                if side_by_side and pi["slots"] and pj["slots"]:
+                    assert pi["slot"] + pi["slots"] <= pj["slot"] or pj["slot"] + pj["slots"] <= pi["slot"]
+    return launches
+
+
+def test_random_batches_become_chains():
+    """What the test above looks at is not all linears that go one by one."""
+    chained = 0
+    for seed in range(20):
+        rng = random.Random(1000 + seed)
+        M, calls, mem = rng.choice([1, 8, 9, 32]), [], Memory()
+        spots = [mem.take(1 << 20) for _ in range(6)]
+        for _ in range(60):
+            N, K = rng.choice([256, 1024, 2048]), rng.choice([256, 1024, 2048])
+            calls.append(linear(M, N, K, rng.choice(spots), mem.take(blob_bytes(N, K)), rng.choice(spots)))
+        launches = _check(calls, plan(calls))
+        chained += max(len(v) for v in launches.values()) > 20
+    assert chained >= 15
+
+
+@pytest.mark.parametrize("seed", range(20))
+def test_places_of_a_step(seed):
+    """Up to 8 rows: no thread block has work of two linears of a step (its four warps count their ends together)."""
+    rng = random.Random(seed)
+    mem = Memory()
+    spots = [mem.take(1 << 20) for _ in range(4)]
+    calls = []
+    for _ in range(100):
+        N, K = rng.choice([128, 256, 1024, 4096]), rng.choice([128, 256, 1024, 2048])
+        calls.append(linear(4, N, K, rng.choice(spots), mem.take(blob_bytes(N, K)), rng.choice(spots)))
+    got = plan(calls)
+    steps = {}
+    for p in got:
+        steps.setdefault((p["launch"], p["wait0"], p["wait1"]), []).append(p)
+    assert max(len(s) for s in steps.values()) > 1
+    for s in steps.values():
+        taken = set()
+        for p in s:
+            per_sm, first_sm, home = -(-p["blocks"] // 148), p["place"] // 4, p["place"] % 4
+            mine = {4 * ((first_sm + v // per_sm) % 148) + (home + v % per_sm) % 4 for v in range(p["blocks"])}
+            assert len(mine) == p["blocks"] and not taken & mine
+            taken |= mine
