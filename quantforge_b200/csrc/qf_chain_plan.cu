@@ -13,15 +13,18 @@ struct Range {
 };
 Range range_of(const void *p, int64_t bytes) { return Range{(uintptr_t)p, (uintptr_t)p + (p ? (uintptr_t)bytes : 0u)}; }
 struct Touched {
-    Range x, r, y;
-    // Whether this linear has to come behind an earlier one: reads what that writes, writes what that reads or writes.
-    bool after(const Touched &o) const { return o.y.meets(x) || o.y.meets(r) || o.y.meets(y) || y.meets(o.x) || y.meets(o.r); }
+    Range x, r, w, y;
+    // Whether this linear has to come behind an earlier one: reads what that writes, writes what that reads or writes. (Weights are
+    // read ahead of all waits: where an earlier result becomes weights, stream_chain_length ends the chain.)
+    bool after(const Touched &o) const {
+        return o.y.meets(x) || o.y.meets(r) || o.y.meets(y) || y.meets(o.x) || y.meets(o.r) || y.meets(o.w);
+    }
 };
 Touched touched(const StreamLinear &l) {
     const qf_linear_desc &d = *l.d;
     const int64_t cols = d.epilogue == QF_EPI_SILU_MUL ? d.N / 2 : d.N, size = d.out_dtype == QF_F32 ? 4 : 2;
     return Touched{range_of(l.X, d.M * d.K * 2), range_of(d.epilogue == QF_EPI_RESIDUAL_ADD ? l.residual : nullptr, d.M * cols * size),
-                   range_of(l.Y, d.M * cols * size)};
+                   range_of(l.blob, d.N / 64 * (d.K / 128) * QF_SLAB_UNIT_BYTES), range_of(l.Y, d.M * cols * size)};
 }
 }  // namespace
 
@@ -151,18 +154,17 @@ int stream_chain_length(const StreamLinear *l, int count) {
         while (m < maps && !(x_of[m] == l[n].X && x_k[m] == d.K)) ++m;
         if (m == kStreamMaxX) break;
         // weights are read ahead of the phases: they must not be an earlier linear's result
-        const Range w = range_of(l[n].blob, d.N / 64 * (d.K / 128) * QF_SLAB_UNIT_BYTES);
+        const Touched t = touched(l[n]);
         bool meets = false;
-        for (const Range &y : written) meets = meets || y.meets(w);
+        for (const Range &y : written) meets = meets || y.meets(t.w);
         if (meets) break;
         if (m == maps) {
             x_of[maps] = l[n].X;
             x_k[maps++] = d.K;
         }
-        const Range y = touched(l[n]).y;
         bool known = false;
-        for (const Range &o : written) known = known || (o.lo <= y.lo && y.hi <= o.hi);
-        if (!known) written.push_back(y);
+        for (const Range &o : written) known = known || (o.lo <= t.y.lo && t.y.hi <= o.hi);
+        if (!known) written.push_back(t.y);
     }
     return n;
 }

@@ -122,6 +122,43 @@ def _check(calls, got):
     return launches
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 20])
+def test_a_result_over_weights_that_an_earlier_linear_reads(M):
+    # the last linear of each layer writes over the weights of the layer's k projection, which nothing waits for
+    calls = layers(M, 2048, 5632, 4)
+    for i in range(6, len(calls), 7):
+        calls[i]["y"] = calls[i - 5]["w"]
+        if i + 1 < len(calls):
+            for c in calls[i + 1:i + 4]:
+                c["x"] = calls[i]["y"]
+    _check(calls, plan(calls))
+    # pairs side by side but for that
+    mem, calls = Memory(), []
+    x = mem.take(M * 4096)
+    for _ in range(8):
+        w = mem.take(blob_bytes(2048, 2048))
+        calls += [linear(M, 2048, 2048, x, w, mem.take(M * 4096)), linear(M, 2048, 2048, x, mem.take(blob_bytes(2048, 2048)), w + 8192)]
+    got = plan(calls)
+    assert {p["launch"] for p in got} == {0}
+    _check(calls, got)
+
+
+@pytest.mark.parametrize("seed", range(60))
+def test_whatever_touches_has_an_order(seed):
+    rng = random.Random(seed)
+    M = rng.choice([1, 2, 5, 8, 9, 16, 17, 32])
+    span = rng.choice([1 << 18, 1 << 21, 1 << 24, 1 << 28])  # a small one makes nearly everything meet
+    mem, calls = Memory(), []
+    spot = lambda: (1 << 36) + rng.randrange(span) // 1024 * 1024  # noqa: E731
+    spots = [spot() for _ in range(rng.choice([3, 6, 12]))]
+    for _ in range(rng.choice([9, 20, 60, 130])):
+        N, K = rng.choice([256, 512, 1024, 2048]), rng.choice([256, 512, 1024, 5632])
+        w = mem.take(blob_bytes(N, K)) if rng.random() < 0.9 else rng.choice(spots)
+        y = rng.choice(spots) if calls == [] or rng.random() < 0.95 else rng.choice(calls)["w"]
+        calls.append(linear(M, N, K, rng.choice(spots), w, y, rng.choice(spots), rng.choice([QF_EPI_NONE, QF_EPI_SILU_MUL, QF_EPI_RESIDUAL_ADD])))
+    _check(calls, plan(calls))
+
+
 def test_random_batches_become_chains():
     """What the test above looks at is not all linears that go one by one."""
     chained = 0
