@@ -217,7 +217,9 @@ __global__ void __launch_bounds__(SLAB_THREADS, SC_BLOCKS_PER_SM) slab_chain_ker
                     }
                     passed[i] = w;
                 }
-                // the results were stored through the generic proxy and are read by the copy engine
+                // Lane 0 has acquired the counters, and all lanes issue copies: a vote orders no memory, the barrier does. Then the
+                // results, which were stored through the generic proxy, are read by the copy engine.
+                __syncwarp();
                 asm volatile("fence.proxy.async;" ::: "memory");
             }
             // (behind a wait that ran out as well: the stages are complete then, and can be waited for)

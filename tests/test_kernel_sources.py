@@ -10,9 +10,23 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 SOURCES = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
 
 
+def _code(path):
+    with open(path) as f:
+        return re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+
+
 @pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
 def test_no_load_through_the_read_only_path(path):
-    with open(path) as f:
-        code = re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+    code = _code(path)
     found = re.findall(r"\b__ldg\s*\(|\bld\.global\S*\.nc\b|\bconst\b[^;,(){}]*\*\s*(?:const\s+)?__restrict__", code)
     assert not found, found
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_what_one_lane_acquires_is_passed_on(path):
+    """One lane polls a counter for its warp, inside a vote. Votes order no memory, so before the lanes' proxy fences, behind which they
+    issue copies of what the counter guards, comes a warp barrier."""
+    code = _code(path)
+    for poll in re.finditer(r"lane\s*!=\s*0\s*\|\|\s*\w*acquire\w*\s*\(", code):
+        fence = code.find("fence.proxy.async", poll.end())
+        assert fence < 0 or "__syncwarp()" in code[poll.end():fence]
