@@ -480,10 +480,12 @@ def run_stack_workload(env, args):
     parity = st.check_parity(oracle_linear, oracle_silu_mul)
     parity["tolerance"] = 1e-2
     parity["ok"] = bool(parity["max_rel_err"] < 1e-2 and parity["ranks_bit_identical"] and
-                        qf.device_status(dev) == 0)
-    parity["checked"] = ("every linear of layer 0 through the call path of the timed step, 64 sampled output columns "
-                         "each, against the numpy restatement of the reference arithmetic (fp64 accumulation); "
-                         "row-parallel linears after the sum over ranks, all ranks compared bit for bit")
+                        parity["step_bits_identical"] is not False and qf.device_status(dev) == 0)
+    parity["checked"] = ("every linear of layer 0, 64 sampled output columns each, against the numpy restatement of the "
+                         "reference arithmetic (fp64 accumulation); row-parallel linears after the sum over ranks, all "
+                         "ranks compared bit for bit; a step that is one batched call: all its output buffers bit for bit "
+                         "against its linears one by one (above 8 rows: against one batch per layer, whose linears are "
+                         "compared with the restatement as well)")
     if not parity["ok"]:
         if rank == 0:
             print(json.dumps({"error": "parity check failed", "parity": parity}), flush=True)

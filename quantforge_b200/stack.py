@@ -286,19 +286,48 @@ class DecodeLinearStack:
         return per_layer * self.L
 
     # ------------------------------------------------------------------------------------------
+    def _step_is_its_parts(self) -> bool:
+        """Whether a step leaves the same bits in every output buffer as its linears one by one, or above SLAB_BATCH rows as its layers,
+        a batch each."""
+        calls = self._chain_calls()
+        outs = list({out.data_ptr(): out for _, _, out, _, _ in calls}.values())
+
+        def bits(run):
+            for out in outs:
+                out.zero_()
+            run()
+            return [out.view(torch.int16).clone() for out in outs]
+
+        def parts():
+            if self.M <= SLAB_BATCH:
+                h = self.buf["h_in"]
+                for ly in self.layers:
+                    h = self._layer(ly, h)
+            else:
+                n = len(calls) // self.L
+                for i in range(0, len(calls), n):
+                    ops.LinearBatch(calls[i:i + n]).run()
+
+        return all(torch.equal(a, b) for a, b in zip(bits(self.step), bits(parts)))
+
     def check_parity(self, oracle_linear: Callable, silu_mul: Callable) -> dict:
-        """Runs every linear of layer 0 through the call path `step` uses (those of a chain one by one) and compares SAMPLE_COLUMNS output columns
-        with `oracle_linear(x, qweight_rows, scales, zeros, group) -> float array [M, rows]` (a CPU restatement the
+        """Runs every linear of layer 0 by itself and compares SAMPLE_COLUMNS output columns with
+        `oracle_linear(x, qweight_rows, scales, zeros, group) -> float array [M, rows]` (a CPU restatement the
         caller provides; this package has none). Row-parallel linears are compared after the sum over ranks, with
         the oracle's partial sums added across ranks in float64; every rank must also hold identical bits.
         The comparison is made on fp32 outputs of the same kernels (rounding an exact result to bf16 alone costs up
         to 1.3e-2 of the output's rms on layers this wide, more than the tolerance the path is specified with).
-        Returns {"max_rel_err", "cases", "ranks_bit_identical"}; errors are max |y - ref| / rms(ref)."""
+        Where a step is one batched call, the whole step is run too. Up to SLAB_BATCH rows it must leave the bits of the linears
+        called one by one. Above, a chain divides K in its own way: the linears of layer 0 are compared with the oracle once more as
+        a batch, and the step must leave the bits of one batch per layer.
+        Returns {"max_rel_err", "cases", "ranks_bit_identical", "step_bits_identical"}; errors are max |y - ref| / rms(ref), and the
+        last is None where a step calls its linears one by one."""
         import numpy as np
         b = self.buf
         ly = self.layers[0]
         M = self.M
         worst, cases, identical = 0.0, 0, True
+        batched = []  # (linear, activations, output buffer, epilogue, reference) of a layer that runs as a chain
 
         def ref_of(lin, x):
             s = lin.sample
@@ -307,6 +336,9 @@ class DecodeLinearStack:
         def err_of(y_cols, ref):
             rms = float(np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
             return float(np.max(np.abs(y_cols.astype(np.float64) - ref)) / max(rms, 1e-30))
+
+        def sampled(lin, out):
+            return out[:, torch.from_numpy(lin.sample["cols"]).to(out.device)].float().cpu().numpy()
 
         def f32(t):
             return torch.empty(t.shape, dtype=torch.float32, device=t.device)
@@ -321,9 +353,9 @@ class DecodeLinearStack:
             if lin.silu:
                 n = len(lin.sample["cols"])
                 ref = silu_mul(ref[:, :n], ref[:, n:])
-            y = out[:, torch.from_numpy(lin.sample["cols"]).to(out.device)].float().cpu().numpy()
-            worst = max(worst, err_of(y, ref))
+            worst = max(worst, err_of(sampled(lin, out), ref))
             cases += 1
+            batched.append((lin, x, buf, epilogue, ref))
 
         def row(lin, x, buf):
             nonlocal worst, cases, identical
@@ -337,9 +369,10 @@ class DecodeLinearStack:
                 every = [torch.empty_like(out) for _ in range(self.world)]
                 dist.all_gather(every, out.contiguous(), group=self.group)
                 identical = identical and all(torch.equal(every[0], t) for t in every)
-            y = out[:, torch.from_numpy(lin.sample["cols"]).to(out.device)].float().cpu().numpy()
-            worst = max(worst, err_of(y, part.cpu().numpy()))
+            part = part.cpu().numpy()
+            worst = max(worst, err_of(sampled(lin, out), part))
             cases += 1
+            batched.append((lin, x, buf, QF_EPI_NONE, part))
 
         h = b["h_in"]
         if self.fuse:
@@ -357,8 +390,15 @@ class DecodeLinearStack:
             column(ly["gate"], b["o"], b["gate"])
             column(ly["up"], b["o"], b["up"])
             row(ly["down"], b["gate"], b["down"])
+        if self.chain and M > SLAB_BATCH:
+            outs = [f32(buf) for _, _, buf, _, _ in batched]
+            ops.LinearBatch([(x, lin.slab, out, epi, None) for (lin, x, _, epi, _), out in zip(batched, outs)]).run()
+            for (lin, _, _, _, ref), out in zip(batched, outs):
+                worst = max(worst, err_of(sampled(lin, out), ref))
+                cases += 1
+        step_identical = self._step_is_its_parts() if self.chain else None
         if self.world > 1:
             t = torch.tensor([worst, 0.0 if identical else 1.0], device=self.dev, dtype=torch.float64)
             dist.all_reduce(t, op=dist.ReduceOp.MAX, group=self.group)
             worst, identical = float(t[0].item()), bool(t[1].item() == 0.0)
-        return {"max_rel_err": worst, "cases": cases, "ranks_bit_identical": identical}
+        return {"max_rel_err": worst, "cases": cases, "ranks_bit_identical": identical, "step_bits_identical": step_identical}
