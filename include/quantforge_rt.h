@@ -192,8 +192,9 @@ int qf_w4a16_linear_fused(qf_ctx *ctx, const qf_linear_desc *desc, const void *X
  * concatenated linear, o with the residual, gate/up with SiLU * mul, down with the residual). Entry i uses
  * descs[i], X[i], qweight[i], scales[i], qzeros[i] (may be NULL), Y[i], residual[i] (`residual` itself may be
  * NULL). Consecutive kernels are chained with programmatic dependent launch; entry i+1 may read what entry i
- * wrote. `workspace` must hold the largest qf_w4a16_workspace_bytes over the entries. Stops at the first entry
- * that fails and returns its status (earlier entries stay enqueued).
+ * wrote. `workspace` must hold the largest qf_w4a16_workspace_bytes over the entries; qf_w4a16_batched_workspace_bytes says how much
+ * it takes for several linears to be one launch, and with less they go one by one. Stops at the first entry that fails and returns
+ * its status (earlier entries stay enqueued).
  * Consecutive entries on QF_LAYOUT_GEMV_SLAB weights that leave path and split_k to the library and have the same M <= 32, the
  * same act_dtype and, above 8 rows, N % 128 == 0 run as ONE cooperative launch (at most 112 linears and 16 different X; weights that
  * an earlier entry writes begin a new one): entries of which none writes what another one reads (weights too) or writes run side by
@@ -205,6 +206,7 @@ int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs,
                             const void *const *qweight, const void *const *scales, const void *const *qzeros,
                             void *const *Y, const void *const *residual, void *workspace, size_t workspace_bytes,
                             void *stream);
+size_t qf_w4a16_batched_workspace_bytes(int count, const qf_linear_desc *descs);
 /* Kernel launches that this call would make (-1: bad arguments). Nothing is enqueued. */
 int qf_w4a16_batched_launches(qf_ctx *ctx, int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight,
                               void *const *Y, const void *const *residual, const void *workspace, size_t workspace_bytes);

@@ -37,7 +37,7 @@ EXPORTS = [
     "qf_launch_count", "qf_prepack_w4", "qf_prepack_w4_tiled", "qf_w4a16_gemv_static_scratch", "qf_ctx_status", "qf_ctx_clear_status",
     "qf_comm_create", "qf_comm_export", "qf_comm_connect", "qf_comm_destroy", "qf_w4a16_linear_allreduce",
     "qf_w4a16_linear_allgather", "qf_w4a16_linear_host_async", "qf_w4a16_linear_fused", "qf_w4a16_linear_batched",
-    "qf_w4a16_batched_launches", "qf_w4a16_batched_plan",
+    "qf_w4a16_batched_launches", "qf_w4a16_batched_plan", "qf_w4a16_batched_workspace_bytes",
     "qf_prepack_bytes", "qf_prepack_gemv_slab", "qf_unpack_gemv_slab", "qf_repack_kn_to_canonical",
     "qf_pack_int4", "qf_quantize_w4",
 ]
@@ -95,6 +95,8 @@ def load() -> ctypes.CDLL:
     lib.qf_w4a16_linear_batched.argtypes = [vp, ctypes.c_int, dp, pvp, pvp, pvp, pvp, pvp, pvp, vp, sz, vp]
     lib.qf_w4a16_batched_launches.argtypes = [vp, ctypes.c_int, dp, pvp, pvp, pvp, pvp, vp, sz]
     lib.qf_w4a16_batched_plan.argtypes = [ctypes.c_int, dp, pvp, pvp, pvp, pvp, vp, sz, ctypes.POINTER(ctypes.c_int32)]
+    lib.qf_w4a16_batched_workspace_bytes.restype = sz
+    lib.qf_w4a16_batched_workspace_bytes.argtypes = [ctypes.c_int, dp]
     lib.qf_prepack_bytes.restype = sz
     lib.qf_prepack_bytes.argtypes = [ctypes.c_int, i64, i64]
     lib.qf_prepack_gemv_slab.argtypes = [vp, dp, vp, vp, vp, vp, vp]

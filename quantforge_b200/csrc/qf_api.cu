@@ -528,12 +528,22 @@ size_t qf_w4a16_workspace_bytes(const qf_linear_desc *desc) {
     Plan plan;
     if (make_plan(desc, &plan, nullptr) != QF_OK) return 0;
     size_t need = plan.ws_partial_bytes + plan.ws_counter_bytes;
-    if (slab_any(desc)) {
-        // enough for either kernel: an exchanging call on the same descriptor takes the one, a batched call the other
-        qf_linear_desc d = *desc;
-        d.path = QF_PATH_GEMV;
-        if (make_plan(&d, &plan, nullptr) == QF_OK) need = std::max(need, plan.ws_partial_bytes + plan.ws_counter_bytes);
-        need = std::max(need, std::max(kCounterBytes + stream_workspace_bytes(d.M), chain_workspace_bytes(d.M)));
+    if (desc->weight_layout == QF_LAYOUT_GEMV_SLAB && desc->split_k == 0) {
+        // An exchanging call on the same descriptor may divide the weights among more thread blocks. That is also what the
+        // streaming GEMV kernel needs where it steps in for the tcgen05 kernel.
+        const int64_t units = desc->N / 64 * (desc->K / 128);
+        need = std::max(need, slab_workspace_bytes((int)std::min<int64_t>(units, slab_exchange_grid(desc, kSmCount)), desc->M));
+    }
+    return need;
+}
+
+size_t qf_w4a16_batched_workspace_bytes(int count, const qf_linear_desc *descs) {
+    size_t need = 0;
+    for (int i = 0; descs && i < count; ++i) {
+        need = std::max(need, qf_w4a16_workspace_bytes(&descs[i]));
+        if (i > 0 && chains(&descs[i]) && chains(&descs[i - 1]) && descs[i].M == descs[i - 1].M &&
+            descs[i].act_dtype == descs[i - 1].act_dtype)
+            need = std::max(need, chain_workspace_bytes(descs[i].M));
     }
     return need;
 }

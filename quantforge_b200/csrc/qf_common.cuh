@@ -282,6 +282,12 @@ constexpr int64_t kSlabGemvRows = 8;
 int slab_m_pad(int64_t M);
 void slab_geometry(int64_t M, int64_t N, int64_t K, int sm_count, int grid_request, int *grid_out, int *depth_out);
 size_t slab_workspace_bytes(int grid, int64_t M);
+// Thread blocks of an exchanging launch on slab weights: a collecting one waits for its peers while it holds its SM slot, so all of them
+// must be resident at once on every rank: whole multiples of the SM count by the plain kernel's size rule.
+inline int slab_exchange_grid(const qf_linear_desc *d, int sm_count) {
+    const long long wbytes = (long long)(d->N / 64) * (d->K / 128) * QF_SLAB_UNIT_BYTES;
+    return (wbytes <= kSlabSmallBytes ? 2 : d->M > 16 ? 3 : 4) * sm_count;
+}
 int launch_gemv_slab(qf_ctx *ctx, const qf_linear_desc *d, const Plan &p, const void *X, const void *blob, void *Y,
                      const void *residual, void *ws, cudaStream_t s);
 int launch_gemv_slab_ar(qf_ctx *ctx, const qf_linear_desc *d, const Plan &p, const void *X, const void *blob,

@@ -429,7 +429,7 @@ class LinearBatch:
             d.act_dtype, d.out_dtype, d.zero_mode, d.zero_const = _DT[x.dtype], _DT[out.dtype], w.zero_mode, w.zero_const
             d.path, d.weight_layout, d.epilogue = QF_PATH_AUTO, QF_LAYOUT_GEMV_SLAB, epilogue
         self._arrays = [(ctypes.c_void_p * n)(*[t.data_ptr() if t is not None else 0 for t in col]) for col in zip(*self._tensors)]
-        self._ws_bytes = max(workspace_bytes(d) for d in self._descs)
+        self._ws_bytes = int(_lib.load().qf_w4a16_batched_workspace_bytes(n, self._descs))
 
     def launches(self) -> int:
         """Kernel launches of a `run()`."""

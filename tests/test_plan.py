@@ -105,3 +105,48 @@ def test_up_to_8_rows_one_kernel_reads_slab_weights(K, N):
     # AUTO is the streaming GEMV kernel, which QF_PATH_GEMV names, at any size: one order of sums for all of them
     for M in range(1, 9):
         assert _plan(M, K, N, _lib.QF_LAYOUT_GEMV_SLAB) == _plan(M, K, N, _lib.QF_LAYOUT_GEMV_SLAB, _lib.QF_PATH_GEMV)
+
+
+def _slab_desc(M, K, N):
+    return _lib.LinearDesc(M=M, N=N, K=K, group_size=128, act_dtype=_lib.QF_BF16, out_dtype=_lib.QF_BF16, zero_mode=_lib.QF_ZERO_U4,
+                           zero_const=8, weight_layout=_lib.QF_LAYOUT_GEMV_SLAB)
+
+
+def _row_tiles(M):
+    return 1 if M <= 8 else 2 if M <= 16 else 4
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16, 17, 32])
+def test_scratch_of_a_slab_linear_is_that_of_its_own_kernels(M):
+    """What one call on a descriptor can reach: the kernel of the plan and an exchange's launch. Chains are asked for by the batch."""
+    lib = _lib.load()
+    for K, N in ((128, 64), (512, 512), (2048, 1024), (2560, 1024), (4096, 4096), (4096, 14336), (8192, 57344)):
+        blob = N // 64 * (K // 128) * 4352
+        units = blob // 4352
+        blocks = min(units, 148 * (2 if blob <= 16 << 20 else 3 if M > 16 else 4))
+        words = blocks * 4 * _row_tiles(M) * 128  # a tile of partial sums per warp
+        tcgen05 = M > 8 and _plan(M, K, N, _lib.QF_LAYOUT_GEMV_SLAB) != _plan(M, K, N, _lib.QF_LAYOUT_GEMV_SLAB, _lib.QF_PATH_GEMV)
+        if tcgen05:  # its counters and slots, four a block
+            words = max(words, 8192 + 4 * 148 * ((M + 1) // 2 * 2) * 128)
+        d = _slab_desc(M, K, N)
+        assert lib.qf_w4a16_workspace_bytes(ctypes.byref(d)) == 8 * words
+    if M <= 8:  # fits what the package makes for a stream at first
+        assert lib.qf_w4a16_workspace_bytes(ctypes.byref(_slab_desc(M, 28672, 57344))) <= 4 << 20
+
+
+def test_scratch_of_a_batch():
+    lib = _lib.load()
+
+    def need(*descs):
+        return lib.qf_w4a16_batched_workspace_bytes(len(descs), (_lib.LinearDesc * len(descs))(*descs))
+
+    alone = lambda d: lib.qf_w4a16_workspace_bytes(ctypes.byref(d))  # noqa: E731
+    small, large = _slab_desc(1, 1024, 1024), _slab_desc(1, 4096, 14336)
+    assert need(small) == alone(small) and need() == 0
+    assert need(small, large) == 65536 + 2 * 4 * 148 * 4096
+    many = _slab_desc(32, 128, 128)
+    assert need(many) == alone(many) == 4 * 4096 * 2 and need(many, many) == 65536 + 4 * 148 * 32 * 128 * 8
+    # what does not chain: other rows, half row blocks above 8 rows
+    assert need(small, _slab_desc(2, 1024, 1024)) == alone(small)
+    half = _slab_desc(9, 1024, 64)
+    assert need(half, half) == alone(half)
