@@ -196,11 +196,11 @@ int qf_w4a16_linear_fused(qf_ctx *ctx, const qf_linear_desc *desc, const void *X
  * it takes for several linears to be one launch, and with less they go one by one. Stops at the first entry that fails and returns
  * its status (earlier entries stay enqueued).
  * Consecutive entries on QF_LAYOUT_GEMV_SLAB weights that leave path and split_k to the library and have the same M <= 32, the
- * same act_dtype and, above 8 rows, N % 128 == 0 run as ONE cooperative launch (at most 112 linears and 16 different X; weights that
- * an earlier entry writes begin a new one): entries of which none writes what another one reads (weights too) or writes run side by
- * side, the others one behind the other, and weights are fetched ahead. Up to 8 rows that is done where it is the faster way (a rule on the sizes), and the
- * results are those of the linears launched one by one, bit for bit; above, the bits that QF_PATH_GEMM gives for the same linear on
- * the other layouts.
+ * same act_dtype and, above 8 rows, N % 128 == 0 run as ONE cooperative launch where that is the faster way (rules on the sizes): at
+ * most 112 linears and 16 different X; weights that an earlier entry writes begin a new one. Entries of which none writes what another
+ * one reads (weights too) or writes run side by side, the others one behind the other, and weights are fetched ahead. Up to 8 rows the
+ * results are those of the linears launched one by one, bit for bit; above, such a launch gives the bits that QF_PATH_GEMM gives for
+ * the same linears on the other layouts.
  */
 int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs, const void *const *X,
                             const void *const *qweight, const void *const *scales, const void *const *qzeros,

@@ -366,7 +366,7 @@ static int chain_from(qf_ctx *ctx, int i, int count, const qf_linear_desc *descs
         run->push_back(StreamLinear{&descs[j], X[j], qweight[j], res, Y[j], plan.split_k, plan.chunks_per_split});
     }
     const int n = run->size() > 1 ? stream_chain_length(run->data(), (int)run->size()) : 1;
-    *pays = n > 1 && (descs[i].M > kSlabGemvRows || slab_chain_pays(run->data(), n));
+    *pays = n > 1 && (descs[i].M > kSlabGemvRows ? stream_chain_pays : slab_chain_pays)(run->data(), n);
     return std::max(n, 1);
 }
 

@@ -169,4 +169,67 @@ int stream_chain_length(const StreamLinear *l, int count) {
     return n;
 }
 
+// Estimated times in us of linears of more than kSlabGemvRows rows, one by one and as a chain; the chain is taken where it is the shorter.
+// One by one a linear costs `base` (it starts beside its predecessor), `member` for each further thread block with a share of a row
+// block, whose partial sums the last one adds one after the other, and `unit` for each unit of 64 x 128 codes of an SM: the streaming
+// GEMV kernel's costs, also where the tcgen05 kernel serves a linear alone (such batches are chains). A chain costs its launch, and for
+// each step `step` from the last product to the next one's first, kChunk for each 128 codes of its longest piece, at least four of them,
+// `split` where partial sums are exchanged, and `round` for each further round of pieces.
+// Fitted to 64 batches at 9 to 32 rows on weights not in L2, graph replays; standard deviation 10 %. Where the estimate picks the slower
+// way it costs 7 % at most, and 10 % on 19 other batches (4 of 76 points), but for sixteen linears of 1024 x 1024 in a row at 9 rows.
+// Measured, one by one -> chain, at 9 / 16 / 24 / 32 rows; * marks what the estimate picks otherwise (N x K):
+//   one reads the other, 2 linears:  512 x 512       8.7 -> 14.0 / 9.2 -> 14.5 / 12.4 -> 17.7 / 13.0 -> 19.4
+//                                    1024 x 2816     12.9 -> 15.7 / 13.7 -> 17.2 / 19.2 -> 19.5 / 20.3 -> 22.3
+//                                    2048 x 5632     17.1 -> 17.3 / 18.5 -> 17.5* / 29.5 -> 20.3 / 31.9 -> 21.4
+//                                    4096 x 4096     17.2 -> 17.8* / 19.7 -> 18.7 / 29.8 -> 21.1 / 32.3 -> 21.6
+//                                    256 x 18944     34.1 -> 17.7 / 34.6 -> 19.0 / 55.8 -> 20.6 / 58.2 -> 21.7
+//                       16 linears:  1024 x 1024     120 -> 97.3* / 123 -> 118* / 181 -> 147 / 186 -> 173
+//                                    1024 x 2816     101 -> 96.9* / 107 -> 113 / 168 -> 129 / 172 -> 149
+//   side by side, 2 linears:         256 x 256       6.1 -> 8.0 / 6.6 -> 8.8 / 8.5 -> 9.7 / 9.1 -> 10.4
+//                                    14336 x 1024    12.9 -> 16.4 / 14.6 -> 18.2 / 21.1 -> 22.4* / 23.6 -> 25.5*
+//                                    4096 x 4096     17.3 -> 14.7 / 19.8 -> 15.2 / 30.1 -> 16.8 / 32.4 -> 17.7
+//                 4 linears:         512 x 512       16.4 -> 9.0 / 16.9 -> 9.3 / 24.0 -> 10.7 / 25.2 -> 11.3
+//   one layer of seven:              512 / 1024      31.3 -> 24.5 / 32.9 -> 28.7 / 44.9 -> 31.7 / 47.1 -> 38.5
+//                                    4096 / 14336    83.6 -> 54.9 / 89.5 -> 58.8 / 131 -> 65.9 / 138 -> 71.4
+//   30 layers of four:               256 / 256       394 -> 431 / 414 -> 465 / 544 -> 564* / 581 -> 621*
+bool stream_chain_pays(const StreamLinear *l, int count) {
+    struct Costs {
+        double base, member, unit, step, split, round;
+    };
+    const Costs c = l[0].d->M <= 16 ? Costs{3.2, 0.43, 0.23, 3.2, 1.2, 2.9} : Costs{4.0, 0.81, 0.37, 4.7, 1.5, 4.0};
+    constexpr double kChunk = 0.48, kLaunch = 4.0;
+    constexpr int64_t kStreams = 2 * kSmCount;
+    double codes = 0, alone = 0;
+    for (int i = 0; i < count; ++i) codes += 0.5 * (double)l[i].d->N * (double)l[i].d->K;
+    if (count >= 4 && codes >= 5e6 * count) return true;  // 1.1 times as fast and more wherever measured
+    for (int i = 0; i < count; ++i) {
+        const qf_linear_desc &d = *l[i].d;
+        const int64_t chunks = d.K / 128, units = d.N / 64 * chunks;
+        int blocks, depth;
+        slab_geometry(d.M, d.N, d.K, kSmCount, 0, &blocks, &depth);
+        const int64_t share = units / blocks;  // where it is even, row blocks may begin with shares
+        const bool even = units % blocks == 0 && (share % chunks == 0 || chunks % share == 0);
+        const int64_t members = even ? std::max<int64_t>(1, chunks / share) : (chunks - 1) * blocks / units + 2;
+        const int64_t per_sm = (units + blocks - 1) / blocks * ((blocks + kSmCount - 1) / kSmCount);
+        alone += c.base + c.member * (double)(members - 1) + c.unit * (double)per_sm;
+    }
+    ChainPlan plan;
+    plan_stream_chain(l, count, (int)kStreams, &plan);
+    double chain = kLaunch;
+    for (size_t q = 0, end; q < plan.phases.size(); q = end) {
+        int64_t pieces = 0, longest = 4;
+        bool split = false;
+        for (end = q; end < plan.phases.size() && plan.phases[end].step == plan.phases[q].step; ++end)
+            for (int k = plan.phases[end].first; k < plan.phases[end].first + plan.phases[end].count; ++k) {
+                const StreamLinear &x = l[plan.order[k]];
+                pieces += row_blocks(*x.d) * x.split;
+                longest = std::max<int64_t>(longest, x.per);
+                split = split || x.split > 1;
+            }
+        const double rounds = (double)((pieces + kStreams - 1) / kStreams);
+        chain += c.step + kChunk * (double)longest * rounds + (split ? c.split : 0) + c.round * (rounds - 1);
+    }
+    return alone > chain;
+}
+
 }  // namespace qf

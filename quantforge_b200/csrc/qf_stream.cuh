@@ -64,6 +64,8 @@ int launch_stream(qf_ctx *ctx, const StreamLinear &l, void *ws, size_t counter_b
 // How many of the linears from the first on one launch can take: the same rows and activation type, weights that no earlier one
 // writes.
 int stream_chain_length(const StreamLinear *l, int count);
+// Whether one launch is the faster way.
+bool stream_chain_pays(const StreamLinear *l, int count);
 // Linears of one launch, each seeing the results of the earlier ones.
 int launch_stream_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s);
 

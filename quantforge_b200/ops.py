@@ -404,9 +404,9 @@ CHAIN_LINEARS = 112  # linears that one launch takes (see qf_w4a16_linear_batche
 class LinearBatch:
     """Linears on slab weights that run one after the other, each seeing the results of the earlier ones, enqueued by one call:
     `calls` is a sequence of (x, SlabWeight, out, epilogue, residual or None) with the meaning they have in `w4a16_linear`. The
-    tensors are kept and read where they are at each `run()`, which may be captured. Linears of 9 to 32 rows go to the GPU as one
-    launch, up to CHAIN_LINEARS of them, with the bits that the tcgen05 kernel gives on other layouts; so do those of up to 8 rows where
-    it is the faster way, with the bits that they have one by one."""
+    tensors are kept and read where they are at each `run()`, which may be captured. Where it is the faster way they go to the GPU as
+    one launch, up to CHAIN_LINEARS of them: up to 8 rows with the bits that they have one by one, above with the bits that the tcgen05
+    kernel gives on other layouts."""
 
     def __init__(self, calls):
         calls = list(calls)

@@ -196,3 +196,61 @@ def test_places_of_a_step(seed):
             mine = {4 * ((first_sm + v // per_sm) % 148) + (home + v % per_sm) % 4 for v in range(p["blocks"])}
             assert len(mine) == p["blocks"] and not taken & mine
             taken |= mine
+
+
+def _row(M, H, F, n):
+    """n linears H -> F -> H -> ..., each reading the one before."""
+    mem = Memory()
+    a, b = mem.take(M * H * 2), mem.take(M * F * 2)
+    return [linear(M, *((F, H) if i % 2 == 0 else (H, F)), (a, b)[i % 2], mem.take(blob_bytes(H, F)), (b, a)[i % 2]) for i in range(n)]
+
+
+def _beside(M, H, F, n):
+    mem = Memory()
+    x = mem.take(M * H * 2)
+    return [linear(M, F, H, x, mem.take(blob_bytes(F, H)), mem.take(M * F * 2)) for _ in range(n)]
+
+
+@pytest.mark.parametrize("M", [9, 16])
+def test_small_linears_that_wait_for_one_another_are_no_chain(M):
+    for calls in (_row(M, 512, 512, 2), _row(M, 512, 512, 8), _row(M, 1024, 2816, 2), _row(M, 1024, 2816, 4), _row(M, 2048, 2048, 3),
+                  _row(M, 768, 768, 6), _beside(M, 256, 256, 2), _beside(M, 1024, 14336, 2)):
+        assert [p["launch"] for p in plan(calls)] == list(range(len(calls)))
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 32])
+def test_what_gains_is_a_chain(M):
+    for calls in (_row(M, 4096, 14336, 2), _row(M, 2048, 5632, 4), _row(M, 256, 18944, 2), _beside(M, 512, 512, 4), _beside(M, 4096, 4096, 2),
+                  layers(M, 512, 1024, 1), layers(M, 2048, 5632, 1), layers(M, 8192, 28672, 1)):
+        assert {p["launch"] for p in plan(calls)} == {0}
+    for calls in (_row(M, 512, 512, 2), _row(M, 512, 512, 8), _beside(M, 256, 256, 2)):
+        assert {p["launch"] for p in plan(calls)} == set(range(len(calls)))
+    assert {p["launch"] for p in plan(_row(M, 1024, 2816, 8))} == (set(range(8)) if M <= 16 else {0})
+
+
+@pytest.mark.parametrize("fuse", [True, False])
+def test_stacks_that_lay_out_for_chains_get_them(fuse):
+    """A stack of 9 to 32 rows chooses its layout by the size of its linears, before there is a batch."""
+    from quantforge_b200.stack import _chain_bytes
+    rng = random.Random(fuse)
+    seen = 0
+    while seen < 150:
+        H, KV, F = 128 * rng.randint(2, 80), rng.choice([128, 512, 1024]), 128 * rng.randint(2, 224)
+        M, n = rng.randint(9, 32), rng.choice([1, 2, 6])
+        if (2 * H * H + 2 * H * KV + 3 * H * F) // 2 < (4 if fuse else 7) * _chain_bytes(M, fuse):
+            continue
+        seen += 1
+        mem, calls = Memory(), []
+        act = {k: mem.take(M * w * 2) for k, w in dict(h=H, attn=H, q=H, k=KV, v=KV, qkv=H + 2 * KV, o=H, gate=F, up=2 * F, act=F, d=H).items()}
+        h = act["h"]
+        for _ in range(n):
+            if fuse:
+                names = [(h, "qkv", H + 2 * KV, H, 0), (act["attn"], "o", H, H, h), (act["o"], "act", 2 * F, H, 0), (act["act"], "d", H, F, act["o"])]
+            else:
+                names = [(h, "q", H, H, 0), (h, "k", KV, H, 0), (h, "v", KV, H, 0), (act["q"], "o", H, H, 0), (act["o"], "gate", F, H, 0),
+                         (act["o"], "up", F, H, 0), (act["gate"], "d", H, F, 0)]
+            for x, y, N, K, r in names:
+                epi = QF_EPI_RESIDUAL_ADD if r else QF_EPI_SILU_MUL if y == "act" else QF_EPI_NONE
+                calls.append(linear(M, N, K, x, mem.take(blob_bytes(N, K)), act[y], r, epi))
+            h = act["d"]
+        assert {p["launch"] for p in plan(calls)} == {0}, (M, H, KV, F, n)

@@ -93,7 +93,7 @@ def _one_by_one(calls):
 
 @pytest.mark.parametrize("M,hidden,kv,ffn,layers,dtype", [
     (9, 1024, 512, 2816, 3, torch.bfloat16), (16, 1152, 128, 1280, 2, torch.float16), (13, 4096, 1024, 14336, 2, torch.bfloat16),
-    (17, 1024, 256, 5632, 2, torch.float16), (32, 2048, 512, 2048, 2, torch.bfloat16), (10, 256, 128, 256, 30, torch.bfloat16),
+    (17, 1024, 256, 5632, 2, torch.float16), (32, 2048, 512, 2048, 2, torch.bfloat16), (10, 512, 128, 1536, 30, torch.bfloat16),
     (9, 256, 128, 18944, 2, torch.float16), (24, 4096, 1024, 14336, 2, torch.bfloat16)])
 def test_chain_is_the_tcgen05_kernel_bit_for_bit(M, hidden, kv, ffn, layers, dtype):
     made = _layers(hidden, kv, ffn, layers, dtype)
@@ -177,10 +177,12 @@ def test_scales_near_the_top_of_bf16():
     want, got = (torch.empty(M, N, device="cuda") for _ in range(2))
     qf.w4a16_linear(x, qf.prepack_w4(qw), sc, zr, out=want, out_dtype=torch.float32, path=QF_PATH_GEMM,
                     weight_layout=qf.QF_LAYOUT_INTERLEAVED)
-    other = torch.empty_like(got)
+    others = [torch.empty_like(got) for _ in range(7)]
     slab = qf.prepack_gemv_slab(qw, sc, zr)
-    ops.LinearBatch([(x, slab, got, qf.QF_EPI_NONE, None), (x, slab, other, qf.QF_EPI_NONE, None)]).run()
-    assert bool(want.isfinite().all()) and torch.equal(want, got) and torch.equal(want, other)
+    batch = ops.LinearBatch([(x, slab, out, qf.QF_EPI_NONE, None) for out in [got] + others])
+    assert batch.launches() == 1
+    batch.run()
+    assert bool(want.isfinite().all()) and torch.equal(want, got) and all(torch.equal(want, other) for other in others)
 
 
 @pytest.mark.parametrize("fuse", [True, False])
