@@ -1,4 +1,5 @@
 """The native host path of the operators (csrc/qf_host.cpp): what it does itself, what it leaves to ops.py, what it raises."""
+import ctypes
 import json
 import os
 import shutil
@@ -329,10 +330,11 @@ def test_streams_and_growing_workspaces(seen, python_path):
                 assert seen.log == [("linear", True)]
     torch.cuda.synchronize()
     assert all(torch.equal(y, want[k]) for k, y in got)
-    used = {k[1] for k in ops._workspaces}
-    fresh = next((s for s in (torch.cuda.Stream() for _ in range(64)) if s.cuda_stream not in used), None)
-    if fresh is None:  # torch hands its streams out in turn
-        pytest.skip("every stream of the pool has a workspace")
+    # a stream of its own: torch hands out those of its pool in turn, and any of them may have a workspace from an earlier test
+    handle = ctypes.c_void_p()
+    assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(handle))) == 0
+    assert (torch.cuda.current_device(), handle.value) not in ops._workspaces
+    fresh = torch.cuda.ExternalStream(handle.value)
     with torch.cuda.stream(fresh):
         answered = []
         for t in (small, small, large, large, small):
