@@ -76,40 +76,21 @@ __device__ __forceinline__ bool sc_last_warp(unsigned *done) {
     return (before & 3u) == 3u;
 }
 
-// The place of a thread block: 4 * SM + its place on the SM. An entry takes `per_sm` places of SMs from `first_sm` on, around, those from
-// `home` on, around, and numbers its blocks SM by SM: shares of the work differ by a unit, and in this order every SM gets the same
-// sum (numbered across the SMs, the larger shares of a linear whose rows repeat after 148 blocks pile up on a few: 772 us a step of
-// 16 layers of 4096 / 14336 at one row against 691).
-__device__ __forceinline__ unsigned sc_number(const SlabChainEntry &e, unsigned place) {
-    const unsigned n_sm = gridDim.x / SC_BLOCKS_PER_SM, i = (place - (unsigned)e.home) % SC_BLOCKS_PER_SM;
-    unsigned sm = place / SC_BLOCKS_PER_SM + n_sm - (unsigned)e.first_sm;
-    if (sm >= n_sm) sm -= n_sm;
-    return i < (unsigned)e.per_sm ? sm * (unsigned)e.per_sm + i : 0xffffffffu;
-}
-
 // Takes a place. The hardware hands consecutive blocks to a few SMs first, so the block's index says nothing.
 __device__ __forceinline__ unsigned sc_claim(unsigned *words) {
     unsigned sm, sms;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
     asm volatile("mov.u32 %0, %%nsmid;" : "=r"(sms));
-    const unsigned n_sm = gridDim.x / SC_BLOCKS_PER_SM;
-    unsigned i = min(atomicAdd(words + SC_SM + sm % SC_SMS, 1u), (unsigned)SC_BLOCKS_PER_SM - 1u);
-    if (sms == n_sm) return sm * SC_BLOCKS_PER_SM + i;  // every SM has as many blocks as it can hold
-    // numbers of SMs with gaps: the first blocks of the SMs take the first places, and so on; where those are used up (on an uneven
-    // placement) others are left
-    for (int k = 0; k < SC_BLOCKS_PER_SM; ++k) {
-        const unsigned n = atomicAdd(words + SC_PLACE + i, 1u);
-        if (n < n_sm) return n * SC_BLOCKS_PER_SM + i;
-        i = (i + 1u) % SC_BLOCKS_PER_SM;
-    }
-    return 0u;  // never: as many places as blocks
+    return sc_place(
+        gridDim.x / SC_BLOCKS_PER_SM, sm, sms, [&] { return atomicAdd(words + SC_SM + sm % SC_SMS, 1u); },
+        [&](unsigned i) { return atomicAdd(words + SC_PLACE + i, 1u); });
 }
 
 // This block's entry of a phase and its number among the entry's blocks, or -1.
 __device__ __forceinline__ int sc_entry(const SlabChainParams &p, int phase, unsigned place, unsigned *v) {
     const int first = p.ph[phase].first, n = p.ph[phase].count;
     for (int e = first; e < first + n; ++e) {
-        *v = sc_number(p.e[e], place);
+        *v = sc_number(gridDim.x / SC_BLOCKS_PER_SM, p.e[e].home, p.e[e].per_sm, p.e[e].first_sm, place);
         if (*v < p.e[e].grid) return e;
     }
     return -1;

@@ -74,15 +74,6 @@ struct StreamEntry {  // one linear
     int x_map;
     int16_t out_dtype, epilogue;
 };
-struct StreamPhase {
-    int first;       // entry
-    int pieces;      // 0: ranges of units; else how many pieces the phase has
-    int q, r;        // ranges: units of the phase = q * G + r, streams 0..r-1 have q + 1
-    int streams;     // ranges: G; pieces: the streams from `home` on that they are dealt to, forwards and backwards in turn
-    int home, flip;  // flip: backwards first
-    int active;      // streams that have work
-    int wait[2];     // phases that are complete before this one reads or writes anything (or -1)
-};
 struct StreamArgs {
     unsigned long long *slots;  // [kStreamSlots][slot_words] (value | token << 32), zero between launches
     unsigned *done;             // [phases] result warps that have finished the phase, [kStreamMaxLinears] all; zero between launches
@@ -122,26 +113,10 @@ struct Segment {
     int e, b, c, len;
     int members, self, slot0, base;
 };
-// Units of stream `id` in a phase: how many, and *u0 the first.
-__device__ __forceinline__ int stream_range(const StreamPhase &ph, int id, int *u0) {
-    *u0 = id * ph.q + min(id, ph.r);
-    return ph.q + (id < ph.r ? 1 : 0);
-}
-// The piece that stream `id` gets in a round of dealing (none: a number from ph.pieces on).
-__device__ __forceinline__ int stream_piece(const StreamPhase &ph, int id, int round) {
-    const int k = id - ph.home;
-    if ((unsigned)k >= (unsigned)ph.streams) return ph.pieces;
-    return round * ph.streams + ((round ^ ph.flip) & 1 ? ph.streams - 1 - k : k);
-}
 template <int CAP>
 __device__ __forceinline__ bool stream_works(const StreamPhase &ph, int id) {
     int u;
     return CAP > 1 ? stream_piece(ph, id, 0) < ph.pieces : stream_range(ph, id, &u) > 0;
-}
-// The stream that has unit u.
-__device__ __forceinline__ int stream_of(const StreamPhase &ph, int u) {
-    const int head = ph.r * (ph.q + 1);
-    return u < head ? u / (ph.q + 1) : ph.r + (u - head) / ph.q;
 }
 // Walks a stream's work segment by segment; f returns whether to go on.
 template <int CAP, typename F>

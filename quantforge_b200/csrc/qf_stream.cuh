@@ -4,6 +4,7 @@
 
 #include <vector>
 
+#include "qf_chain_index.cuh"
 #include "qf_common.cuh"
 
 namespace qf {
@@ -11,7 +12,6 @@ namespace qf {
 constexpr int kStreamMaxLinears = 112;  // of one launch: the tensor maps travel as kernel parameters (32 764 bytes)
 constexpr int kStreamMaxX = 16;         // different activations of one launch, likewise
 constexpr int kStreamSlots = 4 * kSmCount;  // two for each of the two streams of an SM
-constexpr int kSlabChainPlaces = 4;     // thread blocks per SM of a chain of up to kSlabGemvRows rows
 
 // A checked linear on slab weights. In a chain K is cut into `split` pieces of `per` chunks of 128 codes.
 struct StreamLinear {
@@ -40,7 +40,7 @@ void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t
 // What a linear of a chain gets.
 struct ChainLinear {
     int slot, slots;  // of partial sums
-    // up to kSlabGemvRows rows: thread blocks, those of an SM, and where they are (see sc_number in qf_slab_chain.cu)
+    // up to kSlabGemvRows rows: thread blocks, those of an SM, and where they are (see sc_number)
     int grid, per_sm, home, first_sm;
 };
 struct ChainPlan {

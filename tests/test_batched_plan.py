@@ -5,6 +5,7 @@ import random
 
 import pytest
 
+from chain_index import library
 from quantforge_b200 import _lib
 from quantforge_b200._lib import QF_EPI_NONE, QF_EPI_RESIDUAL_ADD, QF_EPI_SILU_MUL
 
@@ -193,7 +194,7 @@ def test_places_of_a_step(seed):
         taken = set()
         for p in s:
             per_sm, first_sm, home = -(-p["blocks"] // 148), p["place"] // 4, p["place"] % 4
-            mine = {4 * ((first_sm + v // per_sm) % 148) + (home + v % per_sm) % 4 for v in range(p["blocks"])}
+            mine = {at for at in range(4 * 148) if 0 <= library().number(148, home, per_sm, first_sm, at) < p["blocks"]}
             assert len(mine) == p["blocks"] and not taken & mine
             taken |= mine
 

@@ -1,29 +1,23 @@
-"""How a chain of linears of up to 8 rows numbers its thread blocks, restated: every block takes a place of its own whatever SMs the
-hardware gives the blocks, and every share of a linear has one place, apart from those of the linears beside it."""
+"""How a chain of linears of up to 8 rows numbers its thread blocks: every block takes a place of its own whatever SMs the hardware
+gives the blocks, and every share of a linear has one place, apart from those of the linears beside it. (The kernel's arithmetic,
+compiled for the host.)"""
+import ctypes
 import random
 
 import pytest
 
+from chain_index import library
+
 PER_SM = 4
 
 
-def _claim(sm, sms, n_sm, seen, given):
-    i = min(seen.get(sm, 0), PER_SM - 1)
-    seen[sm] = seen.get(sm, 0) + 1
-    if sms == n_sm:
-        return sm * PER_SM + i
-    for _ in range(PER_SM):
-        n, given[i] = given[i], given[i] + 1
-        if n < n_sm:
-            return n * PER_SM + i
-        i = (i + 1) % PER_SM
-    raise AssertionError("no place left")
+def _claim(sm, sms, n_sm, started, given):
+    return library().place(n_sm, sm, sms, started, given)
 
 
 def _number(place, n_sm, home, per_sm, first_sm):
-    i = (place - home) % PER_SM
-    sm = (place // PER_SM - first_sm) % n_sm
-    return sm * per_sm + i if i < per_sm else None
+    v = library().number(n_sm, home, per_sm, first_sm, place)
+    return v if v >= 0 else None
 
 
 @pytest.mark.parametrize("n_sm,sms,uneven", [(148, 148, False), (148, 160, False), (148, 160, True), (20, 32, True)])
@@ -33,8 +27,8 @@ def test_places(n_sm, sms, uneven):
         ids = rng.sample(range(sms), n_sm)
         on = [rng.choice(ids) for _ in range(PER_SM * n_sm)] if uneven else ids * PER_SM
         rng.shuffle(on)
-        seen, given = {}, [0] * PER_SM
-        assert sorted(_claim(s, sms, n_sm, seen, given) for s in on) == list(range(PER_SM * n_sm))
+        started, given = (ctypes.c_uint * sms)(), (ctypes.c_uint * PER_SM)()
+        assert sorted(_claim(s, sms, n_sm, started, given) for s in on) == list(range(PER_SM * n_sm))
 
 
 @pytest.mark.parametrize("n_sm", [148, 132, 7])
