@@ -255,3 +255,20 @@ def test_stacks_that_lay_out_for_chains_get_them(fuse):
                 calls.append(linear(M, N, K, x, mem.take(blob_bytes(N, K)), act[y], r, epi))
             h = act["d"]
         assert {p["launch"] for p in plan(calls)} == {0}, (M, H, KV, F, n)
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 32])
+def test_scratch_for_single_linears_only(M):
+    """With what the largest linear alone needs, and anything up to what a chain needs, linears go one by one."""
+    lib = _lib.load()
+    calls = layers(M, 512, 1024, 2)
+    descs = (_lib.LinearDesc * len(calls))()
+    for d, c in zip(descs, calls):
+        d.M, d.N, d.K, d.group_size, d.act_dtype, d.out_dtype = M, c["N"], c["K"], 128, _lib.QF_BF16, _lib.QF_BF16
+        d.zero_mode, d.weight_layout = _lib.QF_ZERO_U4, _lib.QF_LAYOUT_GEMV_SLAB
+    alone = max(lib.qf_w4a16_workspace_bytes(ctypes.byref(d)) for d in descs)
+    chain = lib.qf_w4a16_batched_workspace_bytes(len(calls), descs)
+    assert alone < chain
+    for room in (alone, chain - 1):
+        assert [p["launch"] for p in plan(calls, room)] == list(range(len(calls)))
+    assert {p["launch"] for p in plan(calls, chain)} == {0}
