@@ -510,6 +510,10 @@ int launch_slab_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, s
 //     one in four above 16 MB: 3072 / 8192 492 -> 431, 1024 / 28672 476 -> 466
 //     two: 4096 / 14336 704 -> 663, 1792 / 23040 580 -> 553, 5120 / 13824 (12 layers) 595 -> 569; but 6656 / 2304 (qkv and o) 562 -> 586
 //     more: 5888 / 6400 646 -> 674; above 80 MB: 4096 / 24576 (12 layers) 683 -> 683, 8192 / 28672 (6) 675 -> 738
+// (In these o stands beside qkv, which it does not read here: 4 linears in 3 steps.) Linears of which each waits for the one before it
+// gain nothing: a step of a chain takes longer than a launch that may begin beside its predecessor. 16 in a row, one / eight rows:
+//   1024 x 2816 69 -> 88 / 75 -> 94, 2048 x 5632 87 -> 104 / 94 -> 112, 4096 x 14336 187 -> 197 / 204 -> 204; 8 layers of 4 with o behind
+//   qkv: 1024 / 2816 143 -> 167 / 154 -> 179, 2048 / 5632 205 -> 203 / 220 -> 217, 4096 / 14336 350 -> 372 / 387 -> 390
 // At 8 rows the chain gains 2 to 7 points more. One or two layers pay for the start of the launch (4 us): 1024 / 2816, 4 linears 21 -> 23,
 // 4096 / 14336 46 -> 49; 8 linears 36 -> 39, 90 -> 90; 7 linears of 7.0 MB 47 -> 40, of 15.6 MB 59 -> 59. The line is drawn between these.
 bool slab_chain_pays(const StreamLinear *l, int count) {
@@ -525,6 +529,8 @@ bool slab_chain_pays(const StreamLinear *l, int count) {
         large += bytes * QF_SLAB_UNIT_BYTES / 4096 > (double)kSlabSmallBytes;
         small += grid <= kSmCount;
     }
+    ChainPlan plan;
+    if (!plan_slab_chain(l, count, kSmCount, &plan) || plan.phases.back().step + 1 == count) return false;
     const std::vector<int64_t> any(count, 0);
     std::vector<int> order;
     std::vector<ChainPhase> chain;

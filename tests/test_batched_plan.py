@@ -272,3 +272,16 @@ def test_scratch_for_single_linears_only(M):
     for room in (alone, chain - 1):
         assert [p["launch"] for p in plan(calls, room)] == list(range(len(calls)))
     assert {p["launch"] for p in plan(calls, chain)} == {0}
+
+
+@pytest.mark.parametrize("M", [1, 2, 4, 8])
+def test_linears_of_which_each_waits_for_the_one_before(M):
+    """Up to 8 rows a launch that begins beside its predecessor is shorter than a step of a chain, however many there are."""
+    for H, F, n in ((512, 1408, 16), (1024, 2816, 16), (2048, 5632, 16), (4096, 14336, 32), (1024, 1024, 100)):
+        assert [p["launch"] for p in plan(_row(M, H, F, n))] == list(range(n))
+    calls = layers(M, 2048, 5632, 8)
+    for c, before in zip(calls[1:], calls):
+        c["K"], c["x"] = before["N"], before["y"]
+    assert [p["launch"] for p in plan(calls)] == list(range(56))
+    # what stands side by side shares a step
+    assert {p["launch"] for p in plan(layers(M, 2048, 5632, 8))} == {0}
