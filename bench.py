@@ -388,7 +388,9 @@ def single_gpu_extras(env, args):
             nb = st.bytes_per_step()
             extra[f"cfg2_llama3_8b_decode_linears_batch{bsz}_{mode}"] = {
                 "us_per_token": round(ms * 1e3, 1), "gbs": round(nb / ms / 1e6, 1),
-                "frac_hbm": round(nb / ms / 1e6 / hbm, 3), "launches": st.launches_per_step()}
+                "frac_hbm": round(nb / ms / 1e6 / hbm, 3), "launches": st.launches_per_step(),
+                "note": ("o does not read q/k/v (there is no attention here) and runs beside it" if mode == "fused_epilogues" else
+                         "o does not read q/k/v nor down the result of gate/up: both run beside them")}
             del g
             st.close()
             del st

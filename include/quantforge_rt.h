@@ -50,7 +50,8 @@ typedef enum qf_zero_mode { QF_ZERO_CONST = 0, QF_ZERO_U4 = 1, QF_ZERO_I8 = 2 } 
 
 /* Which kernel family serves a linear.  AUTO: M <= 2 -> GEMV kernel unless the weight matrix is large (32 MB
  * prepacked, 40 MB canonical), M >= 3 -> tcgen05 GEMM kernel (measured crossovers on B200); prepacked weights
- * (QF_LAYOUT_GEMV_SLAB always runs the streaming GEMV kernel, the other prepacked layouts the tcgen05 kernel),
+ * (QF_LAYOUT_GEMV_SLAB runs the streaming GEMV kernel, or from 9 rows and 24 to 33 MiB on the streaming tcgen05 kernel;
+ * QF_PATH_GEMV keeps it on the former; the other prepacked layouts run the tcgen05 kernel),
  * N % 128 != 0 and a fused epilogue override it, see qf_w4a16_plan. */
 typedef enum qf_path { QF_PATH_AUTO = 0, QF_PATH_GEMV = 1, QF_PATH_GEMM = 2 } qf_path;
 
@@ -95,7 +96,7 @@ typedef enum qf_weight_layout {
  *                         fp32 accumulators and rounded once.
  *   QF_EPI_RESIDUAL_ADD : Y[M, N] = X . W^T + R, R [M, N] in out_dtype (the `residual` argument of
  *                         qf_w4a16_linear_fused; R may alias Y), added in fp32 before the one rounding.
- * Served by the streaming GEMV kernel (QF_LAYOUT_GEMV_SLAB) and by the tcgen05 kernel.
+ * Served by the two streaming kernels (QF_LAYOUT_GEMV_SLAB) and by the tcgen05 kernel.
  */
 typedef enum qf_epilogue { QF_EPI_NONE = 0, QF_EPI_SILU_MUL = 1, QF_EPI_RESIDUAL_ADD = 2 } qf_epilogue;
 
@@ -291,7 +292,7 @@ int qf_repack_kn_to_canonical(qf_ctx *ctx, const void *w_kn, int packed_along_n,
 /*
  * Sticky device-side status of this context: QF_OK, or QF_ERR_TIMEOUT when a kernel's bounded wait expired
  * (the kernel then returned without finishing its tile). Reading it does not synchronise; call it after the
- * stream has been synchronised. qf_ctx_clear_status resets it.
+ * stream has been synchronised. qf_ctx_clear_status resets it; the workspace of the call must be zeroed again.
  */
 int qf_ctx_status(const qf_ctx *ctx);
 int qf_ctx_clear_status(qf_ctx *ctx);

@@ -12,11 +12,11 @@
 // whatever the shape is. A chain is a list of phases, each of linears that do not depend on each other, and each with the phases that
 // it waits for. What the next step of the chain does not touch (q, k and v beside o) is a phase of its own that holds nothing up: it
 // goes to streams that have nothing to do in that step, or fills the time in which the others hand over (the linears of 32 layers at
-// 16 rows 1459 -> 1355 us). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same sizes on other
-// layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any other order
-// into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least surprise).
-// The pieces of a phase are dealt to the streams forwards and backwards in turn. Weights are requested as far ahead as the ring of stages allows,
-// across linears and phases; only the activations of a phase wait for the phase before it.
+// 16 rows 1459 -> 1355 us). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same
+// sizes on other layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any
+// other order into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least
+// surprise). The pieces of a phase are dealt to the streams forwards and backwards in turn. Weights are requested as far ahead as the
+// ring of stages allows, across linears and phases; only the activations of a phase wait for the phase before it.
 //
 // A thread block has its SM to itself and runs two streams side by side (one stream's waits are the other's time to convert), each
 // with half of its threads, shared memory and TMEM. (One block per SM because a cooperative launch admits no more of a kernel that
@@ -31,8 +31,8 @@
 // Row blocks whose K range is shared by several streams (its members): a member leaves its partial sums in a slot of the workspace
 // as 8-byte (value, token) words - no fence, no atomic. The members finish the pairs of batch rows in turn (one member
 // reading ten others' sums of 16 rows would be a dozen trips to L2 in a row): whoever finishes a pair polls all members' words
-// (bounded), adds in their order (deterministic), writes Y and clears the words for the next user of the slots. As streams wait for one another, the launch is cooperative, and without programmatic dependent launch:
-// it would find no room beside another kernel's blocks.
+// (bounded), adds in their order (deterministic), writes Y and clears the words for the next user of the slots. As streams wait for one
+// another, the launch is cooperative, and without programmatic dependent launch: it would find no room beside another kernel's blocks.
 //
 // Shared memory takes all but a few KB of the SM's first-level cache, so a spilled register is a trip to L2: the registers are split
 // between the roles such that none is (see setmaxnreg below).

@@ -250,7 +250,7 @@ def _check_linear_tensors(x, qweight, scales, zeros, group_size):
 
 class SlabWeight:
     """Weights of one linear in QF_LAYOUT_GEMV_SLAB (codes, scales and zeros in one blob) and the facts needed to
-    call the streaming GEMV kernel on them. Made by `prepack_gemv_slab`; serves batches of up to 32 rows."""
+    call the streaming kernels on them. Made by `prepack_gemv_slab`; serves batches of up to 32 rows."""
 
     def __init__(self, blob: torch.Tensor, N: int, K: int, group_size: int, act_dtype: torch.dtype, zero_mode: int,
                  zero_const: int):
@@ -264,7 +264,7 @@ class SlabWeight:
 
 def prepack_gemv_slab(qweight: torch.Tensor, scales: torch.Tensor, zeros: Optional[torch.Tensor] = None,
                       group_size: int = 128, zero_const: int = 8) -> SlabWeight:
-    """One-time prepack of canonical weights (+ scales, zeros) for the streaming GEMV kernel (M <= 32)."""
+    """One-time prepack of canonical weights (+ scales, zeros) for the streaming kernels (M <= 32)."""
     made = (_fast or _native()).prepack_slab(qweight, scales, zeros, group_size, zero_const)
     if made is not None:
         blob, N, K, zero_mode = made

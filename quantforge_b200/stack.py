@@ -15,7 +15,12 @@ Modes
                    over NVLink peer memory instead of being followed by an NCCL all-reduce
 Batches of up to 8 rows read QF_LAYOUT_GEMV_SLAB weights (the streaming GEMV kernel), larger ones the
 interleaved layout of the tcgen05 kernel. On one GPU, 9 to 32 rows of large linears read slab weights too and
-run as a chain: one launch for up to 112 linears, the same results bit for bit. So do up to 8 rows where that is the faster way.
+run as a chain: one launch for up to 112 linears, with the bits of the tcgen05 kernel. So do up to 8 rows where that is the
+faster way, with the bits of the linears one by one.
+
+What a chain gains here is more than a decoder has of it: with attention left out, nothing reads q/k/v of the fused variant and o
+runs beside it (without epilogues down runs beside gate/up too). 32 layers of 4096 / 14336 with o behind q/k/v, one by one -> chain:
+1 row 1403 us, no chain; 16 rows 2045 -> 1592 us where this stack takes 1352.
 """
 from __future__ import annotations
 

@@ -77,7 +77,7 @@ class ColumnParallelLinear:
                  group: Optional[dist.ProcessGroup] = None, gather_output: bool = True,
                  compute: Optional[Callable] = None, prepack: bool = False, comm: Optional["ops.Comm"] = None,
                  slab: bool = False):
-        """slab=True additionally prepacks the shard for the streaming GEMV kernel, which then serves batches of up
+        """slab=True additionally prepacks the shard for the streaming kernels, which then serve batches of up
         to 32 rows (N/world must be a multiple of 64)."""
         self.comm = comm
         self.group = group
@@ -133,7 +133,7 @@ class RowParallelLinear:
                  group: Optional[dist.ProcessGroup] = None, input_is_parallel: bool = True,
                  reduce_dtype: torch.dtype = torch.float32, compute: Optional[Callable] = None,
                  prepack: bool = False, comm: Optional["ops.Comm"] = None, slab: bool = False):
-        """slab=True additionally prepacks the shard for the streaming GEMV kernel (batches of up to 32 rows; N must
+        """slab=True additionally prepacks the shard for the streaming kernels (batches of up to 32 rows; N must
         be a multiple of 64)."""
         self.comm = comm
         self.group = group
