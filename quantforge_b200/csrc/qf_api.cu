@@ -62,21 +62,33 @@ static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
 // Which of the two kernels that read slab weights runs a linear called by itself. The streaming tcgen05 kernel takes its SMs whole
 // and starts when its predecessor has ended, about 10 us a call that do not depend on the size; per byte it is faster, the more so
-// the more rows. Measured on weights not in L2, calls back to back, us, GEMV -> tcgen05 (blob in MiB):
-//   rows   8.5           13            30, K 4096    30, K 14336   34            59.5          119           238
-//   4      7.5 -> 10.6   8.4 -> 12.3   11.2 -> 14.6  13.5 -> 15.3  12.8 -> 16.5  18.1 -> 21.7  33.3 -> 34.2  57.9 -> 56.3
-//   8      7.6 -> 10.5   8.4 -> 12.5   11.9 -> 16.6  14.2 -> 15.9  13.3 -> 16.5  19.2 -> 22.7  34.9 -> 33.1  61.9 -> 57.6
-//   9      9.5 -> 10.8   10.5 -> 12.5  15.3 -> 16.6  19.7 -> 15.6  17.6 -> 16.6  23.1 -> 22.7  42.5 -> 33.6  75.6 -> 57.6
-//   16     10.3 -> 11.4  12.0 -> 14.5  16.6 -> 17.6  21.2 -> 16.2  19.1 -> 18.3  24.6 -> 23.0  44.6 -> 35.0  83.2 -> 63.8
-//   24     15.9 -> 15.6  16.1 -> 16.5  23.0 -> 19.2  28.7 -> 19.0  27.0 -> 20.7  35.5 -> 26.8  66.3 -> 37.1  129 -> 67.9
-//   32     17.0 -> 16.5  17.9 -> 18.6  24.8 -> 22.7  31.1 -> 20.0  29.0 -> 21.4  37.8 -> 28.7  70.2 -> 38.7  135 -> 69.9
+// the more rows. The GEMV kernel adds the partial sums of a row block's thread blocks one after the other, which are the more the
+// longer K is. Measured on weights not in L2, calls back to back in a graph, GEMV's time / tcgen05's (blob in MiB):
+//    rows  MiB   K 256   512  1024  2048  3072  4096  5120  6144  8192 14336
+//    9     25    0.81  0.78  0.76  0.84  0.93  0.95  1.02  1.11  1.23  1.35
+//          34    0.90  0.89  0.82  0.84  0.92  0.96  0.98  1.01  1.12  1.22
+//          48    0.93  0.96  0.95  0.93  0.93  0.98  1.04  1.04  1.08  1.27
+//          72    0.98  1.08  1.05  1.03  1.03  1.05  1.06  1.08  1.13  1.17
+//    16    25    0.78  0.74  0.71  0.80  0.92  0.94  1.03  1.09  1.15  1.41
+//          34    0.86  0.86  0.78  0.79  0.87  0.95  0.97  1.03  1.13  1.32
+//          42    0.86  0.88  0.86  0.85  0.88  0.93  1.00  1.04  1.14  1.25
+//          56    0.88  0.93  0.94  0.92  0.94  0.95  1.00  1.06  1.11  1.21
+//          72    0.92  1.01  1.02  1.00  0.99  1.01  1.02  1.07  1.12  1.19
+//          92    0.93  1.05  1.06  1.07  1.09  1.07  1.08  1.10  1.11  1.20
+//    24    25    0.97  0.92  0.86  0.94  1.09  1.17  1.28  1.34  1.55  1.64
+//          34    1.07  1.08  0.99  1.00  1.10  1.19  1.24  1.31  1.42  1.67
+//    32    25    0.92  0.87  0.82  0.89  1.03  1.11  1.23  1.35  1.50  1.75
+//          34    1.02  1.02  0.95  0.95  1.05  1.15  1.18  1.28  1.45  1.81
+//          42    0.99  1.04  1.06  1.02  1.02  1.12  1.21  1.25  1.42  1.64
+// In us: 9 rows 57344 x 8192 75.6 -> 57.6, 8192 x 28672 42.5 -> 33.6; 16 rows 83.2 -> 63.8 and 44.6 -> 35.0, 32 rows 135 -> 69.9 and
+// 70.2 -> 38.7.
 // Up to 8 rows the GEMV kernel serves whatever the size is: what the largest matrices gain waiting for each call is 1 % (4 rows,
 // 57344 x 8192, SiLU * mul: 65.3 -> 64.7), and their sums would be made in another order than those of all smaller ones.
 static bool stream_serves(const qf_linear_desc *d) {
     const int64_t mib = d->N / 64 * (d->K / 128) * QF_SLAB_UNIT_BYTES >> 20;
     if (d->M <= kSlabGemvRows) return false;
-    if (d->M <= 16) return mib >= (d->K >= 8192 ? 24 : 33);
-    return mib >= 24;
+    if (d->M > 16) return mib >= (d->K >= 3072 ? 24 : d->M <= 24 ? 34 : 42);
+    return d->K >= 512 && mib >= (d->K >= 8192 ? 24 : d->K >= 6144 ? 33 : d->K >= 5120 ? 42 : 72);
 }
 
 int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {

@@ -29,12 +29,13 @@ def _silu_mul(y):  # rows in eights of gate and up
     return gate / (1 + torch.exp(-gate)) * up
 
 
-# sizes of the rule's region (at least 24 or 33 MiB), half row blocks at the end, few and many members a row block; the largest of up to
-# 8 rows, which the streaming GEMV kernel serves
+# sizes that the rule gives to this kernel, half row blocks at the end, few and many members a row block; and some beyond its lines, which
+# the streaming GEMV kernel serves (12 and 25 rows of short K, up to 8 rows of any size)
 @pytest.mark.parametrize("M,N,K,dtype,group", [
     (9, 8256, 8192, torch.bfloat16, 128), (16, 2112, 28672, torch.float16, 256), (12, 17408, 4096, torch.float16, 128),
     (17, 6208, 8192, torch.bfloat16, 8192), (25, 24640, 2048, torch.float16, 128), (32, 1792, 28672, torch.bfloat16, 128),
-    (3, 57344, 5760, torch.bfloat16, 128), (8, 11520, 28672, torch.float16, 128)])
+    (3, 57344, 5760, torch.bfloat16, 128), (8, 11520, 28672, torch.float16, 128),
+    (12, 34880, 4096, torch.float16, 128), (25, 81984, 1024, torch.bfloat16, 128)])
 def test_single_linear(M, N, K, dtype, group):
     qw, sc, zr = _weights(N, K, dtype, group)
     slab, x = qf.prepack_gemv_slab(qw, sc, zr, group_size=group), _x(M, K, dtype)

@@ -150,3 +150,18 @@ def test_scratch_of_a_batch():
     assert need(small, _slab_desc(2, 1024, 1024)) == alone(small)
     half = _slab_desc(9, 1024, 64)
     assert need(half, half) == alone(half)
+
+
+@pytest.mark.parametrize("M,K,mib,tcgen05", [
+    # up to 16 rows; the GEMV kernel's time is up to 1.3 times the other's where this says False, and the other way round
+    (9, 14336, 25, True), (16, 8192, 25, True), (9, 8192, 22, False), (16, 6144, 35, True), (9, 6144, 30, False), (12, 5120, 44, True),
+    (16, 5120, 34, False), (16, 4096, 48, False), (9, 4096, 34, False), (16, 1024, 34, False), (9, 2048, 64, False), (16, 4096, 74, True),
+    (9, 512, 74, True), (9, 256, 120, False),
+    (17, 3072, 25, True), (32, 14336, 25, True), (32, 4096, 22, False), (17, 2048, 25, False), (24, 1024, 36, True), (32, 1024, 36, False),
+    (32, 512, 44, True),
+])
+def test_which_kernel_reads_large_slab_weights(M, K, mib, tcgen05):
+    N = round(mib * 2 ** 20 / 4352 / (K // 128)) * 64
+    auto, gemv = (_plan(M, K, N, _lib.QF_LAYOUT_GEMV_SLAB, path) for path in (_lib.QF_PATH_AUTO, _lib.QF_PATH_GEMV))
+    # the tcgen05 kernel divides the weights among two streams of each SM whatever the size is
+    assert gemv[1] != 296 and (auto == (_lib.QF_PATH_GEMV, 296) if tcgen05 else auto == gemv)
