@@ -40,18 +40,34 @@ CHAIN_BATCH = 32
 
 
 def _chain_bytes(batch: int, fuse: bool) -> float:
-    """Mean bytes of codes of a linear from which batches above SLAB_BATCH run as a chain. Measured, us a step, linear by linear ->
-    chain, at 9 / 16 / 24 / 32 rows (16 layers where not said):
-      fused    1.5 MB (hidden 1024)   324 -> 319 / 323 -> 379 / 367 -> 452 / 368 -> 539
-               5.6 MB (2048)          407 -> 384 / 411 -> 406 / 451 -> 485 / 460 -> 550
-               12 MB (3072, 2048)     517 -> 457 / 525 -> 503 / 562 -> 564 / 572 -> 632,  519 -> 477 / 526 -> 483 / 564 -> 548 / 570 -> 590
-               27 MB (4096, 32 layers) 1556 -> 1333 / 1578 -> 1355 / 1607 -> 1511 / 1624 -> 1581
-               107 MB (8192, 6 layers) 774 -> 704 / 777 -> 714 / 798 -> 752 / 802 -> 786
-      unfused  0.8 MB (1024) 521 -> 398 / 521 -> 464 / 570 -> 551 / 571 -> 637,  3.2 MB (2048) 592 -> 440 / 600 -> 464 / 648 -> 534 / 652 -> 593
-               16 MB (4096, 32 layers) 2028 -> 1597 / 2032 -> 1751 / 2131 -> 1973 / 2147 -> 2153"""
+    """Mean bytes of codes of a linear from which batches above SLAB_BATCH run as a chain. Measured, a step's time linear by linear
+    (interleaved weights) / as a chain, 1 to 16 layers, at 9 / 16 / 20 / 24 / 28 / 32 rows:
+      fused     1.5 MB (hidden 1024)    0.88-1.01 / 0.72-0.86 / 0.70-0.85 / 0.71-0.80 / 0.65-0.71 / 0.56-0.66
+                5.6 MB (2048)           1.00-1.07 / 1.00-1.03 / 0.94-0.97 / 0.91-0.95 / 0.86-0.90 / 0.83-0.90
+                12 MB (3072)            1.00-1.14 / 1.00-1.06 / 0.96-1.03 / 0.96-1.00 / 0.88-0.93 / 0.91-0.92
+                14 MB (1792, 18944)     1.00      / 0.99-1.00 / 0.90-0.93 / 0.90-0.96 / 0.84-0.88 / 0.84-0.92
+                22 MB (6912, 3584)      1.08-1.09 / 1.00-1.02 / 0.93-0.96 / 0.93-0.94 / 0.86-0.88 / 0.83-0.85
+                27 MB (4096, 14336)     1.00-1.17 / 1.00-1.15 / 0.98-1.07 / 0.94-1.09 / 0.97-1.04 / 0.97-1.03
+                34 MB (5120, 13824)     1.03-1.12 / 1.00-1.07 / 1.00-1.05 / 1.00-1.05 / 0.94-0.97 / 0.92-0.97
+                90 MB (7680, 25856)     1.00-1.05 / 1.00-1.04 / 0.98-1.00 / 0.98-1.01 / 0.97-0.98 / 0.95-0.96
+                107 MB (8192, 28672)    1.08-1.10 / 1.08-1.09 / 1.04-1.06 / 1.04-1.05 / 1.00-1.01 / 1.01-1.02
+      unfused   0.8 MB (1024)           1.12-1.29 / 1.05-1.16 / 1.00-1.12 / 1.00-1.06 / 0.87-0.96 / 0.84-0.89
+                1.8 MB (1536)           1.23-1.41 / 1.06-1.25 / 1.10-1.22 / 1.09-1.19 / 1.04-1.09 / 1.00-1.06
+                16 MB (4096, 14336)     1.13-1.26 / 1.03-1.15 / 1.03-1.12 / 1.00-1.07 / 0.97-1.01 / 0.95-1.00
+                61 MB (8192, 28672)     1.09-1.12 / 1.09-1.11 / 1.07-1.10 / 1.06-1.09 / 1.03-1.06 / 1.02-1.05"""
     if not fuse:
         return 2e6
-    return 5e6 if batch <= 16 else 13e6 if batch <= 24 else 24e6
+    return 5e6 if batch <= 16 else 24e6 if batch <= 24 else float("inf")
+
+
+def runs_as_chain(cfg: dict, batch: int, fuse: bool, world: int = 1) -> bool:
+    """Whether a step is one batched call on slab weights. Up to SLAB_BATCH rows that call decides by itself whether one launch is the
+    faster way."""
+    H, KV, F = cfg["hidden"], cfg["kv"], cfg["ffn"]
+    if world != 1 or batch > CHAIN_BATCH or H % 128 or KV % 128 or F % 128:
+        return False
+    codes = (2 * H * H + 2 * H * KV + 3 * H * F) // 2  # bytes of a layer's codes
+    return batch <= SLAB_BATCH or codes >= (4 if fuse else 7) * _chain_bytes(batch, fuse)
 
 
 SAMPLE_COLUMNS = 64  # output columns per linear of layer 0 kept on the CPU for `check_parity`
@@ -130,10 +146,7 @@ class DecodeLinearStack:
                 raise ValueError("fused_allreduce needs batch <= 64")
             self.comm = ops.Comm(batch * H, device=self.dev, group=group)
         exch = self.comm is not None and not exchange_in_slab_kernel
-        codes = (2 * H * H + 2 * H * KV + 3 * H * F) // 2  # bytes of a layer's codes
-        # up to SLAB_BATCH rows the batched call decides by itself whether one launch is the faster way
-        self.chain = (world == 1 and batch <= CHAIN_BATCH and H % 128 == 0 and KV % 128 == 0 and F % 128 == 0 and
-                      (batch <= SLAB_BATCH or codes >= (4 if fuse else 7) * _chain_bytes(batch, fuse)))
+        self.chain = runs_as_chain(cfg, batch, fuse, world)
         self._batch = None
         self.layers = []
         for li in range(self.L):

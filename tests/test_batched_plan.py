@@ -232,13 +232,13 @@ def test_what_gains_is_a_chain(M):
 @pytest.mark.parametrize("fuse", [True, False])
 def test_stacks_that_lay_out_for_chains_get_them(fuse):
     """A stack of 9 to 32 rows chooses its layout by the size of its linears, before there is a batch."""
-    from quantforge_b200.stack import _chain_bytes
+    from quantforge_b200.stack import runs_as_chain
     rng = random.Random(fuse)
     seen = 0
     while seen < 150:
         H, KV, F = 128 * rng.randint(2, 80), rng.choice([128, 512, 1024]), 128 * rng.randint(2, 224)
         M, n = rng.randint(9, 32), rng.choice([1, 2, 6])
-        if (2 * H * H + 2 * H * KV + 3 * H * F) // 2 < (4 if fuse else 7) * _chain_bytes(M, fuse):
+        if not runs_as_chain({"hidden": H, "kv": KV, "ffn": F}, M, fuse):
             continue
         seen += 1
         mem, calls = Memory(), []
@@ -285,3 +285,17 @@ def test_linears_of_which_each_waits_for_the_one_before(M):
     assert [p["launch"] for p in plan(calls)] == list(range(56))
     # what stands side by side shares a step
     assert {p["launch"] for p in plan(layers(M, 2048, 5632, 8))} == {0}
+
+
+@pytest.mark.parametrize("hidden,ffn,batch,fuse,chain", [
+    (2048, 5632, 9, True, True), (2048, 5632, 16, True, True), (1024, 2816, 9, True, False), (2048, 5632, 17, True, False),
+    (1792, 18944, 20, True, False), (6912, 3584, 24, True, False), (4096, 14336, 24, True, True), (4096, 14336, 25, True, False),
+    (5120, 13824, 32, True, False), (7680, 25856, 28, True, False), (1536, 4096, 32, False, False), (2048, 5632, 32, False, True),
+    (8192, 28672, 32, False, True), (4096, 14336, 33, False, False), (1024, 2816, 8, True, True)])
+def test_stacks_of_more_than_8_rows_that_run_as_chains(hidden, ffn, batch, fuse, chain):
+    """Where it is the faster way by the times beside the rule; up to 8 rows the batched call decides."""
+    from quantforge_b200.stack import runs_as_chain
+    cfg = {"hidden": hidden, "kv": 1024 if hidden >= 4096 else 512, "ffn": ffn}
+    assert runs_as_chain(cfg, batch, fuse) == chain
+    assert not runs_as_chain(cfg, batch, fuse, world=2)
+    assert not runs_as_chain(dict(cfg, kv=64), batch, fuse)
