@@ -348,7 +348,7 @@ static bool slab_any(const qf_linear_desc *d) {
 // Linears that qf_w4a16_linear_batched runs as one launch. (One without rows goes alone: it has no launch, and its pointers were not
 // looked at.)
 static bool chains(const qf_linear_desc *d) {
-    return d->M > 0 && slab_any(d) && (d->M <= kSlabGemvRows ? slab_chain_takes(d) : d->N % 128 == 0);
+    return d->M > 0 && slab_any(d) && d->N > 0 && d->N % 64 == 0 && d->K > 0 && d->K % 128 == 0 && (d->M <= kSlabGemvRows ? slab_chain_takes(d) : d->N % 128 == 0);
 }
 // The workspace of that launch.
 static size_t chain_workspace_bytes(int64_t M) {
@@ -356,29 +356,41 @@ static size_t chain_workspace_bytes(int64_t M) {
 }
 
 // How many of the linears from entry i on one launch could take, those linears, and whether it does or they go one by one. (A linear
-// with which something is wrong goes alone, and its check says what.)
+// with which something is wrong goes alone, and its check says what. They are checked once it is known that a chain would pay: most
+// batches that go one by one are checked there.)
 static int chain_from(qf_ctx *ctx, int i, int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight,
                       void *const *Y, const void *const *residual, const void *workspace, size_t workspace_bytes,
                       std::vector<StreamLinear> *run, bool *pays) {
     run->clear();
-    for (int j = i; j < count && chains(&descs[j]); ++j) {
-        Plan plan;
-        const void *res = residual ? residual[j] : nullptr;
-        if (check_linear(ctx, &descs[j], X[j], qweight[j], nullptr, nullptr, Y[j], res, workspace, workspace_bytes, &plan) != QF_OK ||
-            workspace_bytes < chain_workspace_bytes(descs[j].M))
-            break;
-        if (descs[j].M <= kSlabGemvRows) {
-            run->push_back(StreamLinear{&descs[j], X[j], qweight[j], res, Y[j], 1, 0});
-            continue;
-        }
+    const bool gemv = descs[i].M <= kSlabGemvRows;
+    Plan plan;
+    for (int j = i; j < count && j - i < kStreamMaxLinears && chains(&descs[j]) && descs[j].M == descs[i].M; ++j) {
+        run->push_back(StreamLinear{&descs[j], X[j], qweight[j], residual ? residual[j] : nullptr, Y[j], 1, 0});
+        if (gemv) continue;
         // K is cut as the tcgen05 kernel cuts it for the same sizes in its own layouts: the sums are the same bits
         qf_linear_desc d = descs[j];
         d.weight_layout = QF_LAYOUT_INTERLEAVED;
-        if (make_plan(&d, &plan, nullptr) != QF_OK || plan.path != QF_PATH_GEMM) break;
-        run->push_back(StreamLinear{&descs[j], X[j], qweight[j], res, Y[j], plan.split_k, plan.chunks_per_split});
+        if (make_plan(&d, &plan, nullptr) != QF_OK || plan.path != QF_PATH_GEMM) {
+            run->pop_back();
+            break;
+        }
+        run->back().split = plan.split_k;
+        run->back().per = plan.chunks_per_split;
     }
-    const int n = run->size() > 1 ? stream_chain_length(run->data(), (int)run->size()) : 1;
-    *pays = n > 1 && (descs[i].M > kSlabGemvRows ? stream_chain_pays : slab_chain_pays)(run->data(), n);
+    int n = run->size() > 1 ? stream_chain_length(run->data(), (int)run->size()) : 1;
+    const auto faster = [&] {
+        return n > 1 && workspace_bytes >= chain_workspace_bytes(descs[i].M) &&
+               (gemv ? slab_chain_pays : stream_chain_pays)(run->data(), n);
+    };
+    *pays = faster();
+    for (int k = 0; *pays && k < n; ++k) {
+        const StreamLinear &x = (*run)[k];
+        if (check_linear(ctx, x.d, x.X, x.blob, nullptr, nullptr, x.Y, x.residual, workspace, workspace_bytes, &plan) != QF_OK) {
+            n = k;
+            *pays = faster();
+            break;
+        }
+    }
     return std::max(n, 1);
 }
 

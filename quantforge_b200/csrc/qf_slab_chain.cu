@@ -517,30 +517,30 @@ int launch_slab_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, s
 // At 8 rows the chain gains 2 to 7 points more. One or two layers pay for the start of the launch (4 us): 1024 / 2816, 4 linears 21 -> 23,
 // 4096 / 14336 46 -> 49; 8 linears 36 -> 39, 90 -> 90; 7 linears of 7.0 MB 47 -> 40, of 15.6 MB 59 -> 59. The line is drawn between these.
 bool slab_chain_pays(const StreamLinear *l, int count) {
-    double sum = 0, most = 0;
-    int large = 0, small = 0;
-    for (int i = 0; i < count; ++i) {
-        const qf_linear_desc &d = *l[i].d;
-        int grid, depth;
-        slab_geometry(d.M, d.N, d.K, kSmCount, 0, &grid, &depth);
-        const double bytes = 0.5 * (double)d.N * (double)d.K;
-        sum += bytes;
-        most = std::max(most, bytes);
-        large += bytes * QF_SLAB_UNIT_BYTES / 4096 > (double)kSlabSmallBytes;
-        small += grid <= kSmCount;
-    }
-    ChainPlan plan;
-    if (!plan_slab_chain(l, count, kSmCount, &plan) || plan.phases.back().step + 1 == count) return false;
     const std::vector<int64_t> any(count, 0);
     std::vector<int> order;
     std::vector<ChainPhase> chain;
     chain_phases(l, count, any.data(), 1, 1, &order, &chain);
     const int steps = chain.back().step + 1;
+    if (steps == count) return false;
+    double sum = 0, most = 0;
+    int large = 0;
+    for (int i = 0; i < count; ++i) {
+        const double bytes = 0.5 * (double)l[i].d->N * (double)l[i].d->K;
+        sum += bytes;
+        most = std::max(most, bytes);
+        large += bytes * QF_SLAB_UNIT_BYTES / 4096 > (double)kSlabSmallBytes;
+    }
     const double mean = sum / count;
-    if (2 * count >= 3 * steps && mean <= 18e6) return count >= 14 || (count >= 7 && mean <= 8e6);
-    if (count < 8 || (count < 16 && (mean < 4e6 || mean > 16e6))) return false;
-    if (large == 0) return small > 0 || mean <= 7e6;
-    return 2 * large <= count && most <= 80e6 && (4 * large <= count || most >= 1.7 * mean);
+    const bool wide = 2 * count >= 3 * steps && mean <= 18e6;
+    if (wide ? count < 7 || (count < 14 && mean > 8e6) : count < 8 || (count < 16 && (mean < 4e6 || mean > 16e6))) return false;
+    if (!wide && large > 0 && (2 * large > count || most > 80e6 || (4 * large > count && most < 1.7 * mean))) return false;
+    // (thread blocks are looked at last: a linear's number of them takes longer to find than all of the above)
+    ChainPlan plan;
+    if (!plan_slab_chain(l, count, kSmCount, &plan) || plan.phases.back().step + 1 == count) return false;
+    bool small = wide || large > 0 || mean <= 7e6;
+    for (const ChainLinear &x : plan.linears) small = small || x.grid <= kSmCount;
+    return small;
 }
 
 bool slab_chain_takes(const qf_linear_desc *d) {
