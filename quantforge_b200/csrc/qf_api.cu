@@ -355,6 +355,11 @@ static size_t chain_workspace_bytes(int64_t M) {
     return kCounterBytes + (M <= kSlabGemvRows ? slab_chain_workspace_bytes() : stream_workspace_bytes(M));
 }
 
+// Slots of partial sums of a chain of more than kSlabGemvRows rows in this workspace.
+static int chain_slots(int64_t M, size_t workspace_bytes) {
+    return workspace_bytes >= kCounterBytes + stream_workspace_bytes(M, kChainSlots) ? kChainSlots : kStreamSlots;
+}
+
 // How many of the linears from entry i on one launch could take, those linears, and whether it does or they go one by one. (A linear
 // with which something is wrong goes alone, and its check says what. They are checked once it is known that a chain would pay: most
 // batches that go one by one are checked there.)
@@ -563,11 +568,19 @@ size_t qf_w4a16_workspace_bytes(const qf_linear_desc *desc) {
 
 size_t qf_w4a16_batched_workspace_bytes(int count, const qf_linear_desc *descs) {
     size_t need = 0;
+    int64_t slots = 0;  // of partial sums, of the linears since one that does not go with the one before
     for (int i = 0; descs && i < count; ++i) {
         need = std::max(need, qf_w4a16_workspace_bytes(&descs[i]));
-        if (i > 0 && chains(&descs[i]) && chains(&descs[i - 1]) && descs[i].M == descs[i - 1].M &&
-            descs[i].act_dtype == descs[i - 1].act_dtype)
-            need = std::max(need, chain_workspace_bytes(descs[i].M));
+        const bool run = i > 0 && chains(&descs[i]) && chains(&descs[i - 1]) && descs[i].M == descs[i - 1].M &&
+                         descs[i].act_dtype == descs[i - 1].act_dtype;
+        if (run) need = std::max(need, chain_workspace_bytes(descs[i].M));
+        if (!run) slots = 0;
+        if (descs[i].M <= kSlabGemvRows || !chains(&descs[i])) continue;
+        qf_linear_desc d = descs[i];
+        d.weight_layout = QF_LAYOUT_INTERLEAVED;
+        Plan plan;
+        if (make_plan(&d, &plan, nullptr) == QF_OK && plan.split_k > 1) slots += row_blocks(d) * plan.split_k;
+        if (run && slots > kStreamSlots) need = std::max(need, kCounterBytes + stream_workspace_bytes(d.M, kChainSlots));
     }
     return need;
 }
@@ -613,8 +626,10 @@ int qf_w4a16_linear_batched(qf_ctx *ctx, int count, const qf_linear_desc *descs,
         const int n = i < alone ? 1 : chain_from(ctx, i, count, descs, X, qweight, Y, residual, workspace, workspace_bytes, &run, &pays);
         alone = std::max(alone, i + n);
         if (pays) {
-            const auto launch = descs[i].M <= kSlabGemvRows ? launch_slab_chain : launch_stream_chain;
-            const int st = launch(ctx, run.data(), n, workspace, kCounterBytes, (cudaStream_t)stream);
+            const int64_t M = descs[i].M;
+            const int st = M <= kSlabGemvRows ? launch_slab_chain(ctx, run.data(), n, workspace, kCounterBytes, (cudaStream_t)stream)
+                                              : launch_stream_chain(ctx, run.data(), n, workspace, kCounterBytes,
+                                                                    chain_slots(M, workspace_bytes), (cudaStream_t)stream);
             if (st != QF_OK && st != kStreamNoRoom) return st;
             if (st == QF_OK) {
                 i += n - 1;
@@ -663,13 +678,13 @@ int qf_w4a16_batched_plan(int count, const qf_linear_desc *descs, const void *co
                 if (descs[i + j].M > 0) o[j * QF_BATCHED_PLAN_WORDS] = launch++;
             continue;
         }
-        if (!gemv) plan_stream_chain(run.data(), n, 2 * kSmCount, &plan);
+        if (!gemv) plan_stream_chain(run.data(), n, 2 * kSmCount, chain_slots(descs[i].M, workspace_bytes), &plan);
         for (size_t q = 0; q < plan.phases.size(); ++q) {
             const ChainPhase &c = plan.phases[q];
             for (int k = c.first; k < c.first + c.count; ++k) {
                 const ChainLinear &x = plan.linears[plan.order[k]];
                 const int32_t words[QF_BATCHED_PLAN_WORDS] = {launch, (int32_t)q, c.wait[0], c.wait[1], x.slot, x.slots,
-                                                              gemv ? kSlabChainPlaces * x.first_sm + x.home : -1, gemv ? x.grid : -1};
+                                                              gemv ? kSlabChainPlaces * x.first_sm + x.home : c.slots_wait, gemv ? x.grid : -1};
                 std::copy(words, words + QF_BATCHED_PLAN_WORDS, o + (size_t)plan.order[k] * QF_BATCHED_PLAN_WORDS);
             }
         }

@@ -18,7 +18,8 @@ struct StreamPhase {
     int streams;     // ranges: G; pieces: the streams from `home` on that they are dealt to, forwards and backwards in turn
     int home, flip;  // flip: backwards first
     int active;      // streams that have work
-    int wait[2];     // phases that are complete before this one reads or writes anything (or -1)
+    int wait[2];     // phases that are complete before this one writes a result (or -1)
+    int slots_wait;  // the phase that, with wait[1], is complete before this one writes partial sums (or -1)
 };
 // Units of stream `id` in a phase: how many, and *u0 the first.
 QF_HD int stream_range(const StreamPhase &ph, int id, int *u0) {

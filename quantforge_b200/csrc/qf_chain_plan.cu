@@ -45,7 +45,7 @@ void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t
         used += room[i];
         step_of.push_back(steps - 1);
     }
-    int last = -1, late_before = -1, late = -1;  // phases: of the step before; late ones two steps back and one
+    int last = -1, last_two = -1, late_before = -1, late = -1;  // phases: of the step before and of two steps back; late ones likewise
     for (int q = 0, i0 = 0, i1, i2; q < steps; ++q, i0 = i1) {
         for (i1 = i0; i1 < count && step_of[i1] == q;) ++i1;
         for (i2 = i1; i2 < count && step_of[i2] == q + 1;) ++i2;
@@ -60,10 +60,12 @@ void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t
         }
         if (!any) waits.assign(i1 - i0, 1);
         const int wait0 = last, wait1 = late_before;
+        const int slots_wait = last_two;
+        last_two = last;
         late_before = late;
         late = -1;
         for (int part = 0; part < 2; ++part) {
-            ChainPhase c{(int)order->size(), 0, {wait0, wait1}, q, part == 1, here, i1, i2, 0, 0, 0};
+            ChainPhase c{(int)order->size(), 0, {wait0, wait1}, slots_wait, q, part == 1, here, i1, i2, 0, 0, 0};
             for (int i = i0; i < i1; ++i)
                 if ((waits[i - i0] != 0) == (part == 0)) order->push_back(i), ++c.count;
             if (c.count == 0) continue;
@@ -73,7 +75,7 @@ void chain_phases(const StreamLinear *l, int count, const int64_t *room, int64_t
     }
 }
 
-void plan_stream_chain(const StreamLinear *l, int count, int streams, ChainPlan *plan) {
+void plan_stream_chain(const StreamLinear *l, int count, int streams, int room, ChainPlan *plan) {
     std::vector<int64_t> slots(count);
     *plan = ChainPlan{};
     plan->linears.resize(count);
@@ -81,12 +83,54 @@ void plan_stream_chain(const StreamLinear *l, int count, int streams, ChainPlan 
         slots[i] = l[i].split > 1 ? row_blocks(*l[i].d) * l[i].split : 0;
         plan->linears[i].slots = (int)slots[i];
     }
-    chain_phases(l, count, slots.data(), kStreamSlots, kStreamSlots, &plan->order, &plan->phases);
+    chain_phases(l, count, slots.data(), room, room, &plan->order, &plan->phases);
+    // Where activations come from. The last linear before this one that writes any of them has made them, if they are its results whole.
+    int64_t flags = 0;
+    for (int i = 0; i < count; ++i) {
+        ChainLinear &x = plan->linears[i];
+        x.maker = kChainThere;
+        x.flags = -1;
+        const Touched t = touched(l[i]);
+        int from = i;
+        while (from-- > 0 && !touched(l[from]).y.meets(t.x)) {
+        }
+        if (from < 0) continue;
+        const qf_linear_desc &d = *l[from].d;
+        const int64_t cols = d.epilogue == QF_EPI_SILU_MUL ? d.N / 2 : d.N;
+        x.maker = kChainMixed;
+        if (l[from].Y != l[i].X || cols != l[i].d->K || d.out_dtype == QF_F32) continue;
+        ChainLinear &m = plan->linears[from];
+        if (m.flags < 0) {
+            if (flags + row_blocks(d) > kStreamFlagWords) continue;
+            m.flags = (int)flags;
+            flags += row_blocks(d);
+        }
+        x.maker = from;
+    }
     auto pieces_of = [&](int i) { return row_blocks(*l[i].d) * l[i].split; };
-    int slot = 0;
+    struct Slots {
+        int lo = 0, hi = 0;
+        bool meets(int a, int b) const { return a < hi && lo < b; }
+    };
+    std::vector<Slots> of_main, of_late;  // by step
+    int used = 0;                         // of the step so far
     for (ChainPhase &c : plan->phases) {
-        // slots: from the lower end and the upper one in turn, so that a late phase and the next step have their own
-        if (!c.late) slot = c.step & 1 ? kStreamSlots - (int)c.room : 0;
+        // slots: from the lower end and the upper one in turn, so that a late phase and the next step have their own, and what is not late
+        // at the very end, where it meets the step before least
+        int own = 0;
+        for (int k = c.first; k < c.first + c.count; ++k) own += (int)slots[plan->order[k]];
+        if (!c.late) {
+            used = 0;
+            of_main.emplace_back();
+            of_late.emplace_back();
+        }
+        int slot = c.step & 1 ? room - used - own : used;
+        (c.late ? of_late : of_main).back() = Slots{slot, slot + own};
+        // What two steps back is complete does not speak for: the step before, and what was late three steps back (for which the step
+        // before does).
+        const int q = c.step;
+        if ((q >= 1 && of_main[q - 1].meets(slot, slot + own)) || (q >= 3 && of_late[q - 3].meets(slot, slot + own))) c.slots_wait = c.wait[0];
+        used += own;
         for (int k = c.first; k < c.first + c.count; ++k) {
             plan->linears[plan->order[k]].slot = slot;
             slot += (int)slots[plan->order[k]];
@@ -214,7 +258,7 @@ bool stream_chain_pays(const StreamLinear *l, int count) {
         alone += c.base + c.member * (double)(members - 1) + c.unit * (double)per_sm;
     }
     ChainPlan plan;
-    plan_stream_chain(l, count, (int)kStreams, &plan);
+    plan_stream_chain(l, count, (int)kStreams, kStreamSlots, &plan);
     double chain = kLaunch;
     for (size_t q = 0, end; q < plan.phases.size(); q = end) {
         int64_t pieces = 0, longest = 4;

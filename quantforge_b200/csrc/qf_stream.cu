@@ -5,14 +5,19 @@
 // instruction) and live in TMEM only, the activations are B from shared memory. What the streaming GEMV kernel (mma.sync) spends
 // on fragments of X and on the MMAs themselves, which take issue slots and packed-half time from the conversion and grow with the
 // rows, is here one thread's work. Without memory, converters and MMAs alone take 283 cycles per 128 x 128 codes and SM; HBM delivers
-// those in 377; the kernel takes about 450, bound by the issue slots that the conversion and its hand-overs share.
+// those in 377; the kernel takes about 450, bound by the issue slots that the conversion and its hand-overs share. In a chain there are 5 to
+// 6 us from the last MMA of a step to the first of the next: partial sums, results, a release (1 us and more behind stores), counters, a
+// copy of activations.
 //
 // Work split. Units of 128 rows x 128 codes. Of a single linear they are numbered row block major, K chunk minor, and stream i of G
 // owns a contiguous range of them (the first r streams one more than the others): every stream moves the same number of bytes
 // whatever the shape is. A chain is a list of phases, each of linears that do not depend on each other, and each with the phases that
 // it waits for. What the next step of the chain does not touch (q, k and v beside o) is a phase of its own that holds nothing up: it
 // goes to streams that have nothing to do in that step, or fills the time in which the others hand over (the linears of 32 layers at
-// 16 rows 1459 -> 1355 us). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same
+// 16 rows 1459 -> 1355 us). Only results wait for whole phases. Activations that are another linear's results are read row block by row
+// block as these are finished (a counter each), and partial sums are exchanged as soon as their slots are free (linears of 32 layers,
+// 4096 / 14336, with the code of the results made smaller: 16 rows 1372 -> 1285 us, 9 rows 1338 -> 1240; seven linears a layer 1760 -> 1570
+// at 16 rows, 1988 -> 1805 at 24). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same
 // sizes on other layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any
 // other order into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least
 // surprise). The pieces of a phase are dealt to the streams forwards and backwards in turn. Weights are requested as far ahead as the
@@ -72,16 +77,27 @@ struct StreamEntry {  // one linear
     int split, per;  // pieces: K is cut into `split` of them, `per` chunks each (the last may be shorter)
     int slot;        // of its first piece, where there are several to a row block
     int x_map;
+    // Where the activations come from: kXThere, kXGate, or the first counter of the row blocks of the linear that makes them, its
+    // results. A counter is complete at x_want; x_two: two row blocks to a chunk (SiLU * mul).
+    int x_from;
+    int flags;       // this linear's first counter (or -1: nobody looks)
+    int16_t x_want, x_two;
     int16_t out_dtype, epilogue;
 };
+constexpr int kXThere = -1;  // no linear of the launch writes them
+constexpr int kXGate = -2;   // they are there when the phase may write its results
+
 struct StreamArgs {
-    unsigned long long *slots;  // [kStreamSlots][slot_words] (value | token << 32), zero between launches
-    unsigned *done;             // [phases] result warps that have finished the phase, [kStreamMaxLinears] all; zero between launches
+    unsigned long long *slots;  // [kStreamSlots or kChainSlots][slot_words] (value | token << 32), zero between launches
+    // [phases] streams that have finished the phase, [kStreamMaxLinears] result warps that have finished everything, from kStreamFlags
+    // on result warps that have finished a row block; `words` of them, zero between launches
+    unsigned *done;
     int *status;
     int slot_words;
     int M, x_rows;              // x_rows: rows of an X box (M rounded up to 8)
-    int phases, linears;
+    int phases, linears, words;
 };
+constexpr int kStreamFlags = (kStreamMaxLinears + 4) / 4 * 4;
 template <int CAP>
 struct StreamParams {
     static constexpr int XCAP = CAP == 1 ? 1 : kStreamMaxX;
@@ -92,7 +108,7 @@ struct StreamParams {
     StreamArgs a;
 };
 static_assert(sizeof(StreamParams<kStreamMaxLinears>) <= 32764, "kernel parameters");
-static_assert((kStreamMaxLinears + 1) * sizeof(unsigned) <= 65536, "the counter region of the workspace");
+static_assert(kStreamFlags > kStreamMaxLinears && kStreamFlags * sizeof(unsigned) <= kCounterBytes, "the counter region of the workspace");
 // The lists of linears and phases, in shared memory: every role reads the next phase's when it gets there, and from the parameter
 // space that was a miss of the constant cache each time.
 template <int CAP>
@@ -177,23 +193,56 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *ptr) {
 // Between ordinary accesses to global memory and accesses of the copy engine.
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-__device__ __forceinline__ float load_elem(const void *R, int out_dtype, int64_t idx) {
-    if (out_dtype == QF_F32) return reinterpret_cast<const float *>(R)[idx];
-    if (out_dtype == QF_F16) return __half2float(reinterpret_cast<const __half *>(R)[idx]);
-    return __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(R)[idx]);
+// Finished sums leave as pairs of neighbouring outputs of a batch row, a pair to a lane: of two neighbouring lanes, which hold two batch
+// rows of neighbouring weight rows, the even one takes the first batch row and the odd one the second. Code that runs once a phase
+// costs what its instructions take to arrive, so there are few of them: 16-bit types differ in one selection, and a pair of outputs
+// is one store. (One output per store with a branch per type and store, 74 KB of code instead of 58: 32 layers of 4096 / 14336 at 16 rows
+// 1362 us instead of 1283.)
+struct StreamOut {
+    int64_t o;  // element of the first of the two outputs, of the first pair of batch rows
+    int step;   // elements from one pair of batch rows to the next
+    int m;      // this lane's batch row of the first pair
+};
+__device__ __forceinline__ StreamOut stream_out(const StreamEntry &e, int n, int m0) {
+    const int m = m0 + (n & 1);
+    return StreamOut{(int64_t)m * e.N + (n & ~1), 2 * e.N, m};
 }
-
-// Writes finished sums: PAIRS pairs of batch rows from row m0 on (as far as M goes) of weight row n. All 32 lanes of a warp, which
-// hold 32 consecutive weight rows. The steps of all pairs go side by side: these warps run a chain of dependent instructions
-// otherwise, 450 cycles a pair.
+// What the residual epilogue adds to PAIRS pairs of batch rows, as it lies in memory.
 template <int PAIRS>
-__device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, int m0, const float (&v)[2 * PAIRS]) {
-    const int type = e.out_dtype;
+__device__ __forceinline__ void stream_residual(const StreamEntry &e, int M, const StreamOut &at, uint2 (&r)[PAIRS]) {
+    const bool f32 = e.out_dtype == QF_F32;
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+        r[i] = make_uint2(0u, 0u);
+        const int64_t o = at.o + (int64_t)i * at.step;
+        if (at.m + 2 * i < M) {
+            if (f32) r[i] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const float *>(e.residual) + o);
+            else r[i].x = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const uint16_t *>(e.residual) + o);
+        }
+    }
+}
+__device__ __forceinline__ void stream_put(const StreamEntry &e, int64_t o, float lo, float hi) {
+    if (e.out_dtype == QF_F32) {
+        *reinterpret_cast<float2 *>(reinterpret_cast<float *>(e.Y) + o) = make_float2(lo, hi);
+        return;
+    }
+    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+    const __half2 h = __floats2half2_rn(lo, hi);
+    *reinterpret_cast<uint32_t *>(reinterpret_cast<uint16_t *>(e.Y) + o) =
+        e.out_dtype == QF_BF16 ? *reinterpret_cast<const uint32_t *>(&b) : *reinterpret_cast<const uint32_t *>(&h);
+}
+// Writes finished sums: PAIRS pairs of batch rows from row m0 on (as far as M goes) of weight row n; `r`: stream_residual's. All 32
+// lanes of a warp, which hold 32 consecutive weight rows. The steps of all pairs go side by side: these warps run a chain of dependent
+// instructions otherwise, 450 cycles a pair.
+template <int PAIRS>
+__device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, int m0, const float (&v)[2 * PAIRS], const StreamOut &at,
+                                            const uint2 (&r)[PAIRS]) {
+    const bool odd = n & 1;
     if (e.epilogue == QF_EPI_SILU_MUL) {
         // rows 0..7 of sixteen are gate rows, 8..15 the matching up rows: of a pair the gate lane does the first batch row, the up lane
         // the second
         const bool up_lane = n & 8;
-        const int64_t cols = e.N >> 1, col = (n >> 4) * 8 + (n & 7);
+        const int cols = e.N >> 1, col = (n >> 4) * 8 + (n & 6);
         float gate[PAIRS], up[PAIRS];
 #pragma unroll
         for (int i = 0; i < PAIRS; ++i) {
@@ -203,25 +252,39 @@ __device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, 
         }
 #pragma unroll
         for (int i = 0; i < PAIRS; ++i) up[i] = gate[i] / (1.f + expf(-gate[i])) * up[i];
+        // neighbouring lanes hold neighbouring outputs of the same batch rows: the even one takes the first of two pairs
+        const int m = m0 + (up_lane ? 1 : 0);
 #pragma unroll
-        for (int i = 0; i < PAIRS; ++i) {
-            const int m = m0 + 2 * i + (up_lane ? 1 : 0);
-            if (m < M) store_out(e.Y, type, m * cols + col, up[i]);
+        for (int i = 0; i < PAIRS; i += 2) {
+            const float mine = odd && i + 1 < PAIRS ? up[i + 1 < PAIRS ? i + 1 : i] : up[i];
+            const float other = __shfl_xor_sync(0xffffffffu, odd || i + 1 >= PAIRS ? up[i] : up[i + 1 < PAIRS ? i + 1 : i], 1);
+            const int row = m + 2 * i + (odd ? 2 : 0);
+            if (row < M && (i + 1 < PAIRS || !odd)) stream_put(e, (int64_t)row * cols + col, odd ? other : mine, odd ? mine : other);
         }
         return;
     }
-    const int64_t o = (int64_t)m0 * e.N + n;
-    float r[2 * PAIRS];
+    const bool add = e.epilogue == QF_EPI_RESIDUAL_ADD;
 #pragma unroll
-    for (int i = 0; i < 2 * PAIRS; ++i)
-        r[i] = e.epilogue == QF_EPI_RESIDUAL_ADD && m0 + i < M ? load_elem(e.residual, type, o + (int64_t)i * e.N) : 0.f;
-#pragma unroll
-    for (int i = 0; i < 2 * PAIRS; ++i)
-        if (m0 + i < M) store_out(e.Y, type, o + (int64_t)i * e.N, e.epilogue == QF_EPI_RESIDUAL_ADD ? v[i] + r[i] : v[i]);
+    for (int i = 0; i < PAIRS; ++i) {
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 1);
+        float lo = odd ? other : v[2 * i], hi = odd ? v[2 * i + 1] : other;
+        if (add) {
+            float a = __uint_as_float(r[i].x), b = __uint_as_float(r[i].y);
+            if (e.out_dtype == QF_BF16) b = __uint_as_float(r[i].x & 0xffff0000u), a = __uint_as_float(r[i].x << 16);
+            if (e.out_dtype == QF_F16) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&r[i].x));
+                a = f.x, b = f.y;
+            }
+            lo += a;
+            hi += b;
+        }
+        if (at.m + 2 * i < M) stream_put(e, at.o + (int64_t)i * at.step, lo, hi);
+    }
 }
 
-__device__ __forceinline__ unsigned long long *slot_of(const StreamArgs &a, const Segment &g, int member) {
-    return a.slots + (size_t)(member == 0 ? g.slot0 : g.base + member) * a.slot_words;
+// Word of a member's slot (32 bits: 888 slots of at most 4096 words).
+__device__ __forceinline__ unsigned slot_of(const StreamArgs &a, const Segment &g, int member) {
+    return (unsigned)((member == 0 ? g.slot0 : g.base + member) * a.slot_words);
 }
 // Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of eight members are requested
 // at a time. Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us,
@@ -230,30 +293,32 @@ __device__ __forceinline__ bool stream_sum(const StreamArgs &a, const Segment &g
                                            volatile int *abort_flag) {
     constexpr int WORDS = 8;
     v[0] = v[1] = 0.f;
+    const unsigned at = (unsigned)(pair * 128 + row) * 2u;
 #pragma unroll 1
     for (int m0 = 0; m0 < g.members; m0 += WORDS) {
-        unsigned long long *src[WORDS], w[WORDS][2];
+        // (where there are fewer, the last member's words take the place of the missing ones; what is added for them is +0, and a sum that
+        // begins with +0 is never -0)
+        unsigned src[WORDS];
+        unsigned long long w[WORDS][2];
 #pragma unroll
-        for (int j = 0; j < WORDS; ++j) src[j] = slot_of(a, g, m0 + j) + (pair * 128 + row) * 2;
+        for (int j = 0; j < WORDS; ++j) src[j] = slot_of(a, g, min(m0 + j, g.members - 1)) + at;
         const long long t0 = clock64();
         while (true) {
-            bool miss = false;
+            unsigned miss = 0u;
 #pragma unroll
-            for (int j = 0; j < WORDS; ++j)
-                if (m0 + j < g.members) ld_words2(src[j], w[j][0], w[j][1]);
+            for (int j = 0; j < WORDS; ++j) ld_words2(a.slots + src[j], w[j][0], w[j][1]);
 #pragma unroll
-            for (int j = 0; j < WORDS; ++j)
-                if (m0 + j < g.members) miss = miss || (uint32_t)(w[j][0] >> 32) != 1u || (uint32_t)(w[j][1] >> 32) != 1u;
-            if (!__any_sync(0xffffffffu, miss)) break;
+            for (int j = 0; j < WORDS; ++j) miss |= ((unsigned)(w[j][0] >> 32) ^ 1u) | ((unsigned)(w[j][1] >> 32) ^ 1u);
+            if (!__any_sync(0xffffffffu, miss != 0u)) break;
             if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles || *abort_flag != 0)) return false;
         }
 #pragma unroll
-        for (int j = 0; j < WORDS; ++j)
-            if (m0 + j < g.members) {
-                v[0] += __uint_as_float((uint32_t)w[j][0]);
-                v[1] += __uint_as_float((uint32_t)w[j][1]);
-                st_words2(src[j], 0ull, 0ull);
-            }
+        for (int j = 0; j < WORDS; ++j) {
+            const bool real = m0 + j < g.members;
+            v[0] += real ? __uint_as_float((uint32_t)w[j][0]) : 0.f;
+            v[1] += real ? __uint_as_float((uint32_t)w[j][1]) : 0.f;
+            st_words2(a.slots + src[j], 0ull, 0ull);
+        }
     }
     return true;
 }
@@ -287,13 +352,69 @@ __device__ __forceinline__ bool stream_wait(uint32_t bar, uint32_t parity, volat
     return stream_try_wait(bar, parity) || stream_wait_on(bar, parity, abort_flag);
 }
 
+// Warp-uniform: waits until the phases behind `gate` are complete; false when another role gave up.
+__device__ __forceinline__ bool stream_gate(volatile int *gates, int gate, volatile int *abort_flag) {
+    bool ok = true;
+    const long long t0 = clock64();
+    while (ok && *gates < gate) {
+        __nanosleep(40);
+        if (*abort_flag) ok = false;
+        else if (clock64() - t0 > kWaitCycles) *abort_flag = 1;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    __threadfence_block();
+    return ok;
+}
+// Waits until phase w (or -1) is complete; one thread.
+__device__ __forceinline__ bool stream_phase_done(const StreamArgs &a, int w, unsigned want, volatile int *abort_flag) {
+    const long long t0 = clock64();
+    while (ld_acquire(a.done + w) < want) {
+        __nanosleep(40);
+        if (*abort_flag) return false;
+        if (clock64() - t0 > kWaitCycles) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+    return true;
+}
+// Waits for the row blocks that chunk c of an entry's activations comes from, and looks at those of the n - 1 chunks behind it: how many
+// chunks are there (at least one), or 0 when it gave up. All 32 lanes, each a chunk's counters.
+__device__ __forceinline__ int stream_arrived(const StreamArgs &a, const StreamEntry &e, int c, int n, int lane, volatile int *abort_flag) {
+    const unsigned want = (unsigned)e.x_want;
+    const unsigned *count = a.done + e.x_from + (e.x_two ? 2 * (c + lane) : c + lane);
+    bool there = lane >= n;
+    const long long t0 = clock64();
+    while (true) {
+        if (!there) there = ld_acquire(count) >= want && (!e.x_two || ld_acquire(count + 1) >= want);
+        const unsigned yet = ~__ballot_sync(0xffffffffu, there);
+        if (!(yet & 1u)) {
+            __syncwarp();
+            // the results were stored through the generic proxy and are read by the copy engine
+            fence_proxy_async_all();
+            return min(n, yet ? __ffs(yet) - 1 : 32);
+        }
+        if (clock64() - t0 > kWaitCycles) *abort_flag = 1;
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) return 0;
+        __nanosleep(20);
+    }
+}
+// Whether this is the last of a stream's four result warps to get here; it then speaks for the stores of all four.
+__device__ __forceinline__ bool stream_last_warp(unsigned *count) {
+    unsigned before;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_u32(count)) : "memory");
+    return (before & 3u) == 3u;
+}
+
 template <bool BF16, int NB, int CAP>
 __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_constant__ StreamParams<CAP> p) {
     using C = StreamCfg<NB>;
     extern __shared__ uint8_t stream_smem[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
-    __shared__ int s_gates[2];  // of a stream: phases whose waits are over (those that it has work in)
+    // Of a stream: of the phases that it has work in, two steps each: partial sums may be written, results may be.
+    __shared__ int s_gates[2];
+    __shared__ unsigned s_finished[2][4];  // result warps that have finished a phase, by its number modulo 4
 
     const int tid = threadIdx.x & 511;
     const int half = threadIdx.x >> 9;
@@ -301,7 +422,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
     const int lane = tid & 31;
     // The single threads of the two streams sit on different schedulers (a warp's is its number mod 4): weights 8 and 10,
     // activations 9 and 11, MMAs 10 and 8.
-    // roles: 0 converts, 1 weights, 2 activations, 3 MMAs, 4 results, 5 none
+    // roles: 0 converts, 1 weights, 2 activations, 3 MMAs, 4 results, 5 waits for phases
     const int role = warp < 8 ? 0 : warp >= 12 ? 4 : (half == 0 ? 0x5321 : 0x2153) >> (4 * (warp - 8)) & 7;
     const int id = half * (int)gridDim.x + (int)blockIdx.x;  // of the stream: two streams of a block differ by at most a unit
     const uint32_t base = ((smem_u32(stream_smem) + 1023u) & ~1023u) + (uint32_t)half * C::STREAM_BYTES;
@@ -344,6 +465,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
             mbar_init(dempty(d), 4);
         }
         s_gates[half] = 0;
+        for (int i = 0; i < 4; ++i) s_finished[half][i] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 10 && half == 0) tmem_alloc<false>(smem_u32(&s_tmem_base), 2 * ST_TMEM_COLS);
@@ -396,50 +518,69 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
     } else if (role == 2) {
         // ------------------------------ activations ------------------------------
         const bool leader = elect_one();
-        if (leader) {
-            int s = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            const uint32_t tx = 2u * (uint32_t)a.x_rows * 128u;
-            int passed[2] = {-1, -1}, opened = 0;
-            for (int phase = 0; phase < phases && ok; ++phase) {
-                bool behind = CAP > 1 && (t.ph[phase].wait[0] >= 0 || t.ph[phase].wait[1] >= 0);
-                for_segments(t, phase, id, [&](const Segment &g) {
-                    if (behind) {
-                        for (int i = 0; i < 2; ++i) {
-                            const int w = t.ph[phase].wait[i];
-                            if (w < 0 || w == passed[i]) continue;
-                            const unsigned want = 4u * (unsigned)t.ph[w].active;
-                            const long long t0 = clock64();
-                            while (ld_acquire(a.done + w) < want) {
-                                if (*abort_flag) return ok = false;
-                                if (clock64() - t0 > kWaitCycles) {
-                                    *abort_flag = 1;
-                                    return ok = false;
-                                }
-                            }
-                            passed[i] = w;
-                        }
-                        // the results were stored through the generic proxy and are read by the copy engine
-                        fence_proxy_async_all();
-                        __threadfence_block();
-                        *gates = ++opened;
-                        behind = false;
+        int s = 0, nth = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        const uint32_t tx = 2u * (uint32_t)a.x_rows * 128u;
+        for (int phase = 0; phase < phases && ok; ++phase) {
+            if (!stream_works<CAP>(t.ph[phase], id)) continue;
+            ++nth;
+            bool open = false;
+            for_segments(t, phase, id, [&](const Segment &g) {
+                const StreamEntry &en = t.e[g.e];
+                const CUtensorMap *map = &p.x[en.x_map];
+                if (leader) tma_prefetch_desc(map);
+                int there = CAP > 1 && en.x_from >= 0 ? 0 : g.len;  // chunks that can be read
+                if (CAP > 1 && en.x_from == kXGate && !open) {
+                    ok = stream_gate(gates, 2 * nth, abort_flag);
+                    if (!ok) return false;
+                    fence_proxy_async_all();
+                    open = true;
+                }
+                for (int i = 0; i < g.len; ++i) {
+                    if (CAP > 1 && i == there) {
+                        const int n = stream_arrived(a, en, g.c + i, g.len - i, lane, abort_flag);
+                        ok = n > 0;
+                        if (!ok) return false;
+                        there += n;
                     }
-                    const CUtensorMap *map = &p.x[t.e[g.e].x_map];
-                    for (int i = 0; i < g.len; ++i) {
-                        if (!stream_wait(xempty(s), ph ^ 1u, abort_flag)) return ok = false;
+                    ok = __all_sync(0xffffffffu, !leader || stream_wait(xempty(s), ph ^ 1u, abort_flag));
+                    if (!ok) return false;
+                    if (leader) {
                         mbar_arrive_expect_tx(xfull(s), tx);
                         tma_load_2d(x_stage(s), map, xfull(s), (g.c + i) * 128, 0);
                         tma_load_2d(x_stage(s) + C::X_BOX_BYTES, map, xfull(s), (g.c + i) * 128 + 64, 0);
-                        ++issued;
-                        if (++s == C::X_STAGES) {
-                            s = 0;
-                            ph ^= 1u;
-                        }
                     }
-                    return true;
-                });
+                    ++issued;
+                    if (++s == C::X_STAGES) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
+                }
+                return true;
+            });
+        }
+        __syncwarp();
+    } else if (role == 5) {
+        // ------------------------------ waits for phases ------------------------------
+        // The results of a phase come behind the phases that it waits for; its activations may be there before (stream_arrived), and its
+        // partial sums may be exchanged as soon as the last phase with the same slots is complete.
+        if (CAP > 1 && elect_one()) {
+            int passed[3] = {-1, -1, -1}, opened = 0;
+            bool ok = true;
+            for (int phase = 0; phase < phases && ok; ++phase) {
+                if (!stream_works<CAP>(t.ph[phase], id)) continue;
+                const int waits[3] = {t.ph[phase].slots_wait, t.ph[phase].wait[1], t.ph[phase].wait[0]};
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int w = waits[i];
+                    if (ok && w >= 0 && w != passed[i]) ok = stream_phase_done(a, w, (unsigned)t.ph[w].active, abort_flag);
+                    passed[i] = w;
+                    if (ok && i > 0) {
+                        __threadfence_block();
+                        *gates = ++opened;
+                    }
+                }
             }
         }
         __syncwarp();
@@ -563,83 +704,112 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
         const int quad = warp & 3;  // TMEM lanes 32 * quad ..
         const int row = quad * 32 + lane;
         const uint32_t lane_tmem = tmem + ((uint32_t)(quad * 32) << 16);
-        int seg = 0;
-        int opened = 0;
+        int seg = 0, nth = 0;
         bool ok = true;
+        // (behind the stores of a row block: whoever waits for it may read it)
+        auto finished = [&](const StreamEntry &en, int b) {
+            if (CAP == 1 || en.flags < 0) return;
+            __syncwarp();
+            if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.done + en.flags + b) : "memory");
+        };
         for (int phase = 0; phase < phases; ++phase) {
             if (!stream_works<CAP>(t.ph[phase], id)) continue;
-            if (CAP > 1 && (t.ph[phase].wait[0] >= 0 || t.ph[phase].wait[1] >= 0)) {
-                // idle until then: the results come behind the activations. (Not a barrier's phase: the other side may be two ahead.)
-                ++opened;
-                const long long t0 = clock64();
-                while (ok && *gates < opened) {
-                    __nanosleep(100);
-                    if (*abort_flag) ok = false;
-                    else if (clock64() - t0 > kWaitCycles) *abort_flag = 1;
-                }
-                ok = __all_sync(0xffffffffu, ok);
-                __threadfence_block();
-            }
+            ++nth;
+            bool open = CAP == 1;  // results may be written
+            if (CAP > 1) ok = ok && stream_gate(gates, 2 * nth - 1, abort_flag);
+            auto opens = [&]() {
+                if (!open) ok = stream_gate(gates, 2 * nth, abort_flag);
+                open = true;
+                return ok;
+            };
             for_segments(t, phase, id, [&](const Segment &g) {
                 const int d = seg & 1;
                 const StreamEntry &en = t.e[g.e];
                 const int n = g.b * 128 + row;
                 const bool in = g.b * 128 + quad * 32 < en.N;  // N is a multiple of 64: the last row block may be half
-                unsigned long long *slot = slot_of(a, g, g.self) + row * 2;
+                unsigned long long *slot = a.slots + slot_of(a, g, g.self) + row * 2;
                 ok = __all_sync(0xffffffffu, ok && stream_wait(dfull(d), (uint32_t)(seg >> 1) & 1u, abort_flag));
                 if (!ok) return false;
                 ++seg;
+                if (g.members == 1 && !opens()) return false;
                 tc_fence_after();
+                if (g.members == 1) {
 #pragma unroll 1
-                for (int m0 = 0; m0 < a.M; m0 += 8) {
-                    uint32_t r[8];
-                    tmem_ld8(lane_tmem + d * NB + m0, r);
-                    tmem_wait_ld();
-                    if (!in) continue;
-                    if (g.members == 1) {
-                        float v[8];
+                    for (int m0 = 0; m0 < a.M; m0 += 4) {
+                        uint32_t r[4];
+                        tmem_ld4(lane_tmem + d * NB + m0, r);
+                        tmem_wait_ld();
+                        if (!in) continue;
+                        const float v[4] = {__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3])};
+                        uint2 add[2];
+                        const StreamOut at = stream_out(en, n, m0);
+                        if (en.epilogue == QF_EPI_RESIDUAL_ADD) stream_residual<2>(en, a.M, at, add);
+                        stream_emit<2>(en, a.M, n, m0, v, at, add);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int m0 = 0; m0 < a.M; m0 += 16, slot += 16 * 128) {
+                        uint32_t r[16];
+                        tmem_ld16(lane_tmem + d * NB + m0, r);
+                        tmem_wait_ld();
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
-                        stream_emit<4>(en, a.M, n, m0, v);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 8; j += 2)
-                            if (m0 + j < a.M) st_words2(slot + (m0 + j) * 128, word_of(r[j]), word_of(r[j + 1]));
+                        for (int j = 0; j < 16; j += 2)
+                            if (in && m0 + j < a.M) st_words2(slot + j * 128, word_of(r[j]), word_of(r[j + 1]));
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dempty(d));
+                if (g.members == 1) finished(en, g.b);
                 return true;
             });
             // The members of a shared row block finish its pairs of batch rows in turn.
             for_segments(t, phase, id, [&](const Segment &g) {
                 const StreamEntry &en = t.e[g.e];
-                if (!ok || g.members == 1 || g.b * 128 + quad * 32 >= en.N) return ok;
+                const int pairs = (a.M + 1) >> 1, first = g.members - 1 - g.self;
+                if (!ok || g.members == 1 || first >= pairs) return ok;
+                if (g.b * 128 + quad * 32 < en.N) {
 #pragma unroll 1
-                for (int pair = g.members - 1 - g.self; pair < (a.M + 1) >> 1; pair += g.members) {
-                    float v[2];
-                    ok = stream_sum(a, g, pair, row, v, abort_flag);
-                    if (!ok) {
-                        *abort_flag = 1;
-                        return false;
+                    for (int pair = first; pair < pairs; pair += g.members) {
+                        float v[2];
+                        uint2 add[1];
+                        const StreamOut at = stream_out(en, g.b * 128 + row, 2 * pair);
+                        const bool adds = en.epilogue == QF_EPI_RESIDUAL_ADD;
+                        // what is added is on its way while the sums are awaited, where it is known to be there
+                        if (!open && __all_sync(0xffffffffu, *gates >= 2 * nth) && !opens()) return false;
+                        const bool early = open;
+                        if (early && adds) stream_residual<1>(en, a.M, at, add);
+                        ok = stream_sum(a, g, pair, row, v, abort_flag);
+                        if (!ok) {
+                            *abort_flag = 1;
+                            return false;
+                        }
+                        if (!early) {
+                            if (!opens()) return false;
+                            if (adds) stream_residual<1>(en, a.M, at, add);
+                        }
+                        stream_emit<1>(en, a.M, g.b * 128 + row, 2 * pair, v, at, add);
                     }
-                    stream_emit<1>(en, a.M, g.b * 128 + row, 2 * pair, v);
                 }
+                finished(en, g.b);
                 return true;
             });
             if (CAP > 1) {
+                // a phase that is complete says that those are that it waits for, also where this stream had no result to write
+                if (ok) opens();
                 __syncwarp();
-                if (lane == 0 && ok) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.done + phase) : "memory");
+                if (lane == 0 && ok && stream_last_warp(&s_finished[half][nth & 3]))
+                    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.done + phase) : "memory");
             }
         }
-        if (CAP > 1 && lane == 0 && ok) {
+        if (CAP > 1) {
             // The last result warp of the launch leaves the counters as they were: behind everybody's last count and wait.
-            unsigned before;
-            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.done + kStreamMaxLinears) : "memory");
-            if (before + 1u == 8u * gridDim.x) {
-                for (int q = 0; q < phases; ++q) a.done[q] = 0u;
-                a.done[kStreamMaxLinears] = 0u;
+            unsigned before = 0;
+            if (lane == 0 && ok)
+                asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.done + kStreamMaxLinears) : "memory");
+            if (__shfl_sync(0xffffffffu, before + 1u, 0) == 8u * gridDim.x && __all_sync(0xffffffffu, ok)) {
+                __syncwarp();
+                for (int q = lane * 4; q < a.words; q += 128) *reinterpret_cast<uint4 *>(a.done + q) = make_uint4(0u, 0u, 0u, 0u);
             }
         }
     }
@@ -693,7 +863,7 @@ int stream_init(qf_ctx *ctx) {
 
 static size_t slot_words(int64_t M) { return (size_t)((M + 1) / 2) * 2 * 128; }
 
-size_t stream_workspace_bytes(int64_t M) { return (size_t)kStreamSlots * slot_words(M) * sizeof(unsigned long long); }
+size_t stream_workspace_bytes(int64_t M, int slots) { return (size_t)slots * slot_words(M) * sizeof(unsigned long long); }
 
 template <bool BF16, int NB, int CAP>
 static cudaError_t stream_go(const StreamParams<CAP> &p, int grid, cudaStream_t s) {
@@ -717,7 +887,7 @@ static cudaError_t stream_dispatch(const StreamParams<CAP> &p, bool bf16, int gr
 }
 
 template <int CAP>
-static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s) {
+static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, int slots, cudaStream_t s) {
     StreamParams<CAP> p;
     const qf_linear_desc &d0 = *l[0].d;
     p.a.slots = (unsigned long long *)((char *)ws + counter_bytes);
@@ -726,6 +896,7 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
     p.a.slot_words = (int)slot_words(d0.M);
     p.a.M = (int)d0.M;
     p.a.x_rows = (int)((d0.M + 7) / 8) * 8;
+    p.a.words = kStreamFlags;
     const void *x_of[StreamParams<CAP>::XCAP];
     int64_t x_k[StreamParams<CAP>::XCAP];
     int maps = 0, phases = 0, next = 0;
@@ -747,6 +918,9 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
         e.epilogue = (int16_t)d.epilogue;
         int st = get_slab_map(ctx, &p.w[next++], l[i].blob, (uint64_t)(d.N / 64), (uint64_t)e.chunks);
         if (st != QF_OK) return st;
+        e.x_from = kXThere;
+        e.flags = -1;
+        e.x_want = e.x_two = 0;
         e.x_map = 0;
         while (e.x_map < maps && !(x_of[e.x_map] == l[i].X && x_k[e.x_map] == d.K)) ++e.x_map;
         if (e.x_map == maps) {
@@ -772,17 +946,35 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
     } else {
         grid = sms;
         ChainPlan plan;
-        plan_stream_chain(l, count, 2 * grid, &plan);
+        plan_stream_chain(l, count, 2 * grid, slots, &plan);
+        std::vector<int> entry_of(count);
         for (const ChainPhase &c : plan.phases) {
             StreamPhase &ph = p.ph[phases++];
-            ph = StreamPhase{next, 0, 0, 0, c.streams, c.home, c.flip, 0, {c.wait[0], c.wait[1]}};
+            ph = StreamPhase{next, 0, 0, 0, c.streams, c.home, c.flip, 0, {c.wait[0], c.wait[1]}, c.slots_wait};
             for (int k = c.first; k < c.first + c.count; ++k) {
                 const int st = enter(plan.order[k]);
                 if (st != QF_OK) return st;
                 p.e[next - 1].slot = plan.linears[plan.order[k]].slot;
+                entry_of[plan.order[k]] = next - 1;
             }
             ph.active = std::min(ph.pieces, ph.streams);
         }
+        for (int i = 0; i < count; ++i) {
+            const ChainLinear &at = plan.linears[i];
+            StreamEntry &e = p.e[entry_of[i]];
+            e.x_from = at.maker == kChainThere ? kXThere : kXGate;
+            if (at.maker < 0 || plan.linears[at.maker].flags < 0) continue;
+            const StreamLinear &from = l[at.maker];
+            e.x_from = kStreamFlags + plan.linears[at.maker].flags;
+            e.x_two = from.d->epilogue == QF_EPI_SILU_MUL;
+            // the warps of the members that finish a pair of batch rows
+            e.x_want = (int16_t)(4 * std::min<int64_t>(from.split, (d0.M + 1) / 2));
+        }
+        for (int i = 0; i < count; ++i)
+            if (plan.linears[i].flags >= 0) {
+                p.e[entry_of[i]].flags = kStreamFlags + plan.linears[i].flags;
+                p.a.words = std::max(p.a.words, kStreamFlags + plan.linears[i].flags + (int)row_blocks(*l[i].d));
+            }
     }
     p.a.phases = phases;
     p.a.linears = count;
@@ -795,11 +987,11 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
 }
 
 int launch_stream(qf_ctx *ctx, const StreamLinear &l, void *ws, size_t counter_bytes, cudaStream_t s) {
-    return stream_launch<1>(ctx, &l, 1, ws, counter_bytes, s);
+    return stream_launch<1>(ctx, &l, 1, ws, counter_bytes, kStreamSlots, s);
 }
 
-int launch_stream_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, cudaStream_t s) {
-    return stream_launch<kStreamMaxLinears>(ctx, l, count, ws, counter_bytes, s);
+int launch_stream_chain(qf_ctx *ctx, const StreamLinear *l, int count, void *ws, size_t counter_bytes, int slots, cudaStream_t s) {
+    return stream_launch<kStreamMaxLinears>(ctx, l, count, ws, counter_bytes, slots, s);
 }
 
 }  // namespace qf
