@@ -276,21 +276,29 @@ __device__ __forceinline__ void gemv_body(const GemvParams &p, const typename Ex
         const int per = (units + p.split_k - 1) / p.split_k;
         const int u_end = min(units, (split + 1) * per);
         const uint32_t tile = (uint32_t)__cvta_generic_to_shared(s_tile);
-        for (int u = split * per + tid; u < u_end; u += GEMV_THREADS) {
+        // (two blocks at least: a thread has one or two of the outputs)
+        constexpr int kUnits = (GEMV_ROWS_PER_BLOCK * (m_pad + (m_pad & 1)) / 2 + GEMV_THREADS - 1) / GEMV_THREADS;
+        float sum[kUnits];
+#pragma unroll
+        for (int i = 0; i < kUnits; ++i) {
+            const int u = split * per + tid + i * GEMV_THREADS;
+            float v[8];
+#pragma unroll
+            for (int sp = 0; sp < 8; ++sp)
+                v[sp] = u < u_end && sp < p.split_k ? ld_dsmem_f1(dsmem_addr(tile + 4u * (uint32_t)u, (uint32_t)sp)) : 0.f;
+            sum[i] = 0.f;
+#pragma unroll
+            for (int sp = 0; sp < 8; ++sp) sum[i] += v[sp];
+        }
+        cluster_arrive();  // has read what it reads of the other blocks
+#pragma unroll
+        for (int i = 0; i < kUnits; ++i) {
+            const int u = split * per + tid + i * GEMV_THREADS;
             const int64_t n = n_blk + (u & (GEMV_ROWS_PER_BLOCK - 1));
             const int64_t mm = (int64_t)mt * 8 + u / GEMV_ROWS_PER_BLOCK;
-            if (n < p.N && mm < p.M) {
-                float v[8];
-#pragma unroll
-                for (int sp = 0; sp < 8; ++sp)
-                    v[sp] = sp < p.split_k ? ld_dsmem_f1(dsmem_addr(tile + 4u * (uint32_t)u, (uint32_t)sp)) : 0.f;
-                float s = 0.f;
-#pragma unroll
-                for (int sp = 0; sp < 8; ++sp) s += v[sp];
-                store_out(p.Y, p.out_dtype, mm * p.N + n, s);
-            }
+            if (u < u_end && n < p.N && mm < p.M) store_out(p.Y, p.out_dtype, mm * p.N + n, sum[i]);
         }
-        cluster_sync_all();  // nobody leaves while its partial outputs may still be read
+        cluster_wait();  // nobody leaves while its partial outputs may still be read
         return;
     }
     if (AR && p.split_k == 1) {
