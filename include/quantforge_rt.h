@@ -52,7 +52,8 @@ typedef enum qf_zero_mode { QF_ZERO_CONST = 0, QF_ZERO_U4 = 1, QF_ZERO_I8 = 2 } 
  * prepacked, 40 MB canonical), M >= 3 -> tcgen05 GEMM kernel (measured crossovers on B200); prepacked weights
  * (QF_LAYOUT_GEMV_SLAB runs the streaming GEMV kernel, or from 9 rows and 24 to 72 MiB on, by K, the streaming tcgen05 kernel;
  * QF_PATH_GEMV keeps it on the former; the other prepacked layouts run the tcgen05 kernel),
- * N % 128 != 0 and a fused epilogue override it, see qf_w4a16_plan. */
+ * N % 128 != 0 (the GEMV kernel, or, for 16-bit results of 3 rows and more on canonical weights from a size on, the tcgen05 kernel) and a
+ * fused epilogue override it, see qf_w4a16_plan. */
 typedef enum qf_path { QF_PATH_AUTO = 0, QF_PATH_GEMV = 1, QF_PATH_GEMM = 2 } qf_path;
 
 /*

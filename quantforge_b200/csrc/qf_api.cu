@@ -91,6 +91,26 @@ static bool stream_serves(const qf_linear_desc *d) {
     return d->K >= 512 && mib >= (d->K >= 8192 ? 24 : d->K >= 6144 ? 33 : d->K >= 5120 ? 42 : 72);
 }
 
+// Whether the tcgen05 kernel takes canonical weights of N % 128 != 0 rows, as the GEMV kernel can. Copies of scales and zeros are
+// multiples of 16 bytes, also those of what is left for the last tile of 128 rows. Measured, GEMV / tcgen05 kernel, times as fast:
+//   K x N          1024x4112  1024x6160  2048x2064  2048x3088  4096x1040  4096x3088  6144x2064  8192x4112  14336x2064  14336x14352  512x40976
+//   codes             4.2 M      6.3        4.2        6.3        4.3       12.6       12.7       33.7       29.6        206          21
+//   3 rows             0.87      1.04       0.87       1.04       0.91       1.21       1.28       1.11       0.93       1.31        0.73
+//   8 rows             0.87      1.13       0.88       1.10       0.95       1.26       1.52       1.29       1.10       2.26        0.76
+// 9 to 16 rows (two tiles of the GEMV kernel): 1024x2064 0.89, 2048x1040 0.88 to 1.06, 4096x528 0.98, 2048x2064 1.20, 8192x528 1.42, 512x11024 1.31,
+// 3968x5136 1.95, 28672x4112 3.7; 17 to 64 rows: 1024x1040 0.81 to 1.02, 1024x2064 1.04 to 1.44, 2048x2064 1.44 to 2.0; 200 rows: 2048x1040
+// 0.58, 2048x2064 1.06, 8192x528 1.18.
+static bool gemm_serves_ragged(const qf_linear_desc *d) {
+    if (d->weight_layout != QF_LAYOUT_CANONICAL || d->epilogue != QF_EPI_NONE || d->M < 3) return false;
+    if (d->zero_mode == QF_ZERO_U4 && d->N % 32 != 0) return false;
+    // Sums of a whole split in one accumulator are 2e-7 to 4e-7 (of the outputs' rms) further off than the GEMV kernel's two accumulators
+    // of shorter splits: 16-bit results, rounded by 1e-4 and more, do not show it; 32-bit ones keep that kernel.
+    if (d->out_dtype == QF_F32) return false;
+    const int64_t codes = d->K * d->N;
+    if (d->M <= 8) return codes >= 6000000 && d->K >= 1024;
+    return codes >= (d->M <= 16 || d->M > 64 ? 4000000 : 2000000);
+}
+
 int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
     auto bad = [&](int st, const char *m) {
         if (why) *why = m;
@@ -169,7 +189,8 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
                        "a fused epilogue needs QF_LAYOUT_GEMV_SLAB weights or the tcgen05 path (N % 128 == 0)");
         path = QF_PATH_GEMM;
     }
-    if (path == QF_PATH_GEMM && d->N % 128 != 0) {
+    // Any multiple of 16 rows of weights where the kernel may be chosen: the last tile of 128 is cut short (gemm_serves_ragged)
+    if (path == QF_PATH_GEMM && d->N % 128 != 0 && !(d->path == QF_PATH_AUTO && gemm_serves_ragged(d))) {
         if (d->path == QF_PATH_GEMM) return bad(QF_ERR_BAD_ARG, "the GEMM path needs N to be a multiple of 128");
         path = QF_PATH_GEMV;
     }
@@ -219,7 +240,7 @@ int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {
         // of 16, 32, 64, 128 or 256 rows ran M = 777 as 1024 rows; 777 x 4096 x 4096 f16, canonical: 38.5 -> 35.1 us.)
         p->m_tiles = d->M > 256 ? (int)((d->M + 255) / 256) : 1;
         const int64_t rows = d->M > p->m_tiles ? (d->M + p->m_tiles - 1) / p->m_tiles : 1;
-        const int64_t tiles = (int64_t)p->m_tiles * (d->N / 128);
+        const int64_t tiles = (int64_t)p->m_tiles * ((d->N + 127) / 128);
         auto width = [&](int step) { return (int)((rows + step - 1) / step * step); };
         // Splits of K for batch tiles of bn rows in k-blocks of bk codes, and k-blocks per split.
         auto splits = [&](int bn, int bk, int *kbps_out) {
@@ -557,6 +578,11 @@ size_t qf_w4a16_workspace_bytes(const qf_linear_desc *desc) {
     Plan plan;
     if (make_plan(desc, &plan, nullptr) != QF_OK) return 0;
     size_t need = plan.ws_partial_bytes + plan.ws_counter_bytes;
+    if (plan.path == QF_PATH_GEMM && desc->N % 128 != 0) {  // an exchanging call takes the GEMV kernel
+        qf_linear_desc d = *desc;
+        d.path = QF_PATH_GEMV;
+        if (make_plan(&d, &plan, nullptr) == QF_OK) need = std::max(need, plan.ws_partial_bytes + plan.ws_counter_bytes);
+    }
     if (desc->weight_layout == QF_LAYOUT_GEMV_SLAB && desc->split_k == 0) {
         // An exchanging call on the same descriptor may divide the weights among more thread blocks. That is also what the
         // streaming GEMV kernel needs where it steps in for the tcgen05 kernel.

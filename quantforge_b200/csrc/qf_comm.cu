@@ -168,7 +168,7 @@ int qf_comm_destroy(qf_comm *comm) {
 }
 
 // Shared body of the two exchange entry points. The path follows the plan of qf_w4a16_linear (GEMV kernel for
-// M <= 2 or when N is not a multiple of 128, tcgen05 kernel otherwise) unless desc->path names one.
+// M <= 2, tcgen05 kernel otherwise) unless desc->path names one or N is not a multiple of 128 (GEMV kernel).
 static int linear_exchange(qf_ctx *ctx, qf_comm *comm, const qf_linear_desc *desc, const void *X,
                            const void *qweight, const void *scales, const void *qzeros_or_null, void *Y,
                            void *workspace, size_t workspace_bytes, void *stream, int gather) {
@@ -186,6 +186,9 @@ static int linear_exchange(qf_ctx *ctx, qf_comm *comm, const qf_linear_desc *des
     if (local_desc.weight_layout == QF_LAYOUT_GEMV_SLAB && local_desc.split_k == 0) {
         // (the launch checks it against the occupancy the kernel really gets)
         local_desc.split_k = slab_exchange_grid(desc, ctx->sm_count);
+        desc = &local_desc;
+    } else if (local_desc.path == QF_PATH_AUTO && local_desc.N % 128 != 0) {
+        local_desc.path = QF_PATH_GEMV;  // the tcgen05 kernel exchanges whole tiles
         desc = &local_desc;
     }
     Plan plan;

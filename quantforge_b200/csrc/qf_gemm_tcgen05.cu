@@ -225,18 +225,19 @@ __device__ __forceinline__ void convert32(const uint4 &v, const ShortConvert<BF1
 // ---------------------------------------------------------------------------------------------
 // EXCH: finished tiles are exchanged across GPUs (sum or gather) before Y is written; `ar` then is an ArParams.
 // The plain instantiations take an empty struct instead, so their parameter block and code stay what they were.
+// RAGGED: the last weight tile has fewer than 128 rows (an instantiation of its own: the same in all cost the others 1 to 2 %).
 // PAIR: the grid runs in clusters of two blocks along x (weight tiles 2i, 2i + 1). A block stages half of the batch tile's
 // rows and its own weights; its converters report to the first block, whose MMA warp issues cta_group::2 MMAs of 256
 // weight rows for both and signals completion to both. With one CTA per MMA a k-block of 64 codes and 256 rows moves 72 KB
 // through a block's shared memory (36 KB in, 32 KB to the tensor core, 4 KB of codes to the converters), 562 cycles at
 // 128 bytes a cycle and more than the 512 the MMAs take; in a pair it is 40 KB. M = 2048, 8192 x 28672: 777 -> 738 us;
 // M = 777, 4096 x 4096: 28.9 -> 27.5 us.
-template <bool BF16, int BN, bool INTER, bool EXCH, bool PAIR>
+template <bool BF16, int BN, bool INTER, bool EXCH, bool PAIR, bool RAGGED = false>
 __global__ void __launch_bounds__(GEMM_THREADS, GemmCfg<BN, PAIR>::CTAS_PER_SM)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
             const GemmParams p, const typename ExchArg<EXCH>::type ar) {
     using C = GemmCfg<BN, PAIR>;
-    static_assert(!(PAIR && EXCH), "the exchange serves the narrow tiles");
+    static_assert(!(PAIR && EXCH) && !(RAGGED && (PAIR || EXCH)), "the exchange serves the narrow tiles, whole ones");
     constexpr int BK = C::BK;
     constexpr int STAGES = C::STAGES;
     constexpr int NA = C::NA;
@@ -284,6 +285,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         mbar_init(dfull_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (RAGGED && n0 + 128 > p.N) {
+        // scales and zeros of rows that there are not: no copy writes them
+        for (int i = tid; i < STAGES * C::SZ_BYTES / 4; i += GEMM_THREADS)
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(bar_base + 256u + 4u * i), "r"(0u) : "memory");
+        fence_proxy_async_shared();
+    }
     if (warp == 8 && lane == 0) {
         tma_prefetch_desc(&tmap_w);
         tma_prefetch_desc(&tmap_x);
@@ -305,10 +312,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         // ------------------------------ TMA producer ------------------------------
         // The whole warp runs the loop (uniform control flow); one elected lane issues the copies.
         const bool leader = elect_one();
-        const uint32_t zbytes = p.zero_mode == QF_ZERO_U4 ? 64u : p.zero_mode == QF_ZERO_I8 ? 128u : 0u;
+        // (of a last tile of fewer than 128 rows what there is of scales and zeros; its codes' other rows are filled with zeros)
+        const uint32_t sbytes = RAGGED ? (uint32_t)min((int64_t)128, p.N - n0) * 2u : 256u;
+        const uint32_t zbytes = p.zero_mode == QF_ZERO_U4 ? sbytes / 4u : p.zero_mode == QF_ZERO_I8 ? sbytes / 2u : 0u;
         const int x_rows = PAIR ? p.bn >> 1 : p.bn;  // this block's share of the batch tile
         const int x_row0 = (int)m0 + (int)rank * x_rows;
-        const uint32_t tx_bytes = C::W_STAGE_BYTES + (uint32_t)(BK / 64) * (uint32_t)x_rows * 128u + 256u + zbytes;
+        const uint32_t tx_bytes = C::W_STAGE_BYTES + (uint32_t)(BK / 64) * (uint32_t)x_rows * 128u + sbytes + zbytes;
         const int group_kb = p.group_size / BK;  // k-blocks per quantisation group (>= 1)
         const int gi = kb0 / group_kb;
         const uint8_t *sc_ptr = (const uint8_t *)(p.scales + n0) + (size_t)gi * p.N * 2;
@@ -326,7 +335,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             const uint32_t fb = full_bar(s);
             mbar_arrive_expect_tx(fb, tx_bytes);
             tma_load_2d(w_stage(s), &tmap_w, fb, w_col(kb), w_row(kb));
-            bulk_load(sz_stage(s), sc_ptr, 256u, fb);
+            bulk_load(sz_stage(s), sc_ptr, sbytes, fb);
             if (zbytes) bulk_load(sz_stage(s) + 256u, z_ptr, zbytes, fb);
             if (++g_rem == group_kb) {
                 g_rem = 0;
@@ -356,7 +365,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 } else if (prefetch) {
                     const int dg = (kb0 + it) / group_kb - gi;  // groups behind the first one
                     tma_prefetch_2d(&tmap_w, w_col(kb0 + it), w_row(kb0 + it));
-                    l2_prefetch(sc_ptr + (size_t)dg * p.N * 2, 256u);
+                    l2_prefetch(sc_ptr + (size_t)dg * p.N * 2, sbytes);
                     if (zbytes) l2_prefetch(z_ptr + (size_t)dg * z_row, zbytes);
                 }
             }
@@ -514,7 +523,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 tmem_wait_ld();
                 if (to_partial) {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) __stcg(part + (int64_t)(col + j) * p.N, __uint_as_float(r[j]));
+                    for (int j = 0; j < 8; ++j)
+                        if (!RAGGED || n < p.N) __stcg(part + (int64_t)(col + j) * p.N, __uint_as_float(r[j]));
                 } else if constexpr (EXCH) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -551,7 +561,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
         // 5.30, 16 x 4096 x 6144 8.45 instead of 8.03, 32 x 14336 x 4096 13.5 instead of 12.8, 64 x 4096 x 1024 6.79 instead of 6.34.)
         const bool silu = p.epilogue == QF_EPI_SILU_MUL;
         const int u_end = s_abort ? 0 : min(32 * p.bn, (split + 1) * per);
-        auto mine = [&](int u) { return u < u_end && m0 + (u >> 5) < p.M && !(silu && (u & 2)); };
+        auto mine = [&](int u) { return u < u_end && m0 + (u >> 5) < p.M && !(silu && (u & 2)) && (!RAGGED || n0 + (u & 31) * 4 < p.N); };
         auto total = [&](uint32_t at) {
             float4 v[8], sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -621,7 +631,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                 for (int u = tid; u < rows * 16; u += GEMM_THREADS) {
                     float v[8];
                     lds_f4<2>(smem_base + (uint32_t)u * 32u, v);
-                    gemm_store<8>(p, m0 + (u >> 4), n0 + (u & 15) * 8, v);
+                    if (!RAGGED || n0 + (u & 15) * 8 < p.N) gemm_store<8>(p, m0 + (u >> 4), n0 + (u & 15) * 8, v);
                 }
             }
         }
@@ -650,7 +660,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
                     const int nl = (u & 31) * 4;
                     const int64_t m = m0 + (u >> 5);
                     const bool silu = !EXCH && p.epilogue == QF_EPI_SILU_MUL;
-                    if (m < p.M && !(silu && (nl & 8))) {
+                    if (m < p.M && !(silu && (nl & 8)) && (!RAGGED || n0 + nl < p.N)) {
                         // sum over the splits of 4 consecutive output columns starting `off` columns into the row
                         auto sum4 = [&](int off) {
                             const float *base = p.partial + (size_t)m * p.N + n0 + nl + off;
@@ -721,6 +731,7 @@ static cudaError_t gemm_set_attr() {
     const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, false, false>, attr, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, true, false, false>, attr, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, false, false, true>, attr, bytes);
     if constexpr (gemm_has_exchange(BN)) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, false, true, false>, attr, bytes);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_kernel<BF16, BN, true, true, false>, attr, bytes);
@@ -769,7 +780,7 @@ static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan
     p.kblocks = (int)(d->K / C::BK);
     p.kblocks_per_split = plan.chunks_per_split;
     // a pair's blocks differ in x: the dimension along which cta_group::2 pairs them
-    dim3 grid((unsigned)plan.m_tiles * (PAIR ? 2u : 1u), (unsigned)(d->N / 128) / (PAIR ? 2u : 1u), (unsigned)plan.split_k);
+    dim3 grid((unsigned)plan.m_tiles * (PAIR ? 2u : 1u), (unsigned)((d->N + 127) / 128) / (PAIR ? 2u : 1u), (unsigned)plan.split_k);
     const dim3 blk(GEMM_THREADS);
     cudaError_t le;
     if (ar) {
@@ -793,10 +804,11 @@ static int gemm_launch_bn(qf_ctx *ctx, const qf_linear_desc *d, const Plan &plan
                 cluster_z = (unsigned)plan.split_k;
             }
         }
-        le = p.interleaved ? launch_kernel_cluster(gemm_kernel<BF16, BN, true, false, PAIR>, grid, blk, C::SMEM_BYTES, s,
-                                             pdl_enabled(), dim3(PAIR ? 2 : 1, 1, cluster_z), tw, tx, p, NoExchange{})
-                           : launch_kernel_cluster(gemm_kernel<BF16, BN, false, false, PAIR>, grid, blk, C::SMEM_BYTES, s,
-                                             pdl_enabled(), dim3(PAIR ? 2 : 1, 1, cluster_z), tw, tx, p, NoExchange{});
+        const dim3 cluster(PAIR ? 2 : 1, 1, cluster_z);
+        auto *fn = p.interleaved ? gemm_kernel<BF16, BN, true, false, PAIR> : gemm_kernel<BF16, BN, false, false, PAIR>;
+        if constexpr (!PAIR)
+            if (d->N % 128 != 0) fn = gemm_kernel<BF16, BN, false, false, false, true>;
+        le = launch_kernel_cluster(fn, grid, blk, C::SMEM_BYTES, s, pdl_enabled(), cluster, tw, tx, p, NoExchange{});
     }
     note_linear(s);
     return launched(ctx, le, "GEMM");
