@@ -8,7 +8,7 @@
 // On the CPU torch divides by 15 and 7; a scale there can be the next 16-bit number (about one in 10^4 f16 scales of fp32
 // weights), and with it some codes.
 // 2 bytes in and 1 byte out per 16-bit weight (the codes are one byte each, the packing is a separate call): 7.7 us for
-// 4096 x 4096 at the copy rate. It takes 13.7 us, bound by issue slots; as elementwise passes over fp32 copies it took 300 us.
+// 4096 x 4096 at the copy rate. It takes 10.0 us; as elementwise passes over fp32 copies it took 300 us.
 #include "qf_common.cuh"
 
 namespace qf {
@@ -64,10 +64,21 @@ __device__ __forceinline__ uint32_t max2_nan(uint32_t a, uint32_t b) {
 
 struct GroupParams {
     float scale;  // after rounding to the stored type
-    float rcp;    // about 1 / scale
+    float rcp;    // 1 / scale, rounded
     float zero;
     uint16_t scale_bits;
+    bool plain;   // quotients of the group's values need no division, see quotient
 };
+
+// w / scale as a division rounds it, by the reciprocal. The product q0 is within 2 ulp of the quotient; its residual w - scale * q0 is a
+// multiple of ulp(q0) * ulp(scale) and less than 2 ulp(q0) * scale, a number of 13 bits as a stored scale has 11 at most, so one fused
+// operation gives it exactly; q0 + residual * rcp is then off by 2^-23 ulp before its own rounding. No quotient by an 11-bit number is
+// that near to a rounding boundary without being on it (the distance is at least 2^-11 of half an ulp, or 0), so the rounding is the
+// division's. Ties of a group's values, w = (k + 1/2) scale, one in 500 for bf16 weights, come out as ties.
+__device__ __forceinline__ float quotient(float w, float scale, float rcp) {
+    const float q0 = w * rcp;
+    return fmaf(fmaf(-scale, q0, w), rcp, q0);
+}
 
 template <bool SYM>
 __device__ __forceinline__ GroupParams group_params(float lo, float hi, int scale_dtype) {
@@ -84,20 +95,18 @@ __device__ __forceinline__ GroupParams group_params(float lo, float hi, int scal
         g.scale = __half2float(h);
     }
     g.rcp = 1.0f / g.scale;
+    // (false for infinities and NaN as well, and where the reciprocal could be subnormal; 256: codes are cut out of 16 bits)
+    g.plain = fmaxf(fabsf(lo), fabsf(hi)) * g.rcp < 256.0f && g.scale < 1e30f;
     if (SYM) {
         g.zero = 8.0f;
     } else {
-        float z = rintf(-lo * g.rcp);
-        if (!(fabsf(fmaf(-lo, g.rcp, -z)) < 0.4999f && fabsf(z) < 256.0f)) z = rintf(-lo / g.scale);  // as code_exact
+        const float z = rintf(g.plain ? quotient(-lo, g.scale, g.rcp) : -lo / g.scale);
         g.zero = fminf(fmaxf(z, 0.0f), 15.0f);
     }
     return g;
 }
 
-// code = clamp(rint(w / scale) + zero, 0, 15). The product with the reciprocal is within 2 ulp of the quotient, so away from
-// the rounding boundary (and for quotients of at most a few tens, what a group's own scale gives) it rounds to the same
-// integer; near the boundary the division decides. Adding 1.5 * 2^23 rounds to the nearest even integer and leaves it in
-// the low bits.
+// code = clamp(rint(w / scale) + zero, 0, 15). Adding 1.5 * 2^23 rounds to the nearest even integer and leaves it in the low bits.
 constexpr float kRound = 12582912.0f;
 __device__ __forceinline__ uint32_t code_exact(float w, const GroupParams &g) {
     return (uint32_t)(int)fminf(fmaxf(rintf(w / g.scale) + g.zero, 0.0f), 15.0f);
@@ -116,20 +125,29 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// Four codes, one per byte; `wmax`: the largest magnitude in the group. Products and roundings are made for two values at a
-// time in fp32, zero point and clamp for two in 16 bits.
-__device__ __forceinline__ uint32_t codes4(const float *v, float wmax, const GroupParams &g) {
-    const uint64_t rcp = f32x2(g.rcp, g.rcp), round = f32x2(kRound, kRound), minus = f32x2(-1.0f, -1.0f);
-    float off = 0.f;
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Four codes, one per byte. Quotients and roundings are made for two values at a time in fp32, zero point and clamp for two in 16 bits.
+// (With the product alone, and the division where that comes near to a half, a warp of bf16 weights took that way for one in four of
+// its 128 values: a fifth of all instructions, and bound by them 4096 x 4096 took 13.6 us instead of 10.0.)
+__device__ __forceinline__ uint32_t codes4(const float *v, const GroupParams &g) {
+    if (!g.plain) return code_exact(v[0], g) | code_exact(v[1], g) << 8 | code_exact(v[2], g) << 16 | code_exact(v[3], g) << 24;
+    const uint64_t rcp = f32x2(g.rcp, g.rcp), minus = f32x2(-g.scale, -g.scale), round = f32x2(kRound, kRound);
     uint32_t m[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const uint64_t w = f32x2(v[2 * h], v[2 * h + 1]);
-        const uint64_t r = fma_f32x2(w, rcp, round);
-        const uint64_t d = fma_f32x2(w, rcp, fma_f32x2(r, minus, round));  // distance from the integer
+        const uint64_t q0 = mul_f32x2(w, rcp);
+        const uint64_t r = add_f32x2(fma_f32x2(fma_f32x2(minus, q0, w), rcp, q0), round);
         float a, b;
-        split_f32x2(d, a, b);
-        off = fmaxf(off, fmaxf(fabsf(a), fabsf(b)));
         split_f32x2(r, a, b);
         m[2 * h] = __float_as_uint(a);
         m[2 * h + 1] = __float_as_uint(b);
@@ -137,23 +155,20 @@ __device__ __forceinline__ uint32_t codes4(const float *v, float wmax, const Gro
     const uint32_t zero = dup16((uint32_t)(int)g.zero);
     const uint32_t a = __viaddmin_s16x2_relu(prmt(m[0], m[1], 0x5410u), zero, 0x000f000fu);
     const uint32_t b = __viaddmin_s16x2_relu(prmt(m[2], m[3], 0x5410u), zero, 0x000f000fu);
-    uint32_t c = prmt(a, b, 0x6420u);
-    if (!(off < 0.4999f && wmax * g.rcp < 256.0f))
-        c = code_exact(v[0], g) | code_exact(v[1], g) << 8 | code_exact(v[2], g) << 16 | code_exact(v[3], g) << 24;
-    return c;
+    return prmt(a, b, 0x6420u);
 }
-__device__ __forceinline__ void codes16(const float (&v)[16], float wmax, const GroupParams &g, uint32_t (&c)[4]) {
+__device__ __forceinline__ void codes16(const float (&v)[16], const GroupParams &g, uint32_t (&c)[4]) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) c[k] = codes4(v + 4 * k, wmax, g);
+    for (int k = 0; k < 4; ++k) c[k] = codes4(v + 4 * k, g);
 }
 
 // Groups of 128: eight lanes hold a group in registers, sixteen values each, so a warp works on four neighbouring groups of
 // a row (1 KB in for 16-bit weights) and the scale's divisions and roundings are paid once per 512 weights. A block covers
 // 16 rows of four groups, so that scales [G, N] leave as whole sectors; all its loads are in flight before the first is used.
 // (32 rows with half of the loads ahead: 1.7 waves for 4096 x 4096. Alone, on weights not in L2, bf16 asymmetric / f16 symmetric:
-// 15.9 / 12.2 -> 13.7 / 10.1 us, 14336 x 4096 47.1 / 36.0 -> 40.8 / 31.3; all bytes at the copy rate 7.7 and 27.) Five blocks of
-// 48 registers per SM for 16-bit weights, for which the asymmetric forms spill ten bytes; fp32 ones need the registers (four blocks
-// 13.3 us, five 14.4). The steps from 32 rows to this (16 rows, loads ahead, two fp32 values per instruction, extremes in one word,
+// 15.9 / 12.2 -> 13.7 / 10.1 us, 14336 x 4096 47.1 / 36.0 -> 40.8 / 31.3; with quotients as above 10.0 / 9.1 and 31.2 / 29.4; all bytes at the
+// copy rate 7.7 and 27.) Five blocks of 48 registers per SM for 16-bit weights (four 10.2 / 9.7, six 10.6 / 10.1, 32 rows a block 10.5 / 9.6); fp32
+// ones need the registers (four blocks 12.8 us, five 14.4 before). The steps from 32 rows to this (16 rows, loads ahead, two fp32 values per instruction, extremes in one word,
 // zero point by reciprocal) were measured together only.
 // With a group per warp the kernel was bound by issue slots (25.2 us for 4096 x 4096 bf16).
 constexpr int QUANT_PASSES = 2;  // rows a warp works on
@@ -222,7 +237,7 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(
         }
         const GroupParams g = group_params<SYM>(lo, hi, scale_dtype);
         uint32_t c[4];
-        codes16(v, fmaxf(fabsf(lo), fabsf(hi)), g, c);
+        codes16(v, g, c);
         if (have && n0 + row < N) {
             uint32_t *dst = codes + (first + pass * 8 * K) / 4;
 #pragma unroll
@@ -278,7 +293,7 @@ __global__ void __launch_bounds__(256) quantize_group_kernel(const void *w, int6
     for (int i = threadIdx.x * 4; i < group; i += blockDim.x * 4) {
         float v[4];
         load4<DT>(w, base + i, v);
-        codes[(base + i) / 4] = codes4(v, fmaxf(fabsf(lo), fabsf(hi)), g);
+        codes[(base + i) / 4] = codes4(v, g);
     }
     if (threadIdx.x == 0) {
         scales[gi * N + n] = g.scale_bits;
