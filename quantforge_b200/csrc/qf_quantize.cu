@@ -162,7 +162,7 @@ __device__ __forceinline__ void codes16(const float (&v)[16], const GroupParams 
     for (int k = 0; k < 4; ++k) c[k] = codes4(v + 4 * k, g);
 }
 
-// Groups of 128: eight lanes hold a group in registers, sixteen values each, so a warp works on four neighbouring groups of
+// Groups of 128 (256, 512): eight (16, 32) lanes hold a group in registers, sixteen values each, so a warp works on four neighbouring groups of
 // a row (1 KB in for 16-bit weights) and the scale's divisions and roundings are paid once per 512 weights. A block covers
 // 16 rows of four groups, so that scales [G, N] leave as whole sectors; all its loads are in flight before the first is used.
 // (32 rows with half of the loads ahead: 1.7 waves for 4096 x 4096. Alone, on weights not in L2, bf16 asymmetric / f16 symmetric:
@@ -170,24 +170,26 @@ __device__ __forceinline__ void codes16(const float (&v)[16], const GroupParams 
 // copy rate 7.7 and 27.) Five blocks of 48 registers per SM for 16-bit weights (four 10.2 / 9.7, six 10.6 / 10.1, 32 rows a block 10.5 / 9.6); fp32
 // ones need the registers (four blocks 12.8 us, five 14.4 before). The steps from 32 rows to this (16 rows, loads ahead, two fp32 values per instruction, extremes in one word,
 // zero point by reciprocal) were measured together only.
-// With a group per warp the kernel was bound by issue slots (25.2 us for 4096 x 4096 bf16).
+// With a group per warp, four values a lane, the kernel was bound by issue slots (25.2 us for 4096 x 4096 bf16). Groups of 256 and 512 took 36.8
+// and 36.1 us as blocks of their own, 10.0 so.
 constexpr int QUANT_PASSES = 2;  // rows a warp works on
-template <int DT, bool SYM, bool TALL>
-__global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(const void *w, int64_t N, int64_t K, uint32_t *codes,
+template <int DT, bool SYM, bool TALL, int LANES>
+__global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize_warp_kernel(const void *w, int64_t N, int64_t K, uint32_t *codes,
                                                           uint16_t *scales, int scale_dtype, int8_t *zeros) {
     griddep_begin();
     constexpr int ROWS = 8 * QUANT_PASSES;
-    __shared__ uint16_t s_scale[4][ROWS];
-    __shared__ int8_t s_zero[4][ROWS];
+    constexpr int GROUPS = 32 / LANES;  // of a warp
+    __shared__ uint16_t s_scale[GROUPS][ROWS];
+    __shared__ int8_t s_zero[GROUPS][ROWS];
     constexpr int VEC = DT == QF_F32 ? 4 : 8;  // values of a 16-byte load
     constexpr int LOADS = 16 / VEC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int q = lane >> 3, t = lane & 7;  // group of the warp's four, lane of the group
-    const int64_t G = K >> 7;
-    const int64_t gi = (int64_t)blockIdx.x * 4 + q;
+    const int q = lane / LANES, t = lane % LANES;  // group of the warp's, lane of the group
+    const int64_t G = K / (16 * LANES);
+    const int64_t gi = (int64_t)blockIdx.x * GROUPS + q;
     const int64_t n0 = TALL ? ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * ROWS : (int64_t)blockIdx.y * ROWS;
     const bool have = gi < G;
-    const int64_t first = (n0 + warp) * K + gi * 128;  // of the row of pass 0; a pass is 8 rows
+    const int64_t first = (n0 + warp) * K + gi * (16 * LANES);  // of the row of pass 0; a pass is 8 rows
     uint4 u[QUANT_PASSES][LOADS];
 #pragma unroll
     for (int pass = 0; pass < QUANT_PASSES; ++pass)
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(
         for (int l = 0; l < LOADS; ++l) {
             u[pass][l] = make_uint4(0u, 0u, 0u, 0u);
             if (have && n0 + pass * 8 + warp < N)  // neighbouring lanes take neighbouring 16-byte pieces
-                u[pass][l] = reinterpret_cast<const uint4 *>(w)[(first + pass * 8 * K) / VEC + l * 8 + t];
+                u[pass][l] = reinterpret_cast<const uint4 *>(w)[(first + pass * 8 * K) / VEC + l * LANES + t];
         }
 #pragma unroll
     for (int pass = 0; pass < QUANT_PASSES; ++pass) {
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(
 #pragma unroll
             for (int k = 1; k < 16; ++k) lo = min_nan(lo, v[k]), hi = max_nan(hi, v[k]);
 #pragma unroll
-            for (int o = 4; o; o >>= 1) {
+            for (int o = LANES / 2; o; o >>= 1) {
                 lo = min_nan(lo, __shfl_xor_sync(0xffffffffu, lo, o));
                 hi = max_nan(hi, __shfl_xor_sync(0xffffffffu, hi, o));
             }
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(
             hi2 ^= 0x80008000u;
             uint32_t e = min2_nan<DT>(prmt(lo2, hi2, 0x5410u), prmt(lo2, hi2, 0x7632u));
 #pragma unroll
-            for (int o = 4; o; o >>= 1) e = min2_nan<DT>(e, __shfl_xor_sync(0xffffffffu, e, o));
+            for (int o = LANES / 2; o; o >>= 1) e = min2_nan<DT>(e, __shfl_xor_sync(0xffffffffu, e, o));
             lo = low_half<DT>(e);
             hi = -high_half<DT>(e);
         }
@@ -242,8 +244,8 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(
             uint32_t *dst = codes + (first + pass * 8 * K) / 4;
 #pragma unroll
             for (int l = 0; l < LOADS; ++l) {
-                if constexpr (VEC == 8) reinterpret_cast<uint2 *>(dst)[l * 8 + t] = make_uint2(c[2 * l], c[2 * l + 1]);
-                else dst[l * 8 + t] = c[l];
+                if constexpr (VEC == 8) reinterpret_cast<uint2 *>(dst)[l * LANES + t] = make_uint2(c[2 * l], c[2 * l + 1]);
+                else dst[l * LANES + t] = c[l];
             }
         }
         if (t == 0) {
@@ -253,17 +255,111 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize128_kernel(
     }
     __syncthreads();
     const int64_t n = n0 + lane;
-    const int64_t go = (int64_t)blockIdx.x * 4 + warp;
-    if (warp < 4 && lane < ROWS && go < G && n < N) {
+    const int64_t go = (int64_t)blockIdx.x * GROUPS + warp;
+    if (warp < GROUPS && lane < ROWS && go < G && n < N) {
         scales[go * N + n] = s_scale[warp][lane];
         if (!SYM) zeros[go * N + n] = s_zero[warp][lane];
     }
 }
 
-// Any group size that is a multiple of 4: a block per (row, group), two passes over the group (the second one reads it
-// from L1 or L2). Only blocks of 256 threads let the next kernel in early: the GPU takes one such signal a nanosecond, and there is
-// one per block, so that in smaller blocks they were all the time (4096 x 4096 bf16 in groups of 64: 270.8 us instead of 137.6,
-// of 256: 68.4 instead of 37.0, of 512: 36.8 instead of 36.3; in groups of 4096 22.7 with the signal, 22.9 without).
+// Larger groups, multiples of 16 values: a block per (row, group), sixteen values a thread in registers as above; what a block of the
+// largest kind cannot hold is read twice, the second time from L1 or L2. 4096 x 4096 bf16, four values a thread at a time in
+// two passes -> this: groups of 1024 38.7 -> 14.1 us, 2048 27.0 -> 14.2, 4096 19.3 -> 15.2; 1024 x 28672 in one group a row 45.5 -> 21.6.
+template <int DT, bool SYM, int THREADS>
+__global__ void __launch_bounds__(THREADS, DT == QF_F32 ? 1024 / THREADS : 1280 / THREADS)
+quantize_block_kernel(const void *w, int64_t N, int64_t K, int group, uint32_t *codes, uint16_t *scales, int scale_dtype, int8_t *zeros) {
+    if (THREADS >= 256) griddep_launch_dependents();  // (see quantize_group_kernel)
+    griddep_wait();
+    constexpr int VEC = DT == QF_F32 ? 4 : 8;  // values of a 16-byte load
+    constexpr int LOADS = 16 / VEC, TILE = THREADS * 16;
+    __shared__ float s_lo[THREADS / 32], s_hi[THREADS / 32];
+    const int64_t G = K / group;
+    const int64_t n = blockIdx.x / G, gi = blockIdx.x % G;
+    const int64_t base = n * K + gi * group;
+    const uint4 *src = reinterpret_cast<const uint4 *>(w) + base / VEC;
+    const int pieces = group / VEC;
+    uint4 u[LOADS];
+    auto load = [&](int first) {
+#pragma unroll
+        for (int l = 0; l < LOADS; ++l) {
+            const int i = first / VEC + l * THREADS + (int)threadIdx.x;
+            u[l] = i < pieces ? src[i] : src[0];  // (in place of what there is not, a value that is in the group anyway)
+        }
+    };
+    float lo = __int_as_float(0x7f800000), hi = -lo;
+    const int tiles = (group + TILE - 1) / TILE;
+    // the last tile first: the first one stays in registers
+    for (int tile = tiles - 1; tile >= 0; --tile) {
+        load(tile * TILE);
+        uint32_t lo2 = u[0].x, hi2 = u[0].x;
+#pragma unroll
+        for (int l = 0; l < LOADS; ++l) {
+            const uint32_t x[4] = {u[l].x, u[l].y, u[l].z, u[l].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if constexpr (DT == QF_F32) {
+                    lo = min_nan(lo, __uint_as_float(x[k]));
+                    hi = max_nan(hi, __uint_as_float(x[k]));
+                } else {
+                    lo2 = min2_nan<DT>(lo2, x[k]);
+                    hi2 = max2_nan<DT>(hi2, x[k]);
+                }
+            }
+        }
+        if constexpr (DT != QF_F32) {
+            lo = min_nan(lo, min_nan(low_half<DT>(lo2), high_half<DT>(lo2)));
+            hi = max_nan(hi, max_nan(low_half<DT>(hi2), high_half<DT>(hi2)));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        lo = min_nan(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max_nan(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (THREADS > 32) {
+        if ((threadIdx.x & 31) == 0) s_lo[threadIdx.x >> 5] = lo, s_hi[threadIdx.x >> 5] = hi;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < THREADS / 32; ++i) lo = min_nan(lo, s_lo[i]), hi = max_nan(hi, s_hi[i]);
+    }
+    const GroupParams g = group_params<SYM>(lo, hi, scale_dtype);
+    uint32_t *dst = codes + base / 4;
+#pragma unroll 1
+    for (int tile = 0; tile < tiles; ++tile) {
+        if (tile > 0) load(tile * TILE);
+        float v[16];
+#pragma unroll
+        for (int l = 0; l < LOADS; ++l) {
+            const uint32_t x[4] = {u[l].x, u[l].y, u[l].z, u[l].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if constexpr (DT == QF_F32) {
+                    v[l * 4 + k] = __uint_as_float(x[k]);
+                } else {
+                    v[l * 8 + 2 * k] = low_half<DT>(x[k]);
+                    v[l * 8 + 2 * k + 1] = high_half<DT>(x[k]);
+                }
+            }
+        }
+        uint32_t c[4];
+        codes16(v, g, c);
+#pragma unroll
+        for (int l = 0; l < LOADS; ++l) {
+            const int i = tile * TILE / VEC + l * THREADS + (int)threadIdx.x;
+            if (i >= pieces) continue;
+            if constexpr (VEC == 8) reinterpret_cast<uint2 *>(dst)[i] = make_uint2(c[2 * l], c[2 * l + 1]);
+            else dst[i] = c[l];
+        }
+    }
+    if (threadIdx.x == 0) {
+        scales[gi * N + n] = g.scale_bits;
+        if (!SYM) zeros[gi * N + n] = (int8_t)(int)g.zero;
+    }
+}
+
+// The other group sizes, multiples of 4: a block per (row, group), two passes over the group (the second one reads it from L1 or L2). Only
+// blocks of 256 threads let the next kernel in early: the GPU takes one such signal a nanosecond, and there is one per block, so that in
+// smaller blocks they were all the time (4096 x 4096 bf16 in groups of 64: 270.8 us instead of 137.6).
 template <int DT, bool SYM>
 __global__ void __launch_bounds__(256) quantize_group_kernel(const void *w, int64_t N, int64_t K, int group,
                                                              uint32_t *codes, uint16_t *scales,
@@ -305,13 +401,23 @@ template <int DT, bool SYM>
 static cudaError_t quantize_launch(const void *w, int64_t N, int64_t K, int group, uint32_t *codes, uint16_t *scales,
                                    int scale_dtype, int8_t *zeros, cudaStream_t s) {
     constexpr int ROWS = 8 * QUANT_PASSES;
-    if (group == 128) {
+    if (group == 128 || group == 256 || group == 512) {
         // Blocks of rows in y and, where there are more than 65535 of them, in z: 1.1 million rows of 128 297 us, a block per group
         // as below 572. (With z in the address everywhere, symmetric 4096 x 14336 took 39.3 us instead of 38.6.)
         const int64_t blocks = (N + ROWS - 1) / ROWS, z = (blocks + 65534) / 65535;
-        const dim3 grid((unsigned)((K / 128 + 3) / 4), (unsigned)((blocks + z - 1) / z), (unsigned)z);
-        auto *fn = z > 1 ? quantize128_kernel<DT, SYM, true> : quantize128_kernel<DT, SYM, false>;
+        const dim3 grid((unsigned)((K + 511) / 512), (unsigned)((blocks + z - 1) / z), (unsigned)z);
+        auto *fn = group == 128   ? (z > 1 ? quantize_warp_kernel<DT, SYM, true, 8> : quantize_warp_kernel<DT, SYM, false, 8>)
+                   : group == 256 ? (z > 1 ? quantize_warp_kernel<DT, SYM, true, 16> : quantize_warp_kernel<DT, SYM, false, 16>)
+                                  : (z > 1 ? quantize_warp_kernel<DT, SYM, true, 32> : quantize_warp_kernel<DT, SYM, false, 32>);
         return launch_kernel(fn, grid, dim3(256), 0, s, pdl_enabled(), w, N, K, codes, scales, scale_dtype, zeros);
+    }
+    if (group > 512 && group % 16 == 0 && group <= 1 << 24) {
+        const int fit = group <= 1024 ? 64 : group <= 2048 ? 128 : group <= 4096 ? 256 : 512;
+        auto *fn = fit == 64    ? quantize_block_kernel<DT, SYM, 64>
+                   : fit == 128 ? quantize_block_kernel<DT, SYM, 128>
+                   : fit == 256 ? quantize_block_kernel<DT, SYM, 256>
+                                : quantize_block_kernel<DT, SYM, 512>;
+        return launch_kernel(fn, dim3((unsigned)(N * (K / group))), dim3(fit), 0, s, pdl_enabled(), w, N, K, group, codes, scales, scale_dtype, zeros);
     }
     const int threads = group >= 1024 ? 256 : group >= 512 ? 128 : group >= 256 ? 64 : 32;
     return launch_kernel(quantize_group_kernel<DT, SYM>, dim3((unsigned)(N * (K / group))), dim3(threads), 0, s, pdl_enabled(), w, N, K,

@@ -19,7 +19,7 @@ def _same(w, group, symmetric, scale_dtype=None):
 
 @pytest.mark.parametrize("dtype,scale_dtype", [(torch.float16, None), (torch.bfloat16, None), (torch.float32, torch.bfloat16), (torch.float32, torch.float16)])
 @pytest.mark.parametrize("symmetric", [False, True])
-@pytest.mark.parametrize("group", [128, 64, 512])
+@pytest.mark.parametrize("group", [128, 64, 256, 512, 1024, 640])
 def test_quotients(dtype, scale_dtype, symmetric, group):
     gen = torch.Generator(device="cuda").manual_seed(group)
     rnd = lambda *shape: torch.randn(*shape, device="cuda", generator=gen)  # noqa: E731
@@ -36,3 +36,20 @@ def test_quotients(dtype, scale_dtype, symmetric, group):
     tiny[:, 0] = 7.0
     rows.append(tiny)
     _same(torch.cat(rows).to(dtype), group, symmetric, scale_dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("symmetric", [False, True])
+@pytest.mark.parametrize("N,K,group", [(3, 768, 256), (17, 1024, 512), (33, 512, 256), (5, 1040, 1040), (2, 4096, 1024), (3, 2064, 2064), (2, 4096, 4096),
+                                       (2, 8192, 4096), (3, 4112, 4112), (1, 8192, 8192), (2, 8208, 8208), (2, 28672, 28672), (70000, 512, 512), (1, 20, 20)])
+def test_large_groups(N, K, group, dtype, symmetric):
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    w = (torch.randn(N, K, device="cuda", generator=gen) * 0.05).to(dtype)
+    _same(w, group, symmetric)
+    if N < 100:  # extremes and NaN at the ends of what a thread, a tile and a group hold
+        for i, at in enumerate((0, group - 1, group // 2, min(group - 1, 15), min(group - 1, 4095), min(group - 1, 8191))):
+            v = w.clone()
+            v[i % N, at], v[i % N, (at + 7) % group] = 3.0, -2.0
+            _same(v, group, symmetric)
+            v[i % N, at] = float("nan")
+            _same(v, group, symmetric)
