@@ -21,7 +21,7 @@
 // sizes on other layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any
 // other order into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least
 // surprise). The pieces of a phase are dealt to the streams forwards and backwards in turn. Weights are requested as far ahead as the
-// ring of stages allows, across linears and phases; only the activations of a phase wait for the phase before it.
+// ring of stages allows, across linears and phases; only activations and results wait.
 //
 // A thread block has its SM to itself and runs two streams side by side (one stream's waits are the other's time to convert), each
 // with half of its threads, shared memory and TMEM. (One block per SM because a cooperative launch admits no more of a kernel that
@@ -29,8 +29,10 @@
 //   warps 0-7    two converter groups, alternating units: thread t owns weight row t of the unit, reads its 64 bytes of codes and
 //                its constants from the swizzled stage, converts and writes them to TMEM lane t (tcgen05.st).
 //   one warp     copies of weights: one TMA box per unit, a chunk of two row blocks of the blob as 64-byte lines.
-//   one warp     copies of activations (MMA B tiles, K-major, 128-byte swizzle), and the wait for the phase before.
+//   one warp     copies of activations (MMA B tiles, K-major, 128-byte swizzle); those that are another linear's results as soon as
+//                their row block is finished.
 //   one warp     one thread issues the MMAs of a unit once its weights and activations are there.
+//   one warp     waits for the phases that results may not overtake, and tells warps 12-15.
 //   warps 12-15  results: a row block's accumulators go from TMEM to Y, or to the workspace where others have chunks of it too.
 //
 // Row blocks whose K range is shared by several streams (its members): a member leaves its partial sums in a slot of the workspace
@@ -242,7 +244,7 @@ __device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, 
         // rows 0..7 of sixteen are gate rows, 8..15 the matching up rows: of a pair the gate lane does the first batch row, the up lane
         // the second
         const bool up_lane = n & 8;
-        const int cols = e.N >> 1, col = (n >> 4) * 8 + (n & 6);
+        const int cols = e.N >> 1, col = (n >> 4) * 8 + (n & 7);
         float gate[PAIRS], up[PAIRS];
 #pragma unroll
         for (int i = 0; i < PAIRS; ++i) {
@@ -252,15 +254,10 @@ __device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, 
         }
 #pragma unroll
         for (int i = 0; i < PAIRS; ++i) up[i] = gate[i] / (1.f + expf(-gate[i])) * up[i];
-        // neighbouring lanes hold neighbouring outputs of the same batch rows: the even one takes the first of two pairs
         const int m = m0 + (up_lane ? 1 : 0);
 #pragma unroll
-        for (int i = 0; i < PAIRS; i += 2) {
-            const float mine = odd && i + 1 < PAIRS ? up[i + 1 < PAIRS ? i + 1 : i] : up[i];
-            const float other = __shfl_xor_sync(0xffffffffu, odd || i + 1 >= PAIRS ? up[i] : up[i + 1 < PAIRS ? i + 1 : i], 1);
-            const int row = m + 2 * i + (odd ? 2 : 0);
-            if (row < M && (i + 1 < PAIRS || !odd)) stream_put(e, (int64_t)row * cols + col, odd ? other : mine, odd ? mine : other);
-        }
+        for (int i = 0; i < PAIRS; ++i)
+            if (m + 2 * i < M) store_out(e.Y, e.out_dtype, (int64_t)(m + 2 * i) * cols + col, up[i]);
         return;
     }
     const bool add = e.epilogue == QF_EPI_RESIDUAL_ADD;
@@ -286,12 +283,14 @@ __device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, 
 __device__ __forceinline__ unsigned slot_of(const StreamArgs &a, const Segment &g, int member) {
     return (unsigned)((member == 0 ? g.slot0 : g.base + member) * a.slot_words);
 }
-// Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of eight members are requested
-// at a time. Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us,
+// Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of WORDS members are requested
+// at a time (missing ones are the last member's again, so a linear of wide N, with two to four members a row block, takes four: together
+// with plain stores of SiLU * mul and eight rows at a time, 32 rows: 5120 x 27648 38.9 -> 35.3 us, 8192 x 57344 73.8 -> 69.9, SiLU * mul of
+// 4096 x 28672 32.6 -> 30.8; four for everybody: 8192 x 8192 22.1 -> 22.6). Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us,
 // then 1500 to 1528.)
+template <int WORDS>
 __device__ __forceinline__ bool stream_sum(const StreamArgs &a, const Segment &g, int pair, int row, float (&v)[2],
                                            volatile int *abort_flag) {
-    constexpr int WORDS = 8;
     v[0] = v[1] = 0.f;
     const unsigned at = (unsigned)(pair * 128 + row) * 2u;
 #pragma unroll 1
@@ -734,17 +733,22 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
                 if (g.members == 1 && !opens()) return false;
                 tc_fence_after();
                 if (g.members == 1) {
+                    // (eight rows at a time are no faster in a chain, and more code)
+                    constexpr int ROWS = CAP == 1 ? 8 : 4;
 #pragma unroll 1
-                    for (int m0 = 0; m0 < a.M; m0 += 4) {
-                        uint32_t r[4];
-                        tmem_ld4(lane_tmem + d * NB + m0, r);
+                    for (int m0 = 0; m0 < a.M; m0 += ROWS) {
+                        uint32_t r[ROWS];
+                        if constexpr (ROWS == 8) tmem_ld8(lane_tmem + d * NB + m0, r);
+                        else tmem_ld4(lane_tmem + d * NB + m0, r);
                         tmem_wait_ld();
                         if (!in) continue;
-                        const float v[4] = {__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3])};
-                        uint2 add[2];
+                        float v[ROWS];
+#pragma unroll
+                        for (int j = 0; j < ROWS; ++j) v[j] = __uint_as_float(r[j]);
+                        uint2 add[ROWS / 2];
                         const StreamOut at = stream_out(en, n, m0);
-                        if (en.epilogue == QF_EPI_RESIDUAL_ADD) stream_residual<2>(en, a.M, at, add);
-                        stream_emit<2>(en, a.M, n, m0, v, at, add);
+                        if (en.epilogue == QF_EPI_RESIDUAL_ADD) stream_residual<ROWS / 2>(en, a.M, at, add);
+                        stream_emit<ROWS / 2>(en, a.M, n, m0, v, at, add);
                     }
                 } else {
 #pragma unroll 1
@@ -779,7 +783,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
                         if (!open && __all_sync(0xffffffffu, *gates >= 2 * nth) && !opens()) return false;
                         const bool early = open;
                         if (early && adds) stream_residual<1>(en, a.M, at, add);
-                        ok = stream_sum(a, g, pair, row, v, abort_flag);
+                        ok = CAP == 1 && g.members <= 4 ? stream_sum<4>(a, g, pair, row, v, abort_flag) : stream_sum<8>(a, g, pair, row, v, abort_flag);
                         if (!ok) {
                             *abort_flag = 1;
                             return false;
