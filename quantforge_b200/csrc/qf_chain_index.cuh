@@ -20,6 +20,7 @@ struct StreamPhase {
     int active;      // streams that have work
     int wait[2];     // phases that are complete before this one writes a result (or -1)
     int slots_wait;  // the phase that, with wait[1], is complete before this one writes partial sums (or -1)
+    int awaited;     // whether a later phase waits for this one
 };
 // Units of stream `id` in a phase: how many, and *u0 the first.
 QF_HD int stream_range(const StreamPhase &ph, int id, int *u0) {

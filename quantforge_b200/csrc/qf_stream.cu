@@ -286,8 +286,8 @@ __device__ __forceinline__ unsigned slot_of(const StreamArgs &a, const Segment &
 // Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of WORDS members are requested
 // at a time (missing ones are the last member's again, so a linear of wide N, with two to four members a row block, takes four: together
 // with plain stores of SiLU * mul and eight rows at a time, 32 rows: 5120 x 27648 38.9 -> 35.3 us, 8192 x 57344 73.8 -> 69.9, SiLU * mul of
-// 4096 x 28672 32.6 -> 30.8; four for everybody: 8192 x 8192 22.1 -> 22.6). Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us,
-// then 1500 to 1528.)
+// 4096 x 28672 32.6 -> 30.8; four for everybody: 8192 x 8192 22.1 -> 22.6). Warp-uniform; false when a wait ran out. (Two pairs at a
+// time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us, then 1500 to 1528.)
 template <int WORDS>
 __device__ __forceinline__ bool stream_sum(const StreamArgs &a, const Segment &g, int pair, int row, float (&v)[2],
                                            volatile int *abort_flag) {
@@ -802,12 +802,14 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
                 // a phase that is complete says that those are that it waits for, also where this stream had no result to write
                 if (ok) opens();
                 __syncwarp();
-                if (lane == 0 && ok && stream_last_warp(&s_finished[half][nth & 3]))
+                if (t.ph[phase].awaited && lane == 0 && ok && stream_last_warp(&s_finished[half][nth & 3]))
                     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.done + phase) : "memory");
             }
         }
-        if (CAP > 1) {
-            // The last result warp of the launch leaves the counters as they were: behind everybody's last count and wait.
+        if (CAP > 1 && a.words > 0) {
+            // The last result warp of the launch leaves the counters as they were: behind everybody's last count and wait. (Where
+            // nothing waits for a phase it is not counted, and a launch without counts ends without this: a release behind stores takes
+            // 1 us. Two of 4096 x 4096 side by side at 9 rows 14.9 -> 13.8 us, four of 512 x 512 8.7 -> 7.3.)
             unsigned before = 0;
             if (lane == 0 && ok)
                 asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.done + kStreamMaxLinears) : "memory");
@@ -900,7 +902,7 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
     p.a.slot_words = (int)slot_words(d0.M);
     p.a.M = (int)d0.M;
     p.a.x_rows = (int)((d0.M + 7) / 8) * 8;
-    p.a.words = kStreamFlags;
+    p.a.words = 0;
     const void *x_of[StreamParams<CAP>::XCAP];
     int64_t x_k[StreamParams<CAP>::XCAP];
     int maps = 0, phases = 0, next = 0;
@@ -938,7 +940,7 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
     const int sms = std::min(ctx->sm_count, kSmCount);
     int grid = 1;
     if (CAP == 1) {
-        p.ph[phases++] = StreamPhase{0, 0, 0, 0, 0, 0, 0, 0, {-1, -1}};
+        p.ph[phases++] = StreamPhase{0, 0, 0, 0, 0, 0, 0, 0, {-1, -1}, -1, 0};
         const int st = enter(0);
         if (st != QF_OK) return st;
         StreamPhase &ph = p.ph[0];
@@ -954,7 +956,9 @@ static int stream_launch(qf_ctx *ctx, const StreamLinear *l, int count, void *ws
         std::vector<int> entry_of(count);
         for (const ChainPhase &c : plan.phases) {
             StreamPhase &ph = p.ph[phases++];
-            ph = StreamPhase{next, 0, 0, 0, c.streams, c.home, c.flip, 0, {c.wait[0], c.wait[1]}, c.slots_wait};
+            ph = StreamPhase{next, 0, 0, 0, c.streams, c.home, c.flip, 0, {c.wait[0], c.wait[1]}, c.slots_wait, 0};
+            for (int w : {c.wait[0], c.wait[1], c.slots_wait})
+                if (w >= 0) p.ph[w].awaited = 1, p.a.words = std::max(p.a.words, kStreamFlags);
             for (int k = c.first; k < c.first + c.count; ++k) {
                 const int st = enter(plan.order[k]);
                 if (st != QF_OK) return st;
