@@ -286,8 +286,10 @@ __device__ __forceinline__ unsigned slot_of(const StreamArgs &a, const Segment &
 // Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of WORDS members are requested
 // at a time (missing ones are the last member's again, so a linear of wide N, with two to four members a row block, takes four: together
 // with plain stores of SiLU * mul and eight rows at a time, 32 rows: 5120 x 27648 38.9 -> 35.3 us, 8192 x 57344 73.8 -> 69.9, SiLU * mul of
-// 4096 x 28672 32.6 -> 30.8; four for everybody: 8192 x 8192 22.1 -> 22.6). Warp-uniform; false when a wait ran out. (Two pairs at a
-// time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us, then 1500 to 1528.)
+// 4096 x 28672 32.6 -> 30.8; four for everybody: 8192 x 8192 22.1 -> 22.6). A chain always takes four, which is less code: the linears of 32
+// layers of 4096 / 14336 at 16 rows 1297 -> 1280 us, eight layers of seven 391 -> 371, at 32 rows 494 -> 465 (with both in the code, by members,
+// 1297 and 484). Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us,
+// then 1500 to 1528.)
 template <int WORDS>
 __device__ __forceinline__ bool stream_sum(const StreamArgs &a, const Segment &g, int pair, int row, float (&v)[2],
                                            volatile int *abort_flag) {
@@ -783,7 +785,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) stream_kernel(const __grid_cons
                         if (!open && __all_sync(0xffffffffu, *gates >= 2 * nth) && !opens()) return false;
                         const bool early = open;
                         if (early && adds) stream_residual<1>(en, a.M, at, add);
-                        ok = CAP == 1 && g.members <= 4 ? stream_sum<4>(a, g, pair, row, v, abort_flag) : stream_sum<8>(a, g, pair, row, v, abort_flag);
+                        ok = CAP > 1 || g.members <= 4 ? stream_sum<4>(a, g, pair, row, v, abort_flag) : stream_sum<8>(a, g, pair, row, v, abort_flag);
                         if (!ok) {
                             *abort_flag = 1;
                             return false;

@@ -62,3 +62,36 @@ def test_sources(M, wide, dtype):
         torch.cuda.synchronize()
         assert all(torch.equal(g, w) for g, w in zip(got, want))
     assert qf.device_status() == 0
+
+
+# Launches in which nothing waits for the only phase, nothing is counted and nothing cleared, between launches that count: each leaves the
+# counters as the next one needs them. Seven members a row block too, whose words are fetched in two goes.
+@pytest.mark.parametrize("M", [9, 16, 17, 32])
+def test_batches_without_waits_between_others(M):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+
+    def linear(N, K):
+        qw = torch.randint(-128, 128, (N, K // 2), dtype=torch.int8, device="cuda", generator=gen)
+        sc = (torch.rand(K // 128, N, device="cuda", generator=gen) * 0.003 + 0.0005).bfloat16()
+        return qf.prepack_gemv_slab(qw, sc, qf.pack_zeros_u4(torch.randint(0, 16, (K // 128, N), dtype=torch.int8, device="cuda",
+                                                                           generator=gen)))
+    x = torch.randn(M, 4096, device="cuda", generator=gen).bfloat16()
+    e = lambda n: torch.zeros(M, n, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+    first, second, third, wide = linear(4096, 4096), linear(4096, 4096), linear(1024, 4096), linear(512, 14336)
+    a, b, c, d, act = e(4096), e(4096), e(1024), e(512), torch.randn(M, 14336, device="cuda", generator=gen).bfloat16()
+    side = ops.LinearBatch([(x, first, a, qf.QF_EPI_NONE, None), (x, second, b, qf.QF_EPI_NONE, None), (x, third, c, qf.QF_EPI_NONE, None),
+                            (act, wide, d, qf.QF_EPI_NONE, None)])
+    row = ops.LinearBatch([(x, first, a, qf.QF_EPI_NONE, None), (a, second, b, qf.QF_EPI_NONE, None), (b, third, c, qf.QF_EPI_NONE, None),
+                           (act, wide, d, qf.QF_EPI_NONE, None)])
+    for batch in (side, row):
+        assert batch.launches() == 1
+    seen = {}
+    for batch in (side, side, row, side, row, row, side):
+        for y in (a, b, c, d):
+            y.zero_()
+        batch.run()
+        got = [y.clone() for y in (a, b, c, d)]
+        for u, v in zip(seen.setdefault(id(batch), got), got):
+            assert torch.equal(u, v)
+    assert torch.equal(seen[id(side)][0], seen[id(row)][0]) and torch.equal(seen[id(side)][3], seen[id(row)][3])
+    assert qf.device_status() == 0
