@@ -34,8 +34,10 @@ __device__ __forceinline__ void unpack_word(uint32_t w, uint32_t &o0, uint32_t &
     o1 = prmt(lo, hi, 0x7362u);
 }
 
-// 16 input bytes per step, four steps in flight per thread, one 32-byte store each (two of 16 bytes where the output is only
-// aligned to that: WIDE is false; 64 MB in 41.3 instead of 32.7 us, a byte per thread 57.2). The up to 15 bytes behind the last whole step are unpacked by the first threads of block 0.
+// 16 input bytes per step, four steps in flight per thread, one 32-byte store each. Where the output is only aligned to 16 bytes (WIDE is
+// false) the sectors lie across two threads: each stores its second half with the first half of the thread behind it (64 MB in 31.7 us; two
+// stores of 16 bytes a thread, half a sector each, 41.3 to 49.9; aligned 32.7, a byte per thread 57.2). The up to 15 bytes behind the last
+// whole step are unpacked by the first threads of block 0.
 // Four loads per thread before the first store, and whole-sector stores, are what the memory system needs: one load and
 // two 16-byte stores 32 bytes apart ran at 4.5 TB/s (28672 x 4096 bytes in 77.4 us).
 constexpr int UNPACK_STEPS = 4;
@@ -47,10 +49,10 @@ __global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *in, uint
     uint4 v[UNPACK_STEPS];
 #pragma unroll
     for (int j = 0; j < UNPACK_STEPS; ++j)
-        if (first + j * 256 < n_vec) v[j] = ld_stream16(in + (first + j * 256) * 16);
+        v[j] = first + j * 256 < n_vec ? ld_stream16(in + (first + j * 256) * 16) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int j = 0; j < UNPACK_STEPS; ++j) {
-        if (first + j * 256 >= n_vec) continue;
+        if (WIDE && first + j * 256 >= n_vec) continue;
         uint4 a, b;
         unpack_word(v[j].x, a.x, a.y);
         unpack_word(v[j].y, a.z, a.w);
@@ -60,8 +62,13 @@ __global__ void __launch_bounds__(256) unpack_vec_kernel(const uint8_t *in, uint
         if (WIDE) {
             st_stream32(dst, a, b);
         } else {
-            reinterpret_cast<uint4 *>(dst)[0] = a;
-            reinterpret_cast<uint4 *>(dst)[1] = b;
+            const int lane = threadIdx.x & 31;
+            const uint4 next = make_uint4(__shfl_down_sync(0xffffffffu, a.x, 1), __shfl_down_sync(0xffffffffu, a.y, 1),
+                                          __shfl_down_sync(0xffffffffu, a.z, 1), __shfl_down_sync(0xffffffffu, a.w, 1));
+            if (first + j * 256 >= n_vec) continue;
+            if (lane == 0) *reinterpret_cast<uint4 *>(dst) = a;
+            if (lane < 31 && first + j * 256 + 1 < n_vec) st_stream32(dst + 16, b, next);
+            else *reinterpret_cast<uint4 *>(dst + 16) = b;
         }
     }
     if (blockIdx.x == 0 && threadIdx.x < tail) {
