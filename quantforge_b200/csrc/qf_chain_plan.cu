@@ -221,20 +221,22 @@ int stream_chain_length(const StreamLinear *l, int count) {
 // `split` where partial sums are exchanged, and `round` for each further round of pieces.
 // Fitted to 64 batches at 9 to 32 rows on weights not in L2, graph replays; standard deviation 10 %. Where the estimate picks the slower
 // way it costs 7 % at most, and 10 % on 19 other batches (4 of 76 points), but for sixteen linears of 1024 x 1024 in a row at 9 rows.
-// Measured, one by one -> chain, at 9 / 16 / 24 / 32 rows; * marks what the estimate picks otherwise (N x K):
+// The fit is older than the present chains (results awaited by row blocks, phases that nobody waits for not counted, sums fetched by
+// fours), which are up to 25 % shorter than estimated; it stands, because the way that is taken decides about the order of the sums.
+// Measured, one by one -> chain, at 9 / 16 / 24 / 32 rows; * marks what the estimate picks otherwise, + present chains (N x K):
 //   one reads the other, 2 linears:  512 x 512       8.7 -> 14.0 / 9.2 -> 14.5 / 12.4 -> 17.7 / 13.0 -> 19.4
 //                                    1024 x 2816     12.9 -> 15.7 / 13.7 -> 17.2 / 19.2 -> 19.5 / 20.3 -> 22.3
 //                                    2048 x 5632     17.1 -> 17.3 / 18.5 -> 17.5* / 29.5 -> 20.3 / 31.9 -> 21.4
-//                                    4096 x 4096     17.2 -> 17.8* / 19.7 -> 18.7 / 29.8 -> 21.1 / 32.3 -> 21.6
+//                                    4096 x 4096     17.2 -> 17.3* / 19.7 -> 17.9 / 29.8 -> 20.9 / 32.3 -> 21.9 +
 //                                    256 x 18944     34.1 -> 17.7 / 34.6 -> 19.0 / 55.8 -> 20.6 / 58.2 -> 21.7
-//                       16 linears:  1024 x 1024     120 -> 97.3* / 123 -> 118* / 181 -> 147 / 186 -> 173
+//                       16 linears:  1024 x 1024     120 -> 97.3* / 123 -> 118* / 181 -> 133+ / 186 -> 154+
 //                                    1024 x 2816     101 -> 96.9* / 107 -> 113 / 168 -> 129 / 172 -> 149
 //   side by side, 2 linears:         256 x 256       6.1 -> 8.0 / 6.6 -> 8.8 / 8.5 -> 9.7 / 9.1 -> 10.4
 //                                    14336 x 1024    12.9 -> 16.4 / 14.6 -> 18.2 / 21.1 -> 22.4* / 23.6 -> 25.5*
-//                                    4096 x 4096     17.3 -> 14.7 / 19.8 -> 15.2 / 30.1 -> 16.8 / 32.4 -> 17.7
-//                 4 linears:         512 x 512       16.4 -> 9.0 / 16.9 -> 9.3 / 24.0 -> 10.7 / 25.2 -> 11.3
-//   one layer of seven:              512 / 1024      31.3 -> 24.5 / 32.9 -> 28.7 / 44.9 -> 31.7 / 47.1 -> 38.5
-//                                    4096 / 14336    83.6 -> 54.9 / 89.5 -> 58.8 / 131 -> 65.9 / 138 -> 71.4
+//                                    4096 x 4096     17.3 -> 13.9 / 19.8 -> 14.3 / 30.1 -> 16.2 / 32.4 -> 17.7 +
+//                 4 linears:         512 x 512       16.4 -> 7.5 / 16.9 -> 7.9 / 24.0 -> 8.7 / 25.2 -> 9.0 +
+//   one layer of seven:              512 / 1024      31.3 -> 22.9 / 32.9 -> 24.7 / 44.9 -> 27.9 / 47.1 -> 28.7 +
+//                                    4096 / 14336    83.6 -> 47.0 / 89.5 -> 49.6 / 131 -> 56.4 / 138 -> 61.2 +
 //   30 layers of four:               256 / 256       394 -> 431 / 414 -> 465 / 544 -> 564* / 581 -> 621*
 bool stream_chain_pays(const StreamLinear *l, int count) {
     struct Costs {

@@ -5,8 +5,8 @@
 // instruction) and live in TMEM only, the activations are B from shared memory. What the streaming GEMV kernel (mma.sync) spends
 // on fragments of X and on the MMAs themselves, which take issue slots and packed-half time from the conversion and grow with the
 // rows, is here one thread's work. Without memory, converters and MMAs alone take 283 cycles per 128 x 128 codes and SM; HBM delivers
-// those in 377; the kernel takes about 450, bound by the issue slots that the conversion and its hand-overs share. In a chain there are 5 to
-// 6 us from the last MMA of a step to the first of the next: partial sums, results, a release (1 us and more behind stores), counters, a
+// those in 377; the kernel takes about 450, bound by the issue slots that the conversion and its hand-overs share. In a chain there are 4 to
+// 5 us from the last MMA of a step to the first of the next: partial sums, results, a release (1 us and more behind stores), counters, a
 // copy of activations.
 //
 // Work split. Units of 128 rows x 128 codes. Of a single linear they are numbered row block major, K chunk minor, and stream i of G
@@ -16,8 +16,8 @@
 // goes to streams that have nothing to do in that step, or fills the time in which the others hand over (the linears of 32 layers at
 // 16 rows 1459 -> 1355 us). Only results wait for whole phases. Activations that are another linear's results are read row block by row
 // block as these are finished (a counter each), and partial sums are exchanged as soon as their slots are free (linears of 32 layers,
-// 4096 / 14336, with the code of the results made smaller: 16 rows 1372 -> 1285 us, 9 rows 1338 -> 1240; seven linears a layer 1760 -> 1570
-// at 16 rows, 1988 -> 1805 at 24). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same
+// 4096 / 14336, with the code of the results made smaller, sums fetched by fours and phases that nobody waits for not counted: 16 rows 1372 -> 1280
+// us, 9 rows 1338 -> 1207; eight layers of seven linears 437 -> 371 at 16 rows, 495 -> 421 at 24). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same
 // sizes on other layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any
 // other order into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least
 // surprise). The pieces of a phase are dealt to the streams forwards and backwards in turn. Weights are requested as far ahead as the

@@ -20,7 +20,7 @@ faster way, with the bits of the linears one by one.
 
 What a chain gains here is more than a decoder has of it: with attention left out, nothing reads q/k/v of the fused variant and o
 runs beside it (without epilogues down runs beside gate/up too). 32 layers of 4096 / 14336 with o behind q/k/v, one by one -> chain:
-1 row 1403 us, no chain; 16 rows 2045 -> 1592 us where this stack takes 1352.
+1 row 1403 us, no chain; 16 rows 2071 -> 1612 us where this stack takes 1262.
 """
 from __future__ import annotations
 
@@ -41,20 +41,22 @@ CHAIN_BATCH = 32
 
 def _chain_bytes(batch: int, fuse: bool) -> float:
     """Mean bytes of codes of a linear from which batches above SLAB_BATCH run as a chain. Measured, a step's time linear by linear
-    (interleaved weights) / as a chain, 1 to 16 layers, at 9 / 16 / 20 / 24 / 28 / 32 rows:
-      fused     1.5 MB (hidden 1024)    0.88-1.01 / 0.72-0.86 / 0.70-0.85 / 0.71-0.80 / 0.65-0.71 / 0.56-0.66
-                5.6 MB (2048)           1.00-1.07 / 1.00-1.03 / 0.94-0.97 / 0.91-0.95 / 0.86-0.90 / 0.83-0.90
-                12 MB (3072)            1.00-1.14 / 1.00-1.06 / 0.96-1.03 / 0.96-1.00 / 0.88-0.93 / 0.91-0.92
-                14 MB (1792, 18944)     1.00      / 0.99-1.00 / 0.90-0.93 / 0.90-0.96 / 0.84-0.88 / 0.84-0.92
-                22 MB (6912, 3584)      1.08-1.09 / 1.00-1.02 / 0.93-0.96 / 0.93-0.94 / 0.86-0.88 / 0.83-0.85
-                27 MB (4096, 14336)     1.00-1.17 / 1.00-1.15 / 0.98-1.07 / 0.94-1.09 / 0.97-1.04 / 0.97-1.03
-                34 MB (5120, 13824)     1.03-1.12 / 1.00-1.07 / 1.00-1.05 / 1.00-1.05 / 0.94-0.97 / 0.92-0.97
-                90 MB (7680, 25856)     1.00-1.05 / 1.00-1.04 / 0.98-1.00 / 0.98-1.01 / 0.97-0.98 / 0.95-0.96
-                107 MB (8192, 28672)    1.08-1.10 / 1.08-1.09 / 1.04-1.06 / 1.04-1.05 / 1.00-1.01 / 1.01-1.02
-      unfused   0.8 MB (1024)           1.12-1.29 / 1.05-1.16 / 1.00-1.12 / 1.00-1.06 / 0.87-0.96 / 0.84-0.89
-                1.8 MB (1536)           1.23-1.41 / 1.06-1.25 / 1.10-1.22 / 1.09-1.19 / 1.04-1.09 / 1.00-1.06
-                16 MB (4096, 14336)     1.13-1.26 / 1.03-1.15 / 1.03-1.12 / 1.00-1.07 / 0.97-1.01 / 0.95-1.00
-                61 MB (8192, 28672)     1.09-1.12 / 1.09-1.11 / 1.07-1.10 / 1.06-1.09 / 1.03-1.06 / 1.02-1.05"""
+    (interleaved weights) / as a chain, 2 to 8 layers, at 9 / 16 / 20 / 24 / 28 / 32 rows:
+      fused     1.5 MB (hidden 1024)    1.12 / 1.00 / 1.03 / 0.97 / 0.88 / 0.82
+                5.6 MB (2048)           1.20 / 1.15 / 1.13 / 1.10 / 1.04 / 1.01
+                12 MB (3072)            1.23 / 1.15 / 1.13 / 1.09 / 1.03 / 1.01
+                14 MB (1792, 18944)     1.11 / 1.09 / 1.04 / 1.02 / 0.99 / 0.97
+                22 MB (6912, 3584)      1.34 / 1.29 / 1.22 / 1.20 / 1.13 / 1.08
+                27 MB (4096, 14336)     1.20-1.28 / 1.17-1.22 / 1.10-1.15 / 1.11-1.14 / 1.09-1.11 / 1.07-1.08
+                34 MB (5120, 13824)     1.18 / 1.13 / 1.12 / 1.11 / 1.06 / 1.06
+                90 MB (7680, 25856)     1.20 / 1.05 / 1.00 / 1.05 / 1.00 / 0.97
+                107 MB (8192, 28672)    1.13 / 1.13 / 1.08 / 1.08 / 1.18 / 1.08
+      unfused   0.8 MB (1024)           1.38 / 1.20 / 1.21 / 1.15 / 1.05 / 0.98
+                2.5 MB (2048)           1.41 / 1.34 / 1.30 / 1.28 / 1.21 / 1.18
+                16 MB (4096, 14336)     1.44-1.48 / 1.36-1.37 / 1.26-1.29 / 1.21-1.24 / 1.17-1.19 / 1.12-1.14
+                61 MB (8192, 28672)     1.17 / 1.15 / 1.14 / 1.13 / 1.19 / 1.11
+    The lines were drawn when chains took 10 to 15 % longer (17 rows and more of small linears lost then, and of any size from 25 rows on).
+    They stand: which layout a stack has its weights in is part of what its callers see."""
     if not fuse:
         return 2e6
     return 5e6 if batch <= 16 else 24e6 if batch <= 24 else float("inf")
