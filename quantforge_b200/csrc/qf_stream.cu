@@ -16,12 +16,13 @@
 // goes to streams that have nothing to do in that step, or fills the time in which the others hand over (the linears of 32 layers at
 // 16 rows 1459 -> 1355 us). Only results wait for whole phases. Activations that are another linear's results are read row block by row
 // block as these are finished (a counter each), and partial sums are exchanged as soon as their slots are free (linears of 32 layers,
-// 4096 / 14336, with the code of the results made smaller, sums fetched by fours and phases that nobody waits for not counted: 16 rows 1372 -> 1280
-// us, 9 rows 1338 -> 1207; eight layers of seven linears 437 -> 371 at 16 rows, 495 -> 421 at 24). In a chain K is cut into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same
-// sizes on other layouts, so that each sum is made of the same partial sums in the same order: a deep stack of 16-bit layers turns any
-// other order into another rounding of everything behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least
-// surprise). The pieces of a phase are dealt to the streams forwards and backwards in turn. Weights are requested as far ahead as the
-// ring of stages allows, across linears and phases; only activations and results wait.
+// 4096 / 14336, with the code of the results made smaller, sums fetched by fours and phases that nobody waits for not counted: 16 rows
+// 1372 -> 1280 us, 9 rows 1338 -> 1207; eight layers of seven linears 437 -> 371 at 16 rows, 495 -> 421 at 24). In a chain K is cut
+// into pieces exactly as the tcgen05 kernel (qf_gemm_tcgen05.cu) cuts it for the same sizes on other layouts, so that each sum is made
+// of the same partial sums in the same order: a deep stack of 16-bit layers turns any other order into another rounding of everything
+// behind it (32 layers: hidden states 0.9 % apart, where the same bits are the least surprise). The pieces of a phase are dealt to the
+// streams forwards and backwards in turn. Weights are requested as far ahead as the ring of stages allows, across linears and phases;
+// only activations and results wait.
 //
 // A thread block has its SM to itself and runs two streams side by side (one stream's waits are the other's time to convert), each
 // with half of its threads, shared memory and TMEM. (One block per SM because a cooperative launch admits no more of a kernel that
@@ -283,13 +284,13 @@ __device__ __forceinline__ void stream_emit(const StreamEntry &e, int M, int n, 
 __device__ __forceinline__ unsigned slot_of(const StreamArgs &a, const Segment &g, int member) {
     return (unsigned)((member == 0 ? g.slot0 : g.base + member) * a.slot_words);
 }
-// Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of WORDS members are requested
-// at a time (missing ones are the last member's again, so a linear of wide N, with two to four members a row block, takes four: together
-// with plain stores of SiLU * mul and eight rows at a time, 32 rows: 5120 x 27648 38.9 -> 35.3 us, 8192 x 57344 73.8 -> 69.9, SiLU * mul of
-// 4096 x 28672 32.6 -> 30.8; four for everybody: 8192 x 8192 22.1 -> 22.6). A chain always takes four, which is less code: the linears of 32
-// layers of 4096 / 14336 at 16 rows 1297 -> 1280 us, eight layers of seven 391 -> 371, at 32 rows 494 -> 465 (with both in the code, by members,
-// 1297 and 484). Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9 to 16 rows 1417 to 1461 us,
-// then 1500 to 1528.)
+// Adds the members' shares of a pair of batch rows, in their order, and clears their words; the words of WORDS members are requested at
+// a time (missing ones are the last member's again, so a linear of wide N, with two to four members a row block, takes four: together
+// with plain stores of SiLU * mul and eight rows at a time, 32 rows: 5120 x 27648 38.9 -> 35.3 us, 8192 x 57344 73.8 -> 69.9, SiLU *
+// mul of 4096 x 28672 32.6 -> 30.8; four for everybody: 8192 x 8192 22.1 -> 22.6). A chain always takes four, which is less code: the
+// linears of 32 layers of 4096 / 14336 at 16 rows 1297 -> 1280 us, eight layers of seven 391 -> 371, at 32 rows 494 -> 465 (with both
+// in the code, by members, 1297 and 484). Warp-uniform; false when a wait ran out. (Two pairs at a time: the linears of 32 layers at 9
+// to 16 rows 1417 to 1461 us, then 1500 to 1528.)
 template <int WORDS>
 __device__ __forceinline__ bool stream_sum(const StreamArgs &a, const Segment &g, int pair, int row, float (&v)[2],
                                            volatile int *abort_flag) {
