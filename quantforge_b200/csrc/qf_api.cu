@@ -102,6 +102,9 @@ static bool stream_serves(const qf_linear_desc *d) {
 // 0.58, 2048x2064 1.06, 8192x528 1.18.
 static bool gemm_serves_ragged(const qf_linear_desc *d) {
     if (d->weight_layout != QF_LAYOUT_CANONICAL || d->epilogue != QF_EPI_NONE || d->M < 3) return false;
+    // A number of splits that the caller names is one of the GEMV kernel's, which runs them in shorter pieces where they are long (4 rows,
+    // 14336 x 1040 in one split: 12.9 us there, 39.6 here).
+    if (d->split_k != 0) return false;
     if (d->zero_mode == QF_ZERO_U4 && d->N % 32 != 0) return false;
     // Sums of a whole split in one accumulator are 2e-7 to 4e-7 (of the outputs' rms) further off than the GEMV kernel's two accumulators
     // of shorter splits: 16-bit results, rounded by 1e-4 and more, do not show it; 32-bit ones keep that kernel.
