@@ -91,6 +91,11 @@ static bool stream_serves(const qf_linear_desc *d) {
     return d->K >= 512 && mib >= (d->K >= 8192 ? 24 : d->K >= 6144 ? 33 : d->K >= 5120 ? 42 : 72);
 }
 
+// Whether the GEMV kernel can run through K: without a split, which needs a counter for each of its tiles of outputs, a block takes 32 chunks.
+static bool gemv_takes(const qf_linear_desc *d) {
+    return d->K <= 32 * 128 || (d->N + 63) / 64 * ((d->M + 7) / 8) <= kMaxCounters;
+}
+
 // Whether the tcgen05 kernel takes canonical weights of N % 128 != 0 rows, as the GEMV kernel can. Copies of scales and zeros are
 // multiples of 16 bytes, also those of what is left for the last tile of 128 rows. Measured, GEMV / tcgen05 kernel, times as fast:
 //   K x N          1024x4112  1024x6160  2048x2064  2048x3088  4096x1040  4096x3088  6144x2064  8192x4112  14336x2064  14336x14352  512x40976
@@ -105,6 +110,8 @@ static bool gemm_serves_ragged(const qf_linear_desc *d) {
     // A number of splits that the caller names is one of the GEMV kernel's, which runs them in shorter pieces where they are long (4 rows,
     // 14336 x 1040 in one split: 12.9 us there, 39.6 here).
     if (d->split_k != 0) return false;
+    // What the GEMV kernel refuses stays refused, 32-bit and 16-bit results alike.
+    if (!gemv_takes(d)) return false;
     if (d->zero_mode == QF_ZERO_U4 && d->N % 32 != 0) return false;
     // Sums of a whole split in one accumulator are 2e-7 to 4e-7 (of the outputs' rms) further off than the GEMV kernel's two accumulators
     // of shorter splits: 16-bit results, rounded by 1e-4 and more, do not show it; 32-bit ones keep that kernel.

@@ -24,3 +24,12 @@ def test_named_splits_are_those_of_the_gemv_kernel(M, K, N):
     assert _plan(M, K, N)[0] == QF_PATH_GEMM
     for split in (1, 2, 3, 8, 16, 100):
         assert _plan(M, K, N, split_k=split) == _plan(M, K, N, path=QF_PATH_GEMV, split_k=split)
+
+
+# the GEMV kernel's tiles of 64 columns x 8 rows: 449 x 37 and 38, 16385 x 1 (16384 have a counter)
+@pytest.mark.parametrize("M,K,N,refused", [(296, 8192, 28688, True), (288, 8192, 28688, False), (300, 4096, 28688, False), (8, 4224, 1048640 - 48, True),
+                                           (8, 4096, 1048640 - 48, False), (8, 4224, 1048640 - 64, False)])
+def test_what_the_gemv_kernel_refuses_stays_refused(M, K, N, refused):
+    for out_dtype in (_lib.QF_BF16, _lib.QF_F32):
+        for path in (QF_PATH_AUTO, QF_PATH_GEMV):
+            assert (_plan(M, K, N, path=path, out_dtype=out_dtype) == -2) == refused  # QF_ERR_UNSUPPORTED
