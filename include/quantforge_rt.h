@@ -175,7 +175,8 @@ int qf_dequant_w4(qf_ctx *ctx, const qf_linear_desc *desc, const void *qweight, 
  * python/quantforge/baseline.py:52-72 `gemv_int4_baseline`).
  * fp32 accumulation.  `workspace` must hold qf_w4a16_workspace_bytes(desc) bytes, be zero-filled
  * once before its first use, and not be shared by calls that overlap in time; the kernels leave
- * it ready for the next call.  It may be NULL when the size is 0.
+ * it ready for the next call.  It may be NULL when the size is 0.  (Canonical weights with N % 128 != 0 also run, on the GEMV kernel, with
+ * what the same descriptor asks for with QF_PATH_GEMV.)
  */
 size_t qf_w4a16_workspace_bytes(const qf_linear_desc *desc);
 int qf_w4a16_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, const void *qweight, const void *scales,

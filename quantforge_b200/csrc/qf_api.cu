@@ -346,6 +346,9 @@ static int check_linear_args(qf_ctx *ctx, const qf_linear_desc *d, const void *X
     return QF_OK;
 }
 
+// A plan that the GEMV kernel can step in for (gemm_serves_ragged).
+static bool ragged_gemm(const qf_linear_desc *d, const Plan &plan) { return plan.path == QF_PATH_GEMM && d->N % 128 != 0; }
+
 // Everything that a linear's launch relies on, and its plan. M == 0 needs no tensors. Without a context: all but the current device.
 static int check_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, const void *qweight, const void *scales,
                         const void *qzeros_or_null, const void *Y, const void *residual, const void *workspace,
@@ -362,7 +365,14 @@ static int check_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, 
         return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_RESIDUAL_ADD needs a 16-byte aligned residual tensor");
     if (desc->epilogue == QF_EPI_SILU_MUL && desc->N % 16 != 0)
         return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_SILU_MUL needs N (gate and up rows together) to be a multiple of 16");
-    const size_t need = plan->ws_partial_bytes + plan->ws_counter_bytes;
+    size_t need = plan->ws_partial_bytes + plan->ws_counter_bytes;
+    if (ragged_gemm(desc, *plan) && (!workspace || workspace_bytes < need)) {
+        // what the GEMV kernel can do with its own scratch (none, where it does not split) is its
+        qf_linear_desc d = *desc;
+        d.path = QF_PATH_GEMV;
+        if ((st = make_plan(&d, plan, &why)) != QF_OK) return fail(ctx, st, why);
+        need = plan->ws_partial_bytes + plan->ws_counter_bytes;
+    }
     if (need > 0) {
         if (!workspace || workspace_bytes < need)
             return fail(ctx, QF_ERR_WORKSPACE, "workspace smaller than qf_w4a16_workspace_bytes(desc)");
@@ -588,7 +598,7 @@ size_t qf_w4a16_workspace_bytes(const qf_linear_desc *desc) {
     Plan plan;
     if (make_plan(desc, &plan, nullptr) != QF_OK) return 0;
     size_t need = plan.ws_partial_bytes + plan.ws_counter_bytes;
-    if (plan.path == QF_PATH_GEMM && desc->N % 128 != 0) {  // an exchanging call takes the GEMV kernel
+    if (ragged_gemm(desc, plan)) {  // an exchanging call takes the GEMV kernel
         qf_linear_desc d = *desc;
         d.path = QF_PATH_GEMV;
         if (make_plan(&d, &plan, nullptr) == QF_OK) need = std::max(need, plan.ws_partial_bytes + plan.ws_counter_bytes);
