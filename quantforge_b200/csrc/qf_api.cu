@@ -366,7 +366,7 @@ static int check_linear(qf_ctx *ctx, const qf_linear_desc *desc, const void *X, 
     if (desc->epilogue == QF_EPI_SILU_MUL && desc->N % 16 != 0)
         return fail(ctx, QF_ERR_BAD_ARG, "QF_EPI_SILU_MUL needs N (gate and up rows together) to be a multiple of 16");
     size_t need = plan->ws_partial_bytes + plan->ws_counter_bytes;
-    if (ragged_gemm(desc, *plan) && (!workspace || workspace_bytes < need)) {
+    if (ragged_gemm(desc, *plan) && need > 0 && (!workspace || workspace_bytes < need)) {
         // what the GEMV kernel can do with its own scratch (none, where it does not split) is its
         qf_linear_desc d = *desc;
         d.path = QF_PATH_GEMV;

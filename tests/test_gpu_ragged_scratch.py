@@ -11,8 +11,8 @@ from quantforge_b200 import _lib, ops
 pytestmark = pytest.mark.gpu
 
 
-# splits of the GEMV kernel: 12 (through memory), 5 (on chip), none, none, 2
-@pytest.mark.parametrize("M,K,N", [(8, 6144, 1040), (16, 8192, 4112), (64, 4096, 4112), (200, 4096, 4112), (300, 8192, 1040)])
+# splits of the GEMV kernel: 12 (through memory), 5 (on chip), none, none, 2, none (as the tcgen05 kernel)
+@pytest.mark.parametrize("M,K,N", [(8, 6144, 1040), (16, 8192, 4112), (64, 4096, 4112), (200, 4096, 4112), (300, 8192, 1040), (300, 512, 28688)])
 def test_scratch_of_the_gemv_kernel(M, K, N):
     lib, dev = _lib.load(), torch.device("cuda", torch.cuda.current_device())
     gen = torch.Generator(device="cuda").manual_seed(K + N)
@@ -35,11 +35,12 @@ def test_scratch_of_the_gemv_kernel(M, K, N):
 
     auto, gemv = desc(_lib.QF_PATH_AUTO), desc(_lib.QF_PATH_GEMV)
     own, both = (int(lib.qf_w4a16_workspace_bytes(ctypes.byref(d))) for d in (gemv, auto))
-    assert own < both
+    assert own < both or both == 0
     st, want = call(gemv, own)
     assert st == 0
     st, y = call(auto, own)
-    assert st == 0 and torch.equal(y, want)
+    # where neither kernel splits there is no reason to leave the faster one, whose order of sums shows in some roundings
+    assert st == 0 and torch.equal(y, want) == (own < both)
     st, y = call(auto, both)
     # both round sums of at most 1e-4 of the outputs' rms apart to bf16
     e = 1e-4 * float(want.float().pow(2).mean().sqrt())
