@@ -96,15 +96,49 @@ static bool gemv_takes(const qf_linear_desc *d) {
     return d->K <= 32 * 128 || (d->N + 63) / 64 * ((d->M + 7) / 8) <= kMaxCounters;
 }
 
+// Millions of codes from which the tcgen05 kernel is the faster one on canonical weights of N % 128 != 0 rows; -1: never. Its blocks take a
+// tile of 128 rows and, up to 64 batch rows, an eighth of K at least; the GEMV kernel's take 64 rows, 8 batch rows and a piece of K that fills
+// the device four times over. So this one loses where there are few tiles of long K, and on small matrices what its start-up and its sums cost.
+// GEMV / tcgen05 kernel, times as fast, weights not in L2:
+//   3, 4 rows    K 1024: N 10256 0.84, 12304 1.02    1536: 7184 0.95, 8208 1.05    2048: 5136 0.95, 6160 1.04    3072: 3088 0.99, 4112 1.02
+//                4096: 2064 0.97, 3088 1.02, 4112 1.17    5120: 1552 0.94, 2064 1.01    6144: 1040 1.30    8192: 784 1.25
+//                12288: 528 to 3600 0.97 to 1.23    14336: 784 to 2576 0.89 to 1.02, 3088 1.00    18944 to 28672: up to 2064 0.73 to 1.04, 3088 1.26
+//   5 to 8       1024: 10256 0.84 to 0.86, 12304 1.11    1280: 8208 0.90, 10256 1.08    1536: 4112 0.93 to 0.99, 5136 1.00
+//                2048: 3600 0.89 to 0.96, 4112 1.05    2560 to 6144: 0.96 and more    24576, 28672: up to 1296 0.85 to 1.04 at 5, 0.91 to 1.19 at 8
+//   9 to 16      up to 512: 0.95 and more but 128 x 57360 0.88    640: up to 18448 0.76 to 0.94, 20496 1.62
+//                768: up to 8208 0.84 to 1.00, 12304 1.01, 18448 0.92    896: 7184, 8208 0.89 to 0.94, 10256 1.09
+//                1152 to 1408: 3088, 4112 0.94 to 1.07    all else 1.0 to 3.7
+//   17 to 64     128: 16400 0.80 to 0.85 up to 24    256: 8208 0.85 to 0.93 up to 40, 12304 0.95 and more    384, 512: 1.02 and more
+//                640: up to 12304 0.80 to 0.93 up to 24, to 8208 0.89 to 0.93 at 32, to 7184 0.84 at 40
+//                768, 896: up to 8208 0.87 to 1.09 up to 24, 3088 and 4112 0.75 to 0.91 to 64, 6160 1.12 from 32 on
+//                1024: 2064, 2576 0.78 to 0.88 up to 24, then 0.99 and more but 2064 0.90 to 0.95 at 33 to 40
+//                1152 to 1408: up to 3088 0.83 to 0.94 up to 24, to 2064 0.84 to 0.93 at 32, 1808 0.87 at 33 to 40    1536: 1552 0.95 and more
+//                28672: 80 and 112 0.82 to 0.97 from 33 on, 144 0.85 to 0.92 up to 56 and 1.24 at 64, 208 0.91 up to 40 and 1.28 from 48 on
+//   65 to 256    1024: 4112, 1536 and 1664: 3088 0.80 to 0.92 up to 72    2048: 2064 0.87 at 96 and 100
+//                14336: 400 0.85 to 0.92 from 96 to 160    20480: 208 0.62 to 0.91 up to 200, 272 0.68 to 0.90 up to 160, then 1.05 and more
+//                28672: 144 0.53 to 0.79, 208 0.60 to 0.78 up to 140, 272 0.73 to 0.97 up to 112, then 0.99 and more
+//   more         1.5 and more
+static double ragged_line(int64_t M, int64_t K, int64_t N) {
+    if (M <= 8) {
+        if (K < 1024 || (M <= 4 && K > 12288 && N < 3072) || (M <= 6 && K >= 24576 && N < 1536)) return -1;
+        if (M > 4) return K < 1536 ? 12 : K < 2560 ? 8 : 6;
+        return K < 1536 ? std::max<double>(12, 12288e-6 * K) : K < 2560 ? 12 : K < 6144 ? 10 : 6;
+    }
+    if (M <= 16) return K <= 512 || K >= 1024 ? 4 : K < 768 ? 12.5 : 9;
+    if (M <= 64) {
+        if (M > 32 && K > 16384 && N < (M > 56 ? 144 : M <= 40 && K >= 24576 ? 256 : 176)) return -1;
+        if (K <= 512 || K >= 1536) return K < 384 && M <= (K < 256 ? 24 : 40) ? 2.5 : 2;
+        if (K < 1024) return M <= 24 ? (K < 768 ? 9 : 7) : K >= 768 || M > 40 ? 4 : M <= 32 ? 6 : 5;
+        return M <= 24 ? (K < 1280 ? 4 : 4.5) : M <= 32 ? (K < 1152 ? 2 : 2.95) : M <= 40 ? 2.4 : 2;
+    }
+    if (M <= 256 && (K > 16384 ? N < 176 || (N < 384 && M * N * K < 930000000) : K > 8192 && N < 512 && M * N < 65536)) return -1;
+    if (M < 80 && K >= 1024 && K < 2048) return 5.2;
+    if (M > 80 && M <= 104 && K > 1536 && K < 2560) return 4.5;
+    return 4;
+}
+
 // Whether the tcgen05 kernel takes canonical weights of N % 128 != 0 rows, as the GEMV kernel can. Copies of scales and zeros are
-// multiples of 16 bytes, also those of what is left for the last tile of 128 rows. Measured, GEMV / tcgen05 kernel, times as fast:
-//   K x N          1024x4112  1024x6160  2048x2064  2048x3088  4096x1040  4096x3088  6144x2064  8192x4112  14336x2064  14336x14352  512x40976
-//   codes             4.2 M      6.3        4.2        6.3        4.3       12.6       12.7       33.7       29.6        206          21
-//   3 rows             0.87      1.04       0.87       1.04       0.91       1.21       1.28       1.11       0.93       1.31        0.73
-//   8 rows             0.87      1.13       0.88       1.10       0.95       1.26       1.52       1.29       1.10       2.26        0.76
-// 9 to 16 rows (two tiles of the GEMV kernel): 1024x2064 0.89, 2048x1040 0.88 to 1.06, 4096x528 0.98, 2048x2064 1.20, 8192x528 1.42, 512x11024 1.31,
-// 3968x5136 1.95, 28672x4112 3.7; 17 to 64 rows: 1024x1040 0.81 to 1.02, 1024x2064 1.04 to 1.44, 2048x2064 1.44 to 2.0; 200 rows: 2048x1040
-// 0.58, 2048x2064 1.06, 8192x528 1.18.
+// multiples of 16 bytes, also those of what is left for the last tile of 128 rows.
 static bool gemm_serves_ragged(const qf_linear_desc *d) {
     if (d->weight_layout != QF_LAYOUT_CANONICAL || d->epilogue != QF_EPI_NONE || d->M < 3) return false;
     // A number of splits that the caller names is one of the GEMV kernel's, which runs them in shorter pieces where they are long (4 rows,
@@ -116,9 +150,8 @@ static bool gemm_serves_ragged(const qf_linear_desc *d) {
     // Sums of a whole split in one accumulator are 2e-7 to 4e-7 (of the outputs' rms) further off than the GEMV kernel's two accumulators
     // of shorter splits: 16-bit results, rounded by 1e-4 and more, do not show it; 32-bit ones keep that kernel.
     if (d->out_dtype == QF_F32) return false;
-    const int64_t codes = d->K * d->N;
-    if (d->M <= 8) return codes >= 6000000 && d->K >= 1024;
-    return codes >= (d->M <= 16 || d->M > 64 ? 4000000 : 2000000);
+    const double line = ragged_line(d->M, d->K, d->N);
+    return line >= 0 && d->K * d->N >= 1e6 * line;
 }
 
 int make_plan(const qf_linear_desc *d, Plan *p, std::string *why) {

@@ -1,5 +1,7 @@
 """Canonical weights whose rows are no multiple of 128, through the tcgen05 kernel: the last tile is cut short. Against float64 products
-of the dequantised weights, at every length of that tile, on both sides of the rule that picks the kernel."""
+of the dequantised weights, at every length of that tile. (tests/test_ragged_plan.py has the rule that picks the kernel.)"""
+import ctypes
+
 import pytest
 import torch
 
@@ -19,13 +21,20 @@ def _inputs(M, K, N, zeros, group, dtype):
     return qw, sc, zr, torch.randn(M, K, device="cuda", generator=gen).to(dtype)
 
 
-# the last tile has 16, 32, 64, 80, 96, 112 rows; one to eight splits on chip, splits through memory (65 rows and more), none
+# the last tile has 16, 32, 48, 64, 80, 96, 112 rows, and is the only one at N = 112; one to eight splits on chip, splits through memory (65 rows
+# and more), none
 @pytest.mark.parametrize("M,K,N,zeros,group,dtype", [
-    (3, 3968, 5136, "i8", 3968, torch.float16), (8, 8192, 1040, "i8", 128, torch.bfloat16), (5, 1024, 6176, "u4", 256, torch.float16),
+    (3, 3968, 5136, "i8", 3968, torch.float16), (8, 8192, 1040, "i8", 128, torch.bfloat16), (5, 4096, 3104, "u4", 256, torch.float16),
     (16, 8192, 544, "u4", 128, torch.bfloat16), (17, 2048, 2128, "const", 2048, torch.float16), (33, 4096, 1120, "u4", 128, torch.bfloat16),
     (64, 2048, 20144, "i8", 128, torch.bfloat16), (100, 8192, 624, "const", 512, torch.float16), (200, 4096, 1136, "i8", 128, torch.bfloat16),
-    (777, 1024, 4176, "const", 128, torch.float16), (300, 512, 28688, "i8", 512, torch.bfloat16)])
+    (777, 1024, 4176, "const", 128, torch.float16), (300, 512, 28688, "i8", 512, torch.bfloat16),
+    (24, 4096, 1088, "u4", 128, torch.float16), (128, 8192, 704, "u4", 128, torch.bfloat16), (32, 28672, 112, "i8", 128, torch.bfloat16)])
 def test_last_tile(M, K, N, zeros, group, dtype):
+    zero_mode = {"u4": _lib.QF_ZERO_U4, "i8": _lib.QF_ZERO_I8, "const": _lib.QF_ZERO_CONST}[zeros]
+    half = _lib.QF_F16 if dtype == torch.float16 else _lib.QF_BF16
+    d = _lib.LinearDesc(M=M, N=N, K=K, group_size=group, act_dtype=half, out_dtype=half, zero_mode=zero_mode, zero_const=8)
+    planned = ctypes.c_int32()
+    assert _lib.load().qf_w4a16_plan(ctypes.byref(d), ctypes.byref(planned), None) == 0 and planned.value == QF_PATH_GEMM
     qw, sc, zr, x = _inputs(M, K, N, zeros, group, dtype)
     ref = x.double() @ qf.dequant_w4(qw, sc, zr, group_size=group).double().t()
     rms = float(ref.pow(2).mean().sqrt())

@@ -19,7 +19,7 @@ def _plan(*args, **kw):
     return st if st != 0 else (path.value, split.value)
 
 
-@pytest.mark.parametrize("M,K,N", [(4, 14336, 1040), (16, 4096, 4112), (64, 28672, 4112), (200, 14336, 1040), (777, 4096, 4176)])
+@pytest.mark.parametrize("M,K,N", [(4, 8192, 4112), (16, 4096, 4112), (64, 28672, 4112), (200, 14336, 1040), (777, 4096, 4176)])
 def test_named_splits_are_those_of_the_gemv_kernel(M, K, N):
     assert _plan(M, K, N)[0] == QF_PATH_GEMM
     for split in (1, 2, 3, 8, 16, 100):
@@ -33,3 +33,41 @@ def test_what_the_gemv_kernel_refuses_stays_refused(M, K, N, refused):
     for out_dtype in (_lib.QF_BF16, _lib.QF_F32):
         for path in (QF_PATH_AUTO, QF_PATH_GEMV):
             assert (_plan(M, K, N, path=path, out_dtype=out_dtype) == -2) == refused  # QF_ERR_UNSUPPORTED
+
+
+def _gemm(M, K, N, **kw):
+    return _plan(M, K, N, **kw)[0] == QF_PATH_GEMM
+
+
+# on either side of each line, by rows of activations: (rows, K, largest N of the GEMV kernel, smallest of the tcgen05 kernel)
+@pytest.mark.parametrize("rows,K,gemv,gemm", [
+    ((3, 4), 896, 40976, None), ((3, 4), 1024, 12272, 12304), ((3, 4), 1408, 12272, 12304), ((3, 4), 1536, 7792, 7824), ((3, 4), 2432, 4912, 4944),
+    ((3, 4), 2560, 3888, 3920), ((3, 4), 4096, 2416, 2448), ((3, 4), 6016, 1648, 1680), ((3, 4), 6144, 976, 1008), ((3, 4), 12288, 464, 496),
+    ((3, 4), 12416, 3056, 3088), ((3, 4), 28672, 3056, 3088),
+    ((5, 6, 7, 8), 896, 40976, None), ((5, 6, 7, 8), 1024, 11696, 11728), ((5, 6, 7, 8), 1536, 5200, 5232), ((5, 6, 7, 8), 2560, 2320, 2352),
+    ((5, 6, 7, 8), 14336, 400, 432), ((5, 6), 24576, 1520, 1552), ((7, 8), 24576, 240, 272),
+    ((9, 12, 16), 512, 7792, 7824), ((9, 16), 640, 19504, 19536), ((9, 16), 896, 10032, 10064), ((9, 16), 1024, 3888, 3920), ((9, 12, 16), 4096, 976, 992), ((9, 16), 28672, 112, 144),
+    ((17, 24), 512, 3888, 3920), ((17, 24), 128, 19504, 19536), ((25, 40), 128, 15600, 15632), ((17, 40), 256, 9744, 9776), ((41, 64), 256, 7792, 7824), ((17, 24), 640, 14048, 14096), ((17, 24), 1024, 3888, 3920), ((17, 24), 1408, 3184, 3216), ((17, 24), 896, 7792, 7824), ((17, 24, 32, 40, 64), 1536, 1296, 1328),
+    ((25, 32), 896, 4432, 4496), ((25, 32), 640, 9360, 9392), ((33, 40), 640, 7792, 7824), ((41, 64), 640, 6224, 6256), ((25, 32), 1024, 1936, 1968), ((25, 32), 1280, 2288, 2320), ((33, 40), 1024, 2320, 2352), ((41, 64), 1024, 1936, 1968),
+    ((17, 32), 28672, 48, 80), ((33, 40), 28672, 240, 272), ((33, 40), 20480, 144, 176), ((41, 56), 28672, 144, 176), ((57, 64), 28672, 112, 144),
+    ((65, 79), 1024, 5072, 5104), ((80, 128), 1024, 3888, 3920), ((65, 79), 2048, 1936, 1968), ((81, 104), 2048, 2192, 2224), ((105, 256), 2048, 1936, 1968),
+    ((96, 128), 14336, 496, 528), ((160,), 14336, 400, 432), ((65, 256), 28672, 144, None), ((112,), 28672, 272, 304), ((140,), 28672, 208, 240),
+    ((257, 777), 28672, 112, 144), ((257, 777), 4096, 976, 992), ((64,), 8192, 240, 272), ((65,), 8192, 480, 496),
+])
+def test_lines(rows, K, gemv, gemm):
+    for M in rows:
+        assert not _gemm(M, K, gemv)
+        for N in (gemm, gemm + 16, gemm + 4096 + 16) if gemm else ():
+            assert N % 128 == 0 or _gemm(M, K, N), (M, N)
+        # one or two rows, and results whose sums are not rounded: the other kernel
+        for N in (gemv, gemm or gemv):
+            assert not _gemm(1, K, N) and not _gemm(2, K, N) and not _gemm(M, K, N, out_dtype=_lib.QF_F32)
+
+
+@pytest.mark.parametrize("M", [3, 8, 16, 64, 200])
+def test_packed_zeros_come_in_multiples_of_sixteen_bytes(M):
+    # four bits a zero: 16 bytes are 32 columns, so what is left for the last tile is a multiple of that (or there are no zeros in memory)
+    for N in range(5136, 5136 + 128, 16):
+        if N % 128:
+            assert _gemm(M, 4096, N, zero_mode=_lib.QF_ZERO_U4) == (N % 32 == 0)
+            assert _gemm(M, 4096, N) and _gemm(M, 4096, N, zero_mode=_lib.QF_ZERO_CONST)
