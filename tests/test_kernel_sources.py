@@ -30,3 +30,12 @@ def test_what_one_lane_acquires_is_passed_on(path):
     for poll in re.finditer(r"lane\s*!=\s*0\s*\|\|\s*\w*acquire\w*\s*\(", code):
         fence = code.find("fence.proxy.async", poll.end())
         assert fence < 0 or "__syncwarp()" in code[poll.end():fence]
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_warps_are_together_at_aligned_cluster_barriers(path):
+    """The aligned forms are undefined for a warp whose threads are apart, as they may be behind any condition: each stands in a wrapper
+    that brings them together first."""
+    for asm in re.finditer(r'asm volatile\(\s*"barrier\.cluster\.[^"]*\.aligned', _code(path)):
+        body = _code(path)[:asm.start()].rpartition("{")[2]
+        assert "__syncwarp();" in body, body
