@@ -519,6 +519,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
             for (int c8 = 0; c8 < cols_per_wg >> 3; ++c8) {
                 const int col = wg * cols_per_wg + c8 * 8;
                 uint32_t r[8];
+                if constexpr (RAGGED) __syncwarp();  // the last tile's stores may be half a warp's
                 tmem_ld8(lane_taddr + col, r);
                 tmem_wait_ld();
                 if (to_partial) {

@@ -39,3 +39,11 @@ def test_warps_are_together_at_aligned_cluster_barriers(path):
     for asm in re.finditer(r'asm volatile\(\s*"barrier\.cluster\.[^"]*\.aligned', _code(path)):
         body = _code(path)[:asm.start()].rpartition("{")[2]
         assert "__syncwarp();" in body, body
+
+
+def test_warps_are_together_at_loads_of_accumulators():
+    """Where a warp's share of the columns may be cut short, its partial sums are stored under a condition that splits the warp, and the
+    next load of accumulators is a whole warp's."""
+    code = _code(os.path.join(CSRC, "qf_gemm_tcgen05.cu"))
+    loop = code[code.index("for (int c8 = 0;"):code.index("__stcg(part")]
+    assert "n < p.N" in loop and loop.index("if constexpr (RAGGED) __syncwarp();") < loop.index("tmem_ld8")
