@@ -265,8 +265,10 @@ __global__ void __launch_bounds__(256, DT == QF_F32 ? 4 : 5) quantize_warp_kerne
 // Larger groups, multiples of 16 values: a block per (row, group), sixteen values a thread in registers as above; what a block of the
 // largest kind cannot hold is read twice, the second time from L1 or L2. 4096 x 4096 bf16, four values a thread at a time in
 // two passes -> this: groups of 1024 38.7 -> 14.1 us, 2048 27.0 -> 14.2, 4096 19.3 -> 15.2; 1024 x 28672 in one group a row 45.5 -> 21.6.
+// Eight sizes of blocks, because threads without values cost nearly what the others do: with 64, 128, 256 and 512 alone rows of 4112 to 6400 and of 8208
+// took as long as those of 8192, longer than in two passes (2048 x 5120 f16 17.7 us, so 10.1, in two passes 13.1; 1024 x 8208 fp32 15.9, 12.0 and 12.8).
 template <int DT, bool SYM, int THREADS>
-__global__ void __launch_bounds__(THREADS, DT == QF_F32 ? 1024 / THREADS : 1280 / THREADS)
+__global__ void __launch_bounds__(THREADS, DT == QF_F32 ? (1024 + THREADS / 2) / THREADS : THREADS == 448 ? 3 : 1280 / THREADS)
 quantize_block_kernel(const void *w, int64_t N, int64_t K, int group, uint32_t *codes, uint16_t *scales, int scale_dtype, int8_t *zeros) {
     if (THREADS >= 256) griddep_launch_dependents();  // (see quantize_group_kernel)
     griddep_wait();
@@ -412,12 +414,18 @@ static cudaError_t quantize_launch(const void *w, int64_t N, int64_t K, int grou
         return launch_kernel(fn, grid, dim3(256), 0, s, pdl_enabled(), w, N, K, codes, scales, scale_dtype, zeros);
     }
     if (group > 512 && group % 16 == 0 && group <= 1 << 24) {
-        const int fit = group <= 1024 ? 64 : group <= 2048 ? 128 : group <= 4096 ? 256 : 512;
-        auto *fn = fit == 64    ? quantize_block_kernel<DT, SYM, 64>
-                   : fit == 128 ? quantize_block_kernel<DT, SYM, 128>
-                   : fit == 256 ? quantize_block_kernel<DT, SYM, 256>
-                                : quantize_block_kernel<DT, SYM, 512>;
-        return launch_kernel(fn, dim3((unsigned)(N * (K / group))), dim3(fit), 0, s, pdl_enabled(), w, N, K, group, codes, scales, scale_dtype, zeros);
+        // the fewest threads whose tiles hold the group (448 in up to two tiles: of four, 512 x 28672 f16 13.3 us instead of 12.4)
+        const int tiles = (group + 8191) / 8192, need = (group + 16 * tiles - 1) / (16 * tiles);
+        const int threads = need <= 64 ? 64 : need <= 128 ? 128 : need <= 192 ? 192 : need <= 256 ? 256 : need <= 320 ? 320 : need <= 384 ? 384 : need <= 448 && tiles <= 2 ? 448 : 512;
+        auto *fn = threads == 64    ? quantize_block_kernel<DT, SYM, 64>
+                   : threads == 128 ? quantize_block_kernel<DT, SYM, 128>
+                   : threads == 192 ? quantize_block_kernel<DT, SYM, 192>
+                   : threads == 256 ? quantize_block_kernel<DT, SYM, 256>
+                   : threads == 320 ? quantize_block_kernel<DT, SYM, 320>
+                   : threads == 384 ? quantize_block_kernel<DT, SYM, 384>
+                   : threads == 448 ? quantize_block_kernel<DT, SYM, 448>
+                                    : quantize_block_kernel<DT, SYM, 512>;
+        return launch_kernel(fn, dim3((unsigned)(N * (K / group))), dim3(threads), 0, s, pdl_enabled(), w, N, K, group, codes, scales, scale_dtype, zeros);
     }
     const int threads = group >= 1024 ? 256 : group >= 512 ? 128 : group >= 256 ? 64 : 32;
     return launch_kernel(quantize_group_kernel<DT, SYM>, dim3((unsigned)(N * (K / group))), dim3(threads), 0, s, pdl_enabled(), w, N, K,
