@@ -297,14 +297,21 @@ int launch_repack_kn(qf_ctx *ctx, const void *w_kn, int packed_along_n, int64_t 
 }
 
 // A block converts 16 rows x 512 codes: a warp covers 512 codes of a row, a thread two neighbouring words of it (8 bytes
-// in, one 32-byte store out), in two rows, both loads in flight. The words of a thread lie in one quantisation group, so
+// in, one 32-byte store out), in two rows (four where those are short), all loads in flight. The words of a thread lie in one quantisation group, so
 // there is one scale and one zero per row; neighbouring rows' scales share sectors, which the block's rows find in L1.
 // One word per thread with a 64-bit division to find its row ran at 3.2 TB/s (14336 x 4096 bf16 in 45.6 us).
 // Grid: blocks of columns in x, so that those that run together write whole rows, blocks of rows in y and, where there are more than 65535 of
 // them, in z. (Blocks of 32 rows, one below the other: 14336 x 4096 bf16 25.1 us instead of 23.9, 28672 x 8192 95.1 instead of 88.4, all bytes at
 // the copy rate 22.6 and 90; 32 rows in the present order 24.3 and 88.9, 64 rows 27.6 and 97.3.)
-constexpr int DEQUANT_ROWS = 2;
-template <bool BF16, int ZMODE, bool WIDE>
+// Rows of one or two groups leave most of a block's threads idle, and many of them are bound by the blocks' starts and ends: they go 32 to
+// a block, four to a thread (16 -> 32 rows a block, f16: 65536 x 128, constant zero 8.01 -> 6.92 us, 262144 x 256 33.3 -> 30.7, 262144 x 128 with
+// packed zeros 32.0 -> 29.6; but 4096 x 128 1.89 -> 2.19, 262144 x 256 with packed zeros 34.9 -> 36.8, 32768 x 384 5.63 -> 6.04, and with 8-bit zeros
+// 524288 x 128 62.0 -> 64.6).
+static int dequant_rows(int zmode, int64_t N, int64_t K) {
+    if (zmode == QF_ZERO_CONST) return K <= 256 && N >= 32768 ? 4 : 2;
+    return zmode == QF_ZERO_U4 && K <= 128 && N >= 65536 ? 4 : 2;
+}
+template <bool BF16, int ZMODE, bool WIDE, int ROWS>
 __global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *qw,
                                                       const uint16_t *scales,
                                                       const void *zeros, int zero_const,
@@ -313,20 +320,20 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *qw,
     griddep_begin();
     const int64_t j = (int64_t)blockIdx.x * 64 + (threadIdx.x & 31) * 2;
     if (j >= words_per_row) return;
-    const int64_t n0 = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * (8 * DEQUANT_ROWS) + (threadIdx.x >> 5);
+    const int64_t n0 = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * (8 * ROWS) + (threadIdx.x >> 5);
     const int64_t gi = (int)j / group_words;
-    uint2 w[DEQUANT_ROWS];
-    ZeroScale<BF16> zs[DEQUANT_ROWS];
+    uint2 w[ROWS];
+    ZeroScale<BF16> zs[ROWS];
 #pragma unroll
-    for (int r = 0; r < DEQUANT_ROWS; ++r)
+    for (int r = 0; r < ROWS; ++r)
         if (n0 + 8 * r < N) w[r] = ld_stream8(qw + (n0 + 8 * r) * words_per_row + j);
 #pragma unroll
-    for (int r = 0; r < DEQUANT_ROWS; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const int64_t n = n0 + 8 * r;
         if (n < N) zs[r].set(load_zero<ZMODE>(zeros, zero_const, gi, n, N), scales[gi * N + n]);
     }
 #pragma unroll
-    for (int r = 0; r < DEQUANT_ROWS; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const int64_t n = n0 + 8 * r;
         if (n >= N) continue;
         uint4 o[2];
@@ -348,12 +355,12 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *qw,
     }
 }
 
-template <bool BF16, bool WIDE>
+template <bool BF16, bool WIDE, int ROWS>
 static cudaError_t dequant_dispatch(int zmode, dim3 grid, cudaStream_t s, const uint32_t *qw, const uint16_t *sc, const void *z,
                                     int zc, uint4 *out, int64_t N, int words_per_row, int group_words) {
-    auto *fn = zmode == QF_ZERO_CONST ? dequant_kernel<BF16, QF_ZERO_CONST, WIDE>
-               : zmode == QF_ZERO_U4  ? dequant_kernel<BF16, QF_ZERO_U4, WIDE>
-                                      : dequant_kernel<BF16, QF_ZERO_I8, WIDE>;
+    auto *fn = zmode == QF_ZERO_CONST ? dequant_kernel<BF16, QF_ZERO_CONST, WIDE, ROWS>
+               : zmode == QF_ZERO_U4  ? dequant_kernel<BF16, QF_ZERO_U4, WIDE, ROWS>
+                                      : dequant_kernel<BF16, QF_ZERO_I8, WIDE, ROWS>;
     return launch_kernel(fn, grid, dim3(256), 0, s, pdl_enabled(), qw, sc, z, zc, out, N, words_per_row, group_words);
 }
 
@@ -362,11 +369,15 @@ int launch_dequant(qf_ctx *ctx, const qf_linear_desc *d, const void *qw, const v
     if (d->N == 0) return QF_OK;
     const int64_t words = d->K / 8;
     const int64_t cols = (words + 63) / 64;
-    const int64_t rows = (d->N + 8 * DEQUANT_ROWS - 1) / (8 * DEQUANT_ROWS), planes = (rows + 65534) / 65535;
+    const int per = dequant_rows(d->zero_mode, d->N, d->K);
+    const int64_t rows = (d->N + 8 * per - 1) / (8 * per), planes = (rows + 65534) / 65535;
     const dim3 grid((unsigned)cols, (unsigned)((rows + planes - 1) / planes), (unsigned)planes);
     const bool wide = (uintptr_t)w_out % 32 == 0;
-    auto *fn = d->act_dtype == QF_BF16 ? (wide ? dequant_dispatch<true, true> : dequant_dispatch<true, false>)
-                                       : (wide ? dequant_dispatch<false, true> : dequant_dispatch<false, false>);
+    const bool bf16 = d->act_dtype == QF_BF16;
+    auto *fn = per == 4 ? (bf16 ? (wide ? dequant_dispatch<true, true, 4> : dequant_dispatch<true, false, 4>)
+                                : (wide ? dequant_dispatch<false, true, 4> : dequant_dispatch<false, false, 4>))
+                        : (bf16 ? (wide ? dequant_dispatch<true, true, 2> : dequant_dispatch<true, false, 2>)
+                                : (wide ? dequant_dispatch<false, true, 2> : dequant_dispatch<false, false, 2>));
     return launched(ctx, fn(d->zero_mode, grid, s, (const uint32_t *)qw, (const uint16_t *)scales, zeros, d->zero_const,
                             (uint4 *)w_out, d->N, (int)words, d->group_size / 8),
                     "dequant");
