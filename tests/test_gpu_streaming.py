@@ -99,25 +99,26 @@ def test_unpack_at_any_alignment(n, offset, shift):
 
 
 def test_unpack_of_sixteen_byte_aligned_outputs_is_no_byte_loop():
-    """An output that starts in the middle of a 32-byte sector takes the vector kernel too: 1.22 times the time of an aligned
-    one (47.3 against 38.7 us), where a byte per thread takes 1.65 times (63.8 us)."""
+    """An output that starts in the middle of a 32-byte sector takes the vector kernel too, and stores whole sectors: 0.98 times the time of
+    an aligned one (31.9 against 32.4 us in calls behind one another), where half sectors take 1.24 times (40.3 us) and a byte per
+    thread 1.75 times."""
     n = 64 << 20
     packed = torch.randint(-128, 128, (n,), dtype=torch.int8, device="cuda")
     buf = torch.empty(2 * n + 16, dtype=torch.int8, device="cuda")
 
     def ms(out):
-        best = 1e9
-        for _ in range(5):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
+        # (twenty behind one another: the first call finds some of its input in L2)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(20):
             _unpack_into(packed, out)
-            b.record()
-            b.synchronize()
-            best = min(best, a.elapsed_time(b))
-        return best
+        b.record()
+        b.synchronize()
+        return a.elapsed_time(b)
 
-    aligned, half = ms(buf[:2 * n]), ms(buf[16:])
-    assert half < 1.35 * aligned
+    times = [(ms(buf[:2 * n]), ms(buf[16:])) for _ in range(12)]
+    aligned, half = (min(t) for t in zip(*times))
+    assert half < 1.12 * aligned
 
 
 def test_dequant_of_very_long_rows():
