@@ -214,11 +214,14 @@ size_t qf_w4a16_batched_workspace_bytes(int count, const qf_linear_desc *descs);
 int qf_w4a16_batched_launches(qf_ctx *ctx, int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight,
                               void *const *Y, const void *const *residual, const void *workspace, size_t workspace_bytes);
 /* How this call would run on a B200 (host only: nothing is enqueued, and no pointer is followed). For entry i,
- * out[QF_BATCHED_PLAN_WORDS * i ..]: the number of its launch (-1: none, M == 0) and, -1 for an entry that goes by itself, its phase in
- * the launch; the two phases that are complete before it writes its results, and up to 8 rows before it reads (-1: none); its first slot of
- * partial sums and their number; up to 8 rows the place of its first thread block (4 * SM + place on the SM) and the number of its blocks.
- * Above, the phase that is complete, with the second of the two, before it writes partial sums, and -1: activations that another entry
- * makes are read row block by row block as they are finished. */
+ * out[QF_BATCHED_PLAN_WORDS * i ..], where words 1 to 7 are -1 for an entry that goes by itself:
+ *   0     the number of its launch (-1: none, M == 0)
+ *   1     its phase in the launch
+ *   2, 3  two phases (-1: none). Up to 8 rows they are complete before it reads or writes anything; above, before it writes its results:
+ *         activations that another entry makes are read row block by row block as they are finished
+ *   4, 5  its first slot of partial sums, and their number
+ *   6, 7  up to 8 rows the place of its first thread block (4 * SM + place on the SM), and the number of its blocks; above, the phase that,
+ *         with that of word 3, is complete before it writes partial sums (-1: none), and -1 */
 #define QF_BATCHED_PLAN_WORDS 8
 int qf_w4a16_batched_plan(int count, const qf_linear_desc *descs, const void *const *X, const void *const *qweight, void *const *Y,
                           const void *const *residual, const void *workspace, size_t workspace_bytes, int32_t *out);

@@ -219,25 +219,25 @@ int stream_chain_length(const StreamLinear *l, int count) {
 // GEMV kernel's costs, also where the tcgen05 kernel serves a linear alone (such batches are chains). A chain costs its launch, and for
 // each step `step` from the last product to the next one's first, kChunk for each 128 codes of its longest piece, at least four of them,
 // `split` where partial sums are exchanged, and `round` for each further round of pieces.
-// Fitted to 64 batches at 9 to 32 rows on weights not in L2, graph replays; standard deviation 10 %. Where the estimate picks the slower
-// way it costs 7 % at most, and 10 % on 19 other batches (4 of 76 points), but for sixteen linears of 1024 x 1024 in a row at 9 rows.
-// The fit is older than the present chains (results awaited by row blocks, phases that nobody waits for not counted, sums fetched by
-// fours), which are up to 25 % shorter than estimated; it stands, because the way that is taken decides about the order of the sums.
-// Measured, one by one -> chain, at 9 / 16 / 24 / 32 rows; * marks what the estimate picks otherwise, + present chains (N x K):
-//   one reads the other, 2 linears:  512 x 512       8.7 -> 14.0 / 9.2 -> 14.5 / 12.4 -> 17.7 / 13.0 -> 19.4
-//                                    1024 x 2816     12.9 -> 15.7 / 13.7 -> 17.2 / 19.2 -> 19.5 / 20.3 -> 22.3
-//                                    2048 x 5632     17.1 -> 17.3 / 18.5 -> 17.5* / 29.5 -> 20.3 / 31.9 -> 21.4
-//                                    4096 x 4096     17.2 -> 17.3* / 19.7 -> 17.9 / 29.8 -> 20.9 / 32.3 -> 21.9 +
-//                                    256 x 18944     34.1 -> 17.7 / 34.6 -> 19.0 / 55.8 -> 20.6 / 58.2 -> 21.7
-//                       16 linears:  1024 x 1024     120 -> 97.3* / 123 -> 118* / 181 -> 133+ / 186 -> 154+
-//                                    1024 x 2816     101 -> 96.9* / 107 -> 113 / 168 -> 129 / 172 -> 149
-//   side by side, 2 linears:         256 x 256       6.1 -> 8.0 / 6.6 -> 8.8 / 8.5 -> 9.7 / 9.1 -> 10.4
-//                                    14336 x 1024    12.9 -> 16.4 / 14.6 -> 18.2 / 21.1 -> 22.4* / 23.6 -> 25.5*
-//                                    4096 x 4096     17.3 -> 13.9 / 19.8 -> 14.3 / 30.1 -> 16.2 / 32.4 -> 17.7 +
-//                 4 linears:         512 x 512       16.4 -> 7.5 / 16.9 -> 7.9 / 24.0 -> 8.7 / 25.2 -> 9.0 +
-//   one layer of seven:              512 / 1024      31.3 -> 22.9 / 32.9 -> 24.7 / 44.9 -> 27.9 / 47.1 -> 28.7 +
-//                                    4096 / 14336    83.6 -> 47.0 / 89.5 -> 49.6 / 131 -> 56.4 / 138 -> 61.2 +
-//   30 layers of four:               256 / 256       394 -> 431 / 414 -> 465 / 544 -> 564* / 581 -> 621*
+// Fitted to 64 batches at 9 to 32 rows on weights not in L2, graph replays, of former chains: activations awaited phase by phase, every phase
+// counted, sums fetched by eights. Of those its standard deviation was 10 % and a wrong pick cost 7 %, 10 % on 19 other batches. Present
+// chains are up to 25 % shorter than it says, so small batches go one by one that would be faster as chains, by 22 % at most below. It
+// stands because the way that is taken decides about the order of the sums. (It plans with the fewest slots: the way does not depend on the
+// workspace either.) Measured, one by one -> chain, at 9 / 16 / 24 / 32 rows; * marks what the estimate picks otherwise (N x K):
+//   one reads the other, 2 linears:  512 x 512       8.3 -> 12.5 / 8.8 -> 12.2 / 12.2 -> 13.6 / 12.7 -> 15.5
+//                                    1024 x 2816     12.8 -> 14.8 / 13.6 -> 16.6 / 18.8 -> 18.4* / 21.3 -> 20.6*
+//                                    2048 x 5632     16.7 -> 16.5* / 18.3 -> 16.9* / 29.5 -> 19.4 / 31.5 -> 20.2
+//                                    4096 x 4096     17.1 -> 17.5* / 19.7 -> 18.1 / 29.8 -> 20.7 / 32.4 -> 21.7
+//                                    256 x 18944     33.0 -> 18.2 / 33.6 -> 18.8 / 58.9 -> 20.6 / 59.5 -> 21.4
+//                       16 linears:  1024 x 1024     121 -> 93.9* / 124 -> 112* / 183 -> 129 / 187 -> 155
+//                                    1024 x 2816     99.8 -> 96.0* / 106 -> 109 / 169 -> 124 / 163 -> 141
+//   side by side, 2 linears:         256 x 256       6.0 -> 6.4 / 6.5 -> 6.8 / 8.6 -> 7.6* / 9.2 -> 7.9*
+//                                    14336 x 1024    12.8 -> 14.5 / 14.4 -> 16.4 / 21.0 -> 19.5 / 23.5 -> 22.1
+//                                    4096 x 4096     17.3 -> 14.0 / 19.7 -> 14.4 / 29.8 -> 16.3 / 32.4 -> 17.7
+//                 4 linears:         512 x 512       16.6 -> 7.3 / 17.3 -> 7.6 / 24.1 -> 8.4 / 25.3 -> 8.7
+//   one layer of seven:              512 / 1024      32.2 -> 22.7 / 33.8 -> 24.3 / 46.8 -> 27.7 / 48.1 -> 28.4
+//                                    4096 / 14336    77.8 -> 47.4 / 84.4 -> 50.0 / 112 -> 56.7 / 120 -> 61.9
+//   28 layers of four, epilogues:    256 / 256       405 -> 336* / 445 -> 432* / 592 -> 466 / 654 -> 595
 bool stream_chain_pays(const StreamLinear *l, int count) {
     struct Costs {
         double base, member, unit, step, split, round;

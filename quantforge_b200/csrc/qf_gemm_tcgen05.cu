@@ -82,8 +82,8 @@ struct GemmParams {
 };
 
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.f + expf(-gate)) * up; }
-// CNT (4 or 8) consecutive elements of the output type, as vectors: element offsets are multiples of CNT, the base is 16-byte
-// aligned and rows are multiples of 128 bytes long.
+// CNT (4 or 8) consecutive elements of the output type, as vectors: element offsets are multiples of CNT, the base is 16-byte aligned
+// and rows have a multiple of 16 elements, 32 bytes of a 16-bit type, so that vectors of up to 16 bytes are aligned.
 template <int CNT>
 __device__ __forceinline__ void store_vec(void *Y, int out_dtype, int64_t o, const float (&v)[CNT]) {
     if (out_dtype == QF_F32) {

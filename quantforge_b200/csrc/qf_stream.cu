@@ -5,9 +5,10 @@
 // instruction) and live in TMEM only, the activations are B from shared memory. What the streaming GEMV kernel (mma.sync) spends
 // on fragments of X and on the MMAs themselves, which take issue slots and packed-half time from the conversion and grow with the
 // rows, is here one thread's work. Without memory, converters and MMAs alone take 283 cycles per 128 x 128 codes and SM; HBM delivers
-// those in 377; the kernel takes about 450, bound by the issue slots that the conversion and its hand-overs share. In a chain there are 4 to
-// 5 us from the last MMA of a step to the first of the next: partial sums, results, a release (1 us and more behind stores), counters, a
-// copy of activations.
+// those in 377; the kernel takes about 450, bound by the issue slots that the conversion and its hand-overs share. In a chain there are 5 to
+// 6 us from the last MMA of a step to the first of the next (the median stream's; eight layers of 4096 / 14336, each linear behind the one
+// before, 9 and 16 rows; 6.5 to 8 at 32 rows): partial sums, results, a release (1 us and more behind stores), counters, a copy of
+// activations.
 //
 // Work split. Units of 128 rows x 128 codes. Of a single linear they are numbered row block major, K chunk minor, and stream i of G
 // owns a contiguous range of them (the first r streams one more than the others): every stream moves the same number of bytes

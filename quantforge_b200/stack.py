@@ -20,7 +20,9 @@ faster way, with the bits of the linears one by one.
 
 What a chain gains here is more than a decoder has of it: with attention left out, nothing reads q/k/v of the fused variant and o
 runs beside it (without epilogues down runs beside gate/up too). 32 layers of 4096 / 14336 with o behind q/k/v, one by one -> chain:
-1 row 1403 us, no chain; 16 rows 2071 -> 1612 us where this stack takes 1262.
+1 row 1403 us, no chain; 16 rows 2071 -> 1612 us where this stack takes 1262. (Of what made chains of 9 to 32 rows faster since, reading
+results row block by row block and exchanging sums early, that form has next to nothing: four layers, 9 / 16 / 32 rows, 200 -> 196, 205 -> 205,
+240 -> 240 us, where this stack's went from 172, 175 and 201 to 155, 163 and 192.)
 """
 from __future__ import annotations
 
@@ -56,7 +58,9 @@ def _chain_bytes(batch: int, fuse: bool) -> float:
                 16 MB (4096, 14336)     1.44-1.48 / 1.36-1.37 / 1.26-1.29 / 1.21-1.24 / 1.17-1.19 / 1.12-1.14
                 61 MB (8192, 28672)     1.17 / 1.15 / 1.14 / 1.13 / 1.19 / 1.11
     The lines were drawn when chains took 10 to 15 % longer (17 rows and more of small linears lost then, and of any size from 25 rows on).
-    They stand: which layout a stack has its weights in is part of what its callers see."""
+    They are kept although the results are the same bits either way: tests hold stacks to them, and moving them is a change of its own.
+    What they give away, as of the table: on fused stacks 9 to 13 % at 17 to 24 rows of 5.6 and 12 MB and 20 to 22 % of 22 MB, from 25 rows on 6
+    to 13 % of 22 to 34 MB and 8 to 18 % of 107 MB; on unfused ones of 0.8 MB 15 to 38 % up to 24 rows."""
     if not fuse:
         return 2e6
     return 5e6 if batch <= 16 else 24e6 if batch <= 24 else float("inf")
