@@ -91,20 +91,16 @@ static bool stream_serves(const qf_linear_desc *d) {
     return d->K >= 512 && mib >= (d->K >= 8192 ? 24 : d->K >= 6144 ? 33 : d->K >= 5120 ? 42 : 72);
 }
 
-// Whether the GEMV kernel can run through K: without a split, which needs a counter for each of its tiles of outputs, a block takes 32 chunks.
-static bool gemv_takes(const qf_linear_desc *d) {
-    return d->K <= 32 * 128 || (d->N + 63) / 64 * ((d->M + 7) / 8) <= kMaxCounters;
-}
-
 // Millions of codes from which the tcgen05 kernel is the faster one on canonical weights of N % 128 != 0 rows; -1: never. Its blocks take a
 // tile of 128 rows and, up to 64 batch rows, an eighth of K at least; the GEMV kernel's take 64 rows, 8 batch rows and a piece of K that fills
 // the device four times over. So this one loses where there are few tiles of long K, and on small matrices what its start-up and its sums cost.
 // GEMV / tcgen05 kernel, times as fast, weights not in L2:
 //   3, 4 rows    K 1024: N 10256 0.84, 12304 1.02    1536: 7184 0.95, 8208 1.05    2048: 5136 0.95, 6160 1.04    3072: 3088 0.99, 4112 1.02
-//                4096: 2064 0.97, 3088 1.02, 4112 1.17    5120: 1552 0.94, 2064 1.01    6144: 1040 1.30    8192: 784 1.25
-//                12288: 528 to 3600 0.97 to 1.23    14336: 784 to 2576 0.89 to 1.02, 3088 1.00    18944 to 28672: up to 2064 0.73 to 1.04, 3088 1.26
-//   5 to 8       1024: 10256 0.84 to 0.86, 12304 1.11    1280: 8208 0.90, 10256 1.08    1536: 4112 0.93 to 0.99, 5136 1.00
-//                2048: 3600 0.89 to 0.96, 4112 1.05    2560 to 6144: 0.96 and more    24576, 28672: up to 1296 0.85 to 1.04 at 5, 0.91 to 1.19 at 8
+//                4096: 2064 0.97, 3088 1.02, 4112 1.17    5120: 1552 0.94, 2064 1.01    with more than 8 splits: 4608: 1904 1.31
+//                5504: 1296 1.37    6144: 1040 1.30    8192: 784 1.25    12416 to 14208: 0.87 to 1.22    14336: 784 to 2576 0.89 to 1.02, 3088 1.00
+//                18944 to 28672: up to 2064 0.73 to 1.04 (16256: 592 1.11), 2960 and 3088 1.26
+//   5 to 8       1024: 11840 0.79, 12304 1.11    1280: 9376 0.87, 10256 1.08    1536: 4112 0.93 to 0.99, 5136 1.00
+//                2048: 3600 0.89 to 0.96, 4112 1.05    2560 to 16384: 0.93 and more    18944: 0.89 to 1.17 at 5    22784 to 28672: up to 1296 0.82 to 1.10 at 5 and 6, 0.88 to 1.19 at 8
 //   9 to 16      up to 512: 0.95 and more but 128 x 57360 0.88    640: up to 18448 0.76 to 0.94, 20496 1.62
 //                768: up to 8208 0.84 to 1.00, 12304 1.01, 18448 0.92    896: 7184, 8208 0.89 to 0.94, 10256 1.09
 //                1152 to 1408: 3088, 4112 0.94 to 1.07    all else 1.0 to 3.7
@@ -118,11 +114,12 @@ static bool gemv_takes(const qf_linear_desc *d) {
 //                14336: 400 0.85 to 0.92 from 96 to 160    20480: 208 0.62 to 0.91 up to 200, 272 0.68 to 0.90 up to 160, then 1.05 and more
 //                28672: 144 0.53 to 0.79, 208 0.60 to 0.78 up to 140, 272 0.73 to 0.97 up to 112, then 0.99 and more
 //   more         1.5 and more
-static double ragged_line(int64_t M, int64_t K, int64_t N) {
+// (`on_chip`: the GEMV kernel has at most 8 splits, which a cluster sums.)
+static double ragged_line(int64_t M, int64_t K, int64_t N, bool on_chip) {
     if (M <= 8) {
-        if (K < 1024 || (M <= 4 && K > 12288 && N < 3072) || (M <= 6 && K >= 24576 && N < 1536)) return -1;
-        if (M > 4) return K < 1536 ? 12 : K < 2560 ? 8 : 6;
-        return K < 1536 ? std::max<double>(12, 12288e-6 * K) : K < 2560 ? 12 : K < 6144 ? 10 : 6;
+        if (K < 1024 || (M <= 4 && K > 14208 && N < 2688) || (M <= 6 && K > 20480 && N < 1536)) return -1;
+        if (M > 4) return K < 1536 ? 12.5 : K < 2560 ? 8 : 6;
+        return K < 1536 ? std::max<double>(12, 12288e-6 * K) : K < 2560 ? 12 : on_chip ? 10 : 6;
     }
     if (M <= 16) return K <= 512 || K >= 1024 ? 4 : K < 768 ? 12.5 : 9;
     if (M <= 64) {
@@ -145,12 +142,15 @@ static bool gemm_serves_ragged(const qf_linear_desc *d) {
     // 14336 x 1040 in one split: 12.9 us there, 39.6 here).
     if (d->split_k != 0) return false;
     // What the GEMV kernel refuses stays refused, 32-bit and 16-bit results alike.
-    if (!gemv_takes(d)) return false;
+    qf_linear_desc other = *d;
+    other.path = QF_PATH_GEMV;
+    Plan gemv;
+    if (make_plan(&other, &gemv, nullptr) != QF_OK) return false;
     if (d->zero_mode == QF_ZERO_U4 && d->N % 32 != 0) return false;
     // Sums of a whole split in one accumulator are 2e-7 to 4e-7 (of the outputs' rms) further off than the GEMV kernel's two accumulators
     // of shorter splits: 16-bit results, rounded by 1e-4 and more, do not show it; 32-bit ones keep that kernel.
     if (d->out_dtype == QF_F32) return false;
-    const double line = ragged_line(d->M, d->K, d->N);
+    const double line = ragged_line(d->M, d->K, d->N, gemv.split_k <= 8);
     return line >= 0 && d->K * d->N >= 1e6 * line;
 }
 

@@ -42,10 +42,10 @@ def _gemm(M, K, N, **kw):
 # on either side of each line, by rows of activations: (rows, K, largest N of the GEMV kernel, smallest of the tcgen05 kernel)
 @pytest.mark.parametrize("rows,K,gemv,gemm", [
     ((3, 4), 896, 40976, None), ((3, 4), 1024, 12272, 12304), ((3, 4), 1408, 12272, 12304), ((3, 4), 1536, 7792, 7824), ((3, 4), 2432, 4912, 4944),
-    ((3, 4), 2560, 3888, 3920), ((3, 4), 4096, 2416, 2448), ((3, 4), 6016, 1648, 1680), ((3, 4), 6144, 976, 1008), ((3, 4), 12288, 464, 496),
-    ((3, 4), 12416, 3056, 3088), ((3, 4), 28672, 3056, 3088),
-    ((5, 6, 7, 8), 896, 40976, None), ((5, 6, 7, 8), 1024, 11696, 11728), ((5, 6, 7, 8), 1536, 5200, 5232), ((5, 6, 7, 8), 2560, 2320, 2352),
-    ((5, 6, 7, 8), 14336, 400, 432), ((5, 6), 24576, 1520, 1552), ((7, 8), 24576, 240, 272),
+    ((3, 4), 2560, 3888, 3920), ((3, 4), 4096, 2416, 2448), ((3, 4), 4480, 2224, 2256), ((3, 4), 4608, 1296, 1328), ((3, 4), 5120, 1936, 1968),
+    ((3, 4), 5248, 1136, 1168), ((3, 4), 12288, 464, 496), ((3, 4), 14208, 400, 432), ((3, 4), 14336, 2672, 2704), ((3, 4), 28672, 2672, 2704),
+    ((5, 6, 7, 8), 896, 40976, None), ((5, 6, 7, 8), 1024, 12176, 12208), ((5, 6, 7, 8), 1536, 5200, 5232), ((5, 6, 7, 8), 2560, 2320, 2352),
+    ((5, 6, 7, 8), 14336, 400, 432), ((5, 6), 20480, 272, 304), ((5, 6), 20608, 1520, 1552), ((7, 8), 24576, 240, 272),
     ((9, 12, 16), 512, 7792, 7824), ((9, 16), 640, 19504, 19536), ((9, 16), 896, 10032, 10064), ((9, 16), 1024, 3888, 3920), ((9, 12, 16), 4096, 976, 992), ((9, 16), 28672, 112, 144),
     ((17, 24), 512, 3888, 3920), ((17, 24), 128, 19504, 19536), ((25, 40), 128, 15600, 15632), ((17, 40), 256, 9744, 9776), ((41, 64), 256, 7792, 7824), ((17, 24), 640, 14048, 14096), ((17, 24), 1024, 3888, 3920), ((17, 24), 1408, 3184, 3216), ((17, 24), 896, 7792, 7824), ((17, 24, 32, 40, 64), 1536, 1296, 1328),
     ((25, 32), 896, 4432, 4496), ((25, 32), 640, 9360, 9392), ((33, 40), 640, 7792, 7824), ((41, 64), 640, 6224, 6256), ((25, 32), 1024, 1936, 1968), ((25, 32), 1280, 2288, 2320), ((33, 40), 1024, 2320, 2352), ((41, 64), 1024, 1936, 1968),
