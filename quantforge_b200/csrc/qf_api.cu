@@ -100,7 +100,8 @@ static bool stream_serves(const qf_linear_desc *d) {
 //                5504: 1296 1.37    6144: 1040 1.30    8192: 784 1.25    12416 to 14208: 0.87 to 1.22    14336: 784 to 2576 0.89 to 1.02, 3088 1.00
 //                18944 to 28672: up to 2064 0.73 to 1.04 (16256: 592 1.11), 2960 and 3088 1.26
 //   5 to 8       1024: 11840 0.79, 12304 1.11    1280: 9376 0.87, 10256 1.08    1536: 4112 0.93 to 0.99, 5136 1.00
-//                2048: 3600 0.89 to 0.96, 4112 1.05    2560 to 16384: 0.93 and more    18944: 0.89 to 1.17 at 5    22784 to 28672: up to 1296 0.82 to 1.10 at 5 and 6, 0.88 to 1.19 at 8
+//                2048: 3600 0.89 to 0.96, 4112 1.05    2560 to 16384: 0.93 and more    18944: 0.89 to 1.17 at 5
+//                22784 to 28672: up to 1296 0.82 to 1.10 at 5 and 6, 0.88 to 1.19 at 8
 //   9 to 16      up to 512: 0.95 and more but 128 x 57360 0.88    640: up to 18448 0.76 to 0.94, 20496 1.62
 //                768: up to 8208 0.84 to 1.00, 12304 1.01, 18448 0.92    896: 7184, 8208 0.89 to 0.94, 10256 1.09
 //                1152 to 1408: 3088, 4112 0.94 to 1.07    all else 1.0 to 3.7
